@@ -165,8 +165,7 @@ __device__ __forceinline__ T block_min(T v, T* smem) {
   __syncthreads();
   if (lane_id() == 0) smem[warp_id()] = v;
   __syncthreads();
-  T r = smem[0];
-  for (int w = 1; w < nw; ++w) r = smem[w] < r ? smem[w] : r;
+  const T r = warp_min(smem[(int)lane_id() < nw ? lane_id() : 0u]);
   __syncthreads();
   return r;
 }
@@ -184,14 +183,16 @@ __device__ __forceinline__ int64_t block_excl_sum(int64_t v, int64_t* smem, int6
   __syncthreads();
   if (lane_id() == 31) smem[warp_id()] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int w = 0; w < nw; ++w) {
-      int64_t t = smem[w];
-      smem[w] = run;
-      run += t;
+  if (warp_id() == 0) {  // the warp totals, scanned by one warp (a serial loop cost ~1 us a call)
+    const int64_t t = (int)lane_id() < nw ? smem[lane_id()] : 0;
+    int64_t run = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t w = __shfl_up_sync(0xffffffffu, run, o);
+      if ((int)lane_id() >= o) run += w;
     }
-    smem[32] = run;
+    smem[lane_id()] = run - t;
+    if (lane_id() == 31) smem[32] = run;
   }
   __syncthreads();
   int64_t r = smem[warp_id()] + incl - v;

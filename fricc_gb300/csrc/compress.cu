@@ -4,21 +4,22 @@
 // (include/sparse_tensor.hpp:46-56).
 //
 // Pipeline (x resident in HBM, N elements, keep m):
-//   1. histogram of the top 12 bits of |x| -> host picks the digit holding
-//      the m-th largest magnitude (a few KB copied back);
-//   2. stable compaction of every element at or above that digit
-//      (decoupled look-back, one pass) and an LSD radix sort of the
-//      candidates by descending |x|, ties by ascending index: the first m
-//      are argsort(x, m) (:11-36);
-//   3. one_norm (:164-171) as an exact sequential chain (exactsum.cuh);
-//   4. the remaining-norm chain R -= |x_(d)| over the sorted candidates and
+//   1. one pass over x: histogram of the top 12 bits of |x| and the chunk
+//      sums of one_norm, then one_norm (:164-171) as an exact sequential
+//      chain (exactsum.cuh);
+//   2. a select digit: the elements at or above it hold every entry D can
+//      take (k_select_digit), which is 0.2-2% of the m largest on MP2-like
+//      amplitudes; their stable compaction (decoupled look-back, one pass)
+//      and their sort by descending |x|, ties by ascending index: the order
+//      of argsort(x, m) (:11-36), as far as it is needed;
+//   3. the remaining-norm chain R -= |x_(d)| over the sorted candidates and
 //      the acceptance test (m-d)|x_(d)| >= R-|x_(d)| && R > 1e-14
-//      (:411-421), evaluated for every d from exact chain values;
-//   5. p_i = |x_i| / R * m' (:375, this operation order), the p > 1 check
+//      (:411-421), evaluated from exact chain values up to its first failure;
+//   4. p_i = |x_i| / R * m' (:375, this operation order), the p > 1 check
 //      (:383-395), the exact partial sums of p (:142-143) and, for every
 //      interval [I_j, I_{j+1}), the samples u_k = k + rn that land in it
 //      (:136, :147-157); unmatched samples keep index 0, as in the reference;
-//   6. output D in sorted order then S ascending, values x_D and x_S/p_S.
+//   5. output D in sorted order then S ascending, values x_D and x_S/p_S.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -55,18 +56,41 @@ struct Rep {
   int64_t n = 0, m = 0, tile = 0, one = 0;
 };
 
-// histogram of the first select digit (1 << bits bins of dynamic shared memory)
-__global__ void __launch_bounds__(256) k_hist_sel(const double* __restrict__ x, int64_t n, unsigned* __restrict__ hist,
-                                                  int bits, Rep rp = Rep{}) {
+// histogram of the first select digit (1 << bits bins of dynamic shared
+// memory) and, with csum, the approximate sum of |x| over each exact::CH
+// chunk, in one read of x (the one_norm chain's first pass).  Persistent
+// blocks over chunks, so the bins are zeroed and flushed once per block.
+__global__ void __launch_bounds__(256) k_hist_sums(const double* __restrict__ x, int64_t n, unsigned* __restrict__ hist,
+                                                   int bits, double* __restrict__ csum, Rep rp = Rep{}) {
+  const int64_t nch = fricc_cdiv(n, (int64_t)exact::CH);
   x += blockIdx.y * rp.n;
   hist += blockIdx.y * rp.one * NDIG;
+  if (csum) csum += blockIdx.y * rp.one * (nch + 1);
   extern __shared__ unsigned h[];
+  __shared__ double red[32];
   const int nb = 1 << bits, shift = 63 - bits;
   for (int i = threadIdx.x; i < nb; i += 256) h[i] = 0;
   __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * 256;
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride)
-    atomicAdd(&h[abs_key(x[i]) >> shift], 1u);
+  for (int64_t c = blockIdx.x; c < nch; c += gridDim.x) {
+    const int64_t base = c * exact::CH;
+    double v[exact::CH / 256];
+#pragma unroll
+    for (int r = 0; r < exact::CH / 256; ++r) {
+      const int64_t i = base + r * 256 + threadIdx.x;
+      v[r] = i < n ? x[i] : 0.0;
+    }
+    double acc = 0.0;
+#pragma unroll
+    for (int r = 0; r < exact::CH / 256; ++r) {
+      const int64_t i = base + r * 256 + threadIdx.x;
+      if (i < n) atomicAdd(&h[abs_key(v[r]) >> shift], 1u);
+      acc += fabs(v[r]);
+    }
+    if (csum) {
+      const double tot = block_sum_det(acc, red);
+      if (threadIdx.x == 0) csum[c] = tot;
+    }
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += 256)
     if (h[i]) atomicAdd(&hist[i], h[i]);
@@ -76,6 +100,9 @@ __global__ void __launch_bounds__(256) k_hist_sel(const double* __restrict__ x, 
 struct Ctl {
   int64_t dmin;       // first select digit kept as a candidate
   int64_t ncand;      // candidates (every element at or above dmin)
+  int64_t mchain;     // length of the remaining-norm chain: min(m, ncand)
+  double norm;        // one_norm
+  int64_t found;      // 1: |D| already found by the chain's first chunks (k_rem_first)
   int64_t nd;         // |D|
   int64_t mp;         // m - |D|
   unsigned long long dkey;  // |x| bits of the last element of D
@@ -127,17 +154,27 @@ __global__ void __launch_bounds__(256) k_compact(const double* __restrict__ x, i
   if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
   __syncthreads();
   const int tile = s_tile;
-  const int64_t base = (int64_t)tile * TILE + threadIdx.x * ITEMS;
+  // a warp owns 512 consecutive elements, 32 per load (coalesced), and ranks
+  // its keepers with ballots; one thread per 16 consecutive elements read
+  // 128 bytes apart and took 148 us on 20 M elements
+  const int64_t base = (int64_t)tile * TILE + (threadIdx.x >> 5) * (32 * ITEMS) + (threadIdx.x & 31);
   unsigned long long key[ITEMS];
-  int cnt = 0;
+  unsigned mask[ITEMS];
+  int wtot = 0;
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
-    const int64_t i = base + k;
+    const int64_t i = base + 32 * k;
     key[k] = i < n ? abs_key(x[i]) : 0ull;
-    if (i < n && (unsigned)(key[k] >> shift) >= dmin) ++cnt;
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const int64_t i = base + 32 * k;
+    mask[k] = __ballot_sync(0xffffffffu, i < n && (unsigned)(key[k] >> shift) >= dmin);
+    wtot += __popc(mask[k]);
   }
   int64_t tot;
-  const int64_t excl = block_excl_sum(cnt, sm, &tot);
+  const int64_t excl_lane = block_excl_sum((threadIdx.x & 31) == 0 ? wtot : 0, sm, &tot);
+  const int64_t excl = __shfl_sync(0xffffffffu, excl_lane, 0);
   if (threadIdx.x == 0) {
     int64_t pre = 0;
     if (tile == 0) {
@@ -178,12 +215,12 @@ __global__ void __launch_bounds__(256) k_compact(const double* __restrict__ x, i
   int64_t o = s_pre + excl;
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
-    const int64_t i = base + k;
-    if (i < n && (unsigned)(key[k] >> shift) >= dmin) {
-      ckey[o] = key[k];
-      cidx[o] = (unsigned)i;
-      ++o;
+    if ((mask[k] >> (threadIdx.x & 31)) & 1u) {
+      const int64_t at = o + __popc(mask[k] & ((1u << (threadIdx.x & 31)) - 1u));
+      ckey[at] = key[k];
+      cidx[at] = (unsigned)(base + 32 * k);
     }
+    o += __popc(mask[k]);
   }
 }
 
@@ -240,25 +277,35 @@ struct GenPv {
   __device__ __forceinline__ double value(int64_t i) const { return P[i]; }
 };
 
-// get_d_largest's acceptance test for every position d of the sorted list.
+// get_d_largest's acceptance test for the positions d of the sorted list;
+// each thread keeps its first failure and a warp publishes one minimum (an
+// atomic per failing position serialised ~2 M of them on one word: 1.28 ms).
 struct ConsAccept {
   int64_t m;
-  double* Rb;                    // [m+1]: R before element d (Rb[m]: after the last)
+  double* Rb;                    // [m+1]: R before element d; Rb[mchain]: after the last
   unsigned long long* first_fail;
+  const Ctl* c;
   int64_t one = 0;               // 1 in a replica batch
+  int64_t mchain = 0;
+  unsigned long long mine = ~0ull;
   __device__ __forceinline__ ConsAccept at(int r) const {
-    return ConsAccept{m, Rb + r * one * (m + 1), first_fail + r * one, one};
+    const Ctl* cr = c + r * one;
+    return ConsAccept{m, Rb + r * one * (m + 1), first_fail + r * one, cr, one, cr->mchain};
   }
-  __device__ __forceinline__ void operator()(int64_t d, double before, double after, double a) const {
+  __device__ __forceinline__ void operator()(int64_t d, double before, double after, double a) {
     Rb[d] = before;
-    if (d == m - 1) Rb[m] = after;
+    if (d == mchain - 1) Rb[mchain] = after;
     const bool acc = (__dmul_rn((double)(unsigned long long)(m - d), a) >= after) && (before > 1e-14);
-    if (!acc) atomicMin(first_fail, (unsigned long long)d);
+    if (!acc && (unsigned long long)d < mine) mine = (unsigned long long)d;
+  }
+  __device__ __forceinline__ void finish() {
+    const unsigned long long w = warp_min(mine);
+    if (lane_id() == 0 && w != ~0ull) atomicMin(first_fail, w);
   }
 };
 
 // number of k in [0, mp) with fl(k + rn) < I  (u_k increases with k)
-__device__ __forceinline__ int64_t count_below(double I, double rn, int64_t mp) {
+__device__ __noinline__ int64_t count_below(double I, double rn, int64_t mp) {
   if (!(I > rn)) return 0;
   double g = floor(I - rn);
   int64_t k = g < 0.0 ? 0 : (g > (double)mp ? mp : (int64_t)g);
@@ -267,19 +314,56 @@ __device__ __forceinline__ int64_t count_below(double I, double rn, int64_t mp) 
   return k;
 }
 
-// sample_systematic's interval search: the samples of interval j.
+// v in [0, 2^31) as floor(v 2^32), from its bits; false for anything else
+__device__ __forceinline__ bool fix32(double v, long long& f) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)(u >> 52);  // the sign bit makes e >= 2048
+  if (e >= 1023 + 31) return false;
+  const unsigned long long M = (u & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+  const int sh = e - (1075 - 32);  // M 2^(e-1075) 2^32
+  f = (long long)(sh >= 0 ? M << sh : (sh > -64 ? M >> -sh : 0ull));
+  return true;
+}
+
+// sample_systematic's interval search: the samples of interval j.  The two
+// counts come from 32-bit fixed point on the integer pipe (FP64 floor, add
+// and compare per element made this pass FP64-bound, and a dependent chain
+// of them ran for every item of a thread): with D = floor(I 2^32) -
+// floor(rn 2^32) within 2^32 units of I - rn, a fraction of D at least 2^12
+// units from an integer decides every k, since fl(k + rn) is off by at most
+// 2^-23 (2^9 units) below 2^31; nearer ones (1 in 5e5) take count_below.
 struct ConsSample {
   const Ctl* c;
   unsigned* S;
   int64_t cs = 0, ss = 0;  // replica strides of c and S
-  __device__ __forceinline__ ConsSample at(int r) const { return ConsSample{c + r * cs, S + r * ss, cs, ss}; }
+  double rn = 0.0;
+  int64_t mp = 0;
+  long long frn = 0;
+  int ok = 0;  // 1: samples can land; 2: and rn has a fixed-point form
+  __device__ __forceinline__ ConsSample at(int r) const {
+    ConsSample q{c + r * cs, S + r * ss, cs, ss};
+    q.rn = q.c->rn;
+    q.mp = q.c->mp;
+    q.ok = q.c->sample ? (fix32(q.rn, q.frn) && q.mp < (1ll << 31) ? 2 : 1) : 0;
+    return q;
+  }
+  __device__ __forceinline__ int64_t count(double I) const {
+    long long f;
+    if (ok == 2 && fix32(I, f)) {
+      const long long D = f - frn;
+      const unsigned fr = (unsigned)D;
+      if (fr - (1u << 12) <= 0xffffffffu - (1u << 13)) {
+        const long long k = (D >> 32) + 1;
+        return k < 0 ? 0 : (k > mp ? mp : k);
+      }
+    }
+    return count_below(I, rn, mp);
+  }
   __device__ __forceinline__ void operator()(int64_t j, double lo, double hi, double p) const {
-    if (!c->sample || !(p > 0.0)) return;
-    const double rn = c->rn;
-    const int64_t mp = c->mp;
-    const int64_t k0 = count_below(lo, rn, mp);
-    const int64_t k1 = count_below(hi, rn, mp);
-    for (int64_t k = k0; k < k1; ++k) S[k] = (unsigned)j;
+    const long long pb = __double_as_longlong(p);
+    if (!ok || !(pb > 0 && pb <= 0x7ff0000000000000ll)) return;  // p > 0
+    const int64_t k1 = count(hi);
+    for (int64_t k = count(lo); k < k1; ++k) S[k] = (unsigned)j;
   }
 };
 
@@ -295,60 +379,187 @@ struct ConsSample2 {
   }
 };
 
-// The select digit: the largest d with count(digit >= d) >= m (one thread).
-__global__ void k_select_digit(const unsigned* __restrict__ hist, int64_t m, Ctl* c, int bits, Rep rp = Rep{}) {
+// The select digit (one block of 1024): the candidates are the elements at
+// or above it.  For "largest" (c->norm unused, fri = 0) the largest digit d
+// with count(digit >= d) >= m.  For FRI a higher one when the histogram
+// already shows where get_d_largest must stop: with C elements at or above
+// bin b, their sum at most S (counts times the bins' upper edges) and every
+// other |x| below b's lower edge e, position C of the sorted list fails the
+// acceptance test when (m - C) e < norm - S - e, so |D| <= C and only those C
+// elements have to be sorted and chained.  (slack covers the chain's own
+// rounding, at most C half-ulps of the norm, and that of S.)  A norm or a
+// sum that is infinite or NaN keeps the m largest.  One thread walking the bins took
+// 147 us; this takes ~6.
+__global__ void __launch_bounds__(1024) k_select_digit(const unsigned* __restrict__ hist, int64_t m, Ctl* c, int bits,
+                                                       int fri, Rep rp = Rep{}) {
   hist += blockIdx.x * rp.one * NDIG;
   c += blockIdx.x * rp.one;
-  int64_t cum = 0;
-  int d = (1 << bits) - 1;
-  for (; d >= 0; --d) {
-    cum += hist[d];
-    if (cum >= m) break;
+  __shared__ int64_t sm[33];
+  __shared__ double wsum[33];
+  __shared__ int s_best;
+  const int nb = 1 << bits, shift = 63 - bits, per = nb >> 10;  // bits >= 10
+  // thread t owns the bins nb-1 - (t per + j), j < per: descending
+  int64_t cnt = 0;
+  double sum = 0.0;
+  for (int j = 0; j < per; ++j) {
+    const int b = nb - 1 - ((int)threadIdx.x * per + j);
+    const unsigned h = hist[b];
+    cnt += h;
+    if (h) sum += (double)h * __longlong_as_double((long long)((unsigned long long)(b + 1) << shift));
   }
-  c->dmin = d < 0 ? 0 : d;
-  c->ncand = cum;
+  int64_t tot;
+  int64_t C = block_excl_sum(cnt, sm, &tot);
+  double incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double w = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((int)lane_id() >= o) incl += w;
+  }
+  if (lane_id() == 31) wsum[warp_id()] = incl;
+  if (threadIdx.x == 0) s_best = INT_MAX;
+  __syncthreads();
+  double S = 0.0;  // the sums of the warps before this one, then of the lanes
+  for (int w = 0; w < (int)warp_id(); ++w)
+    if (wsum[w] != 0.0) S += wsum[w];
+  {
+    const double ex = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane_id() > 0) S += ex;
+  }
+  const double norm = fri ? c->norm : 0.0;
+  const bool bound = fri && norm > 0.0 && norm < __longlong_as_double(0x7ff0000000000000ll);
+  for (int j = 0; j < per; ++j) {
+    const int b = nb - 1 - ((int)threadIdx.x * per + j);
+    const unsigned h = hist[b];
+    if (h) S += (double)h * __longlong_as_double((long long)((unsigned long long)(b + 1) << shift));
+    C += h;
+    bool stop = C >= m;
+    // only where the next bin holds something can the bound improve
+    if (!stop && bound && b > 0 && hist[b - 1]) {
+      const double e = __longlong_as_double((long long)((unsigned long long)b << shift));
+      const double slack = norm * ((double)(C + 2) * 0x1p-52 + 0x1p-38);
+      stop = (double)(m - C) * e < (norm - S - e - slack) * (1.0 - 0x1p-20);
+    }
+    if (stop) {
+      atomicMin(&s_best, (int)threadIdx.x * per + j);
+      break;
+    }
+  }
+  __syncthreads();
+  if (s_best != INT_MAX && s_best / per == (int)threadIdx.x) {
+    c->dmin = nb - 1 - s_best;  // this thread's C stopped at that bin
+    c->ncand = C;
+    c->mchain = m < C ? m : C;
+  }
+  if (s_best == INT_MAX && threadIdx.x == 0) {  // fewer than m elements: not reached (m <= n)
+    c->dmin = 0;
+    c->ncand = tot;
+    c->mchain = m < tot ? m : tot;
+  }
 }
 
-// After the remaining-norm chain: |D|, R, the D threshold, m' (one thread).
-__global__ void k_finish_d(const unsigned long long* __restrict__ ffail, const double* __restrict__ Rb,
-                           const unsigned long long* __restrict__ ckey, const unsigned* __restrict__ cidx, int64_t m,
-                           Ctl* c, Rep rp = Rep{}) {
-  {
-    const int64_t r = blockIdx.x;
-    ffail += r * rp.one;
-    Rb += r * rp.one * (m + 1);
-    ckey += r * rp.n;
-    cidx += r * rp.n;
-    c += r * rp.one;
-  }
-  const int64_t nd = (int64_t)*ffail;
+// |D|, R, the D threshold and m' into the state of this compression.
+__device__ __forceinline__ void set_d(Ctl* c, int64_t nd, double R, const unsigned long long* ckey,
+                                      const unsigned* cidx, int64_t m) {
   c->nd = nd;
   c->mp = m - nd;
   c->mprime = (double)(unsigned long long)(m - nd);
-  c->R = Rb[nd];
+  c->R = R;
   c->dkey = nd > 0 ? ckey[nd - 1] : 0ull;
   c->didx = nd > 0 ? (int64_t)cidx[nd - 1] : -1;
   c->sample = (c->R > 0.0 && isfinite(c->R)) ? 1 : 0;
 }
 
-__global__ void k_zero_u32(unsigned* p, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = 0;
+// The first chunks of the remaining-norm chain, in one block, until the
+// acceptance test first fails (D is usually a few thousand entries: one or
+// two chunks).  Sets c->found, and the chain's general kernels then have
+// nothing to do; a longer D leaves them the whole chain.
+constexpr int REM_CHUNKS = 4;
+__global__ void __launch_bounds__(1024) k_rem_first(ConsAccept ca0, const unsigned long long* ckey,
+                                                    const unsigned* cidx, Ctl* c, Rep rp = Rep{}) {
+  const int rep = blockIdx.x;
+  ConsAccept ca = exact::replica_of(ca0, rep);
+  ckey += rep * rp.n;
+  cidx += rep * rp.n;
+  c += rep * rp.one;
+  __shared__ exact::ChunkSmem csm;
+  __shared__ unsigned long long s_min[32];
+  const GenSorted gen{ckey};
+  const int64_t len = ca.mchain;
+  double s = c->norm;
+  if (len == 0) {  // no element can pass: D is empty
+    if (threadIdx.x == 0) {
+      set_d(c, 0, s, ckey, cidx, ca.m);
+      c->found = 1;
+    }
+    return;
+  }
+  for (int64_t ch = 0; ch < REM_CHUNKS && ch * exact::CH < len; ++ch) {
+    const int64_t base = ch * exact::CH;
+    const int n_in = (int)(len - base < exact::CH ? len - base : exact::CH);
+    s = exact::block_exact_chunk<1024, exact::CH / 1024>(gen, base, n_in, s, true, ca, csm);
+    const unsigned long long f = block_min<unsigned long long>(ca.mine, s_min);
+    const bool end = f == ~0ull && base + n_in == len;
+    if (f != ~0ull || end) {
+      const int64_t nd = end ? len : (int64_t)f;
+      if (threadIdx.x == 0) {
+        set_d(c, nd, ca.Rb[nd], ckey, cidx, ca.m);  // Rb[nd] was written before block_min's barriers
+        c->found = 1;
+      }
+      return;
+    }
+  }
+}
+
+// After the general chain: |D|, R, the D threshold, m' (unless found before).
+__global__ void k_finish_d(const unsigned long long* __restrict__ ffail, const double* __restrict__ Rb,
+                           const unsigned long long* __restrict__ ckey, const unsigned* __restrict__ cidx, int64_t m,
+                           Ctl* c, Ctl* c2, double rn2, const double* rn2_dev, int64_t rn_stride, Rep rp = Rep{}) {
+  const int64_t r = blockIdx.x;
+  c += r * rp.one;
+  if (!c->found) {
+    const int64_t nd = (int64_t)ffail[r * rp.one];
+    const int64_t at = nd < c->mchain ? nd : c->mchain;
+    set_d(c, at, Rb[r * rp.one * (m + 1) + at], ckey + r * rp.n, cidx + r * rp.n, m);
+  }
+  if (c2) {  // a paired compression's second state: the same, with its own draw
+    c2 += r * rp.one;
+    *c2 = *c;
+    c2->rn = rn2_dev ? rn2_dev[r * rn_stride] : rn2;
+  }
+}
+
+// Everything a compression needs zeroed or set, in one launch (six memsets,
+// a copy and two fills before): one grid row per replica.
+__global__ void k_init(unsigned* hist, unsigned long long* tstate, int64_t ntile1, unsigned* S, unsigned* S2,
+                       int64_t m, Ctl* c, double rn, const double* rn_dev, int64_t rn_stride, unsigned* err,
+                       unsigned* ticket, unsigned long long* ffail, double* dzero, unsigned* bar, double* psum,
+                       int64_t nch1) {
+  const int64_t r = blockIdx.y;
+  hist += r * NDIG;
+  tstate += r * ntile1;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t0; i < NDIG; i += stride) hist[i] = 0;
+  for (int64_t i = t0; i < ntile1; i += stride) tstate[i] = 0;
+  if (S)
+    for (int64_t i = t0; i < m; i += stride) S[r * m + i] = 0;
+  if (S2)
+    for (int64_t i = t0; i < m; i += stride) S2[r * m + i] = 0;
+  for (int64_t i = t0; i < nch1; i += stride) psum[r * nch1 + i] = 0.0;
+  if (t0 == 0) {
+    Ctl z{};
+    z.rn = rn_dev ? rn_dev[r * rn_stride] : rn;
+    c[r] = z;
+    err[r] = 0;
+    ticket[r] = 0;
+    ffail[r] = (unsigned long long)m;
+    dzero[0] = 0.0;
+    if (r == 0) bar[0] = 0;
+  }
 }
 
 // D part of the output: flat = sorted index, value = x (src/fri_utils.cpp:494,498-500)
-__global__ void k_out_d(const double* __restrict__ x, const unsigned* __restrict__ sidx, int64_t nd_max,
-                        const Ctl* __restrict__ c, int64_t* __restrict__ flat, double* __restrict__ vals,
-                        Rep rp = Rep{}) {
-  {
-    const int64_t r = blockIdx.y;
-    x += r * rp.n;
-    sidx += r * rp.n;
-    if (c) c += r * rp.one;
-    flat += r * rp.m;
-    vals += r * rp.m;
-  }
-  const int64_t nd = c ? c->nd : nd_max;
+__global__ void k_out_d(const double* __restrict__ x, const unsigned* __restrict__ sidx, int64_t nd,
+                        int64_t* __restrict__ flat, double* __restrict__ vals) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
     const unsigned j = sidx[i];
     flat[i] = j;
@@ -356,19 +567,30 @@ __global__ void k_out_d(const double* __restrict__ x, const unsigned* __restrict
   }
 }
 
-// S part: flat = S_k, value = x / p (src/fri_utils.cpp:495,502-504)
+// The whole output: D in sorted order (flat = index, value = x), then S,
+// flat = S_k, value = x / p (src/fri_utils.cpp:494-504); with meta, |D| and
+// the error word of this compression.
 template <class G>
-__global__ void k_out_s(G gp0, const unsigned* __restrict__ S, int64_t* __restrict__ flat,
-                        double* __restrict__ vals, Rep rp = Rep{}) {
-  const G gp = exact::replica_of(gp0, blockIdx.y);
-  S += blockIdx.y * rp.m;
-  flat += blockIdx.y * rp.m;
-  vals += blockIdx.y * rp.m;
-  const int64_t mp = gp.c->mp, nd = gp.c->nd;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < mp; k += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned j = S[k];
-    flat[nd + k] = j;
-    vals[nd + k] = __ddiv_rn(gp.x[j], gp.value(j));
+__global__ void k_out(G gp0, int64_t n, const unsigned* __restrict__ sidx, const unsigned* __restrict__ S, int64_t m,
+                      int64_t* __restrict__ flat, double* __restrict__ vals, const unsigned* err,
+                      unsigned long long* meta, Rep rp = Rep{}) {
+  const int64_t r = blockIdx.y;
+  const G gp = exact::replica_of(gp0, r);
+  sidx += r * rp.n;
+  S += r * rp.m;
+  flat += r * rp.m;
+  vals += r * rp.m;
+  const int64_t nd = gp.c->nd;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+    const bool d = i < nd;
+    unsigned j = d ? sidx[i] : S[i - nd];
+    if (j >= n) j = 0;  // only after a sort that gave up (its error bit is set): stay inside x
+    flat[i] = j;
+    vals[i] = d ? gp.x[j] : __ddiv_rn(gp.x[j], gp.value(j));
+  }
+  if (meta && blockIdx.x == 0 && threadIdx.x == 0) {
+    meta[2 * r * rp.one] = (unsigned long long)nd;
+    meta[2 * r * rp.one + 1] |= (unsigned long long)err[r * rp.one];
   }
 }
 
@@ -376,7 +598,7 @@ __global__ void k_unpack(const int64_t* __restrict__ flat, int64_t m, int64_t d0
                          int* __restrict__ slots, unsigned* err, Rep rp = Rep{}) {
   flat += blockIdx.y * rp.m;
   slots += 4 * blockIdx.y * rp.m;
-  err += blockIdx.y * rp.one;
+  err += 4 * blockIdx.y * rp.one;  // the low half of each status block's second word (16 bytes a replica)
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < m; s += (int64_t)gridDim.x * blockDim.x) {
     unsigned long long f = (unsigned long long)flat[s];
     const unsigned long long D1 = d1, D2 = d2, D3 = d3;
@@ -416,17 +638,38 @@ __global__ void k_unpack(const int64_t* __restrict__ flat, int64_t m, int64_t d0
 // element emits, bit 2 it emits the pivot.
 constexpr unsigned char PV_TAKE = 1, PV_EMIT = 2, PV_PIVOT = 4;
 
-__global__ void k_pvec(GenP gp0, int64_t n, double* __restrict__ P, unsigned* err, Rep rp = Rep{}) {
+// P = the p vector, with the p > 1 check and (psum, zeroed beforehand) the
+// approximate sum of each exact::CH chunk of the addends its chain takes.
+// Four blocks share a chunk, so that a small tensor's divisions (FP64, ~12
+// slow instructions each) spread over the chip.
+constexpr int PV_SUB = 4;
+__global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __restrict__ P, unsigned* err,
+                                              double* __restrict__ psum, Rep rp = Rep{}) {
+  constexpr int SUB = exact::CH / PV_SUB;
   const GenP gp = gp0.at(blockIdx.y);
   P += blockIdx.y * rp.n;
   err += blockIdx.y * rp.one;
+  __shared__ double red[32];
+  const int64_t base = (int64_t)blockIdx.x * SUB;
   bool bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double p = gp.value(i);
-    P[i] = p;
-    bad |= p > 1.0;
+  double acc = 0.0;
+#pragma unroll
+  for (int r = 0; r < SUB / 256; ++r) {
+    const int64_t i = base + r * 256 + threadIdx.x;
+    if (i < n) {
+      const double p = gp.value(i);
+      P[i] = p;
+      bad |= p > 1.0;
+      acc += p;
+    }
   }
   if (bad) atomicOr(err, FRICC_DEV_P_GT_ONE);
+  if (psum && gp.c->sample) {  // R <= 0 or not finite: the chain runs over zeros (GenPv)
+    const double tot = block_sum_det(acc, red);
+    const int64_t nch1 = fricc_cdiv(n, (int64_t)exact::CH) + 1;
+    // (the order of these four additions moves only the chain's prediction)
+    if (threadIdx.x == 0) atomicAdd(&psum[blockIdx.y * rp.one * nch1 + blockIdx.x / PV_SUB], tot);
+  }
 }
 
 // One warp.  Lane t of a batch of 32 elements keeps a_j and the wrap flag
@@ -652,18 +895,11 @@ __global__ void k_piv_final(const double* __restrict__ A, int64_t n, Ctl* c, uns
   if (bad) atomicOr(err, FRICC_DEV_PIVOTAL);
 }
 
-__global__ void k_set_u64(unsigned long long* p, unsigned long long v) { *p = v; }
-
-// |D| (m for "largest") and the error word into a handle's status block
-__global__ void k_put_meta(const Ctl* c, int64_t nd_fixed, const unsigned* err, unsigned long long* meta,
-                           Rep rp = Rep{}) {
-  if (c) c += blockIdx.x * rp.one;
-  err += blockIdx.x * rp.one;
-  meta += 2 * blockIdx.x * rp.one;
-  meta[0] = (unsigned long long)(c ? c->nd : nd_fixed);
+// the error word into a handle's status block, with |D| = m ("largest")
+__global__ void k_put_meta(int64_t nd, const unsigned* err, unsigned long long* meta) {
+  meta[0] = (unsigned long long)nd;
   meta[1] |= (unsigned long long)*err;
 }
-__global__ void k_set_f64(double* p, double v) { *p = v; }
 
 inline unsigned grid_for(int64_t n, int nt) {
   int64_t g = fricc_cdiv(n, nt);
@@ -685,10 +921,15 @@ struct CompressScratch {
   unsigned long long* tstate = nullptr;
   unsigned* ticket = nullptr;
   double* dzero = nullptr;
+  double* psum = nullptr;
+  unsigned* bar = nullptr;
   double* Rb = nullptr;
   unsigned long long* ffail = nullptr;
   unsigned* S = nullptr;
+  unsigned* S2 = nullptr;
   double* P = nullptr;
+  Ctl* ctl = nullptr;
+  Ctl* ctl2 = nullptr;  // a paired compression's second state
   exact::ChainScratch chain;
 };
 
@@ -703,6 +944,11 @@ static void free_scratch(CompressScratch& s, cudaStream_t st) {
   fricc_free(s.tstate, st);
   fricc_free(s.ticket, st);
   fricc_free(s.dzero, st);
+  fricc_free(s.psum, st);
+  fricc_free(s.bar, st);
+  fricc_free(s.S2, st);
+  fricc_free(s.ctl, st);
+  fricc_free(s.ctl2, st);
   fricc_free(s.Rb, st);
   fricc_free(s.ffail, st);
   fricc_free(s.S, st);
@@ -957,9 +1203,8 @@ extern "C" int fricc_phase_timing_read(double sec[5]) {
   return FRICC_OK;
 }
 
-static int pivotal(const double* x, int64_t n, int64_t m, const GenP& gp, Ctl* ctl, CompressScratch& s,
-                   unsigned* glibc_hist, int64_t* n_draws, cudaStream_t st) {
-  (void)x;
+static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsigned* glibc_hist, int64_t* n_draws,
+                   cudaStream_t st) {
   double *P = nullptr, *A = nullptr, *R = nullptr;
   unsigned char* code = nullptr;
   int64_t *tlast = nullptr, *tcnt = nullptr;
@@ -969,15 +1214,13 @@ static int pivotal(const double* x, int64_t n, int64_t m, const GenP& gp, Ctl* c
   if (!rc) rc = fricc_alloc_t(&code, n, st);
   if (!rc) rc = fricc_alloc_t(&tlast, ntile, st);
   if (!rc) rc = fricc_alloc_t(&tcnt, ntile, st);
-  if (!rc) rc = fricc_alloc_t(&s.S, m, st);
   int64_t jend = 0;
   unsigned e = 0;
   if (!rc) {
-    k_zero_u32<<<grid_for(m, 256), 256, 0, st>>>(s.S, m);
-    k_pvec<<<grid_for(n, 256), 256, 0, st>>>(gp, n, P, s.err);
+    k_pvec<<<(unsigned)fricc_cdiv(n, exact::CH / PV_SUB), 256, 0, st>>>(gp, n, P, s.err, nullptr);
     phase_mark(2, st);
     k_piv_chain<<<1, 32, 0, st>>>(P, n, ctl, A, code);
-    fricc_note_launch(3);
+    fricc_note_launch(2);
     rc = fricc_cuda_check(cudaGetLastError(), "pivotal chain");
   }
   if (!rc) rc = fricc_cuda_check(cudaMemcpyAsync(&jend, &ctl->jend, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "jend");
@@ -1019,6 +1262,124 @@ static int pivotal(const double* x, int64_t n, int64_t m, const GenP& gp, Ctl* c
   return rc;
 }
 
+// The uniform draws of a compression and (paired) of its second one: host
+// values, or device words (replica r's at a_dev[r * stride]).
+struct Draws {
+  double a = 0.0, b = 0.0;
+  const double* a_dev = nullptr;
+  const double* b_dev = nullptr;
+  int64_t stride = 0;
+};
+
+// One compression's (or a batch of R's) first half: scratch, histogram,
+// one_norm, candidates, their sort, and for mode 0 and 2 the
+// remaining-norm chain: |D|, R and m' in s.ctl (and s.ctl2 when paired).
+static int compress_front(const double* x, int64_t n, int64_t m, int R, int mode, bool paired, const Draws& dr,
+                          const Rep& rp, CompressScratch& s, cudaStream_t st) {
+  const int64_t ntile = fricc_cdiv(n, 4096);
+  const int64_t nch_n = fricc_cdiv(n, exact::CH), nch_m = fricc_cdiv(m, exact::CH);
+  const int64_t nch1 = (nch_n > nch_m ? nch_n : nch_m) + 1;
+  const int64_t rhw = radix::hist_words(n);
+  const size_t r_ = (size_t)R;
+  const bool fri = mode != 1;
+  int rc = fricc_alloc_t(&s.ctl, r_, st);
+  if (!rc && paired) rc = fricc_alloc_t(&s.ctl2, r_, st);
+  if (!rc) rc = fricc_alloc_t(&s.hist, r_ * NDIG, st);
+  if (!rc) rc = fricc_alloc_t(&s.err, r_, st);
+  if (!rc) rc = fricc_alloc_t(&s.ckey, r_ * n, st);
+  if (!rc) rc = fricc_alloc_t(&s.cidx, r_ * n, st);
+  if (!rc) rc = fricc_alloc_t(&s.ktmp, r_ * n, st);
+  if (!rc) rc = fricc_alloc_t(&s.vtmp, r_ * n, st);
+  if (!rc) rc = fricc_alloc_t(&s.tstate, r_ * (ntile + 1), st);  // + a zero word no tile writes (the test-only wait)
+  if (!rc) rc = fricc_alloc_t(&s.ticket, r_, st);
+  if (!rc) rc = fricc_alloc_t(&s.rhist, r_ * rhw, st);
+  if (!rc) rc = fricc_alloc_t(&s.bar, 1, st);
+  if (!rc) rc = fricc_alloc_t(&s.dzero, 1, st);
+  if (!rc) rc = fricc_alloc_t(&s.ffail, r_, st);
+  if (!rc) rc = fricc_alloc_t(&s.psum, r_ * nch1, st);
+  if (!rc && fri) rc = exact::chain_scratch(s.chain, R * nch1, st);
+  if (!rc && fri) rc = fricc_alloc_t(&s.Rb, r_ * (m + 1), st);
+  if (!rc && fri) rc = fricc_alloc_t(&s.S, r_ * m, st);
+  if (!rc && paired) rc = fricc_alloc_t(&s.S2, r_ * m, st);
+  if (rc) return rc;
+
+  k_init<<<dim3(grid_for(fri ? m : NDIG, 512), R), 256, 0, st>>>(s.hist, s.tstate, ntile + 1, s.S, s.S2, m, s.ctl,
+                                                                 dr.a, dr.a_dev, dr.stride, s.err, s.ticket, s.ffail,
+                                                                 s.dzero, s.bar, s.psum, nch_n + 1);
+  phase_mark(0, st);
+  const int bits = select_bits();
+  const int64_t gh = nch_n < 152 * 6 ? nch_n : 152 * 6;
+  k_hist_sums<<<dim3((unsigned)gh, R), 256, sizeof(unsigned) << bits, st>>>(x, n, s.hist, bits,
+                                                                            fri ? s.chain.csum : nullptr, rp);
+  fricc_note_launch(2);
+  const int64_t cw = (int64_t)(sizeof(Ctl) / sizeof(int64_t));  // a Ctl in 8-byte words
+  static_assert(sizeof(Ctl) % sizeof(int64_t) == 0, "Ctl must be a whole number of int64 words");
+  exact::ChainStride zero_start, ctl_start;
+  ctl_start.s_init = cw;
+  if (fri) {  // one_norm
+    rc = exact::run_chain<GenAbs, exact::ConsNull, false>(GenAbs{x, rp.n}, exact::Len{n}, s.dzero, false,
+                                                          exact::ConsNull{}, s.chain, st, R, zero_start, true,
+                                                          &s.ctl->norm, cw);
+    if (rc) return rc;
+  }
+  k_select_digit<<<R, 1024, 0, st>>>(s.hist, m, s.ctl, bits, fri ? 1 : 0, rp);
+  k_compact<<<dim3((unsigned)ntile, R), 256, 0, st>>>(x, n, s.ctl, s.ktmp, s.vtmp, s.tstate, s.ticket, s.err,
+                                                      s.tstate + ntile,
+                                                      (long long)fricc_tune_get(FRICC_TUNE_TEST_WAIT), 63 - bits, rp);
+  fricc_note_launch(2);
+  // argsort (src/fri_utils.cpp:11-36) of the candidates
+  radix::Batch bt;
+  bt.kv_stride = rp.n;
+  bt.hist_stride = rhw;
+  bt.n_stride = cw;
+  rc = radix::sort_desc_dev(s.ktmp, s.vtmp, s.ckey, s.cidx, n, &s.ctl->ncand, s.rhist, s.bar, s.err, st, R, bt);
+  if (rc || !fri) return rc;
+
+  const ConsAccept ca{m, s.Rb, s.ffail, s.ctl, rp.one};
+  k_rem_first<<<R, 1024, 0, st>>>(ca, s.ckey, s.cidx, s.ctl, rp);
+  fricc_note_launch();
+  exact::Len ln;
+  ln.n = m;
+  ln.dev = &s.ctl->mchain;
+  ln.stride = cw;
+  ln.skip = reinterpret_cast<const int*>(&s.ctl->found);
+  ln.sstride = 2 * cw;
+  if (m > REM_CHUNKS * exact::CH) {
+    rc = exact::run_chain<GenSorted, ConsAccept, true>(GenSorted{s.ckey, rp.n}, ln, &s.ctl->norm, true, ca, s.chain,
+                                                       st, R, ctl_start);
+    if (rc) return rc;
+  }
+  if (m > REM_CHUNKS * exact::CH || paired) {
+    k_finish_d<<<R, 1, 0, st>>>(s.ffail, s.Rb, s.ckey, s.cidx, m, s.ctl, s.ctl2, dr.b, dr.b_dev, dr.stride, rp);
+    fricc_note_launch();
+  }
+  return fricc_cuda_check(cudaGetLastError(), "compression");
+}
+
+// Probabilities (once, with the p > 1 check), their exact partial sums and
+// the systematic samples of one or (s.ctl2) both draws.  With m' = 0 every p
+// is 0 (or NaN); with R <= 0 or not finite no interval matches: in both
+// cases all samples keep index 0, as in the reference.
+static int compress_systematic(const double* x, int64_t n, int64_t m, int R, const Rep& rp, CompressScratch& s,
+                               cudaStream_t st) {
+  int rc = fricc_alloc_t(&s.P, (size_t)R * n, st);
+  if (rc) return rc;
+  k_pvec<<<dim3((unsigned)fricc_cdiv(n, exact::CH / PV_SUB), R), 256, 0, st>>>(GenP{x, s.ctl, rp.n, rp.one}, n, s.P,
+                                                                               s.err, s.psum, rp);
+  fricc_note_launch();
+  phase_mark(2, st);
+  const GenPv gpv{s.P, x, s.ctl, rp.n, rp.one};
+  const ConsSample cs{s.ctl, s.S, rp.one, rp.m};
+  exact::ChainScratch sc = s.chain;  // the same scratch, with the chunk sums k_pvec left
+  sc.csum = s.psum;
+  if (s.ctl2)
+    return exact::run_chain<GenPv, ConsSample2, true>(gpv, exact::Len{n}, s.dzero, false,
+                                                      ConsSample2{cs, ConsSample{s.ctl2, s.S2, rp.one, rp.m}}, sc, st,
+                                                      R, exact::ChainStride{}, true);
+  return exact::run_chain<GenPv, ConsSample, true>(gpv, exact::Len{n}, s.dzero, false, cs, sc, st, R,
+                                                   exact::ChainStride{}, true);
+}
+
 // mode 2: "fri" with pivotal sampling.  Its draws (one per visited element)
 // come from the glibc stream whose history is glibc_hist[31] (host, oldest
 // first; advanced past the draws on return), or with glibc_hist == nullptr
@@ -1044,9 +1405,6 @@ int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, doubl
     return FRICC_ERR_ARG;
   }
   CompressScratch s;
-  Ctl* ctl = nullptr;
-  Ctl* ctl2 = nullptr;  // a paired compression's second state
-  unsigned* S2 = nullptr;
   int rc = FRICC_OK;
 #define TRY(x)                  \
   do {                          \
@@ -1055,54 +1413,23 @@ int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, doubl
   } while (0)
 
   {
-    const int64_t ntile = fricc_cdiv(n, 4096);
-    TRY(fricc_alloc_t(&ctl, 1, st));
-    TRY(fricc_alloc_t(&s.hist, NDIG, st));
-    TRY(fricc_alloc_t(&s.err, 1, st));
-    TRY(fricc_alloc_t(&s.ckey, n, st));
-    TRY(fricc_alloc_t(&s.cidx, n, st));
-    TRY(fricc_alloc_t(&s.ktmp, n, st));
-    TRY(fricc_alloc_t(&s.vtmp, n, st));
-    TRY(fricc_alloc_t(&s.tstate, ntile + 1, st));  // + a zero word no tile writes (the test-only wait)
-    TRY(fricc_alloc_t(&s.ticket, 1, st));
-    TRY(fricc_alloc_t(&s.rhist, radix::hist_words(n), st));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.hist, 0, NDIG * sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.err, 0, sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.tstate, 0, (ntile + 1) * sizeof(unsigned long long), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.ticket, 0, sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st), "memset"));
-    if (rn_dev) {
-      // the draw already in device memory (stream-ordered; capturable)
-      TRY(fricc_cuda_check(cudaMemcpyAsync(&ctl->rn, rn_dev, sizeof(double), cudaMemcpyDeviceToDevice, st), "rn"));
-    } else {
-      // the draw goes through a device word (a pageable-source copy completes
-      // before cudaMemcpyAsync returns, so a stack value is safe)
-      const double rn_h = rn;
-      TRY(fricc_cuda_check(cudaMemcpyAsync(&ctl->rn, &rn_h, sizeof(double), cudaMemcpyHostToDevice, st), "rn"));
+    Draws dr;
+    dr.a = rn;
+    dr.a_dev = rn_dev;
+    if (pair) {
+      dr.b = pair->rn;
+      dr.b_dev = pair->rn_dev;
     }
-
-    // 1-2. select digit, candidates, sort (argsort, src/fri_utils.cpp:11-36)
-    phase_mark(0, st);
-    {
-      const int bits = select_bits();
-      k_hist_sel<<<grid_for(n, 256), 256, sizeof(unsigned) << bits, st>>>(x, n, s.hist, bits);
-      k_select_digit<<<1, 1, 0, st>>>(s.hist, m, ctl, bits);
-      k_compact<<<(unsigned)ntile, 256, 0, st>>>(x, n, ctl, s.ckey, s.cidx, s.tstate, s.ticket, s.err,
-                                                 s.tstate + ntile, (long long)fricc_tune_get(FRICC_TUNE_TEST_WAIT),
-                                                 63 - bits);
-    }
-    fricc_note_launch(3);
-    TRY(radix::sort_pairs(s.ckey, s.cidx, s.ktmp, s.vtmp, n, 64, true, s.rhist, st, &ctl->ncand));
-
+    TRY(compress_front(x, n, m, 1, mode, pair != nullptr, dr, Rep{}, s, st));
     if (mode == 1) {  // "largest": argsort(x, m) with unscaled values
       phase_mark(1, st);
       phase_mark(2, st);
       phase_mark(3, st);
-      k_out_d<<<grid_for(m, 256), 256, 0, st>>>(x, s.cidx, m, nullptr, flat, vals);
+      k_out_d<<<grid_for(m, 256), 256, 0, st>>>(x, s.cidx, m, flat, vals);
       fricc_note_launch();
       phase_mark(4, st);
       if (meta) {
-        k_put_meta<<<1, 1, 0, st>>>(nullptr, m, s.err, meta);
+        k_put_meta<<<1, 1, 0, st>>>(m, s.err, meta);
         fricc_note_launch();
       }
       TRY(fricc_cuda_check(cudaGetLastError(), "largest"));
@@ -1115,102 +1442,23 @@ int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, doubl
       }
       goto done;
     }
-
-    // 3. one_norm
-    TRY(fricc_alloc_t(&s.dzero, 1, st));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.dzero, 0, sizeof(double), st), "memset"));
-    TRY((exact::run_chain<GenAbs, exact::ConsNull, false, false>(GenAbs{x}, n, s.dzero, false, exact::ConsNull{},
-                                                                 s.chain, s.err, st)));
-    const int64_t nch_n = fricc_cdiv(n, exact::CH);
-    double* R0 = nullptr;
-    TRY(fricc_alloc_t(&R0, 1, st));
-    cudaMemcpyAsync(R0, s.chain.cstart + nch_n, sizeof(double), cudaMemcpyDeviceToDevice, st);
-
-    // 4. remaining-norm chain over the sorted top m, acceptance test
-    TRY(fricc_alloc_t(&s.Rb, m + 1, st));
-    TRY(fricc_alloc_t(&s.ffail, 1, st));
-    k_set_u64<<<1, 1, 0, st>>>(s.ffail, (unsigned long long)m);
-    fricc_note_launch();
-    ConsAccept ca{m, s.Rb, s.ffail};
-    rc = exact::run_chain<GenSorted, ConsAccept, false, true>(GenSorted{s.ckey}, m, R0, true, ca, s.chain, s.err, st);
-    fricc_free(R0, st);
-    if (rc) goto done;
-    k_finish_d<<<1, 1, 0, st>>>(s.ffail, s.Rb, s.ckey, s.cidx, m, ctl);
-    fricc_note_launch();
     phase_mark(1, st);
-    if (pair) {  // the second compression: the same state, its own draw
-      TRY(fricc_alloc_t(&ctl2, 1, st));
-      TRY(fricc_cuda_check(cudaMemcpyAsync(ctl2, ctl, sizeof(Ctl), cudaMemcpyDeviceToDevice, st), "ctl"));
-      if (pair->rn_dev) {
-        TRY(fricc_cuda_check(cudaMemcpyAsync(&ctl2->rn, pair->rn_dev, sizeof(double), cudaMemcpyDeviceToDevice, st),
-                             "rn"));
-      } else {
-        const double rn_h = pair->rn;
-        TRY(fricc_cuda_check(cudaMemcpyAsync(&ctl2->rn, &rn_h, sizeof(double), cudaMemcpyHostToDevice, st), "rn"));
-      }
-    }
-
-    GenP gp{x, ctl};
+    const GenP gp{x, s.ctl};
     if (mode == 2) {
-      TRY(pivotal(x, n, m, gp, ctl, s, glibc_hist, n_draws, st));
+      TRY(pivotal(n, gp, s.ctl, s, glibc_hist, n_draws, st));
       phase_mark(3, st);
-      k_out_d<<<grid_for(m, 256), 256, 0, st>>>(x, s.cidx, m, ctl, flat, vals);
-      k_out_s<<<grid_for(m, 256), 256, 0, st>>>(gp, s.S, flat, vals);
-      fricc_note_launch(2);
+      k_out<GenP><<<grid_for(m, 256), 256, 0, st>>>(gp, n, s.cidx, s.S, m, flat, vals, s.err, meta);
+      fricc_note_launch();
       phase_mark(4, st);
-      if (meta) {
-        k_put_meta<<<1, 1, 0, st>>>(ctl, 0, s.err, meta);
-        fricc_note_launch();
-      }
-      TRY(fricc_cuda_check(cudaGetLastError(), "output"));
-      if (n_largest) {
-        int64_t nd = 0;
-        TRY(fricc_cuda_check(cudaMemcpyAsync(&nd, &ctl->nd, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "nd"));
-        TRY(fricc_cuda_check(cudaStreamSynchronize(st), "compression"));
-        *n_largest = nd;
-      }
-      goto done;
-    }
-
-    // 5. probabilities (once, with the p > 1 check), exact partial sums,
-    //    systematic samples
-    TRY(fricc_alloc_t(&s.S, m, st));
-    TRY(fricc_alloc_t(&s.P, n, st));
-    k_zero_u32<<<grid_for(m, 256), 256, 0, st>>>(s.S, m);
-    k_pvec<<<grid_for(n, 256), 256, 0, st>>>(gp, n, s.P, s.err);
-    fricc_note_launch(2);
-    phase_mark(2, st);
-    // with m' = 0 every p is 0 (or NaN); with R <= 0 or not finite no
-    // interval matches (ConsSample checks ctl->sample): in both cases all
-    // samples keep index 0, as in the reference
-    const GenPv gpv{s.P, x, ctl};
-    ConsSample cs{ctl, s.S};
-    if (pair) {
-      TRY(fricc_alloc_t(&S2, m, st));
-      k_zero_u32<<<grid_for(m, 256), 256, 0, st>>>(S2, m);
-      fricc_note_launch();
-      ConsSample2 cs2{cs, ConsSample{ctl2, S2}};
-      TRY((exact::run_chain<GenPv, ConsSample2, false, true>(gpv, n, s.dzero, false, cs2, s.chain, s.err, st)));
     } else {
-      TRY((exact::run_chain<GenPv, ConsSample, false, true>(gpv, n, s.dzero, false, cs, s.chain, s.err, st)));
-    }
-
-    // 6. output
-    phase_mark(3, st);
-    k_out_d<<<grid_for(m, 256), 256, 0, st>>>(x, s.cidx, m, ctl, flat, vals);
-    k_out_s<<<grid_for(m, 256), 256, 0, st>>>(gpv, s.S, flat, vals);
-    fricc_note_launch(2);
-    if (!pair) phase_mark(4, st);
-    if (meta) {
-      k_put_meta<<<1, 1, 0, st>>>(ctl, 0, s.err, meta);
-      fricc_note_launch();
-    }
-    if (pair) {
-      const GenPv gpv2{s.P, x, ctl2};
-      k_out_d<<<grid_for(m, 256), 256, 0, st>>>(x, s.cidx, m, ctl2, pair->flat, pair->vals);
-      k_out_s<<<grid_for(m, 256), 256, 0, st>>>(gpv2, S2, pair->flat, pair->vals);
-      k_put_meta<<<1, 1, 0, st>>>(ctl2, 0, s.err, pair->meta);
-      fricc_note_launch(3);
+      TRY(compress_systematic(x, n, m, 1, Rep{}, s, st));
+      phase_mark(3, st);
+      k_out<GenPv><<<grid_for(m, 256), 256, 0, st>>>(GenPv{s.P, x, s.ctl}, n, s.cidx, s.S, m, flat, vals, s.err,
+                                                         meta);
+      if (pair)
+        k_out<GenPv><<<grid_for(m, 256), 256, 0, st>>>(GenPv{s.P, x, s.ctl2}, n, s.cidx, s.S2, m, pair->flat,
+                                                           pair->vals, s.err, pair->meta);
+      fricc_note_launch(pair ? 2 : 1);
       phase_mark(4, st);
     }
     TRY(fricc_cuda_check(cudaGetLastError(), "output"));
@@ -1218,7 +1466,7 @@ int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, doubl
       unsigned e = 0;
       int64_t nd = 0;
       TRY(fricc_cuda_check(cudaMemcpyAsync(&e, s.err, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "err"));
-      TRY(fricc_cuda_check(cudaMemcpyAsync(&nd, &ctl->nd, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "nd"));
+      TRY(fricc_cuda_check(cudaMemcpyAsync(&nd, &s.ctl->nd, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "nd"));
       TRY(fricc_cuda_check(cudaStreamSynchronize(st), "compression"));
       TRY(dev_status(e));
       *n_largest = nd;
@@ -1227,9 +1475,6 @@ int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, doubl
 done:
 #undef TRY
   free_scratch(s, st);
-  fricc_free(ctl, st);
-  fricc_free(ctl2, st);
-  fricc_free(S2, st);
   return rc;
 }
 
@@ -1239,35 +1484,6 @@ done:
 // of the single path with the replica on its grid's y (or x) dimension, each
 // replica's arithmetic that of its own single compression, so each output is
 // bit for bit the one fricc_sp_recompress_pair would give.
-namespace {
-
-__global__ void k_fill_u64_b(unsigned long long* p, unsigned long long v, int R) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < R) p[r] = v;
-}
-
-// R0[r] = the exact one_norm of replica r (the end of its chain)
-__global__ void k_chain_end_b(const double* cstart, int64_t nch, double* R0, int R) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < R) R0[r] = cstart[(int64_t)r * (nch + 1) + nch];
-}
-
-// the replicas' draws into their two compression states
-__global__ void k_set_rn_b(Ctl* a, Ctl* b, const double* rn, int R) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < R) {
-    a[r].rn = rn[2 * r];
-    b[r].rn = rn[2 * r + 1];
-  }
-}
-
-__global__ void k_meta_or_b(const unsigned* err, unsigned long long* meta, int R) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < R) meta[2 * r + 1] |= (unsigned long long)err[r];
-}
-
-}  // namespace
-
 int fricc_compress_pair_batch_device(const double* x, int64_t n, int64_t m, int R, const double* rn_dev,
                                      int64_t* flatA, double* valsA, unsigned long long* metaA, int64_t* flatB,
                                      double* valsB, unsigned long long* metaB, cudaStream_t st) {
@@ -1280,142 +1496,26 @@ int fricc_compress_pair_batch_device(const double* x, int64_t n, int64_t m, int 
                     (long long)n);
     return FRICC_ERR_ARG;
   }
-  const int64_t ntile = fricc_cdiv(n, 4096);
-  const int64_t nch_n = fricc_cdiv(n, exact::CH), nch_m = fricc_cdiv(m, exact::CH);
-  const int64_t rhw = radix::hist_words(n);
   Rep rp;
   rp.n = n;
   rp.m = m;
-  rp.tile = ntile + 1;
+  rp.tile = fricc_cdiv(n, 4096) + 1;
   rp.one = 1;
   CompressScratch s;
-  Ctl *ctl = nullptr, *ctl2 = nullptr;
-  unsigned* S2 = nullptr;
-  double* R0 = nullptr;
-  int rc = FRICC_OK;
-#define TRY(x)         \
-  do {                 \
-    rc = (x);          \
-    if (rc) goto done; \
-  } while (0)
-  {
-    const unsigned rb = (unsigned)fricc_cdiv(R, 256);
-    TRY(fricc_alloc_t(&ctl, R, st));
-    TRY(fricc_alloc_t(&ctl2, R, st));
-    TRY(fricc_alloc_t(&s.hist, (size_t)R * NDIG, st));
-    TRY(fricc_alloc_t(&s.err, R, st));
-    TRY(fricc_alloc_t(&s.ckey, (size_t)R * n, st));
-    TRY(fricc_alloc_t(&s.cidx, (size_t)R * n, st));
-    TRY(fricc_alloc_t(&s.ktmp, (size_t)R * n, st));
-    TRY(fricc_alloc_t(&s.vtmp, (size_t)R * n, st));
-    TRY(fricc_alloc_t(&s.tstate, (size_t)R * (ntile + 1), st));
-    TRY(fricc_alloc_t(&s.ticket, R, st));
-    TRY(fricc_alloc_t(&s.rhist, (size_t)R * rhw, st));
-    TRY(fricc_alloc_t(&s.dzero, 1, st));
-    TRY(fricc_alloc_t(&R0, R, st));
-    TRY(fricc_alloc_t(&s.Rb, (size_t)R * (m + 1), st));
-    TRY(fricc_alloc_t(&s.ffail, R, st));
-    TRY(fricc_alloc_t(&s.S, (size_t)R * m, st));
-    TRY(fricc_alloc_t(&S2, (size_t)R * m, st));
-    TRY(fricc_alloc_t(&s.P, (size_t)R * n, st));
-    {
-      const int64_t nch = nch_n > nch_m ? nch_n : nch_m;
-      TRY(fricc_alloc_t(&s.chain.csum, (size_t)R * (nch + 1), st));
-      TRY(fricc_alloc_t(&s.chain.cbin, (size_t)R * (nch + 1), st));
-      TRY(fricc_alloc_t(&s.chain.cmap, (size_t)R * (nch + 1), st));
-      TRY(fricc_alloc_t(&s.chain.cstart, (size_t)R * (nch + 1), st));
-      s.chain.cap = R * (nch + 1);
-    }
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.hist, 0, (size_t)R * NDIG * sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.err, 0, (size_t)R * sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.tstate, 0, (size_t)R * (ntile + 1) * sizeof(unsigned long long), st),
-                         "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.ticket, 0, (size_t)R * sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(ctl, 0, (size_t)R * sizeof(Ctl), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.dzero, 0, sizeof(double), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(s.S, 0, (size_t)R * m * sizeof(unsigned), st), "memset"));
-    TRY(fricc_cuda_check(cudaMemsetAsync(S2, 0, (size_t)R * m * sizeof(unsigned), st), "memset"));
-    const unsigned gn = grid_for(n, 256), gm = grid_for(m, 256);
-
-    // 1-2. select digit, candidates, sort
-    const int bits = select_bits();
-    k_hist_sel<<<dim3(gn, R), 256, sizeof(unsigned) << bits, st>>>(x, n, s.hist, bits, rp);
-    k_select_digit<<<R, 1, 0, st>>>(s.hist, m, ctl, bits, rp);
-    k_compact<<<dim3((unsigned)ntile, R), 256, 0, st>>>(x, n, ctl, s.ckey, s.cidx, s.tstate, s.ticket, s.err,
-                                                        s.tstate + ntile,
-                                                        (long long)fricc_tune_get(FRICC_TUNE_TEST_WAIT), 63 - bits,
-                                                        rp);
-    fricc_note_launch(3);
-    {
-      radix::Batch bt;
-      bt.kv_stride = n;
-      bt.hist_stride = rhw;
-      bt.n_stride = (int64_t)(sizeof(Ctl) / sizeof(int64_t));
-      static_assert(sizeof(Ctl) % sizeof(int64_t) == 0, "Ctl must be a whole number of int64 words");
-      TRY(radix::sort_pairs(s.ckey, s.cidx, s.ktmp, s.vtmp, n, 64, true, s.rhist, st, &ctl->ncand, R, bt));
-    }
-
-    // 3. one_norm
-    {
-      exact::ChainStride cs;
-      cs.s_init = 0;
-      cs.err = 1;
-      TRY((exact::run_chain<GenAbs, exact::ConsNull, false, false>(GenAbs{x, n}, n, s.dzero, false,
-                                                                   exact::ConsNull{}, s.chain, s.err, st, R, cs)));
-      k_chain_end_b<<<rb, 256, 0, st>>>(s.chain.cstart, nch_n, R0, R);
-      fricc_note_launch();
-    }
-
-    // 4. remaining-norm chain and acceptance test
-    k_fill_u64_b<<<rb, 256, 0, st>>>(s.ffail, (unsigned long long)m, R);
-    fricc_note_launch();
-    {
-      exact::ChainStride cs;
-      cs.s_init = 1;
-      cs.err = 1;
-      ConsAccept ca{m, s.Rb, s.ffail, 1};
-      TRY((exact::run_chain<GenSorted, ConsAccept, false, true>(GenSorted{s.ckey, n}, m, R0, true, ca, s.chain,
-                                                                s.err, st, R, cs)));
-    }
-    k_finish_d<<<R, 1, 0, st>>>(s.ffail, s.Rb, s.ckey, s.cidx, m, ctl, rp);
-    fricc_note_launch();
-    // the second compression: the same state, its own draw
-    TRY(fricc_cuda_check(cudaMemcpyAsync(ctl2, ctl, (size_t)R * sizeof(Ctl), cudaMemcpyDeviceToDevice, st), "ctl"));
-    k_set_rn_b<<<rb, 256, 0, st>>>(ctl, ctl2, rn_dev, R);
-    fricc_note_launch();
-
-    // 5. probabilities, exact partial sums, both samplers
-    const GenP gp{x, ctl, n, 1};
-    k_pvec<<<dim3(gn, R), 256, 0, st>>>(gp, n, s.P, s.err, rp);
-    fricc_note_launch();
-    const GenPv gpv{s.P, x, ctl, n, 1};
-    {
-      exact::ChainStride cs;
-      cs.s_init = 0;
-      cs.err = 1;
-      ConsSample2 cs2{ConsSample{ctl, s.S, 1, m}, ConsSample{ctl2, S2, 1, m}};
-      TRY((exact::run_chain<GenPv, ConsSample2, false, true>(gpv, n, s.dzero, false, cs2, s.chain, s.err, st, R,
-                                                             cs)));
-    }
-
-    // 6. outputs
-    k_out_d<<<dim3(gm, R), 256, 0, st>>>(x, s.cidx, m, ctl, flatA, valsA, rp);
-    k_out_s<<<dim3(gm, R), 256, 0, st>>>(gpv, s.S, flatA, valsA, rp);
-    k_put_meta<<<R, 1, 0, st>>>(ctl, 0, s.err, metaA, rp);
-    const GenPv gpv2{s.P, x, ctl2, n, 1};
-    k_out_d<<<dim3(gm, R), 256, 0, st>>>(x, s.cidx, m, ctl2, flatB, valsB, rp);
-    k_out_s<<<dim3(gm, R), 256, 0, st>>>(gpv2, S2, flatB, valsB, rp);
-    k_put_meta<<<R, 1, 0, st>>>(ctl2, 0, s.err, metaB, rp);
-    fricc_note_launch(6);
-    TRY(fricc_cuda_check(cudaGetLastError(), "compress batch"));
+  Draws dr;
+  dr.a_dev = rn_dev;
+  dr.b_dev = rn_dev + 1;
+  dr.stride = 2;
+  int rc = compress_front(x, n, m, R, 0, true, dr, rp, s, st);
+  if (!rc) rc = compress_systematic(x, n, m, R, rp, s, st);
+  if (!rc) {
+    const dim3 g(grid_for(m, 256), R);
+    k_out<GenPv><<<g, 256, 0, st>>>(GenPv{s.P, x, s.ctl, n, 1}, n, s.cidx, s.S, m, flatA, valsA, s.err, metaA, rp);
+    k_out<GenPv><<<g, 256, 0, st>>>(GenPv{s.P, x, s.ctl2, n, 1}, n, s.cidx, s.S2, m, flatB, valsB, s.err, metaB, rp);
+    fricc_note_launch(2);
+    rc = fricc_cuda_check(cudaGetLastError(), "compress batch");
   }
-done:
-#undef TRY
   free_scratch(s, st);
-  fricc_free(ctl, st);
-  fricc_free(ctl2, st);
-  fricc_free(S2, st);
-  fricc_free(R0, st);
   return rc;
 }
 
@@ -1423,39 +1523,25 @@ done:
 // an out-of-range index is ORed into the replica's meta[1].
 int fricc_unpack_batch_async(const int64_t* flat, int64_t m, int R, const int64_t dims[4], int* slots,
                              unsigned long long* meta, cudaStream_t st) {
-  unsigned* err = nullptr;
-  int rc = fricc_alloc_t(&err, R, st);
-  if (rc) return rc;
-  cudaMemsetAsync(err, 0, (size_t)R * sizeof(unsigned), st);
   Rep rp;
   rp.m = m;
   rp.one = 1;
-  k_unpack<<<dim3(grid_for(m, 256), R), 256, 0, st>>>(flat, m, dims[0], dims[1], dims[2], dims[3], slots, err, rp);
-  k_meta_or_b<<<(unsigned)fricc_cdiv(R, 256), 256, 0, st>>>(err, meta, R);
-  fricc_note_launch(2);
-  cudaError_t ce = cudaGetLastError();
-  fricc_free(err, st);
-  return ce == cudaSuccess ? FRICC_OK : fricc_cuda_fail(ce, "unpack batch", __FILE__, __LINE__);
+  k_unpack<<<dim3(grid_for(m, 256), R), 256, 0, st>>>(flat, m, dims[0], dims[1], dims[2], dims[3], slots,
+                                                      reinterpret_cast<unsigned*>(meta + 1), rp);
+  fricc_note_launch();
+  return fricc_cuda_check(cudaGetLastError(), "unpack batch");
 }
 
 // The error bits of a deferred status word, as a status code (and message).
 int fricc_dev_status(unsigned e) { return dev_status(e); }
 
-__global__ void k_meta_or(const unsigned* err, unsigned long long* meta) { meta[1] |= (unsigned long long)*err; }
-
 // Unpack without waiting: an out-of-range index is ORed into meta[1].
 int fricc_unpack_async(const int64_t* flat, int64_t m, const int64_t dims[4], int* slots, unsigned long long* meta,
                        cudaStream_t st) {
-  unsigned* err = nullptr;
-  int rc = fricc_alloc_t(&err, 1, st);
-  if (rc) return rc;
-  cudaMemsetAsync(err, 0, sizeof(unsigned), st);
-  k_unpack<<<grid_for(m, 256), 256, 0, st>>>(flat, m, dims[0], dims[1], dims[2], dims[3], slots, err);
-  k_meta_or<<<1, 1, 0, st>>>(err, meta);
-  fricc_note_launch(2);
-  cudaError_t ce = cudaGetLastError();
-  fricc_free(err, st);
-  return ce == cudaSuccess ? FRICC_OK : fricc_cuda_fail(ce, "unpack", __FILE__, __LINE__);
+  k_unpack<<<grid_for(m, 256), 256, 0, st>>>(flat, m, dims[0], dims[1], dims[2], dims[3], slots,
+                                             reinterpret_cast<unsigned*>(meta + 1));
+  fricc_note_launch();
+  return fricc_cuda_check(cudaGetLastError(), "unpack");
 }
 
 int fricc_unpack_device(const int64_t* flat, int64_t m, const int64_t dims[4], int* slots, cudaStream_t st) {
@@ -1490,17 +1576,13 @@ int fricc_seq_cumsum_device(const double* x, int64_t n, double* out, cudaStream_
   if (n == 0) return FRICC_OK;
   exact::ChainScratch sc;
   double* dzero = nullptr;
-  unsigned* err = nullptr;
   int rc = fricc_alloc_t(&dzero, 1, st);
-  if (!rc) rc = fricc_alloc_t(&err, 1, st);
   if (!rc) {
     cudaMemsetAsync(dzero, 0, sizeof(double), st);
-    cudaMemsetAsync(err, 0, sizeof(unsigned), st);
-    rc = exact::run_chain<GenAbs, ConsWrite, false, true>(GenAbs{x}, n, dzero, false, ConsWrite{out}, sc, err, st);
+    rc = exact::run_chain<GenAbs, ConsWrite, true>(GenAbs{x}, exact::Len{n}, dzero, false, ConsWrite{out}, sc, st);
   }
   exact::free_chain(sc, st);
   fricc_free(dzero, st);
-  fricc_free(err, st);
   return rc;
 }
 
@@ -1632,10 +1714,9 @@ int fricc_parallel_sample_device(const double* q, int64_t n, int64_t n_sample, i
     PTRY(fricc_cuda_check(cudaMemsetAsync(err, 0, sizeof(unsigned), st), "memset"));
     for (int j = 0; j <= T; ++j) {
       const int64_t lo = j < T ? j * step : 0, hi = j < T ? ((j + 1 == T) ? n : lo + step) : n;
-      PTRY((exact::run_chain<GenAbs, exact::ConsNull, false, false>(GenAbs{q + lo}, hi - lo, dzero, false,
-                                                                     exact::ConsNull{}, sc, err, st)));
-      PTRY(fricc_cuda_check(cudaMemcpyAsync(d_norm + j, sc.cstart + fricc_cdiv(hi - lo, exact::CH), sizeof(double),
-                                            cudaMemcpyDeviceToDevice, st), "norm"));
+      PTRY((exact::run_chain<GenAbs, exact::ConsNull, false>(GenAbs{q + lo}, exact::Len{hi - lo}, dzero, false,
+                                                              exact::ConsNull{}, sc, st, 1, exact::ChainStride{},
+                                                              false, d_norm + j)));
     }
     std::vector<double> hn((size_t)T + 1);
     PTRY(fricc_cuda_check(cudaMemcpyAsync(hn.data(), d_norm, sizeof(double) * (T + 1), cudaMemcpyDeviceToHost, st),

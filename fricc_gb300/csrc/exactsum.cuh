@@ -54,7 +54,6 @@ __device__ __forceinline__ G replica_of(const G& g, int r) {
 // scratch arrays always hold nch + 1 entries per replica.
 struct ChainStride {
   int64_t s_init = 0;  // the start values
-  int64_t err = 0;     // the error words
 };
 
 constexpr int64_t TWO52 = 1LL << 52;
@@ -99,6 +98,9 @@ __device__ __forceinline__ void decomp(double a, int b, int64_t& q, int& cls) {
   const int ef = (int)(bits >> 52);
   unsigned long long M = bits & ((1ull << 52) - 1);
   if (ef) M |= 1ull << 52;
+  // a running value that is infinite or NaN: finite addends leave it alone,
+  // others take the real operation
+  if (b >= 2047) { q = ef == 2047 ? SAT : 0; cls = 0; return; }
   const int efp = ef < 1 ? 1 : ef;
   const int shift = b - efp;
   if (shift < 0) { q = SAT; cls = 0; return; }  // a itself is beyond the binade
@@ -163,14 +165,23 @@ __device__ __forceinline__ Map block_excl_scan_map(Map v, Map* smem, Map* total)
   __syncthreads();
   if (lane_id() == 31) smem[warp_id()] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    Map run = map_id();
-    for (int w = 0; w < NW; ++w) {
-      Map t = smem[w];
-      smem[w] = run;
-      run = compose(run, t);
+  // the warp totals, scanned by warp 0 with shuffles: composing them one
+  // after another in one thread was most of a round (2 of 4 us at 32 warps)
+  if (warp_id() == 0) {
+    Map run = (int)lane_id() < NW ? smem[lane_id()] : map_id();
+#pragma unroll
+    for (int o = 1; o < NW; o <<= 1) {
+      Map w;
+      w.d0 = __shfl_up_sync(0xffffffffu, run.d0, o);
+      w.d1 = __shfl_up_sync(0xffffffffu, run.d1, o);
+      if ((int)lane_id() >= o) run = compose(w, run);
     }
-    smem[NW] = run;
+    Map ex;
+    ex.d0 = __shfl_up_sync(0xffffffffu, run.d0, 1);
+    ex.d1 = __shfl_up_sync(0xffffffffu, run.d1, 1);
+    if (lane_id() == 0) ex = map_id();
+    if ((int)lane_id() < NW) smem[lane_id()] = ex;
+    if (lane_id() == NW - 1) smem[NW] = run;
   }
   __syncthreads();
   Map r = compose(smem[warp_id()], wex);
@@ -189,13 +200,37 @@ struct ConsNull {
   __device__ __forceinline__ void operator()(int64_t, double, double, double) const {}
 };
 
+// A consumer with a method finish() is told once per thread, after the
+// thread's last element (so it can keep a per-thread result and publish it
+// with one atomic per warp).
+template <class C, class = void>
+struct has_finish : std::false_type {};
+template <class C>
+struct has_finish<C, std::void_t<decltype(std::declval<C&>().finish())>> : std::true_type {};
+
+// A chain's length: n elements, or (dev) the count at dev[rep * stride],
+// never above n; nothing at all where the word skip[rep * sstride] is set.
+struct Len {
+  int64_t n = 0;
+  const int64_t* dev = nullptr;
+  int64_t stride = 0;
+  const int* skip = nullptr;
+  int64_t sstride = 0;
+  __device__ __forceinline__ int64_t get(int rep) const {
+    if (skip && skip[rep * sstride]) return 0;
+    if (!dev) return n;
+    const int64_t d = dev[rep * stride];
+    return d < n ? d : n;
+  }
+};
+
 // Exact processing of one chunk by the whole block.  Thread t owns the
 // contiguous elements [t*ITEMS, t*ITEMS+ITEMS).  cons(i, before, after, a)
 // is called once for every element, in no particular order.  Returns the
 // exact running value after the chunk (the same in every thread).
 template <int NT, int ITEMS, class Gen, class Cons>
 __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, double s_start, bool sub,
-                                    const Cons& cons, ChunkSmem& sm) {
+                                    Cons& cons, ChunkSmem& sm) {
   double a[ITEMS];
   const int t = threadIdx.x;
 #pragma unroll
@@ -229,22 +264,28 @@ __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, doub
     int first_bad = INT_MAX;
     int64_t n_bad = 0;
     int k_bad = 0;
+    int istar = INT_MAX;
+    // the running value is monotone, so when the run's end is still inside
+    // the binade every step is: the search for the step that leaves it (a
+    // second pass over the items and a block minimum) runs only otherwise
+    if (!run_valid(apply(tot, n0), b, sub)) {
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const int i = t * ITEMS + k;
-      if (i >= p && i < n_in && first_bad == INT_MAX) {
-        int64_t nn;
-        if (step(n, a[k], b, sub, nn)) {
-          n = nn;
-        } else {
-          first_bad = i;
-          n_bad = n;
-          k_bad = k;
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = t * ITEMS + k;
+        if (i >= p && i < n_in && first_bad == INT_MAX) {
+          int64_t nn;
+          if (step(n, a[k], b, sub, nn)) {
+            n = nn;
+          } else {
+            first_bad = i;
+            n_bad = n;
+            k_bad = k;
+          }
         }
       }
+      istar = block_min<int>(first_bad, sm.imin);
+      n = apply(pre, n0);
     }
-    const int istar = block_min<int>(first_bad, sm.imin);
-    n = apply(pre, n0);
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       const int i = t * ITEMS + k;
@@ -276,61 +317,68 @@ __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, doub
 
 // ---------------------------------------------------------------- kernels
 
-// K_A: approximate sum of each chunk (fixed reduction tree).  With CHECK_P,
-// any addend above 1 sets FRICC_DEV_P_GT_ONE (make_probability_vector's check).
-template <class Gen, bool CHECK_P>
-__global__ void __launch_bounds__(256) k_chunk_sums(Gen gen0, int64_t len, double* csum, unsigned* err,
-                                                    ChainStride cs) {
+// K_A: approximate sum of each chunk (fixed reduction tree).
+template <class Gen>
+__global__ void __launch_bounds__(256) k_chunk_sums(Gen gen0, Len ln, double* csum) {
   const int rep = blockIdx.y;
-  const Gen gen = replica_of(gen0, rep);
-  csum += (int64_t)rep * (fricc_cdiv(len, CH) + 1);
-  err += rep * cs.err;
-  __shared__ double red[32];
+  const int64_t len = ln.get(rep);
   const int64_t base = (int64_t)blockIdx.x * CH;
+  if (base >= len) return;
+  const Gen gen = replica_of(gen0, rep);
+  csum += (int64_t)rep * (fricc_cdiv(ln.n, CH) + 1);
+  __shared__ double red[32];
   double acc = 0.0;
-  bool bad = false;
   for (int r = 0; r < CH / 256; ++r) {
     const int64_t i = base + r * 256 + threadIdx.x;
-    if (i < len) {
-      const double v = gen(i);
-      if (CHECK_P && v > 1.0) bad = true;
-      acc += v;
-    }
+    if (i < len) acc += gen(i);
   }
-  if (CHECK_P && bad) atomicOr(err, FRICC_DEV_P_GT_ONE);
   const double tot = block_sum_det(acc, red);
   if (threadIdx.x == 0) csum[blockIdx.x] = tot;
 }
 
 // K_B (one block of 1024): approximate prefix of the chunk sums and the
-// per-chunk binade prediction: cbin[c] = binade if clean, 0 if not.
-static __global__ void __launch_bounds__(1024) k_classify(const double* csum, int64_t nch, const double* s_init_dev,
+// per-chunk binade prediction: cbin[c] = binade if clean, 0 if not.  The
+// prefix is a shuffle scan: one thread adding 1024 partials (dependent FP64
+// additions, ~55 ns each on this part) took 58 us a call, three calls a
+// compression; now 4-5 us.
+static __global__ void __launch_bounds__(1024) k_classify(const double* csum, Len ln, const double* s_init_dev,
                                                    int sub, int* cbin, ChainStride cs) {
   const int rep = blockIdx.x;
-  csum += (int64_t)rep * (nch + 1);
-  cbin += (int64_t)rep * (nch + 1);
+  const int64_t nch = fricc_cdiv(ln.get(rep), CH), cap = fricc_cdiv(ln.n, CH) + 1;
+  csum += (int64_t)rep * cap;
+  cbin += (int64_t)rep * cap;
   const double s_init = s_init_dev[rep * cs.s_init];
-  __shared__ double part[1024];
-  __shared__ double red[32];
+  __shared__ double wtot[33];
   const int64_t per = fricc_cdiv(nch, 1024);
   const int64_t c0 = threadIdx.x * per;
   const int64_t c1 = c0 + per < nch ? c0 + per : nch;
   double loc = 0.0;
   for (int64_t c = c0; c < c1; ++c) loc += csum[c];
-  part[threadIdx.x] = loc;
-  const double total = block_sum_det(loc, red);
+  double incl = loc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double w = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((int)lane_id() >= o) incl += w;
+  }
+  double excl = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane_id() == 0) excl = 0.0;
+  if (lane_id() == 31) wtot[warp_id()] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double run = 0.0;
-    for (int w = 0; w < 1024; ++w) {
-      const double v = part[w];
-      part[w] = run;
-      run += v;
+  if (warp_id() == 0) {
+    double run = wtot[lane_id()];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double w = __shfl_up_sync(0xffffffffu, run, o);
+      if ((int)lane_id() >= o) run += w;
     }
+    double ex = __shfl_up_sync(0xffffffffu, run, 1);
+    if (lane_id() == 0) ex = 0.0;
+    wtot[lane_id()] = ex;
+    if (lane_id() == 31) wtot[32] = run;
   }
   __syncthreads();
-  const double scale = fabs(s_init) + total;
-  double pre = part[threadIdx.x];
+  const double scale = fabs(s_init) + wtot[32];
+  double pre = wtot[warp_id()] + excl;
   for (int64_t c = c0; c < c1; ++c) {
     const double P0 = sub ? s_init - pre : s_init + pre;
     pre += csum[c];
@@ -349,16 +397,19 @@ static __global__ void __launch_bounds__(1024) k_classify(const double* csum, in
 
 // K_C: composite map of each clean chunk under its predicted binade.
 template <class Gen>
-__global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, int64_t len, int sub, const int* cbin, Map* cmap) {
+__global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, const int* cbin, Map* cmap) {
   constexpr int NT = 256, ITEMS = CH / NT;
   const int rep = blockIdx.y;
+  const int64_t len = ln.get(rep);
+  const int64_t base = (int64_t)blockIdx.x * CH;
+  if (base >= len) return;
   const Gen gen = replica_of(gen0, rep);
-  cbin += (int64_t)rep * (fricc_cdiv(len, CH) + 1);
-  cmap += (int64_t)rep * (fricc_cdiv(len, CH) + 1);
+  const int64_t cap = fricc_cdiv(ln.n, CH) + 1;
+  cbin += (int64_t)rep * cap;
+  cmap += (int64_t)rep * cap;
   __shared__ Map smaps[33];
   const int b = cbin[blockIdx.x];
   if (b == 0) return;  // uniform per block
-  const int64_t base = (int64_t)blockIdx.x * CH;
   Map agg = map_id();
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
@@ -371,14 +422,17 @@ __global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, int64_t len, int s
 }
 
 // K_D (one block of 1024): the exact chain over chunks.  cstart[c] receives
-// the exact running value at the start of chunk c, cstart[nch] the total.
+// the exact running value at the start of chunk c, cstart[nch] the total,
+// which also goes to *end (if given).
 template <class Gen>
-__global__ void __launch_bounds__(1024) k_walk(Gen gen0, int64_t len, const double* s_init_dev, int sub,
-                                               const int* cbin, const Map* cmap, double* cstart, ChainStride cs) {
+__global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s_init_dev, int sub,
+                                               const int* cbin, const Map* cmap, double* cstart, double* end,
+                                               int64_t end_stride, ChainStride cs) {
   const int rep = blockIdx.x;
+  const int64_t len = ln.get(rep);
   const Gen gen = replica_of(gen0, rep);
   {
-    const int64_t st = (int64_t)rep * (fricc_cdiv(len, CH) + 1);
+    const int64_t st = (int64_t)rep * (fricc_cdiv(ln.n, CH) + 1);
     cbin += st;
     cmap += st;
     cstart += st;
@@ -391,56 +445,65 @@ __global__ void __launch_bounds__(1024) k_walk(Gen gen0, int64_t len, const doub
   const int64_t nch = fricc_cdiv(len, CH);
   double s = s_init;
   int64_t c = 0;
-  for (int64_t guard = 0; guard <= nch && c < nch; ++guard) {
+  for (int64_t guard = 0; guard <= 2 * nch && c < nch; ++guard) {
     if (sub && !(s > SUB_STOP)) break;
     const int b = binade_of(s);
     const int64_t n0 = n_of(s, b);
     const int64_t ct = c + threadIdx.x;
     const bool ok = ct < nch && cbin[ct] == b;
     const int L = block_min<int>(ok ? INT_MAX : (int)threadIdx.x, simin);
-    const Map mine = (ok && (int)threadIdx.x < L) ? cmap[ct] : map_id();
-    Map tot;
-    const Map pre = block_excl_scan_map<NT>(mine, smaps, &tot);
-    const Map incl = compose(pre, mine);
-    const int64_t n_end = apply(incl, n0);
-    const bool bad = (int)threadIdx.x < L && !run_valid(n_end, b, sub != 0);
-    int J = block_min<int>(bad ? (int)threadIdx.x : INT_MAX, simin);
-    if (J > L) J = L;
-    if (J > NT) J = NT;
-    if ((int)threadIdx.x < J) cstart[ct] = s_of(b, apply(pre, n0));
-    if (J > 0) {
-      // the thread J-1 holds the end value; every thread can recompute it
-      // from the block data only through smem, so pass it along.
-      if ((int)threadIdx.x == J - 1) csm.s = s_of(b, n_end);
-      __syncthreads();
-      s = csm.s;
-      __syncthreads();
-      c += J;
-      continue;
+    if (L > 0) {
+      const Map mine = (ok && (int)threadIdx.x < L) ? cmap[ct] : map_id();
+      Map tot;
+      const Map pre = block_excl_scan_map<NT>(mine, smaps, &tot);
+      const Map incl = compose(pre, mine);
+      const int64_t n_end = apply(incl, n0);
+      const bool bad = (int)threadIdx.x < L && !run_valid(n_end, b, sub != 0);
+      int J = block_min<int>(bad ? (int)threadIdx.x : INT_MAX, simin);
+      if (J > L) J = L;
+      if (J > NT) J = NT;
+      if ((int)threadIdx.x < J) cstart[ct] = s_of(b, apply(pre, n0));
+      if (J > 0) {
+        // the thread J-1 holds the end value; every thread can recompute it
+        // from the block data only through smem, so pass it along.
+        if ((int)threadIdx.x == J - 1) csm.s = s_of(b, n_end);
+        __syncthreads();
+        s = csm.s;
+        __syncthreads();
+        c += J;
+        continue;
+      }
     }
     if (threadIdx.x == 0) cstart[c] = s;
     const int64_t base = c * CH;
     const int n_in = (int)(len - base < CH ? len - base : CH);
-    s = block_exact_chunk<NT, CH / NT>(gen, base, n_in, s, sub != 0, ConsNull{}, csm);
+    ConsNull none;
+    s = block_exact_chunk<NT, CH / NT>(gen, base, n_in, s, sub != 0, none, csm);
     c += 1;
   }
   // chunks after an exhausted remaining-norm chain keep the final value
   for (int64_t cc = c + threadIdx.x; cc < nch; cc += NT) cstart[cc] = s;
-  if (threadIdx.x == 0) cstart[nch] = s;
+  if (threadIdx.x == 0) {
+    cstart[nch] = s;
+    if (end) end[rep * end_stride] = s;
+  }
 }
 
 // K_E: every element's exact before/after values, from the exact chunk starts.
 template <class Gen, class Cons>
-__global__ void __launch_bounds__(256) k_emit(Gen gen0, Cons cons0, int64_t len, int sub, const double* cstart) {
-  constexpr int NT = 256;
+__global__ void __launch_bounds__(512) k_emit(Gen gen0, Cons cons0, Len ln, int sub, const double* cstart) {
+  constexpr int NT = 512;
   const int rep = blockIdx.y;
-  const Gen gen = replica_of(gen0, rep);
-  const Cons cons = replica_of(cons0, rep);
-  cstart += (int64_t)rep * (fricc_cdiv(len, CH) + 1);
-  __shared__ ChunkSmem csm;
+  const int64_t len = ln.get(rep);
   const int64_t base = (int64_t)blockIdx.x * CH;
+  if (base >= len) return;
+  const Gen gen = replica_of(gen0, rep);
+  Cons cons = replica_of(cons0, rep);
+  cstart += (int64_t)rep * (fricc_cdiv(ln.n, CH) + 1);
+  __shared__ ChunkSmem csm;
   const int n_in = (int)(len - base < CH ? len - base : CH);
   block_exact_chunk<NT, CH / NT>(gen, base, n_in, cstart[blockIdx.x], sub != 0, cons, csm);
+  if constexpr (has_finish<Cons>::value) cons.finish();
 }
 
 struct ChainScratch {
@@ -452,39 +515,48 @@ struct ChainScratch {
 };
 
 // Runs the chain over gen(0..len-1) from s_init.  On return (stream order)
-// scratch.cstart[nch] holds the exact final value; with EMIT, cons has seen
-// every element.
-template <class Gen, class Cons, bool CHECK_P, bool EMIT>
-int run_chain(const Gen& gen, int64_t len, const double* s_init_dev, bool sub, const Cons& cons,
-              ChainScratch& sc, unsigned* dev_err, cudaStream_t st, int R = 1, ChainStride cs = ChainStride{}) {
-  const int64_t nch = fricc_cdiv(len, CH);
+// scratch.cstart[nch] holds the exact final value, which also goes to *end
+// (device, end_stride doubles per replica) when given; with EMIT, cons has
+// seen every element.  have_sums: sc.csum already holds the chunk sums (a
+// kernel that made the addends summed them in the same pass).
+inline int chain_scratch(ChainScratch& sc, int64_t entries, cudaStream_t st) {
+  if (sc.cap >= entries) return FRICC_OK;
+  fricc_free(sc.csum, st);
+  fricc_free(sc.cbin, st);
+  fricc_free(sc.cmap, st);
+  fricc_free(sc.cstart, st);
+  int rc = fricc_alloc_t(&sc.csum, entries, st);
+  if (!rc) rc = fricc_alloc_t(&sc.cbin, entries, st);
+  if (!rc) rc = fricc_alloc_t(&sc.cmap, entries, st);
+  if (!rc) rc = fricc_alloc_t(&sc.cstart, entries, st);
+  if (!rc) sc.cap = entries;
+  return rc;
+}
+
+template <class Gen, class Cons, bool EMIT>
+int run_chain(const Gen& gen, const Len& len, const double* s_init_dev, bool sub, const Cons& cons,
+              ChainScratch& sc, cudaStream_t st, int R = 1, ChainStride cs = ChainStride{}, bool have_sums = false,
+              double* end = nullptr, int64_t end_stride = 0) {
+  const int64_t nch = fricc_cdiv(len.n, CH);
   if (nch > INT_MAX / 2 || R < 1 || R > 65535) return FRICC_ERR_ARG;
   if (R > 1) {  // the batch's scratch: nch + 1 entries per replica, sized by the caller
     if (sc.cap < R * (nch + 1)) return FRICC_ERR_ARG;
     if (nch == 0) return FRICC_ERR_ARG;
-  } else if (sc.cap < nch + 1) {
-    fricc_free(sc.csum, st);
-    fricc_free(sc.cbin, st);
-    fricc_free(sc.cmap, st);
-    fricc_free(sc.cstart, st);
-    int rc = fricc_alloc_t(&sc.csum, nch + 1, st);
-    if (!rc) rc = fricc_alloc_t(&sc.cbin, nch + 1, st);
-    if (!rc) rc = fricc_alloc_t(&sc.cmap, nch + 1, st);
-    if (!rc) rc = fricc_alloc_t(&sc.cstart, nch + 1, st);
-    if (rc) return rc;
-    sc.cap = nch + 1;
+  } else if (int rc = chain_scratch(sc, nch + 1, st)) {
+    return rc;
   }
   if (nch == 0) {
     FRICC_CUDA(cudaMemcpyAsync(sc.cstart, s_init_dev, sizeof(double), cudaMemcpyDeviceToDevice, st));
+    if (end) FRICC_CUDA(cudaMemcpyAsync(end, s_init_dev, sizeof(double), cudaMemcpyDeviceToDevice, st));
     return FRICC_OK;
   }
   const dim3 gch((unsigned)nch, (unsigned)R);
-  k_chunk_sums<Gen, CHECK_P><<<gch, 256, 0, st>>>(gen, len, sc.csum, dev_err, cs);
-  k_classify<<<R, 1024, 0, st>>>(sc.csum, nch, s_init_dev, sub ? 1 : 0, sc.cbin, cs);
+  if (!have_sums) k_chunk_sums<Gen><<<gch, 256, 0, st>>>(gen, len, sc.csum);
+  k_classify<<<R, 1024, 0, st>>>(sc.csum, len, s_init_dev, sub ? 1 : 0, sc.cbin, cs);
   k_chunk_maps<Gen><<<gch, 256, 0, st>>>(gen, len, sub ? 1 : 0, sc.cbin, sc.cmap);
-  k_walk<Gen><<<R, 1024, 0, st>>>(gen, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.cmap, sc.cstart, cs);
-  if (EMIT) k_emit<Gen, Cons><<<gch, 256, 0, st>>>(gen, cons, len, sub ? 1 : 0, sc.cstart);
-  fricc_note_launch(EMIT ? 5 : 4);
+  k_walk<Gen><<<R, 1024, 0, st>>>(gen, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.cmap, sc.cstart, end, end_stride, cs);
+  if (EMIT) k_emit<Gen, Cons><<<gch, 512, 0, st>>>(gen, cons, len, sub ? 1 : 0, sc.cstart);
+  fricc_note_launch(3 + (have_sums ? 0 : 1) + (EMIT ? 1 : 0));
   FRICC_LAUNCH_CHECK();
   return FRICC_OK;
 }

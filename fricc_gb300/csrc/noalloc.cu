@@ -37,8 +37,7 @@ constexpr int64_t kMaxChunks = (kMaxN + exact::CH - 1) / exact::CH + 1;
 
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kOffZero = 0;                                   // double 0.0
-constexpr size_t kOffErr = 256;                                  // unsigned error word
-constexpr size_t kOffCsum = 512;
+constexpr size_t kOffCsum = 256;
 constexpr size_t kOffCbin = kOffCsum + align256(kMaxChunks * sizeof(double));
 constexpr size_t kOffCmap = kOffCbin + align256(kMaxChunks * sizeof(int));
 constexpr size_t kOffCstart = kOffCmap + align256(kMaxChunks * sizeof(exact::Map));
@@ -103,15 +102,13 @@ extern "C" int fricc_seq_cumsum_noalloc(const double* x, int64_t n, double* out,
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   double* dzero = reinterpret_cast<double*>(base + kOffZero);
-  unsigned* err = reinterpret_cast<unsigned*>(base + kOffErr);
   FRICC_CUDA(cudaMemsetAsync(dzero, 0, sizeof(double), st));
-  FRICC_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
   exact::ChainScratch sc;
   sc.csum = reinterpret_cast<double*>(base + kOffCsum);
   sc.cbin = reinterpret_cast<int*>(base + kOffCbin);
   sc.cmap = reinterpret_cast<exact::Map*>(base + kOffCmap);
   sc.cstart = reinterpret_cast<double*>(base + kOffCstart);
   sc.cap = kMaxChunks;  // run_chain allocates only when cap is too small; it never is here
-  return exact::run_chain<GenAbsNA, ConsWriteNA, false, true>(GenAbsNA{x}, n, dzero, false, ConsWriteNA{out}, sc,
-                                                              err, st);
+  return exact::run_chain<GenAbsNA, ConsWriteNA, true>(GenAbsNA{x}, exact::Len{n}, dzero, false, ConsWriteNA{out}, sc,
+                                                       st);
 }
