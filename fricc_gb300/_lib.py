@@ -50,6 +50,20 @@ SIGNATURES = [
                                                  ctypes.POINTER(ctypes.c_double), _vp]),
     ("fricc_spmm", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
                                   _dp, _i64, _dp, _vp]),
+    ("fricc_spmm_mod", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
+                                      _dp, _vp, _i64, _dp, _vp]),
+    ("fricc_spmm_takes_mod", ctypes.c_int, [_i64p, _i64, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _i64,
+                                            ctypes.c_int, ctypes.c_int]),
+    ("fricc_mod_select", ctypes.c_int, [ctypes.c_int]),
+    ("fricc_mod_mode", ctypes.c_int, []),
+    ("fricc_mod_bytes", _i64, [_i64, _i64]),
+    ("fricc_mod_prepare", ctypes.c_int, [_dp, _i64, _i64, _i64, _i64, _vp, _vp]),
+    ("fricc_gemm_f64_mod", ctypes.c_int, [_dp, _vp, _dp, _vp, _dp, _i64, _i64, _i64, _i64, _i64, _i64p, _i64p, _i64p,
+                                          ctypes.c_double, ctypes.c_double, _vp]),
+    ("fricc_gemm_takes_mod", ctypes.c_int, [_i64, _i64, _i64, _i64, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                            ctypes.c_int, ctypes.c_int]),
+    ("fricc_spb_spmm_mod", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                          ctypes.c_double, _dp, _vp, _i64, _dp, _i64, _vp]),
     ("fricc_spmm_f2", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                      ctypes.c_double, _dp, _i64, _dp, _vp]),
     ("fricc_split_f2", ctypes.c_int, [_dp, _i64, _i64, _dp, _vp]),

@@ -205,12 +205,20 @@ def request_stream(n: int, rate: float, seed: int = 0, nocc=(5, 30), ratio=(4.0,
 def footprint_bytes(o: int, v: int, precision: str = "df64") -> int:
     """HBM a resident solve needs: integral blocks and the layouts derived from
     them (vvvv and its float-pair form, ovvv in nine layouts or forms),
-    amplitudes and work arrays (~16 o^2v^2).  Split precision keeps (vv|vv)
+    amplitudes and work arrays (~16 o^2v^2), and the converted blocks and
+    scratch of the modular tensor-core products.  Split precision keeps (vv|vv)
     only as the FP32 block it rebuilds (v^4 / 2 doubles) and adds the
     BF16x3 operand splits (~4.5 o v^3 doubles)."""
     vvvv = 0.5 * v**4 if precision == "split" else 2 * v**4
     ovvv = 13.5 * o * v**3 if precision == "split" else 9 * o * v**3
-    return int(8 * (vvvv + ovvv + 16 * o * o * v * v + 4 * o**4 + 8 * o**3 * v))
+    mod = 0
+    if precision != "split":
+        # blocks kept converted for the modular products: 32 bytes an element of
+        # (vv|vv), the two halves of X/Y and four GEMM operands, up to
+        # DeviceERIs.MOD_BYTES, and the scratch of one product (two panels)
+        from .rccsd_dense import DeviceERIs
+        mod = min(32 * (v**4 + 6.5 * o * v**3), DeviceERIs.MOD_BYTES) + min(64 * v**4, 12 << 30)
+    return int(8 * (vvvv + ovvv + 16 * o * o * v * v + 4 * o**4 + 8 * o**3 * v) + mod)
 
 
 class _Live:

@@ -7,6 +7,7 @@
 
 #include "../../include/fricc_gb300.h"
 #include "common.cuh"
+#include "gemm_mod.cuh"
 #include "sparse.cuh"
 
 int fricc_compress_device(const double* x, int64_t n, int64_t m, int mode, double rn, cudaStream_t st, int64_t* flat,
@@ -25,7 +26,7 @@ int fricc_contract_device(const char* term, const double* W, const int64_t Wd[4]
                           double* out, const int64_t Od[4], const int64_t Os[4], cudaStream_t st);
 double fricc_contract_flops_impl(const char* term, const FriccSparse* T);
 int fricc_spmm_device(FriccSparse* T, int pa, int pb, int ka, int kb, double coef, const double* Wp, int64_t QS,
-                      double* Op, cudaStream_t st);
+                      double* Op, cudaStream_t st, const void* w_mod = nullptr);
 int fricc_spmm_f2_device(FriccSparse* T, int pa, int pb, int ka, int kb, double coef, const float4* Wp, int64_t QS,
                          double* Op, cudaStream_t st);
 int fricc_split_f2_device(const double* x, int64_t rows, int64_t qs, float4* out, cudaStream_t st);
@@ -38,7 +39,8 @@ int fricc_gemm_df_device(const double* A, const double* B, double* C, int64_t ba
                          cudaStream_t st, int64_t batch2, const int64_t* s2);
 int fricc_gemm_f64_device(const double* A, const double* B, double* C, int64_t batch, int64_t M, int64_t N,
                           int64_t K, const int64_t sA[3], const int64_t sB[3], const int64_t sC[3], double alpha,
-                          double beta, cudaStream_t st, int64_t batch2, const int64_t* s2);
+                          double beta, cudaStream_t st, int64_t batch2, const int64_t* s2,
+                          const void* a_mod = nullptr, const void* b_mod = nullptr);
 int fricc_combine_device(const int64_t dims[5], int n_in, const double* const* x, const int64_t* sx, int n_prod,
                          const double* const* p, const int64_t* sp, int n_out, double* const* out, const int64_t* so,
                          const double* coef, int accumulate, cudaStream_t st);
@@ -52,7 +54,9 @@ int fricc_unpack_batch_async(const int64_t* flat, int64_t m, int R, const int64_
                              unsigned long long* meta, cudaStream_t st);
 int fricc_batch_spmm_device(FriccSparseBatch* B, int which, int pa, int pb, int ka, int kb, double coef,
                             const void* Wp, int64_t w_stride, int64_t QS, double* Op, int64_t o_stride, bool f2,
-                            cudaStream_t st);
+                            cudaStream_t st, const void* w_mod = nullptr);
+bool fricc_spmm_takes_mod(const int64_t dims[4], int64_t m, int pa, int pb, int ka, int kb, int64_t QS, bool prepared,
+                          bool pairs);
 int fricc_batch_densify_device(FriccSparseBatch* B, int which, int pa, int pb, int ka, int kb, double coef, void* Ap,
                                int64_t kp, cudaStream_t st);
 int fricc_energy_update_batch_device(int R, const double* t1num, const double* t2num, const double* eia,
@@ -102,6 +106,7 @@ void fricc_note_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxe
 
 static thread_local int g_tune[FRICC_TUNE_KNOBS] = {-1, -1, -1, -1, -1, -1};
 int fricc_tune_get(int knob) { return knob >= 0 && knob < FRICC_TUNE_KNOBS ? g_tune[knob] : -1; }
+static thread_local int g_mod_mode = -1;
 bool fricc_prof_on() { return g_prof.load(std::memory_order_relaxed); }
 
 void fricc_prof_record(cudaStream_t st, bool start, double flops, int ch) {
@@ -604,6 +609,73 @@ int fricc_spmm(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, con
   return rc;
 }
 
+int fricc_spmm_mod(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, const double* Wp, const void* Wm,
+                   int64_t QS, double* Op, void* stream) {
+  cudaStream_t st = as_stream(stream);
+  int rc = fricc_spmm_device(T, pa, pb, ka, kb, coef, Wp, QS, Op, st, Wm);
+  if (!rc && T) T->owner_stream = st;
+  return rc;
+}
+
+int fricc_spmm_takes_mod(const int64_t dims[4], int64_t m, int pa, int pb, int ka, int kb, int64_t QS, int prepared,
+                         int pairs) {
+  if (bad_dims(dims) || m <= 0 || QS <= 0 || pa < 0 || pa > 3 || pb < 0 || pb > 3 || ka < 0 || ka > 3 || kb < 0 ||
+      kb > 3)
+    return 0;
+  return fricc_spmm_takes_mod(dims, m, pa, pb, ka, kb, QS, prepared != 0, pairs != 0) ? 1 : 0;
+}
+
+int fricc_gemm_takes_mod(int64_t batch, int64_t M, int64_t N, int64_t K, int a_batched, int b_batched, int a_prepared,
+                         int b_prepared, int pairs) {
+  if (batch < 1 || M < 1 || N < 1 || K < 1) return 0;
+  return fricc_mod_chosen(batch, M, N, K, a_batched != 0, b_batched != 0, a_prepared != 0, b_prepared != 0,
+                          fricc_mod_alt_us(batch, M, N, K, pairs != 0))
+             ? 1
+             : 0;
+}
+
+int fricc_mod_select(int mode) {
+  if (mode < -1 || mode > 1) {
+    fricc_set_error("mod_select: -1 (by the time model), 0 (never) or 1 (wherever possible)");
+    return FRICC_ERR_ARG;
+  }
+  g_mod_mode = mode;
+  return FRICC_OK;
+}
+
+int fricc_mod_mode(void) { return g_mod_mode; }
+
+int64_t fricc_mod_bytes(int64_t rows, int64_t k) { return rows > 0 && k > 0 ? fricc_mod_operand_bytes(rows, k) : 0; }
+
+int fricc_mod_prepare(const double* x, int64_t rows, int64_t k, int64_t row_stride, int64_t k_stride, void* out,
+                      void* stream) {
+  if (!x || !out || rows <= 0 || k <= 0 || reinterpret_cast<uintptr_t>(out) % 16) {
+    fricc_set_error("mod_prepare: bad arguments (the output 16-byte aligned)");
+    return FRICC_ERR_ARG;
+  }
+  ModView v;
+  v.x = x;
+  v.rows.outer(rows, row_stride);
+  v.sk = k_stride;
+  return fricc_mod_operand(v, rows, k, out, as_stream(stream));
+}
+
+int fricc_gemm_f64_mod(const double* A, const void* Am, const double* B, const void* Bm, double* C, int64_t batch,
+                       int64_t batch2, int64_t M, int64_t N, int64_t K, const int64_t sA[4], const int64_t sB[4],
+                       const int64_t sC[4], double alpha, double beta, void* stream) {
+  if (!sA || !sB || !sC) {
+    fricc_set_error("gemm_f64_mod: null strides");
+    return FRICC_ERR_ARG;
+  }
+  // a prepared operand is one matrix shared by every product of the batch
+  if ((Am && (sA[2] || sA[3])) || (Bm && (sB[2] || sB[3]))) {
+    fricc_set_error("gemm_f64_mod: a prepared operand is shared (batch strides 0)");
+    return FRICC_ERR_ARG;
+  }
+  const int64_t s2[3] = {sA[3], sB[3], sC[3]};
+  return fricc_gemm_f64_device(A, B, C, batch, M, N, K, sA, sB, sC, alpha, beta, as_stream(stream), batch2, s2, Am, Bm);
+}
+
 int fricc_spmm_f2(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, const float* Wp4, int64_t QS,
                   double* Op, void* stream) {
   cudaStream_t st = as_stream(stream);
@@ -810,6 +882,11 @@ int fricc_spb_spmm(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, 
                    int64_t w_stride, int64_t QS, double* Op, int64_t o_stride, void* stream) {
   return fricc_batch_spmm_device(B, which, pa, pb, ka, kb, coef, Wp, w_stride, QS, Op, o_stride, false,
                                  as_stream(stream));
+}
+
+int fricc_spb_spmm_mod(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, double coef, const double* Wp,
+                       const void* Wm, int64_t QS, double* Op, int64_t o_stride, void* stream) {
+  return fricc_batch_spmm_device(B, which, pa, pb, ka, kb, coef, Wp, 0, QS, Op, o_stride, false, as_stream(stream), Wm);
 }
 
 int fricc_spb_spmm_f2(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, double coef, const void* W2,

@@ -20,6 +20,7 @@
 
 #include <cuda_bf16.h>
 
+#include "gemm_mod.cuh"
 #include "radix.cuh"
 #include "sparse.cuh"
 
@@ -382,6 +383,28 @@ __global__ void k_densify_bf16x3(const int* __restrict__ slots, const double* __
   }
 }
 
+// The compressed T as a dense FP64 matrix [nP][R] in zeroed memory: the A
+// operand of the modular tensor-core product (gemm_mod.cu), which skips
+// elements whose bits are all zero, so a stored zero is written as -0.  (P, r)
+// is unique per nonzero but for the flat index 0, where every unmatched
+// sample of a systematic compression sits: those add up (equal values, or
+// an infinity among them, so their order does not matter).
+__global__ void k_densify_f64(const int* __restrict__ slots, const double* __restrict__ vals, int64_t m, int pa, int pb,
+                              int64_t dpb, int ka, int kb, int64_t dkb, int64_t R, double* __restrict__ out,
+                              int64_t rep) {
+  slots += 4 * (int64_t)blockIdx.y * m;
+  vals += (int64_t)blockIdx.y * m;
+  out += (int64_t)blockIdx.y * rep;
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < m; s += (int64_t)gridDim.x * blockDim.x) {
+    const int4 q = reinterpret_cast<const int4*>(slots)[s];
+    const int sl[4] = {q.x, q.y, q.z, q.w};
+    const double x = vals[s];
+    const int64_t at = ((int64_t)sl[pa] * dpb + sl[pb]) * R + (int64_t)sl[ka] * dkb + sl[kb];
+    if (at == 0) atomicAdd(&out[0], x);
+    else out[at] = x == 0.0 ? -0.0 : x;
+  }
+}
+
 // The same contraction against an FP32 W (the split-precision (vv|vv) block
 // rebuilt on the tensor cores): row r of W holds ldw floats, read as pairs
 // (W[r][2t], W[r][2t+1]); the compressed T values stay float pairs, so
@@ -596,6 +619,60 @@ bool is_contig_perm(const int64_t dims[4], const int64_t strides[4], const int p
 
 double fricc_contract_flops_impl(const char* term, const FriccSparse* T);
 
+// Whether a sparse term of this shape runs as a modular tensor-core product
+// of the zero-filled T (gemm_mod.cu): where its estimate, the densify
+// included, is below 0.8 of the sparse kernel's (FP64: 1.2 TFLOP/s measured;
+// float pairs: 4.5, both on whole q tiles; plus ~60 us of bucketing).  The zeros cost 1/density more products, so
+// the line moves with m; at 5-10% kept it lies near o = 10 (o20v100 at 5%: 2323
+// 3.3 ms on k_spmm).  Not for slots that leave (P, r) ambiguous.
+bool fricc_spmm_takes_mod(const int64_t dims[4], int64_t m, int pa, int pb, int ka, int kb, int64_t QS, bool prepared,
+                          bool pairs) {
+  const int force = fricc_mod_mode();
+  if (force == 0 || ((1 << pa) | (1 << pb) | (1 << ka) | (1 << kb)) != 15) return false;
+  const int64_t nP = dims[pa] * dims[pb], R = dims[ka] * dims[kb];
+  if (R > (1ll << 22)) return false;
+  if (force == 1) return true;
+  const double qpad = (double)(fricc_cdiv(QS, pairs ? 512 : 256) * (pairs ? 512 : 256));  // whole q tiles
+  const double sparse_us = 60.0 + 2.0 * (double)m * qpad / (pairs ? 4.5e6 : 1.2e6);
+  const double mod_us = fricc_mod_time_us(nP, QS, R, 1, true, true, true, !prepared) +
+                        ((double)nP * (double)R * 16.0 + (double)m * 56.0) / 4.5e6 + 6.0;
+  return mod_us < 0.8 * sparse_us;
+}
+
+namespace {
+
+// out[P][q] += coef sum_r T[P][r] W[r][q] as a modular product; W given as the view
+// of its rows q (and prepared or not), reps > 1: one T (and W unless shared) per replica
+int spmm_mod(const int* slots, const double* vals, int64_t m, const int64_t dims[4], int pa, int pb, int ka, int kb,
+             const ModView& W, ModOut out, int64_t QS, int64_t reps, bool w_shared, cudaStream_t st) {
+  const int64_t nP = dims[pa] * dims[pb], R = dims[ka] * dims[kb];
+  double* Td = nullptr;
+  int rc = fricc_alloc_t(&Td, (size_t)reps * nP * R, st);
+  if (rc) return rc;
+  cudaError_t e = cudaMemsetAsync(Td, 0, sizeof(double) * (size_t)(reps * nP * R), st);
+  if (e == cudaSuccess) {
+    k_densify_f64<<<dim3(grid_for(m, 256), (unsigned)reps), 256, 0, st>>>(slots, vals, m, pa, pb, dims[pb], ka, kb,
+                                                                          dims[kb], R, Td, nP * R);
+    fricc_note_launch();
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) rc = fricc_cuda_fail(e, "densify", __FILE__, __LINE__);
+  if (!rc) {
+    ModView A;
+    A.x = Td;
+    A.rows.outer(reps * nP, R);
+    A.sk = 1;
+    if (w_shared)  // the replicas are more rows of one product
+      rc = fricc_mod_gemm(A, W, out, reps * nP, QS, R, 1, true, true, true, st);
+    else
+      rc = fricc_mod_gemm(A, W, out, nP, QS, R, reps, false, false, true, st);
+  }
+  fricc_free(Td, st);
+  return rc;
+}
+
+}  // namespace
+
 // A re-compression keeps every bucketing's arrays (m and dims do not change)
 // and only marks it stale; it is rebuilt in place on first use, so a steady
 // iteration allocates nothing that outlives it (which also keeps it
@@ -661,14 +738,14 @@ int fricc_sparse_bucketing(FriccSparse* T, int pa, int pb, cudaStream_t st, Buck
   return FRICC_OK;
 }
 
-int fricc_contract_device(const char* term, const double* W, const int64_t Wd[4], const int64_t Ws[4], FriccSparse* T,
+int fricc_contract_device(const char* term, const double* Win, const int64_t Wd[4], const int64_t Ws[4], FriccSparse* T,
                           double* out, const int64_t Od[4], const int64_t Os[4], cudaStream_t st) {
   const TermSpec* ts = find_term(term);
   if (!ts) {
     fricc_set_error("CASE NOT IMPLEMENTED: contraction term '%s'", term ? term : "(null)");
     return FRICC_ERR_TERM;
   }
-  if (!W || !out || !T) {
+  if (!Win || !out || !T) {
     fricc_set_error("contract: null argument");
     return FRICC_ERR_ARG;
   }
@@ -695,9 +772,31 @@ int fricc_contract_device(const char* term, const double* W, const int64_t Wd[4]
   const int64_t nW = we[0] * we[1] * QS;
   const int64_t nO = oe[0] * oe[1] * QS;
   if (T->m == 0 || nO == 0) return FRICC_OK;
+  int rc = FRICC_OK;
+  if (fricc_spmm_takes_mod(td, T->m, ts->pa, ts->pb, ts->ka, ts->kb, QS, false, false)) {
+    // any strides of W and out are read and written in place
+    ModView W;
+    W.x = Win;
+    W.rows.outer(we[3], wsp[3]);
+    W.rows.outer(we[2], wsp[2]);
+    W.sk = wsp[1];
+    if (we[0] > 1 && wsp[0] != we[1] * wsp[1]) {
+      W.kn = we[1];
+      W.sko = wsp[0];
+    }
+    ModOut o;
+    o.C = out;
+    o.alpha = ts->coef;
+    o.beta = 1.0;
+    o.row.outer(oe[1], osp[1]);
+    o.row.outer(oe[0], osp[0]);
+    o.col.outer(oe[3], osp[3]);
+    o.col.outer(oe[2], osp[2]);
+    return spmm_mod(T->slots, T->vals, T->m, td, ts->pa, ts->pb, ts->ka, ts->kb, W, o, QS, 1, true, st);
+  }
 
   Bucketing* bk = nullptr;
-  int rc = fricc_sparse_bucketing(T, ts->pa, ts->pb, st, &bk);
+  rc = fricc_sparse_bucketing(T, ts->pa, ts->pb, st, &bk);
   if (rc) return rc;
 
   const bool w_direct = is_contig_perm(Wd, Ws, ts->permW);
@@ -714,11 +813,11 @@ int fricc_contract_device(const char* term, const double* W, const int64_t Wd[4]
     k_entries<<<grid_for(T->m, 256), 256, 0, st>>>(T->slots, T->vals, bk->order, T->m, ts->ka, ts->kb, td[ts->kb],
                                                    ts->coef, erow, eval);
     if (!w_direct)
-      k_gather4<<<grid_for(nW, 256), 256, 0, st>>>(W, wsp[0], wsp[1], wsp[2], wsp[3], we[0], we[1], we[2], we[3], Wp);
+      k_gather4<<<grid_for(nW, 256), 256, 0, st>>>(Win, wsp[0], wsp[1], wsp[2], wsp[3], we[0], we[1], we[2], we[3], Wp);
     if (!o_direct)
       k_gather4<<<grid_for(nO, 256), 256, 0, st>>>(out, osp[0], osp[1], osp[2], osp[3], oe[0], oe[1], oe[2], oe[3],
                                                    Op);
-    const double* Wuse = w_direct ? W : Wp;
+    const double* Wuse = w_direct ? Win : Wp;
     double* Ouse = o_direct ? out : Op;
     const int64_t ntq = fricc_cdiv(QS, SP_NT * SP_QPT);
     if (ntq > 65535 || bk->nbuckets > 0x7fffffffLL) {
@@ -748,14 +847,29 @@ int fricc_contract_device(const char* term, const double* W, const int64_t Wd[4]
 // Generic form: out'[P, q] += coef * sum_{e in bucket P} W'[key_e, q] * value_e
 // with P = slot[pa]*dims[pb] + slot[pb], key = slot[ka]*dims[kb] + slot[kb],
 // W' contiguous [dims[ka]*dims[kb]][QS] and out' contiguous [dims[pa]*dims[pb]][QS].
+// w_mod: W' prepared by fricc_mod_prepare (rows q, K the keys), or null.
 int fricc_spmm_device(FriccSparse* T, int pa, int pb, int ka, int kb, double coef, const double* Wp, int64_t QS,
-                      double* Op, cudaStream_t st) {
+                      double* Op, cudaStream_t st, const void* w_mod) {
   if (!T || !Wp || !Op || QS <= 0 || pa < 0 || pa > 3 || pb < 0 || pb > 3 || ka < 0 || ka > 3 || kb < 0 || kb > 3 ||
       pa == pb || ka == kb) {
     fricc_set_error("spmm: bad arguments");
     return FRICC_ERR_ARG;
   }
   if (T->m == 0) return FRICC_OK;
+  if (fricc_spmm_takes_mod(T->dims, T->m, pa, pb, ka, kb, QS, w_mod != nullptr, false)) {
+    ModView W;
+    W.x = Wp;
+    W.rows.outer(QS, 1);
+    W.sk = QS;
+    W.prepared = w_mod;
+    ModOut o;
+    o.C = Op;
+    o.alpha = coef;
+    o.beta = 1.0;
+    o.row.outer(T->dims[pa] * T->dims[pb], QS);
+    o.col.outer(QS, 1);
+    return spmm_mod(T->slots, T->vals, T->m, T->dims, pa, pb, ka, kb, W, o, QS, 1, true, st);
+  }
   Bucketing* bk = nullptr;
   int rc = fricc_sparse_bucketing(T, pa, pb, st, &bk);
   if (rc) return rc;
@@ -1066,7 +1180,7 @@ int fricc_batch_bucketing(FriccSparseBatch* B, int which, int pa, int pb, cudaSt
 // f2: W' in the q-pair float layout of fricc_spmm_f2 (w_stride in float4s).
 int fricc_batch_spmm_device(FriccSparseBatch* B, int which, int pa, int pb, int ka, int kb, double coef,
                             const void* Wp, int64_t w_stride, int64_t QS, double* Op, int64_t o_stride, bool f2,
-                            cudaStream_t st) {
+                            cudaStream_t st, const void* w_mod) {
   if (!B || !Wp || !Op || which < 0 || which > 1 || QS <= 0 || pa < 0 || pa > 3 || pb < 0 || pb > 3 || ka < 0 ||
       ka > 3 || kb < 0 || kb > 3 || pa == pb || ka == kb || w_stride < 0 || o_stride < 0) {
     fricc_set_error("batch spmm: bad arguments");
@@ -1082,6 +1196,28 @@ int fricc_batch_spmm_device(FriccSparseBatch* B, int which, int pa, int pb, int 
   }
   const int R = B->R;
   const int64_t m = B->m;
+  // (one replica's estimate: a replica takes its lone call's route)
+  if (!f2 && fricc_spmm_takes_mod(B->dims, m, pa, pb, ka, kb, QS, w_mod != nullptr, false)) {
+    ModView W;
+    W.x = static_cast<const double*>(Wp);
+    W.rows.outer(QS, 1);
+    W.sk = QS;
+    W.prepared = w_mod;
+    ModOut o;
+    o.C = Op;
+    o.alpha = coef;
+    o.beta = 1.0;
+    o.row.outer(B->dims[pa] * B->dims[pb], QS);
+    o.col.outer(QS, 1);
+    if (w_stride == 0 || R == 1) {
+      o.row.outer(R, o_stride);
+    } else {
+      W.rows.outer(R, w_stride);
+      o.rep.outer(R, o_stride);
+    }
+    return spmm_mod(B->slots[which], B->vals[which], m, B->dims, pa, pb, ka, kb, W, o, QS, R, w_stride == 0 || R == 1,
+                    st);
+  }
   BatchBucketing* bk = nullptr;
   int rc = fricc_batch_bucketing(B, which, pa, pb, st, &bk);
   if (rc) return rc;

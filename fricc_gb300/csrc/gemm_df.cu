@@ -13,7 +13,7 @@
 // output ~1e-14.  A long K is split over blockIdx.x (beside the N tiles;
 // blockIdx.z is the batch); the partial tiles are
 // summed afterwards in a fixed order, so results are deterministic.
-#include "common.cuh"
+#include "gemm_mod.cuh"
 
 namespace {
 
@@ -319,6 +319,11 @@ int fricc_gemm_df_device(const double* A, const double* B, double* C, int64_t ba
   if (fricc_cdiv(M, BM) > 65535 || batch > 65535 || g.ntn * splits > 0x7fffffff) {
     fricc_set_error("gemm_df: grid too large (M=%lld, batch=%lld)", (long long)M, (long long)batch);
     return FRICC_ERR_ARG;
+  }
+  // large products run on the tensor cores, at FP64 accuracy (gemm_mod.cu)
+  if (K > 0) {
+    const int rc = fricc_mod_try(A, B, C, g.nb1, batch2, M, N, K, sA, sB, sC, s2, alpha, beta, true, nullptr, nullptr, st);
+    if (rc >= 0) return rc;
   }
   double* part = nullptr;
   if (splits > 1) {

@@ -12,7 +12,7 @@
 // k order (deterministic); a long K with few output tiles is split over
 // blockIdx.x (beside the N tiles; blockIdx.z is the batch) and the partial
 // tiles summed afterwards in slice order.
-#include "common.cuh"
+#include "gemm_mod.cuh"
 
 namespace {
 
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_gemv_cols(GemmArgs g) {
 
 int fricc_gemm_f64_device(const double* A, const double* B, double* C, int64_t batch, int64_t M, int64_t N, int64_t K,
                           const int64_t sA[3], const int64_t sB[3], const int64_t sC[3], double alpha, double beta,
-                          cudaStream_t st, int64_t batch2, const int64_t* s2) {
+                          cudaStream_t st, int64_t batch2, const int64_t* s2, const void* a_mod, const void* b_mod) {
   if (((!A || !B) && K > 0) || !C || batch <= 0 || M <= 0 || N <= 0 || K < 0 || !sA || !sB || !sC) {
     fricc_set_error("gemm_f64: bad arguments");
     return FRICC_ERR_ARG;
@@ -336,6 +336,11 @@ int fricc_gemm_f64_device(const double* A, const double* B, double* C, int64_t b
   if (fricc_cdiv(M, BM) > 65535 || batch > 65535 || g.ntn * splits > 0x7fffffff) {
     fricc_set_error("gemm_f64: grid too large (M=%lld, batch=%lld)", (long long)M, (long long)batch);
     return FRICC_ERR_ARG;
+  }
+  // large products run on the tensor cores, at FP64 accuracy
+  if (K > 0) {
+    const int rc = fricc_mod_try(A, B, C, g.nb1, batch2, M, N, K, sA, sB, sC, s2, alpha, beta, false, a_mod, b_mod, st);
+    if (rc >= 0) return rc;
   }
   double* part = nullptr;
   if (splits > 1) {

@@ -188,7 +188,7 @@ class FRICCSDGPU:
         self._tc_status = torch.zeros(1, dtype=torch.int32, device=eris.device)
         self.lib = L.load()
         if precision == "df64":
-            eris.prepare_splits()
+            eris.prepare_splits(eris.pair_blocks(int(s["m_keep"]), self._tuner is not None))
         elif precision == "split":
             o_, v_ = eris.nocc, eris.mo_energy.numel() - eris.nocc
             eris.prepare_f32({"ovvv_XY": 2 * o_ * v_, "ovov": o_ * v_, "ovov_0313_0113": o_ * v_,
@@ -241,7 +241,19 @@ class FRICCSDGPU:
             # (half the bytes of the float-pair layout)
             W32 = self.eris.f32(const, QS) if const else D.to_f32_rows(Wp, QS)
             L.check(self._spmm32(T, pa, pb, ka, kb, float(coef), _ptr(W32), int(QS), W32.shape[1], _ptr(Op), stream))
+            return
+        term = (pa, pb, ka, kb, int(QS))
+        m = int(self.settings["m_keep"])
+        Wm = None
+        if const and self._tuner is None and D.takes_mod(self._dims, m, term, True, self._df):
+            Wm = self.eris.mod_w(const, QS)
+        if Wm is not None or (self._tuner is None and D.takes_mod(self._dims, m, term, False, self._df)):
+            # FP64-accurate on the tensor cores (in either precision)
+            L.check(self.lib.fricc_spmm_mod(T, pa, pb, ka, kb, float(coef), _ptr(Wp),
+                                            _ptr(Wm) if Wm is not None else None, int(QS), _ptr(Op), stream))
         elif self._df:
+            if const:
+                self.eris.prepare_splits((const,))
             W2 = self.eris.split(const) if const else D.split_f2(Wp, QS)
             assert W2.numel() == (Wp.numel() // QS) * ((QS + 1) // 2) * 4, "float-pair W' split with another QS"
 
@@ -402,6 +414,9 @@ class FRICCSDGPU:
 
             def mm(A_, B_, C_, alpha=1.0, beta=0.0, const=None, const_b=None):
                 if tuner is None:
+                    Am, Bm = D.mod_constants(E, A_, B_, C_, const, const_b, self._df)
+                    if Am is not None or Bm is not None:
+                        return D.gemm_f64(A_, B_, C_, alpha, beta, Am, Bm)
                     return mm0(A_, B_, C_, alpha, beta)
                 from .autotune import GEMM_CANDIDATES
                 key = ("gemm", tuple(A_.shape), A_.stride(), tuple(B_.shape), B_.stride(), tuple(C_.shape),

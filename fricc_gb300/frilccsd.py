@@ -66,7 +66,7 @@ class FRILCCSDGPU(FRICCSDGPU):
         self.lib = L.load()
         eris.prepare_linear()
         if precision == "df64":
-            eris.prepare_splits(("vvvvT",) + D.DeviceERIs.LIN_BLOCKS)
+            eris.prepare_splits(eris.pair_blocks(int(s["m_keep"]), False, ("vvvvT",) + D.DeviceERIs.LIN_BLOCKS))
         self.independent = bool(s["Independent Compressions"])
         self._handles = [_Handle() for _ in range(len(SPARSE_ORDER) if self.independent else 1)]
         self._res = torch.zeros(4, dtype=torch.float64, device=eris.device)
@@ -96,6 +96,7 @@ class FRILCCSDGPU(FRICCSDGPU):
         comp = s["compressed_contractions"]
         o, v = t1.shape
         ov = o * v
+        self._dims = tuple(t2.shape)
         st = L.cur_stream()
         t2 = t2.contiguous()
         e_o = E.mo_energy[:o]

@@ -17,8 +17,8 @@ only as vvvvT[c,d,a,b] = (ac|bd), the layout the O^2V^4 term streams.
 """
 from __future__ import annotations
 
+import functools
 import math
-
 import threading
 
 import numpy as np
@@ -90,6 +90,7 @@ class DeviceERIs:
         self.ovvv_kacd = ovvv.permute(0, 2, 3, 1).contiguous()           # Wvovo t1 term
         self._dense_wvvvv = None
         self._splits = {}
+        self._mod_bytes = 0
         self._lock = threading.Lock()
 
     SPLIT_BLOCKS = ("vvvvT", "ovvv_XY", "ovov", "ovov_0312", "ovov_0313_0113", "ovov_cdkl")
@@ -104,6 +105,23 @@ class DeviceERIs:
                 if name not in self._splits and getattr(self, name) is not None:
                     self._splits[name] = split_f2(getattr(self, name))
             torch.cuda.current_stream().synchronize()
+
+    def pair_blocks(self, m, every, names=None):
+        """The constant W' blocks a df64 solver keeping m entries contracts in
+        float pairs: all of them with ``every`` (an autotuner compares the
+        float-pair launches), else those whose term does not run as a modular
+        tensor-core product."""
+        names = self.SPLIT_BLOCKS if names is None else names
+        if every:
+            return names
+        o, v = self.nocc, self.mo_energy.numel() - self.nocc
+        ov = o * v
+        use = {"vvvvT": [(0, 1, 2, 3, v * v)], "ovvv_XY": [(0, 1, 2, 3, 2 * ov)], "ovov": [(3, 0, 1, 2, ov)],
+               "ovov_0312": [(3, 0, 1, 2, ov)], "ovov_0313_0113": [(2, 0, 1, 3, ov)],
+               "ovov_cdkl": [(0, 1, 2, 3, o * o)], "oooo_klij": [(2, 3, 0, 1, o * o)],
+               "lin_WA": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)], "lin_WB": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)],
+               "lin_W2AB": [(1, 3, 0, 2, ov)]}
+        return tuple(n for n in names if not all(takes_mod((o, o, v, v), m, t, True, True) for t in use[n]))
 
     LIN_BLOCKS = ("oooo_klij", "lin_WA", "lin_WB", "lin_W2AB")
 
@@ -164,6 +182,40 @@ class DeviceERIs:
         if got is None or got[0] != role:
             raise RuntimeError(f"split operand {role} of {name} missing: call prepare_tc() first")
         return got[1]
+
+    # device bytes of integral blocks kept converted for the modular products
+    # (all of them at o30v150 take 39 GB); a block beyond that is converted by
+    # each call that uses it
+    MOD_BYTES = 40 << 30
+
+    def _mod(self, key, name, rows, k, row_stride, k_stride):
+        got = self._splits.get(key)
+        if got is None:
+            with self._lock:
+                got = self._splits.get(key)
+                if got is None:
+                    need = L.load().fricc_mod_bytes(rows, k)
+                    if self._mod_bytes + need > self.MOD_BYTES:
+                        return None
+                    got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
+                    torch.cuda.current_stream().synchronize()
+                    self._mod_bytes += need
+                    self._splits[key] = got
+        return got
+
+    def mod_w(self, name, qs):
+        """A constant W' block viewed as [keys][qs], its rows q prepared for
+        the modular products, built on first use under a lock and waited for
+        (None past MOD_BYTES)."""
+        return self._mod(("modW", name, qs), name, qs, getattr(self, name).numel() // qs, 1, qs)
+
+    def mod_a(self, name, m, k):
+        """A constant block as the A operand [m, k] of a dense product."""
+        return self._mod(("modA", name, m, k), name, m, k, k, 1)
+
+    def mod_b(self, name, k, n):
+        """A constant block as the B operand [k, n] of a dense product."""
+        return self._mod(("modB", name, k, n), name, n, k, 1, n)
 
     def f32(self, name, qs):
         """FP32 rows (qs columns, padded to even) of a constant block, built
@@ -361,9 +413,72 @@ def gemm_df(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1.
     return _gemm_call("fricc_gemm_df", A, B, C, alpha, beta)
 
 
-def gemm_f64(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1.0, beta: float = 0.0):
-    """The same contract in FP64 on the library's DFMA GEMM kernel."""
-    return _gemm_call("fricc_gemm_f64", A, B, C, alpha, beta)
+def gemm_f64(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1.0, beta: float = 0.0,
+             a_mod=None, b_mod=None):
+    """The same contract in FP64: the library's DFMA kernel, or, for large
+    products, its modular tensor-core product at the same accuracy.
+    ``a_mod`` / ``b_mod``: a 2-D operand prepared once (``mod_operand``)."""
+    if a_mod is None and b_mod is None:
+        return _gemm_call("fricc_gemm_f64", A, B, C, alpha, beta)
+    import ctypes
+
+    sA, bA, b2A = _bstrides(A)
+    sB, bB, b2B = _bstrides(B)
+    sC, batch, batch2 = _bstrides(C)
+    M, N, K = C.shape[-2], C.shape[-1], A.shape[-1]
+    assert A.shape[-2] == M and B.shape[-2] == K and B.shape[-1] == N
+    assert bA in (1, batch) and bB in (1, batch) and b2A in (1, batch2) and b2B in (1, batch2)
+    sA = (sA[0], sA[1], sA[2] if bA == batch and batch > 1 else 0, sA[3] if b2A == batch2 and batch2 > 1 else 0)
+    sB = (sB[0], sB[1], sB[2] if bB == batch and batch > 1 else 0, sB[3] if b2B == batch2 and batch2 > 1 else 0)
+    vp = ctypes.c_void_p
+    L.check(L.load().fricc_gemm_f64_mod(
+        vp(A.data_ptr()), vp(a_mod.data_ptr()) if a_mod is not None else None, vp(B.data_ptr()),
+        vp(b_mod.data_ptr()) if b_mod is not None else None, vp(C.data_ptr()), batch, batch2, M, N, K, L.i64arr(sA),
+        L.i64arr(sB), L.i64arr(sC), float(alpha), float(beta), L.cur_stream()))
+    return C
+
+
+def takes_mod(dims, m, term, prepared, pairs) -> bool:
+    """Whether the sparse term (pa, pb, ka, kb, QS) of a T with m entries runs
+    as a modular tensor-core product (fricc_spmm_takes_mod)."""
+    return _spmm_route(tuple(dims), int(m), term, bool(prepared), bool(pairs), L.load().fricc_mod_mode())
+
+
+# (the routes are pure functions of the sizes and the thread's fricc_mod_select
+# mode; an iteration asks ~30 times, ~3 us each through ctypes)
+@functools.lru_cache(maxsize=4096)
+def _spmm_route(dims, m, term, prepared, pairs, mode):
+    pa, pb, ka, kb, qs = term
+    return bool(L.load().fricc_spmm_takes_mod(L.i64arr(dims), m, pa, pb, ka, kb, qs, int(prepared), int(pairs)))
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_route(M, N, K, a_prepared, b_prepared, pairs, mode):
+    return bool(L.load().fricc_gemm_takes_mod(1, M, N, K, 0, 0, int(a_prepared), int(b_prepared), int(pairs)))
+
+
+def mod_constants(E, A, B, C, const, const_b, pairs):
+    """The prepared forms (A, B) of the constant integral operands of a dense
+    product A @ B (named const / const_b), where it runs as a modular one
+    with them; (None, None) elsewhere."""
+    if const is None and const_b is None:
+        return None, None
+    M, N, K = C.shape[-2], C.shape[-1], A.shape[-1]
+    if not _gemm_route(M, N, K, const is not None, const_b is not None, bool(pairs), L.load().fricc_mod_mode()):
+        return None, None
+    return (E.mod_a(const, M, K) if const else None), (E.mod_b(const_b, K, N) if const_b else None)
+
+
+def mod_operand(x: torch.Tensor, rows: int, k: int, row_stride: int, k_stride: int) -> torch.Tensor:
+    """rows x k elements of x converted once for the modular tensor-core
+    products (fricc_mod_prepare), as a byte buffer."""
+    import ctypes
+
+    lib = L.load()
+    buf = torch.empty(lib.fricc_mod_bytes(rows, k), dtype=torch.uint8, device=x.device)
+    L.check(lib.fricc_mod_prepare(ctypes.c_void_p(x.data_ptr()), rows, k, row_stride, k_stride,
+                                  ctypes.c_void_p(buf.data_ptr()), L.cur_stream()))
+    return buf
 
 
 def _as3(x: torch.Tensor, shape3):

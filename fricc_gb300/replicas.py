@@ -86,6 +86,13 @@ def einsum_rep(spec: str, A: torch.Tensor, B: torch.Tensor, gemm, za: bool, zb: 
     return C.view([R] + [size[c] for c in order]).permute([0] + [1 + order.index(c) for c in outs])
 
 
+def _lift(x: torch.Tensor) -> torch.Tensor:
+    """An operand of a product over replicas as [replica, 1, rows, cols]
+    ([1, 1, ...] when shared), so that the replica is the GEMM's second
+    batch level and each product takes the route of its lone call."""
+    return x if x.dim() == 4 else (x.unsqueeze(1) if x.dim() == 3 else x.unsqueeze(0).unsqueeze(0))
+
+
 class FusedReplicaBatch:
     """R replicas of one system, one launch per kernel for all of them.
 
@@ -117,7 +124,7 @@ class FusedReplicaBatch:
         self.precision = precision
         self.df = precision == "df64"
         if self.df:
-            eris.prepare_splits()
+            eris.prepare_splits(eris.pair_blocks(int(s["m_keep"]), False))
         if self.split:
             from .cholesky import dense_spmm_ok
             o_, v_ = eris.nocc, eris.mo_energy.numel() - eris.nocc
@@ -182,7 +189,19 @@ class FusedReplicaBatch:
             return gemm_tc_rep(A, B, C, alpha, beta, self.R, status=self._tc_status,
                                a_split=E.tc(const, "A") if const else None,
                                b_split=E.tc(const_b, "B") if const_b else None)
-        return (D.gemm_df if self.df else D.gemm_f64)(A, B, C, alpha, beta)
+        A, B, C4 = _lift(A), _lift(B), _lift(C)
+        Am, Bm = D.mod_constants(self.E, A, B, C4, const, const_b, self.df)
+        if Am is not None or Bm is not None:
+            D.gemm_f64(A, B, C4, alpha, beta, Am, Bm)
+        else:
+            (D.gemm_df if self.df else D.gemm_f64)(A, B, C4, alpha, beta)
+        return C
+
+    @staticmethod
+    def _mmf(A, B, C, alpha=1.0, beta=0.0):
+        """The FP64 GEMM for every replica."""
+        D.gemm_f64(_lift(A), _lift(B), _lift(C), alpha, beta)
+        return C
 
     def _spmm(self, which, pa, pb, ka, kb, coef, W, QS, Op, st, const=None):
         """A sparse term of every replica: W shared (``const`` names a
@@ -198,8 +217,17 @@ class FusedReplicaBatch:
             done = dense_spmm_rep(self.spb, which, R, tuple(self.t2.shape[1:]), pa, pb, ka, kb, coef, Bt, b_rep, QS,
                                   Op, self._tc_status)
             assert done, "checked at construction"
-        elif self.df:
+            return
+        term, dims = (pa, pb, ka, kb, int(QS)), tuple(self.t2.shape[1:])
+        Wm = None
+        if const is not None and D.takes_mod(dims, self.m, term, True, self.df):
+            Wm = self.E.mod_w(const, QS)
+        if Wm is not None:
+            L.check(self.lib.fricc_spb_spmm_mod(self.spb, which, pa, pb, ka, kb, float(coef), _ptr(W), _ptr(Wm), int(QS),
+                                                _ptr(Op), o_stride, st))
+        elif self.df and not D.takes_mod(dims, self.m, term, False, True):
             if const is not None:
+                self.E.prepare_splits((const,))
                 W2, w_stride = self.E.split(const), 0
             else:
                 rows = W[0].numel() // QS
@@ -294,7 +322,7 @@ class FusedReplicaBatch:
         E, R, o, v = self.E, self.R, self.o, self.v
         ov, ovv, oov = o * v, o * v * v, o * o * v
         f64, dev = t2.dtype, t2.device
-        comb, mmf, mm = D.combine, D.gemm_f64, self._mm
+        comb, mmf, mm = D.combine, self._mmf, self._mm
         C = self.C
         fov = C["fov"]
 

@@ -172,9 +172,43 @@ int fricc_sp_recompress_batch(int64_t count, fricc_sparse* const* T, const doubl
  * key_e = slot[ka]*dims[kb] + slot[kb] (slots 0..3 = the tensor's four
  * indices).  Wp is contiguous [dims[ka]*dims[kb]][QS], Op contiguous
  * [dims[pa]*dims[pb]][QS].  Each Op element receives its contributions in
- * nonzero-slot order.  Stream-ordered. */
+ * nonzero-slot order, or as one exact sum (below).  Stream-ordered. */
 int fricc_spmm(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, const double* Wp, int64_t QS,
                double* Op, void* stream);
+
+/* Where the sizes make it pay, fricc_spmm, fricc_contract, fricc_spb_spmm
+ * (FP64) and the dense fricc_gemm_f64 / fricc_gemm_df run as modular integer
+ * products on the tensor cores: sums over the nonzeros (or k) taken exactly
+ * on operands rounded at 2^-60 of their row's norm, then rounded once, which
+ * no order of summation changes; outputs for which that could be less
+ * accurate than an FP64 FMA chain, and rows with infinities or NaNs, are
+ * recomputed in FP64 in index order.  No reference counterpart.
+ *
+ * A constant operand can be converted once: fricc_mod_prepare turns rows x k
+ * FP64 elements (element (r, j) at x + r row_stride + j k_stride) into `out`
+ * (fricc_mod_bytes(rows, k) bytes, 16-byte aligned); fricc_spmm_mod and
+ * fricc_spb_spmm_mod take W' prepared as its rows q (rows = QS, k = the keys:
+ * row_stride 1, k_stride QS) beside W' itself, fricc_gemm_f64_mod a prepared
+ * A (rows m) and / or B (rows n), either null, with strides {row, column,
+ * batch, second batch}.  The results are those of the calls without it.
+ * fricc_spmm_takes_mod / fricc_gemm_takes_mod say whether a shape takes that
+ * route (pairs: against the FP32-pair kernels); fricc_mod_select makes the
+ * calling thread take it never (0), wherever possible (1), or by the time
+ * model (-1, the default). */
+int fricc_mod_select(int mode);
+int fricc_mod_mode(void); /* the calling thread's mode */
+int64_t fricc_mod_bytes(int64_t rows, int64_t k);
+int fricc_mod_prepare(const double* x, int64_t rows, int64_t k, int64_t row_stride, int64_t k_stride, void* out,
+                      void* stream);
+int fricc_spmm_mod(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, const double* Wp, const void* Wm,
+                   int64_t QS, double* Op, void* stream);
+int fricc_spmm_takes_mod(const int64_t dims[4], int64_t m, int pa, int pb, int ka, int kb, int64_t QS, int prepared,
+                         int pairs);
+int fricc_gemm_f64_mod(const double* A, const void* Am, const double* B, const void* Bm, double* C, int64_t batch,
+                       int64_t batch2, int64_t M, int64_t N, int64_t K, const int64_t sA[4], const int64_t sB[4],
+                       const int64_t sC[4], double alpha, double beta, void* stream);
+int fricc_gemm_takes_mod(int64_t batch, int64_t M, int64_t N, int64_t K, int a_batched, int b_batched, int a_prepared,
+                         int b_prepared, int pairs);
 
 /* fricc_spmm in FP32-pair arithmetic (no reference counterpart): Wp4 is W'
  * split by fricc_split_f2 into its q-pair layout (16-byte aligned); every
@@ -313,6 +347,8 @@ int fricc_spb_export(fricc_spbatch* B, int which, int r, int64_t* flat_host, dou
  * out'_r = Op + r o_stride.  Stream-ordered. */
 int fricc_spb_spmm(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, double coef, const double* Wp,
                    int64_t w_stride, int64_t QS, double* Op, int64_t o_stride, void* stream);
+int fricc_spb_spmm_mod(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, double coef, const double* Wp,
+                       const void* Wm, int64_t QS, double* Op, int64_t o_stride, void* stream);
 int fricc_spb_spmm_f2(fricc_spbatch* B, int which, int pa, int pb, int ka, int kb, double coef, const void* W2,
                       int64_t w2_stride, int64_t QS, double* Op, int64_t o_stride, void* stream);
 /* fricc_densify_bf16x3 for every replica of a batch: replica r's
