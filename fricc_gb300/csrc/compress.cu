@@ -112,6 +112,8 @@ struct Ctl {
   int sample;         // 1: R > 0 and finite, so samples can land in intervals
   double rn;          // the uniform draw
   // pivotal sampling
+  int64_t bad;        // the first segment of the parallel walk whose end is not the next one's start
+  int64_t serial;     // 1: the walk has to be the serial one (k_piv_chain)
   int64_t jend;       // last element the sampler visits (it stops once m' indices are out)
   int64_t npush;      // indices emitted up to jend (chain), then in total (final)
   int64_t plast;      // the pivot after jend
@@ -629,9 +631,9 @@ __global__ void k_unpack(const int64_t* __restrict__ flat, int64_t m, int64_t d0
 //
 // Only the carried weight is a true recurrence (sequential FP64 with a
 // wrap), and it does not depend on the draws, nor does which elements emit.
-// So: (1) one warp walks the weight and records a_j and the wrap flag for
-// every element, which fixes where the sampler stops and how many draws it
-// consumes; (2) the draws arrive; (3) every decision is independent given
+// So: (1) the weight is walked, in parallel segments (below), recording a_j
+// and the wrap flag of every element, which fixes where the sampler stops and
+// how many draws it consumes; (2) the draws arrive; (3) every decision is independent given
 // a_j, p_j and rn_j; (4) the pivot an element emits is the last "take"
 // before it, a max-scan; its slot in S is the count of emits before it, a
 // sum-scan.  Per-element codes: bit 0 the pivot moves here, bit 1 the
@@ -672,11 +674,304 @@ __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __res
   }
 }
 
-// One warp.  Lane t of a batch of 32 elements keeps a_j and the wrap flag
+// The weight walk in parallel.  After a wrap the weight is a multiple of
+// 2^-52 (a sum in [1, 2) minus 1, exactly), and every later step rounds at
+// 2^-53 or finer until the sum passes 1 again: two walks whose weights differ
+// by a multiple d of 2^-52 round alike and stay d apart, as long as no sum of
+// theirs falls on different sides of a power of two, except that a tie at the
+// wrap itself (ulp 2^-52) goes by the parity of d.  Over a segment from one
+// wrap to another the walk is therefore a map n -> n + (n odd ? d1 : d0) on
+// n = a 2^52 near a predicted n, and such maps compose.
+//
+// The tensor is cut into regions of S elements; a segment starts at the
+// first wrap of its region that the exact fixed-point prefix sums (mod 1, in
+// 2^-64) predict.  k_piv_walk<1> walks every segment from its predicted
+// start, once per parity, and leaves its map; k_piv_claims composes them to
+// the start of each segment; k_piv_walk<2> walks each segment again from
+// there with the sampler's own FP64 operations, writes a_j and the flags, and
+// compares its end with the next segment's start.  If they all agree the
+// recurrence holds from end to end: the result does not rest on the argument
+// above.  Where one does not (a prediction within ~1e-12 of a power of
+// two), the claims behind it are recomputed from its true end, twice; what
+// then remains (and p outside [0, 1], m' = 0) is left to the serial walk.
+//
+// Bound by the latency of two dependent FP64 additions per element over one
+// segment (~70 ns each): o13v57 (549,081 elements) 73 ms serial, 60 us so.
+constexpr int PW_MIN = 128;          // elements per region, at least
+constexpr int64_t PW_SEGS = 32768;   // regions, at most
+constexpr double PW_ULP = 0x1p-52;
+
+struct PivSegs {
+  int64_t n, S, nseg;
+  unsigned long long* f;    // sums of floor(p 2^64) per region, then exclusive prefixes
+  int64_t* start;           // the segment's first element (a wrap), -1: none
+  exact::Map* map;
+  double* claim;            // the weight after element start
+  double* end;              // the weight at the end of the segment
+  int* cnt;                 // its wraps
+};
+
+__device__ __forceinline__ unsigned long long frac64(double p) {  // floor(p 2^64) mod 2^64, p in [0, 1]
+  const unsigned long long u = (unsigned long long)__double_as_longlong(p);
+  const int e = (int)(u >> 52);
+  const unsigned long long m = (u & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+  const int sh = e - (1075 - 64);
+  return sh >= 64 || sh <= -64 ? 0ull : (sh >= 0 ? m << sh : m >> -sh);
+}
+
+// region sums (one warp each) and the check of p
+__global__ void __launch_bounds__(256) k_piv_sums(const double* __restrict__ P, PivSegs g, Ctl* c) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t s = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); s < g.nseg; s += (int64_t)gridDim.x * 8) {
+    const int64_t j1 = (s + 1) * g.S < g.n ? (s + 1) * g.S : g.n;
+    unsigned long long f = 0;
+    bool odd = false;
+    for (int64_t j = s * g.S + lane; j < j1; j += 32) {
+      const double p = P[j];
+      f += frac64(p);
+      odd |= (unsigned long long)__double_as_longlong(p) > 0x3ff0000000000000ull;  // not in [0, 1] (or -0, NaN)
+    }
+    f = warp_sum(f);
+    if (__any_sync(0xffffffffu, odd) && lane == 0) c->serial = 1;
+    if (lane == 0) g.f[s] = f;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c->bad = g.nseg;
+    if (c->mp == 0) c->serial = 1;
+  }
+}
+
+// exclusive prefixes of the region sums (one block)
+__global__ void __launch_bounds__(1024) k_piv_prefix(PivSegs g, const Ctl* c) {
+  if (c->serial) return;
+  __shared__ int64_t sm[33];
+  int64_t run = 0;
+  for (int64_t b = 0; b < g.nseg; b += 1024) {
+    const int64_t s = b + threadIdx.x;
+    const int64_t v = s < g.nseg ? (int64_t)g.f[s] : 0;
+    int64_t tot;
+    const int64_t ex = block_excl_sum(v, sm, &tot);  // wraps mod 2^64, as wanted
+    if (s < g.nseg) g.f[s] = (unsigned long long)(run + ex);
+    run += tot;
+  }
+}
+
+__device__ __forceinline__ bool ge_one(double s) { return (__double_as_longlong(s) >> 32) >= 0x3ff00000ll; }
+
+// one step of the sampler's weight
+__device__ __forceinline__ bool piv_step(double& a, double p) {
+  const double sum = __dadd_rn(a, p);
+  const bool w = ge_one(sum);
+  a = w ? __dsub_rn(sum, 1.0) : sum;
+  return w;
+}
+
+// One thread per segment.  PASS 1: find the start, walk both parities of the
+// predicted weight to the next segment's start, leave the map (segment 0:
+// its true end).  PASS 2: walk from the claimed weight, write a_j, the wrap
+// flags and their number, and report an end that is not the next claim.
+template <int PASS>
+__global__ void __launch_bounds__(64) k_piv_walk(const double* __restrict__ P, PivSegs g, Ctl* c,
+                                                 double* __restrict__ A, unsigned char* __restrict__ code,
+                                                 int64_t from_bad) {
+  if (c->serial) return;
+  const int64_t s = (int64_t)blockIdx.x * 64 + threadIdx.x;
+  if (s >= g.nseg) return;
+  // a later round walks only what follows the segment that failed
+  int64_t first = 0;
+  if (PASS == 2 && from_bad) {
+    first = from_bad == 1 ? g.cnt[g.nseg] : g.cnt[g.nseg + 1];  // the last round's bad segment
+    if (first >= g.nseg || s <= first) return;
+  }
+  int64_t j = s * g.S;
+  unsigned long long F = g.f[s];
+  double a0, a1 = 0.0;
+  if (PASS == 1) {
+    if (s == 0) {
+      a0 = P[0];
+      F += frac64(a0);
+      g.start[0] = 0;
+      j = 1;
+    } else {
+      const int64_t j1 = j + g.S < g.n ? j + g.S : g.n;
+      int64_t at = -1;
+      for (; j < j1; ++j) {
+        const unsigned long long F1 = F + frac64(P[j]);
+        const bool w = F1 < F;
+        F = F1;
+        if (w) {
+          at = j++;
+          break;
+        }
+      }
+      g.start[s] = at;
+      if (at < 0) {
+        g.map[s] = exact::map_id();
+        return;
+      }
+      const unsigned long long n = F >> 12;  // the weight in units of 2^-52
+      a0 = (double)(long long)(n & ~1ull) * PW_ULP;
+      a1 = (double)(long long)(n | 1ull) * PW_ULP;
+    }
+  } else {
+    const int64_t at = g.start[s];
+    if (at < 0) return;
+    j = at + 1;
+    a0 = s == 0 ? P[0] : g.claim[s];
+    if (s == 0) {
+      A[0] = a0;
+      code[0] = 0;
+    }
+  }
+  const double b0 = a0, b1 = a1;
+  // to the next segment's start: the first predicted wrap past this region
+  // (PASS 2 knows where it is)
+  int64_t last = g.n - 1, nxt = g.nseg;
+  if (PASS == 2) {
+    for (int64_t t = s + 1; t < g.nseg; ++t)
+      if (g.start[t] >= 0) {
+        last = g.start[t];
+        nxt = t;
+        break;
+      }
+  }
+  const int64_t edge = (s + 1) * g.S;
+  int cnt = 0;
+  bool w0 = false, w1 = false, done = false;
+  constexpr int U = 8;  // elements loaded ahead
+  double buf[U];
+#pragma unroll
+  for (int q = 0; q < U; ++q) buf[q] = j + q <= last ? P[j + q] : 0.0;
+  while (j <= last && !done) {
+    double cur[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) cur[q] = buf[q];
+#pragma unroll
+    for (int q = 0; q < U; ++q) buf[q] = j + U + q <= last ? P[j + U + q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      if (j + q <= last && !done) {
+        w0 = piv_step(a0, cur[q]);
+        if (PASS == 1) {
+          w1 = piv_step(a1, cur[q]);
+          const unsigned long long F1 = F + frac64(cur[q]);
+          done = F1 < F && j + q >= edge;
+          F = F1;
+        } else {
+          A[j + q] = a0;
+          code[j + q] = w0 ? PV_EMIT : 0;
+          cnt += w0 ? 1 : 0;
+        }
+      }
+    }
+    j += U;
+  }
+  if (PASS == 1) {
+    if (s == 0) {
+      g.end[0] = a0;
+    } else {
+      // (an end that is no wrap has no map: its claim will not hold)
+      const bool ok = w0 && w1;
+      g.map[s] = ok ? exact::Map{(int64_t)((a0 - b0) * 0x1p52), (int64_t)((a1 - b1) * 0x1p52)} : exact::map_id();
+    }
+  } else {
+    g.end[s] = a0;
+    g.cnt[s] = cnt;
+    if (nxt < g.nseg && __double_as_longlong(g.claim[nxt]) != __double_as_longlong(a0))
+      atomicMin(reinterpret_cast<unsigned long long*>(&c->bad), (unsigned long long)s);
+  }
+}
+
+// The weights at the segments' starts (one block): the maps composed from
+// the end of segment 0, or (a later round) from the true end of the segment
+// that failed, whose number moves to cnt[nseg] (cnt[nseg + 1]).
+__global__ void __launch_bounds__(1024) k_piv_claims(PivSegs g, Ctl* c, int round) {
+  if (c->serial) return;
+  __shared__ exact::Map smaps[33];
+  const int64_t bad = c->bad;
+  __syncthreads();
+  if (round > 0) {
+    if (threadIdx.x == 0) g.cnt[g.nseg + round - 1] = (int)bad;
+    if (bad >= g.nseg) return;
+    if (threadIdx.x == 0) c->bad = g.nseg;
+  }
+  const int64_t s0 = round > 0 ? bad + 1 : 1;
+  const double a = round > 0 ? g.end[bad] : g.end[0];
+  int64_t first = s0;  // the next live segment
+  while (first < g.nseg && g.start[first] < 0) ++first;
+  int64_t n = (int64_t)(a * 0x1p52);
+  for (int64_t b = s0; b < g.nseg; b += 1024) {
+    const int64_t s = b + threadIdx.x;
+    const bool live = s < g.nseg && g.start[s] >= 0;
+    exact::Map tot;
+    const exact::Map pre = exact::block_excl_scan_map<1024>(live ? g.map[s] : exact::map_id(), smaps, &tot);
+    // (the segment behind one that failed takes the weight itself, on or off the 2^-52 grid)
+    if (live) g.claim[s] = s == first ? a : (double)exact::apply(pre, n) * PW_ULP;
+    n = exact::apply(tot, n);
+  }
+}
+
+// Where the sampler stops: the element of the m'-th wrap (one block).
+__global__ void __launch_bounds__(1024) k_piv_end(PivSegs g, const unsigned char* __restrict__ code, Ctl* c) {
+  if (c->serial) return;
+  if (c->bad < g.nseg) {  // not proven after the last round
+    if (threadIdx.x == 0) c->serial = 1;
+    return;
+  }
+  __shared__ int64_t sm[33];
+  __shared__ int64_t s_seg, s_left;
+  if (threadIdx.x == 0) s_seg = -1;
+  __syncthreads();
+  const int64_t mp = c->mp;
+  int64_t run = 0;
+  for (int64_t b = 0; b < g.nseg; b += 1024) {
+    const int64_t s = b + threadIdx.x;
+    const int64_t k = s < g.nseg && g.start[s] >= 0 ? g.cnt[s] : 0;
+    int64_t tot;
+    const int64_t ex = run + block_excl_sum(k, sm, &tot);
+    if (k > 0 && ex < mp && ex + k >= mp) {
+      s_seg = s;
+      s_left = mp - ex;
+    }
+    run += tot;
+  }
+  __syncthreads();
+  if (s_seg < 0) {
+    if (threadIdx.x == 0) {
+      c->jend = g.n - 1;
+      c->npush = run;
+      c->broke = 0;
+    }
+    return;
+  }
+  if (threadIdx.x < 32) {  // the left-th wrap of that segment
+    int64_t left = s_left;
+    for (int64_t j0 = g.start[s_seg] + 1;; j0 += 32) {
+      const int64_t j = j0 + threadIdx.x;
+      const unsigned w = __ballot_sync(0xffffffffu, j < g.n && code[j] != 0);
+      if (__popc(w) >= left) {
+        unsigned m = w;
+        for (int64_t q = 1; q < left; ++q) m &= m - 1;
+        if (threadIdx.x == 0) {
+          c->jend = j0 + __ffs((int)m) - 1;
+          c->npush = mp;
+          c->broke = 1;
+        }
+        break;
+      }
+      left -= __popc(w);
+      if (j0 + 32 >= g.n) break;  // not reached: the wraps were counted
+    }
+  }
+}
+
+// The serial walk, for what the parallel one leaves (c->serial).  One warp.
+// Lane t of a batch of 32 elements keeps a_j and the wrap flag
 // of element j0 + t; every lane walks the same chain (the p_j come in by
 // shuffle, the next batch's are loaded while this one runs).
 __global__ void __launch_bounds__(32) k_piv_chain(const double* __restrict__ P, int64_t n, Ctl* c,
                                                   double* __restrict__ A, unsigned char* __restrict__ code) {
+  if (!c->serial) return;
   const int lane = threadIdx.x;
   const int64_t mp = c->mp;
   double a = P[0];
@@ -1207,6 +1502,7 @@ static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsi
                    cudaStream_t st) {
   double *P = nullptr, *A = nullptr, *R = nullptr;
   unsigned char* code = nullptr;
+  void* seg = nullptr;
   int64_t *tlast = nullptr, *tcnt = nullptr;
   const int64_t ntile = fricc_cdiv(n, PV_TILE);
   int rc = fricc_alloc_t(&P, n, st);
@@ -1219,8 +1515,35 @@ static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsi
   if (!rc) {
     k_pvec<<<(unsigned)fricc_cdiv(n, exact::CH / PV_SUB), 256, 0, st>>>(gp, n, P, s.err, nullptr);
     phase_mark(2, st);
-    k_piv_chain<<<1, 32, 0, st>>>(P, n, ctl, A, code);
-    fricc_note_launch(2);
+    PivSegs g;
+    g.n = n;
+    g.S = fricc_cdiv(n, PW_SEGS) > PW_MIN ? fricc_cdiv(fricc_cdiv(n, PW_SEGS), 32) * 32 : PW_MIN;
+    g.nseg = fricc_cdiv(n, g.S);
+    // one block for all of the segments' arrays: 8-byte items first
+    const int64_t q = g.nseg;
+    rc = fricc_alloc(&seg, (size_t)(q * (8 + 8 + 16 + 8 + 8) + (q + 2) * 4), st);
+    if (!rc) {
+      char* b = static_cast<char*>(seg);
+      g.map = reinterpret_cast<exact::Map*>(b);
+      g.f = reinterpret_cast<unsigned long long*>(b + 16 * q);
+      g.start = reinterpret_cast<int64_t*>(b + 24 * q);
+      g.claim = reinterpret_cast<double*>(b + 32 * q);
+      g.end = reinterpret_cast<double*>(b + 40 * q);
+      g.cnt = reinterpret_cast<int*>(b + 48 * q);
+      const unsigned gw = (unsigned)fricc_cdiv(g.nseg, 64);
+      k_piv_sums<<<grid_for(g.nseg, 8), 256, 0, st>>>(P, g, ctl);
+      k_piv_prefix<<<1, 1024, 0, st>>>(g, ctl);
+      k_piv_walk<1><<<gw, 64, 0, st>>>(P, g, ctl, A, code, 0);
+      for (int round = 0; round < 3; ++round) {
+        k_piv_claims<<<1, 1024, 0, st>>>(g, ctl, round);
+        k_piv_walk<2><<<gw, 64, 0, st>>>(P, g, ctl, A, code, round);
+      }
+      k_piv_end<<<1, 1024, 0, st>>>(g, code, ctl);
+      k_piv_chain<<<1, 32, 0, st>>>(P, n, ctl, A, code);
+      fricc_note_launch(12);
+    }
+  }
+  if (!rc) {
     rc = fricc_cuda_check(cudaGetLastError(), "pivotal chain");
   }
   if (!rc) rc = fricc_cuda_check(cudaMemcpyAsync(&jend, &ctl->jend, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "jend");
@@ -1257,6 +1580,7 @@ static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsi
   fricc_free(A, st);
   fricc_free(R, st);
   fricc_free(code, st);
+  fricc_free(seg, st);
   fricc_free(tlast, st);
   fricc_free(tcnt, st);
   return rc;

@@ -46,7 +46,9 @@ __global__ void k_glibc_starts(const unsigned* __restrict__ J, const unsigned* _
 
 // chunk c: draws [c*GCH, min((c+1)*GCH, k)); the thread holding the last draw
 // writes the history that follows it
-__global__ void k_glibc_gen(const unsigned* __restrict__ starts, int64_t nch, int64_t k, double* __restrict__ out,
+// (the words only: the FP64 division of each draw, in the same thread, made a
+// draw ~370 ns, 0.73 ms a chunk; k_glibc_uniform divides in parallel)
+__global__ void k_glibc_gen(const unsigned* __restrict__ starts, int64_t nch, int64_t k, unsigned* __restrict__ out,
                             unsigned* __restrict__ hist_out) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nch) return;
@@ -63,7 +65,7 @@ __global__ void k_glibc_gen(const unsigned* __restrict__ starts, int64_t nch, in
       if (done + d < cnt) {
         const unsigned w = r[d] + r[(d + RDEG - RSEP) % RDEG];
         r[d] = w;
-        out[base + done + d] = (double)(int)(w >> 1) / 2147483647.0;
+        out[base + done + d] = w;
       }
     }
     done += RDEG;
@@ -74,6 +76,11 @@ __global__ void k_glibc_gen(const unsigned* __restrict__ starts, int64_t nch, in
 #pragma unroll
     for (int t = 0; t < RDEG; ++t) hist_out[t] = r[(off + t) % RDEG];
   }
+}
+
+__global__ void k_glibc_uniform(const unsigned* __restrict__ w, int64_t k, double* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = (double)(int)(w[i] >> 1) / 2147483647.0;
 }
 
 using Mat = std::vector<unsigned>;
@@ -117,11 +124,13 @@ int fricc_glibc_uniforms_device(unsigned* hist, int64_t k, double* out, cudaStre
   if (k == 0) return FRICC_OK;
   const int64_t nch = fricc_cdiv(k, GCH);
   static const Mat J = step_power(GCH);
-  unsigned *dJ = nullptr, *dh = nullptr, *starts = nullptr;
+  unsigned *dJ = nullptr, *dh = nullptr, *starts = nullptr, *words = nullptr;
   int rc = fricc_alloc_t(&dJ, RDEG * RDEG + 2 * RDEG, st);
   if (!rc) rc = fricc_alloc_t(&starts, nch * RDEG, st);
+  if (!rc) rc = fricc_alloc_t(&words, k, st);
   if (rc) {
     fricc_free(dJ, st);
+    fricc_free(starts, st);
     return rc;
   }
   dh = dJ + RDEG * RDEG;
@@ -131,13 +140,16 @@ int fricc_glibc_uniforms_device(unsigned* hist, int64_t k, double* out, cudaStre
   if (e == cudaSuccess) e = cudaMemcpyAsync(dh, hist, sizeof(unsigned) * RDEG, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
     k_glibc_starts<<<1, 32, 0, st>>>(dJ, dh, nch, starts);
-    k_glibc_gen<<<(unsigned)fricc_cdiv(nch, 128), 128, 0, st>>>(starts, nch, k, out, dout);
-    fricc_note_launch(2);
+    k_glibc_gen<<<(unsigned)fricc_cdiv(nch, 32), 32, 0, st>>>(starts, nch, k, words, dout);
+    const int64_t g = fricc_cdiv(k, 256);
+    k_glibc_uniform<<<(unsigned)(g < 152 * 16 ? g : 152 * 16), 256, 0, st>>>(words, k, out);
+    fricc_note_launch(3);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(hist, dout, sizeof(unsigned) * RDEG, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   fricc_free(starts, st);
+  fricc_free(words, st);
   fricc_free(dJ, st);
   return e == cudaSuccess ? FRICC_OK : fricc_cuda_fail(e, "glibc_uniforms", __FILE__, __LINE__);
 }
