@@ -32,7 +32,7 @@
 // tiling, batch or split of K.
 //
 // Measured on a GB300 (operands prepared; DFMA kernel): 900 x 22500 x 22500
-// 11.8 ms; 4500^3 2.5 ms (152 ms); 2000^3 0.29 ms (14.0 ms); 400^3 31 us
+// 9.1 ms; 4500^3 2.05 ms (152 ms); 2000^3 0.26 ms (14.0 ms); 400^3 30 us
 // (279 us); 675000 x 30 x 150 0.97 ms (5.25 ms).  Converting an operand: 11-12 ps
 // an element.  Error (2-norm, against 64 bits) of the o30v150 iteration: 7e-16,
 // 2.3e-15 on the FP64 pipe.
@@ -555,16 +555,15 @@ __global__ void __launch_bounds__(MNT, 1)
   const uint32_t tmem = tbase;
 
   if (warp == 0) {
-    if (lane == 0) {  // TMA producer
-      int q = 0;      // k blocks issued over all units
+    if (elect_one()) {  // TMA producer
+      int q = 0, s = 0;  // k blocks issued over all units; stage q % STAGES
+      uint32_t ph = 0;   // and its use's parity
       for (int u = blockIdx.x; u < nunits && !*(volatile int*)&failed; u += gridDim.x) {
         const Unit x = unit_of(g, u);
         const int ya = x.plane * nk * g.a_rows + x.rep * g.a_rep + x.mt * BM;
         const int yb = x.plane * nk * g.b_rows + x.rep * g.b_rep + x.nt * g.bn;
         const int kb1 = min(nk, (x.slice + 1) * cpk * KC);
         for (int kb = x.slice * cpk * KC; kb < kb1; ++kb, ++q) {
-          const int s = q % STAGES;
-          const uint32_t ph = (uint32_t)(q / STAGES) & 1u;
           if (q >= STAGES && !mbar_wait(smem_u32(&empty[s]), ph ^ 1u)) {
             atomicOr(err, FRICC_DEV_TIMEOUT);
             failed = 1;
@@ -573,6 +572,10 @@ __global__ void __launch_bounds__(MNT, 1)
           mbar_expect_tx(smem_u32(&full[s]), a_bytes + b_bytes);
           tma_load_2d(sA + s * A_BYTES, &tma, 0, ya + kb * g.a_rows, smem_u32(&full[s]));
           tma_load_2d(sB + s * b_bytes, &tmb, 0, yb + kb * g.b_rows, smem_u32(&full[s]));
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
       if (*(volatile int*)&failed) {
@@ -582,10 +585,17 @@ __global__ void __launch_bounds__(MNT, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // MMA issuer
+    if (elect_one()) {  // MMA issuer
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.bn >> 3) << 17) |
                              ((uint32_t)(BM >> 4) << 24);
-      int q = 0, i = 0;  // k blocks, runs
+      // The chain wait, MMAs, commit of a k block must stay below its MMAs' time: no
+      // division by the stage count, descriptors by one addition.  (With both and
+      // a branch on the lane number it took ~900 clocks: 1204 TFLOP/s at 4500^3,
+      // whatever the loads did; now ~400.)
+      const uint64_t da = sw128_desc(sA), db = sw128_desc(sB);
+      const uint32_t b_step = b_bytes >> 4;
+      int i = 0, s = 0;  // runs; the stage
+      uint32_t ph = 0;
       for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int slice = unit_of(g, u).slice;
         const int kb1 = min(nk, (slice + 1) * cpk * KC);
@@ -600,19 +610,22 @@ __global__ void __launch_bounds__(MNT, 1)
           tc_fence_after();
           const uint32_t acc = tmem + (uint32_t)(b * 256);
           const int kb_end = min(kb1, kb0 + KC);
-          for (int kb = kb0; kb < kb_end; ++kb, ++q) {
-            const int s = q % STAGES;
-            if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(q / STAGES) & 1u)) {
+          for (int kb = kb0; kb < kb_end; ++kb) {
+            if (!mbar_wait(smem_u32(&full[s]), ph)) {
               atomicOr(err, FRICC_DEV_TIMEOUT);
               failed = 1;
               break;
             }
             tc_fence_after();
-            const uint32_t a0 = sA + s * A_BYTES, b0 = sB + s * b_bytes;
+            const uint64_t a0 = da + (uint32_t)s * (A_BYTES >> 4), b0 = db + (uint32_t)s * b_step;
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
-              tc_mma(acc, sw128_desc(a0 + k * 32), sw128_desc(b0 + k * 32), idesc, ((kb - kb0) | k) != 0);
+              tc_mma(acc, a0 + 2 * k, b0 + 2 * k, idesc, ((kb - kb0) | k) != 0);
             tc_commit(smem_u32(&empty[s]));
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
           tc_commit(smem_u32(&tfull[b]));  // arrives when this run's MMAs have completed
           if (*(volatile int*)&failed) break;
@@ -974,10 +987,13 @@ __global__ void __launch_bounds__(256) k_mod_fix(CombineArgs a, const ModView A,
 // ------------------------------------------------------------ host
 // The tile width and orientation by a model in clocks: rounds of units over
 // the SMs times a unit's K steps or its drains, whichever is longer.  An MMA
-// of 128 x bn x 16 takes bn/2 clocks of tensor pipe, 32 + bn/4 of
-// shared-memory reads, and its operands 32 (128 + bn) bytes of L2 at the ~58
-// per clock and SM that a 128 x 256 tile was measured at (1.27 PFLOP/s); a
-// drain issues ~6 clocks a column, ~1200 clocks a unit overlap with nothing.
+// of 128 x bn x 16 takes bn/2 clocks of tensor pipe, ~100 of the issuing
+// thread, and its operands 32 (128 + bn) bytes of L2 at the 68-74 per clock and
+// SM that tiles of 96 to 256 columns were measured at (4500^3: 3.1 ms at 96, 2.3
+// at 128, 1.77 at 224, 1.80 at 256); a drain issues ~6 clocks a column, ~1200
+// clocks a unit overlap with nothing.  Pairs of CTAs on 256 x 256 tiles
+// (cta_group::2: 49 bytes per clock) were 3% faster there and 5% slower at
+// 400 x 10000 x 10000: the drains then set the pace.
 struct Plan {
   int bn = 256, ks = 1;
   bool swap = false;
@@ -992,8 +1008,8 @@ Plan plan_for(int64_t M, int64_t N, int64_t K, int64_t reps, int nsm) {
       const int64_t tiles = fricc_cdiv(m, BM) * fricc_cdiv(n, bn) * PLANES * reps;
       int ks = 1;
       while (ks < MAX_KS && tiles * ks < 2 * nsm && chunks / (2 * ks) >= 2) ks *= 2;
-      const double smem = 32 + bn / 4, l2 = ((m < BM ? m : BM) + bn) * 32 / 58.0;
-      double step = bn / 2 > smem ? bn / 2 : smem;
+      const double l2 = ((m < BM ? m : BM) + bn) * 32 / 70.0;
+      double step = bn / 2 > 100 ? bn / 2 : 100;
       if (l2 > step) step = l2;
       const double runs = (double)fricc_cdiv(chunks, ks);
       const double mma = (nk < KC ? (double)nk : runs * KC) * 4.0 * step, drain = runs * (200.0 + 6.0 * bn);

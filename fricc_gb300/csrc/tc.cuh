@@ -37,6 +37,15 @@ __device__ __forceinline__ uint64_t gtime() {
   return t;
 }
 
+// True in one lane of a converged warp.  A branch on elect.sync (rather than
+// on a lane number) tells the compiler that a single thread runs it, so that the
+// descriptors of an MMA go straight to uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
 }
