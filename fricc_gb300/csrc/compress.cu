@@ -1621,7 +1621,7 @@ static int compress_front(const double* x, int64_t n, int64_t m, int R, int mode
   if (!rc) rc = fricc_alloc_t(&s.dzero, 1, st);
   if (!rc) rc = fricc_alloc_t(&s.ffail, r_, st);
   if (!rc) rc = fricc_alloc_t(&s.psum, r_ * nch1, st);
-  if (!rc && fri) rc = exact::chain_scratch(s.chain, R * nch1, st);
+  if (!rc && fri) rc = exact::chain_scratch(s.chain, R * nch1, st, R);
   if (!rc && fri) rc = fricc_alloc_t(&s.Rb, r_ * (m + 1), st);
   if (!rc && fri) rc = fricc_alloc_t(&s.S, r_ * m, st);
   if (!rc && paired) rc = fricc_alloc_t(&s.S2, r_ * m, st);

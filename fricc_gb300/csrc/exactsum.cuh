@@ -21,10 +21,13 @@
 // * The binade of the running sum is predicted from an approximate
 //   (parallel) prefix sum with a safety margin; chunks whose predicted
 //   range stays inside one binade are "clean".
+// * A chunk whose predicted range crosses binades (the first one crosses a
+//   dozen) is cut at the elements whose step may leave a binade: the maps of the
+//   segments between them come from one segmented scan, and the cuts are
+//   single steps of real FP64 additions.
 // * A single-block walk applies the chunk maps to the exact running value,
 //   verifies every assumption (start in the predicted binade, end inside
-//   it) and, where a chunk crosses a binade or was mispredicted, processes
-//   that chunk exactly: scan under the current binade, find the first
+//   it) and, where one fails, processes that chunk exactly: scan under the current binade, find the first
 //   element whose step would leave it, perform that one step with a real
 //   FP64 add, continue.  Correctness never depends on the prediction.
 #pragma once
@@ -190,11 +193,213 @@ __device__ __forceinline__ Map block_excl_scan_map(Map v, Map* smem, Map* total)
   return r;
 }
 
+// One segment of a chunk that crosses binades: `map` composes the elements
+// between two cuts under binade b (0: none), then the cut element a is added
+// for real (unless `last`).
+struct Piece {
+  Map map;
+  double a;
+  int b, last;
+};
+constexpr int PIECES = 64;  // per chunk
+constexpr int SLOTS = 32;   // chunks of a chain with pieces: its binade crossings, as a rule
+struct Slots {
+  Piece p[SLOTS][PIECES];
+  int cnt[SLOTS];
+};
+
+// Composes s through the pieces of a chunk, checking every prediction;
+// `at` (if given) receives {before, after} of each cut, with the segments'
+// start values at[j].y of the cut before.
+__device__ __forceinline__ bool walk_pieces(const Piece* p, int cnt, double& s, double2* at) {
+  double v = s;
+  for (int j = 0; j < cnt; ++j) {
+    const Piece q = p[j];
+    if (q.b) {
+      if (binade_of(v) != q.b) return false;
+      const int64_t n = apply(q.map, n_of(v, q.b));
+      if (!run_valid(n, q.b, false)) return false;
+      v = s_of(q.b, n);
+    }
+    const double before = v;
+    if (!q.last) v = __dadd_rn(v, q.a);
+    if (at) at[j] = make_double2(before, v);
+  }
+  s = v;
+  return true;
+}
+
+struct SplitSmem {
+  Piece p[PIECES];
+  double2 at[PIECES];
+  Map m[33];
+  double sum[33];
+  int seg[33], cnt[33];  // a segment's binade | CUT once a cut lies in the range
+  int ok;
+};
+constexpr int CUT = 1 << 16;
+
+struct Seg {
+  Map m;
+  int f;  // binade | CUT
+  int n;  // cuts
+};
+__device__ __forceinline__ Seg then(const Seg& x, const Seg& y) {
+  Seg r;
+  r.m = (y.f & CUT) ? y.m : compose(x.m, y.m);
+  r.f = (y.f & CUT) ? y.f : (y.f ? (x.f & CUT) | y.f : x.f);
+  r.n = x.n + y.n;
+  return r;
+}
+__device__ __forceinline__ Seg seg_up(const Seg& x, int o) {
+  Seg r;
+  r.m.d0 = __shfl_up_sync(0xffffffffu, x.m.d0, o);
+  r.m.d1 = __shfl_up_sync(0xffffffffu, x.m.d1, o);
+  r.f = __shfl_up_sync(0xffffffffu, x.f, o);
+  r.n = __shfl_up_sync(0xffffffffu, x.n, o);
+  return r;
+}
+
 struct ChunkSmem {
   Map maps[33];
   int imin[32];
   double s;
+  SplitSmem split;
 };
+
+// Cuts a chunk of additions (element t ITEMS + k at thread t's a[k]) that
+// starts at about P0, `slack` units of its last place off at most, and writes
+// the pieces to out.  An element is a cut unless the approximate values before
+// and after it, slackened, lie in one binade.  Returns the number of pieces (the
+// same in every thread), 0 if they are more than PIECES.  pre: the composite
+// before the thread's first element, in the segment pre.n; cuts: the thread's
+// cut elements, as bits.  Integer comparisons of the bit patterns: GB300 adds
+// 2 FP64 numbers per SM and clock.  Bound by its dependent steps: ~25 us, where a
+// round per crossing (scan, search, one addition) took 4-9 us each and a first
+// chunk has a dozen (compressing o10v40's 160000 elements: the two walks 319 ->
+// 50 us, the sampling pass 130 -> 37, the chunk maps 17 -> 62; 613 -> 292 in all).
+template <int NT, int ITEMS>
+__device__ __forceinline__ int split_chunk(const double* a, int n_in, double P0, int64_t slack, SplitSmem& sm, Piece* out,
+                                           Seg& pre, unsigned& cuts) {
+  constexpr int NW = NT / 32;
+  const int t = threadIdx.x, lane = (int)lane_id(), warp = (int)warp_id();
+  double loc = 0.0;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) loc += a[k];  // (zeros past n_in)
+  double incl = loc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double w = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += w;
+  }
+  double ex = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) ex = 0.0;
+  __syncthreads();
+  if (lane == 31) sm.sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    double run = lane < NW ? sm.sum[lane] : 0.0;
+#pragma unroll
+    for (int o = 1; o < NW; o <<= 1) {
+      const double w = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += w;
+    }
+    double e = __shfl_up_sync(0xffffffffu, run, 1);
+    if (lane == 0) e = 0.0;
+    if (lane < NW) sm.sum[lane] = e;
+  }
+  __syncthreads();
+  const double P = P0 + (sm.sum[warp] + ex);
+  auto binade = [&](double p, double q, int& b) {  // false: a cut
+    const long long lo = __double_as_longlong(p) - slack, hi = __double_as_longlong(q) + slack;
+    if (!(q < 1e300)) return false;  // (NaN too)
+    const int bl = lo < 0 ? 0 : (int)(lo >> 52), bh = (int)(hi >> 52);
+    b = bl < 1 ? 1 : bl;
+    return b == (bh < 1 ? 1 : bh);
+  };
+  Seg mine{map_id(), 0, 0};
+  cuts = 0;
+  double p = P;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    if (t * ITEMS + k < n_in) {
+      const double q = p + a[k];
+      int b;
+      if (binade(p, q, b)) {
+        mine.m = compose(mine.m, elem_map(a[k], b, false));
+        mine.f = (mine.f & CUT) | b;
+      } else {
+        cuts |= 1u << k;
+        mine.m = map_id();
+        mine.f = CUT;
+        ++mine.n;
+      }
+      p = q;
+    }
+  }
+  Seg inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Seg w = seg_up(inc, o);
+    if (lane >= o) inc = then(w, inc);
+  }
+  Seg wex = seg_up(inc, 1);
+  if (lane == 0) wex = Seg{map_id(), 0, 0};
+  if (lane == 31) {
+    sm.m[warp] = inc.m;
+    sm.seg[warp] = inc.f;
+    sm.cnt[warp] = inc.n;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    Seg run = lane < NW ? Seg{sm.m[lane], sm.seg[lane], sm.cnt[lane]} : Seg{map_id(), 0, 0};
+#pragma unroll
+    for (int o = 1; o < NW; o <<= 1) {
+      const Seg w = seg_up(run, o);
+      if (lane >= o) run = then(w, run);
+    }
+    Seg e = seg_up(run, 1);
+    if (lane == 0) e = Seg{map_id(), 0, 0};
+    if (lane < NW) {
+      sm.m[lane] = e.m;
+      sm.seg[lane] = e.f;
+      sm.cnt[lane] = e.n;
+    }
+    if (lane == NW - 1) {
+      sm.m[NW] = run.m;
+      sm.seg[NW] = run.f;
+      sm.cnt[NW] = run.n;
+    }
+  }
+  __syncthreads();
+  pre = then(Seg{sm.m[warp], sm.seg[warp], sm.cnt[warp]}, wex);
+  const int total = sm.cnt[NW] + 1;
+  if (total > PIECES) return 0;
+  if (cuts) {
+    Map m = pre.m;
+    int f = pre.f & ~CUT, j = pre.n;
+    p = P;
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      if (t * ITEMS + k < n_in) {
+        const double q = p + a[k];
+        if ((cuts >> k) & 1u) {
+          out[j++] = Piece{m, a[k], f, 0};
+          m = map_id();
+          f = 0;
+        } else {
+          int b;
+          binade(p, q, b);
+          m = compose(m, elem_map(a[k], b, false));
+          f = b;
+        }
+        p = q;
+      }
+    }
+  }
+  if (t == 0) out[total - 1] = Piece{sm.m[NW], 0.0, sm.seg[NW] & ~CUT, 1};
+  return total;
+}
 
 struct ConsNull {
   __device__ __forceinline__ void operator()(int64_t, double, double, double) const {}
@@ -269,6 +474,42 @@ __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, doub
     // the binade every step is: the search for the step that leaves it (a
     // second pass over the items and a block minimum) runs only otherwise
     if (!run_valid(apply(tot, n0), b, sub)) {
+      if (!sub && round == 0) {
+        // all crossings at once: the rounds below take one each (4-9 us; the
+        // first chunk of a chain has a dozen)
+        Seg seg;
+        unsigned cuts;
+        const int cnt = split_chunk<NT, ITEMS>(a, n_in, s, 256 + n_in, sm.split, sm.split.p, seg, cuts);
+        __syncthreads();
+        if (t == 0) {
+          double v = s;
+          sm.split.ok = cnt > 0 && walk_pieces(sm.split.p, cnt, v, sm.split.at);
+          sm.s = v;
+        }
+        __syncthreads();
+        if (sm.split.ok) {
+          int j = seg.n, bj = sm.split.p[j].b;
+          const double s0 = j ? sm.split.at[j - 1].y : s;
+          int64_t nj = bj ? apply(seg.m, n_of(s0, bj)) : 0;
+#pragma unroll
+          for (int k = 0; k < ITEMS; ++k) {
+            const int i = t * ITEMS + k;
+            if (i < n_in) {
+              if ((cuts >> k) & 1u) {
+                const double2 v = sm.split.at[j];
+                cons(base + i, v.x, v.y, a[k]);
+                bj = sm.split.p[++j].b;
+                nj = n_of(v.y, bj);
+              } else {
+                const int64_t nn = apply(elem_map(a[k], bj, false), nj);
+                cons(base + i, s_of(bj, nj), s_of(bj, nn), a[k]);
+                nj = nn;
+              }
+            }
+          }
+          return sm.s;
+        }
+      }
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
         const int i = t * ITEMS + k;
@@ -337,18 +578,22 @@ __global__ void __launch_bounds__(256) k_chunk_sums(Gen gen0, Len ln, double* cs
 }
 
 // K_B (one block of 1024): approximate prefix of the chunk sums and the
-// per-chunk binade prediction: cbin[c] = binade if clean, 0 if not.  The
+// per-chunk binade prediction: cbin[c] = binade if clean; else minus the slot
+// for its pieces, counted from 1 (0: none left, or a chain of subtractions), and
+// csum[c] becomes the approximate value at the chunk's start.  The
 // prefix is a shuffle scan: one thread adding 1024 partials (dependent FP64
 // additions, ~55 ns each on this part) took 58 us a call, three calls a
 // compression; now 4-5 us.
-static __global__ void __launch_bounds__(1024) k_classify(const double* csum, Len ln, const double* s_init_dev,
-                                                   int sub, int* cbin, ChainStride cs) {
+static __global__ void __launch_bounds__(1024) k_classify(double* csum, Len ln, const double* s_init_dev,
+                                                   int sub, int* cbin, int slots, ChainStride cs) {
   const int rep = blockIdx.x;
   const int64_t nch = fricc_cdiv(ln.get(rep), CH), cap = fricc_cdiv(ln.n, CH) + 1;
   csum += (int64_t)rep * cap;
   cbin += (int64_t)rep * cap;
   const double s_init = s_init_dev[rep * cs.s_init];
   __shared__ double wtot[33];
+  __shared__ int used;
+  if (threadIdx.x == 0) used = 0;
   const int64_t per = fricc_cdiv(nch, 1024);
   const int64_t c0 = threadIdx.x * per;
   const int64_t c1 = c0 + per < nch ? c0 + per : nch;
@@ -391,13 +636,20 @@ static __global__ void __launch_bounds__(1024) k_classify(const double* csum, Le
       const int b_lo = binade_of(lo), b_hi = binade_of(hi);
       if (b_lo == b_hi) b = b_lo;
     }
+    if (b == 0 && slots && !sub) {
+      const int k = atomicAdd(&used, 1);
+      if (k < SLOTS) b = -(k + 1);
+      csum[c] = P0;
+    }
     cbin[c] = b;
   }
 }
 
-// K_C: composite map of each clean chunk under its predicted binade.
+// K_C: composite map of each clean chunk under its predicted binade; the
+// pieces of the others.
 template <class Gen>
-__global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, const int* cbin, Map* cmap) {
+__global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, const int* cbin, Map* cmap,
+                                                    const double* csum, Slots* slots) {
   constexpr int NT = 256, ITEMS = CH / NT;
   const int rep = blockIdx.y;
   const int64_t len = ln.get(rep);
@@ -408,8 +660,27 @@ __global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, c
   cbin += (int64_t)rep * cap;
   cmap += (int64_t)rep * cap;
   __shared__ Map smaps[33];
+  __shared__ SplitSmem ssm;
   const int b = cbin[blockIdx.x];
   if (b == 0) return;  // uniform per block
+  if (b < 0) {
+    const int n_in = (int)(len - base < CH ? len - base : CH);
+    double a[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int i = threadIdx.x * ITEMS + k;
+      a[k] = i < n_in ? gen(base + i) : 0.0;
+    }
+    Seg pre;
+    unsigned cuts;
+    slots += rep;
+    // the chain's own rounding: half a unit per element; the prediction's: a
+    // unit per addition of its trees
+    const int cnt = split_chunk<NT, ITEMS>(a, n_in, csum[rep * cap + blockIdx.x], base + n_in + cap / 256 + 256, ssm,
+                                           slots->p[-b - 1], pre, cuts);
+    if (threadIdx.x == 0) slots->cnt[-b - 1] = cnt;
+    return;
+  }
   Map agg = map_id();
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
@@ -421,13 +692,17 @@ __global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, c
   if (threadIdx.x == 0) cmap[blockIdx.x] = tot;
 }
 
+// Up to this many chunks one thread applies their maps one after another
+// (~0.1 us each), where a block scan per binade takes ~4 us.
+constexpr int WALK_SERIAL = 256;
+
 // K_D (one block of 1024): the exact chain over chunks.  cstart[c] receives
 // the exact running value at the start of chunk c, cstart[nch] the total,
 // which also goes to *end (if given).
 template <class Gen>
 __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s_init_dev, int sub,
-                                               const int* cbin, const Map* cmap, double* cstart, double* end,
-                                               int64_t end_stride, ChainStride cs) {
+                                               const int* cbin, const Map* cmap, const Slots* slots, double* cstart,
+                                               double* end, int64_t end_stride, ChainStride cs) {
   const int rep = blockIdx.x;
   const int64_t len = ln.get(rep);
   const Gen gen = replica_of(gen0, rep);
@@ -436,22 +711,54 @@ __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s
     cbin += st;
     cmap += st;
     cstart += st;
+    slots += rep;
   }
   const double s_init = s_init_dev[rep * cs.s_init];
   constexpr int NT = 1024;
   __shared__ Map smaps[33];
   __shared__ int simin[32];
   __shared__ ChunkSmem csm;
+  __shared__ Map cm[WALK_SERIAL];
+  __shared__ int cb[WALK_SERIAL], cnext;
   const int64_t nch = fricc_cdiv(len, CH);
+  const bool serial = nch <= WALK_SERIAL;
   double s = s_init;
   int64_t c = 0;
+  if (serial) {
+    for (int k = threadIdx.x; k < (int)nch; k += NT) {
+      cb[k] = cbin[k];
+      if (cb[k] > 0) cm[k] = cmap[k];
+    }
+    __syncthreads();
+  }
   for (int64_t guard = 0; guard <= 2 * nch && c < nch; ++guard) {
     if (sub && !(s > SUB_STOP)) break;
+    if (serial) {
+      if (threadIdx.x == 0) {
+        double v = s;
+        int k = (int)c;
+        for (; k < (int)nch && cb[k] > 0 && !(sub && !(v > SUB_STOP)); ++k) {
+          const int b = binade_of(v);
+          if (cb[k] != b) break;
+          const int64_t n = apply(cm[k], n_of(v, b));
+          if (!run_valid(n, b, sub != 0)) break;
+          cstart[k] = v;
+          v = s_of(b, n);
+        }
+        csm.s = v;
+        cnext = k;
+      }
+      __syncthreads();
+      s = csm.s;
+      c = cnext;
+      __syncthreads();
+      if (c == nch || (sub && !(s > SUB_STOP))) break;
+    }
     const int b = binade_of(s);
     const int64_t n0 = n_of(s, b);
     const int64_t ct = c + threadIdx.x;
-    const bool ok = ct < nch && cbin[ct] == b;
-    const int L = block_min<int>(ok ? INT_MAX : (int)threadIdx.x, simin);
+    const bool ok = !serial && ct < nch && cbin[ct] == b;
+    const int L = serial ? 0 : block_min<int>(ok ? INT_MAX : (int)threadIdx.x, simin);
     if (L > 0) {
       const Map mine = (ok && (int)threadIdx.x < L) ? cmap[ct] : map_id();
       Map tot;
@@ -475,6 +782,25 @@ __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s
       }
     }
     if (threadIdx.x == 0) cstart[c] = s;
+    const int slot = -cbin[c] - 1, cnt = slot >= 0 ? slots->cnt[slot] : 0;
+    if (cnt > 0) {
+      if ((int)threadIdx.x < cnt) csm.split.p[threadIdx.x] = slots->p[slot][threadIdx.x];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double v = s;
+        csm.split.ok = walk_pieces(csm.split.p, cnt, v, nullptr);
+        csm.s = v;
+      }
+      __syncthreads();
+      const bool done = csm.split.ok != 0;
+      const double v = csm.s;
+      __syncthreads();
+      if (done) {
+        s = v;
+        c += 1;
+        continue;
+      }
+    }
     const int64_t base = c * CH;
     const int n_in = (int)(len - base < CH ? len - base : CH);
     ConsNull none;
@@ -511,7 +837,9 @@ struct ChainScratch {
   int* cbin = nullptr;
   Map* cmap = nullptr;
   double* cstart = nullptr;
+  Slots* slots = nullptr;  // one per replica
   int64_t cap = 0;
+  int reps = 0;
 };
 
 // Runs the chain over gen(0..len-1) from s_init.  On return (stream order)
@@ -519,7 +847,13 @@ struct ChainScratch {
 // (device, end_stride doubles per replica) when given; with EMIT, cons has
 // seen every element.  have_sums: sc.csum already holds the chunk sums (a
 // kernel that made the addends summed them in the same pass).
-inline int chain_scratch(ChainScratch& sc, int64_t entries, cudaStream_t st) {
+inline int chain_scratch(ChainScratch& sc, int64_t entries, cudaStream_t st, int reps = 1) {
+  if (sc.reps < reps) {
+    fricc_free(sc.slots, st);
+    sc.reps = 0;
+    if (int rc = fricc_alloc_t(&sc.slots, reps, st)) return rc;
+    sc.reps = reps;
+  }
   if (sc.cap >= entries) return FRICC_OK;
   fricc_free(sc.csum, st);
   fricc_free(sc.cbin, st);
@@ -540,7 +874,7 @@ int run_chain(const Gen& gen, const Len& len, const double* s_init_dev, bool sub
   const int64_t nch = fricc_cdiv(len.n, CH);
   if (nch > INT_MAX / 2 || R < 1 || R > 65535) return FRICC_ERR_ARG;
   if (R > 1) {  // the batch's scratch: nch + 1 entries per replica, sized by the caller
-    if (sc.cap < R * (nch + 1)) return FRICC_ERR_ARG;
+    if (sc.cap < R * (nch + 1) || sc.reps < R) return FRICC_ERR_ARG;
     if (nch == 0) return FRICC_ERR_ARG;
   } else if (int rc = chain_scratch(sc, nch + 1, st)) {
     return rc;
@@ -552,9 +886,10 @@ int run_chain(const Gen& gen, const Len& len, const double* s_init_dev, bool sub
   }
   const dim3 gch((unsigned)nch, (unsigned)R);
   if (!have_sums) k_chunk_sums<Gen><<<gch, 256, 0, st>>>(gen, len, sc.csum);
-  k_classify<<<R, 1024, 0, st>>>(sc.csum, len, s_init_dev, sub ? 1 : 0, sc.cbin, cs);
-  k_chunk_maps<Gen><<<gch, 256, 0, st>>>(gen, len, sub ? 1 : 0, sc.cbin, sc.cmap);
-  k_walk<Gen><<<R, 1024, 0, st>>>(gen, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.cmap, sc.cstart, end, end_stride, cs);
+  k_classify<<<R, 1024, 0, st>>>(sc.csum, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.slots != nullptr, cs);
+  k_chunk_maps<Gen><<<gch, 256, 0, st>>>(gen, len, sub ? 1 : 0, sc.cbin, sc.cmap, sc.csum, sc.slots);
+  k_walk<Gen><<<R, 1024, 0, st>>>(gen, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.cmap, sc.slots, sc.cstart, end,
+                                  end_stride, cs);
   if (EMIT) k_emit<Gen, Cons><<<gch, 512, 0, st>>>(gen, cons, len, sub ? 1 : 0, sc.cstart);
   fricc_note_launch(3 + (have_sums ? 0 : 1) + (EMIT ? 1 : 0));
   FRICC_LAUNCH_CHECK();
@@ -566,6 +901,7 @@ inline void free_chain(ChainScratch& sc, cudaStream_t st) {
   fricc_free(sc.cbin, st);
   fricc_free(sc.cmap, st);
   fricc_free(sc.cstart, st);
+  fricc_free(sc.slots, st);
   sc = ChainScratch{};
 }
 

@@ -13,7 +13,7 @@
 // * n <= FRICC_NOALLOC_MAX_N (2^26 = 67,108,864 elements, the largest
 //   amplitude tensor of the o40v200 workload); larger n is rejected with
 //   FRICC_ERR_ARG before any device work.
-// * The scratch array (about 0.6 MB) is held by every GPU that loads the
+// * The scratch array (about 0.7 MB) is held by every GPU that loads the
 //   library, until the process exits.
 // * The first call on a device looks up the array's device address for
 //   that device (cudaGetSymbolAddress, once per device, with that device
@@ -41,7 +41,8 @@ constexpr size_t kOffCsum = 256;
 constexpr size_t kOffCbin = kOffCsum + align256(kMaxChunks * sizeof(double));
 constexpr size_t kOffCmap = kOffCbin + align256(kMaxChunks * sizeof(int));
 constexpr size_t kOffCstart = kOffCmap + align256(kMaxChunks * sizeof(exact::Map));
-constexpr size_t kScratchBytes = kOffCstart + align256(kMaxChunks * sizeof(double));
+constexpr size_t kOffSlots = kOffCstart + align256(kMaxChunks * sizeof(double));
+constexpr size_t kScratchBytes = kOffSlots + align256(sizeof(exact::Slots));
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -108,6 +109,8 @@ extern "C" int fricc_seq_cumsum_noalloc(const double* x, int64_t n, double* out,
   sc.cbin = reinterpret_cast<int*>(base + kOffCbin);
   sc.cmap = reinterpret_cast<exact::Map*>(base + kOffCmap);
   sc.cstart = reinterpret_cast<double*>(base + kOffCstart);
+  sc.slots = reinterpret_cast<exact::Slots*>(base + kOffSlots);
+  sc.reps = 1;
   sc.cap = kMaxChunks;  // run_chain allocates only when cap is too small; it never is here
   return exact::run_chain<GenAbsNA, ConsWriteNA, true>(GenAbsNA{x}, exact::Len{n}, dzero, false, ConsWriteNA{out}, sc,
                                                        st);

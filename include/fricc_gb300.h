@@ -418,7 +418,7 @@ int fricc_seq_cumsum(const double* x, int64_t n, double* out, void* stream);
  * (an application whose device memory is reserved up front by its own
  * allocator, or a latency-critical loop that must not enter the CUDA
  * allocator).  No counterpart in the reference.  It allocates nothing: its
- * scratch (about 0.6 MB) is a fixed array inside the library, held by every
+ * scratch (about 0.7 MB) is a fixed array inside the library, held by every
  * GPU that loads it until exit.  n <= 2^26 (67,108,864), larger n fails
  * with FRICC_ERR_ARG.  The first call on a device looks up the array's
  * address for that device; make it before any stream capture begins.  All
