@@ -97,6 +97,40 @@ __global__ void __launch_bounds__(256) k_hist_sums(const double* __restrict__ x,
 }
 
 // Values decided on the device between the phases of one compression.
+// fl(a / R) for many a and one R without FP64 divisions (~10 dependent FP64
+// instructions each, at 2 per SM and clock: most of the 503 us that 20 M
+// probabilities took; now 180).  With the 53-bit significands ma, mr and V =
+// floor(2^116 / mr), Q = floor(2^11 ma V / 2^64) lies at most 2 below
+// 2^63 ma / mr, a number of 63 or 64 bits: where the 10 or 11 bits to be rounded
+// off are not within 3 of the halfway case, the nearest double follows from Q;
+// else (0.3%) from comparing ma 2^63 with that case times mr.  What is not normal
+// takes the division.
+__device__ __forceinline__ unsigned long long recip_word(double R) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(R);
+  const unsigned e = (unsigned)(u >> 52);
+  if (e < 1 || e > 2046) return 0;  // zero, subnormal, negative, infinite or NaN
+  const unsigned long long mr = (u & 0xfffffffffffffull) | (1ull << 52);
+  return mr == 1ull << 52 ? ~0ull : (unsigned long long)(((unsigned __int128)1 << 116) / mr);
+}
+__device__ __forceinline__ double div_by(double a, double R, unsigned long long rv) {  // a >= 0 or NaN
+  const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+  const int ea = (int)(u >> 52), e = ea - (int)((unsigned long long)__double_as_longlong(R) >> 52) + 1023;
+  const unsigned long long ma = (u & 0xfffffffffffffull) | (1ull << 52), q = __umul64hi(ma << 11, rv);
+  const int drop = 10 + (int)(q >> 63);  // bits to round off
+  const unsigned low = (unsigned)q & ((1u << drop) - 1), half = 1u << (drop - 1);
+  bool up = low > half;
+  if (low - (half - 3) <= 3u) {
+    const unsigned long long mr = ((unsigned long long)__double_as_longlong(R) & 0xfffffffffffffull) | (1ull << 52);
+    const unsigned long long h = (q & ~((1ull << drop) - 1)) + half, hi = __umul64hi(h, mr), lo = h * mr;
+    const unsigned long long t_hi = ma >> 1, t_lo = ma << 63;
+    up = t_hi > hi || (t_hi == hi && (t_lo > lo || (t_lo == lo && ((q >> drop) & 1))));
+  }
+  // (the significand's leading bit adds one to the exponent)
+  const double r = __longlong_as_double((long long)(((unsigned long long)(e - 12 + drop) << 52) + (q >> drop) + up));
+  if (rv != 0 && ea >= 1 && ea <= 2046 && e >= 3 && e <= 2044) return r;
+  return u == 0 && rv != 0 ? 0.0 : __ddiv_rn(a, R);
+}
+
 struct Ctl {
   int64_t dmin;       // first select digit kept as a candidate
   int64_t ncand;      // candidates (every element at or above dmin)
@@ -108,6 +142,7 @@ struct Ctl {
   unsigned long long dkey;  // |x| bits of the last element of D
   int64_t didx;       // its index (-1: D is empty)
   double R;           // remaining norm
+  unsigned long long rv;  // recip_word(R)
   double mprime;      // (double)(m - |D|)
   int sample;         // 1: R > 0 and finite, so samples can land in intervals
   double rn;          // the uniform draw
@@ -252,7 +287,7 @@ struct GenP {
     const unsigned long long k = abs_key(a);
     const int64_t didx = c->didx;
     if (didx >= 0 && (k > c->dkey || (k == c->dkey && i <= didx))) return 0.0;
-    const double p = __dmul_rn(__ddiv_rn(a, c->R), c->mprime);
+    const double p = __dmul_rn(div_by(a, c->R, c->rv), c->mprime);
     // with R <= 0 or not finite no sample can land anywhere: feed the exact
     // chain zeros (NaN addends would only slow it down), but keep any p > 1
     // visible to the check of make_probability_vector
@@ -263,7 +298,7 @@ struct GenP {
     const unsigned long long k = abs_key(a);
     const int64_t didx = c->didx;
     if (didx >= 0 && (k > c->dkey || (k == c->dkey && i <= didx))) return 0.0;
-    return __dmul_rn(__ddiv_rn(a, c->R), c->mprime);
+    return __dmul_rn(div_by(a, c->R, c->rv), c->mprime);
   }
 };
 
@@ -464,6 +499,7 @@ __device__ __forceinline__ void set_d(Ctl* c, int64_t nd, double R, const unsign
                                       const unsigned* cidx, int64_t m) {
   c->nd = nd;
   c->mp = m - nd;
+  c->rv = recip_word(R);
   c->mprime = (double)(unsigned long long)(m - nd);
   c->R = R;
   c->dkey = nd > 0 ? ckey[nd - 1] : 0ull;
@@ -642,8 +678,7 @@ constexpr unsigned char PV_TAKE = 1, PV_EMIT = 2, PV_PIVOT = 4;
 
 // P = the p vector, with the p > 1 check and (psum, zeroed beforehand) the
 // approximate sum of each exact::CH chunk of the addends its chain takes.
-// Four blocks share a chunk, so that a small tensor's divisions (FP64, ~12
-// slow instructions each) spread over the chip.
+// Four blocks share a chunk, so that a small tensor's spread over the chip.
 constexpr int PV_SUB = 4;
 __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __restrict__ P, unsigned* err,
                                               double* __restrict__ psum, Rep rp = Rep{}) {
@@ -661,7 +696,9 @@ __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __res
     if (i < n) {
       const double p = gp.value(i);
       P[i] = p;
-      bad |= p > 1.0;
+      // p > 1, by its bits (a comparison is an FP64 instruction)
+      const long long u = __double_as_longlong(p);
+      bad |= u > 0x3ff0000000000000ll && u <= 0x7ff0000000000000ll;
       acc += p;
     }
   }
