@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_hist_sums(const double* __restrict__ x,
     for (int r = 0; r < exact::CH / 256; ++r) {
       const int64_t i = base + r * 256 + threadIdx.x;
       if (i < n) atomicAdd(&h[abs_key(v[r]) >> shift], 1u);
-      acc += fabs(v[r]);
+      acc += exact::abs_bits(v[r]);
     }
     if (csum) {
       const double tot = block_sum_det(acc, red);
@@ -96,10 +96,9 @@ __global__ void __launch_bounds__(256) k_hist_sums(const double* __restrict__ x,
     if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-// Values decided on the device between the phases of one compression.
 // fl(a / R) for many a and one R without FP64 divisions (~10 dependent FP64
 // instructions each, at 2 per SM and clock: most of the 503 us that 20 M
-// probabilities took; now 180).  With the 53-bit significands ma, mr and V =
+// probabilities took; now 153).  With the 53-bit significands ma, mr and V =
 // floor(2^116 / mr), Q = floor(2^11 ma V / 2^64) lies at most 2 below
 // 2^63 ma / mr, a number of 63 or 64 bits: where the 10 or 11 bits to be rounded
 // off are not within 3 of the halfway case, the nearest double follows from Q;
@@ -131,6 +130,7 @@ __device__ __forceinline__ double div_by(double a, double R, unsigned long long 
   return u == 0 && rv != 0 ? 0.0 : __ddiv_rn(a, R);
 }
 
+// Values decided on the device between the phases of one compression.
 struct Ctl {
   int64_t dmin;       // first select digit kept as a candidate
   int64_t ncand;      // candidates (every element at or above dmin)
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) k_compact(const double* __restrict__ x, i
 struct GenAbs {
   const double* x;
   int64_t rs = 0;  // replica stride of x
-  __device__ __forceinline__ double operator()(int64_t i) const { return fabs(x[i]); }
+  __device__ __forceinline__ double operator()(int64_t i) const { return exact::abs_bits(x[i]); }
   __device__ __forceinline__ GenAbs at(int r) const { return GenAbs{x + r * rs, rs}; }
 };
 
@@ -283,7 +283,7 @@ struct GenP {
   int64_t rs = 0, cs = 0;  // replica strides of x and c
   __device__ __forceinline__ GenP at(int r) const { return GenP{x + r * rs, c + r * cs, rs, cs}; }
   __device__ __forceinline__ double operator()(int64_t i) const {
-    const double a = fabs(x[i]);
+    const double a = exact::abs_bits(x[i]);
     const unsigned long long k = abs_key(a);
     const int64_t didx = c->didx;
     if (didx >= 0 && (k > c->dkey || (k == c->dkey && i <= didx))) return 0.0;
@@ -294,7 +294,7 @@ struct GenP {
     return (c->sample || p > 1.0) ? p : 0.0;
   }
   __device__ __forceinline__ double value(int64_t i) const {  // the reference's p_i itself
-    const double a = fabs(x[i]);
+    const double a = exact::abs_bits(x[i]);
     const unsigned long long k = abs_key(a);
     const int64_t didx = c->didx;
     if (didx >= 0 && (k > c->dkey || (k == c->dkey && i <= didx))) return 0.0;
@@ -396,6 +396,25 @@ struct ConsSample {
     }
     return count_below(I, rn, mp);
   }
+  // the next sample and where it lies, u_k = fl(k + rn) >= 0, as bits
+  struct Run {
+    int64_t k;
+    long long u;
+  };
+  __device__ __forceinline__ bool runs() const { return ok == 2; }
+  __device__ __forceinline__ long long place(int64_t k) const {
+    return k < mp ? __double_as_longlong(__dadd_rn((double)k, rn)) : LLONG_MAX;
+  }
+  __device__ __forceinline__ Run start(double s) const {
+    const int64_t k = count(s);
+    return Run{k, place(k)};
+  }
+  __device__ __forceinline__ void step(Run& r, int64_t j, double s) const {
+    while (r.u < __double_as_longlong(s)) {
+      S[r.k] = (unsigned)j;
+      r.u = place(++r.k);
+    }
+  }
   __device__ __forceinline__ void operator()(int64_t j, double lo, double hi, double p) const {
     const long long pb = __double_as_longlong(p);
     if (!ok || !(pb > 0 && pb <= 0x7ff0000000000000ll)) return;  // p > 0
@@ -410,6 +429,15 @@ struct ConsSample {
 struct ConsSample2 {
   ConsSample a, b;
   __device__ __forceinline__ ConsSample2 at(int r) const { return ConsSample2{a.at(r), b.at(r)}; }
+  struct Run {
+    ConsSample::Run a, b;
+  };
+  __device__ __forceinline__ bool runs() const { return a.runs() && b.runs(); }
+  __device__ __forceinline__ Run start(double s) const { return Run{a.start(s), b.start(s)}; }
+  __device__ __forceinline__ void step(Run& r, int64_t j, double s) const {
+    a.step(r.a, j, s);
+    b.step(r.b, j, s);
+  }
   __device__ __forceinline__ void operator()(int64_t j, double lo, double hi, double p) const {
     a(j, lo, hi, p);
     b(j, lo, hi, p);

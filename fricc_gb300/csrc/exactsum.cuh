@@ -128,6 +128,27 @@ __device__ __forceinline__ Map elem_map(double a, int b, bool sub) {
   return map_of(q, cls, sub);
 }
 
+// |x| by its bits: fabs is an FP64 instruction
+__device__ __forceinline__ double abs_bits(double x) {
+  return __longlong_as_double(__double_as_longlong(x) & 0x7fffffffffffffffll);
+}
+
+// a >= 0 rounded to units of binade b, where no tie leaves the direction to the
+// parity and a is below the binade: the map is then the same for both parities, a
+// run's is the sum, and a third of the instructions suffice (they bound every
+// pass: the maps of 20 M addends took 105 us at 82% of the integer pipe, the
+// sampling pass 280; now 77-91 and 149).
+__device__ __forceinline__ bool plain_step(double a, int b, int64_t& r) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+  const int ef = (int)(u >> 52) & 0x7ff;
+  const unsigned long long M = (u & 0xfffffffffffffull) | (ef ? 1ull << 52 : 0ull);
+  const int shift = b - (ef ? ef : 1) - 1;  // M 2^-shift: halves of a unit
+  const int sh = shift < 0 ? 0 : (shift > 63 ? 63 : shift);
+  const unsigned long long h = M >> sh;
+  r = (int64_t)((h + 1) >> 1);
+  return shift >= 0 && !((h & 1) && (h << sh) == M);
+}
+
 // One step of the model from n, with exactness check.
 __device__ __forceinline__ bool step(int64_t n, double a, int b, bool sub, int64_t& n_out) {
   int64_t q;
@@ -237,7 +258,7 @@ struct SplitSmem {
   int seg[33], cnt[33];  // a segment's binade | CUT once a cut lies in the range
   int ok;
 };
-constexpr int CUT = 1 << 16;
+constexpr int CUT = 1 << 16, CLASH = 1 << 17;  // CLASH: two binades in one segment
 
 struct Seg {
   Map m;
@@ -247,7 +268,9 @@ struct Seg {
 __device__ __forceinline__ Seg then(const Seg& x, const Seg& y) {
   Seg r;
   r.m = (y.f & CUT) ? y.m : compose(x.m, y.m);
-  r.f = (y.f & CUT) ? y.f : (y.f ? (x.f & CUT) | y.f : x.f);
+  const int bx = x.f & 0xffff, by = y.f & 0xffff;
+  r.f = (y.f & CUT) ? y.f | (x.f & CLASH)
+                    : ((x.f | y.f) & (CUT | CLASH)) | (by ? by : bx) | (bx && by && bx != by ? CLASH : 0);
   r.n = x.n + y.n;
   return r;
 }
@@ -267,6 +290,50 @@ struct ChunkSmem {
   SplitSmem split;
 };
 
+// Exclusive scan of segments in thread order; the whole goes to entry NT / 32 of
+// sm's arrays.
+template <int NT>
+__device__ __forceinline__ Seg block_scan_seg(const Seg& mine, SplitSmem& sm) {
+  constexpr int NW = NT / 32;
+  const int lane = (int)lane_id(), warp = (int)warp_id();
+  Seg inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Seg w = seg_up(inc, o);
+    if (lane >= o) inc = then(w, inc);
+  }
+  Seg wex = seg_up(inc, 1);
+  if (lane == 0) wex = Seg{map_id(), 0, 0};
+  if (lane == 31) {
+    sm.m[warp] = inc.m;
+    sm.seg[warp] = inc.f;
+    sm.cnt[warp] = inc.n;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    Seg run = lane < NW ? Seg{sm.m[lane], sm.seg[lane], sm.cnt[lane]} : Seg{map_id(), 0, 0};
+#pragma unroll
+    for (int o = 1; o < NW; o <<= 1) {
+      const Seg w = seg_up(run, o);
+      if (lane >= o) run = then(w, run);
+    }
+    Seg e = seg_up(run, 1);
+    if (lane == 0) e = Seg{map_id(), 0, 0};
+    if (lane < NW) {
+      sm.m[lane] = e.m;
+      sm.seg[lane] = e.f;
+      sm.cnt[lane] = e.n;
+    }
+    if (lane == NW - 1) {
+      sm.m[NW] = run.m;
+      sm.seg[NW] = run.f;
+      sm.cnt[NW] = run.n;
+    }
+  }
+  __syncthreads();
+  return then(Seg{sm.m[warp], sm.seg[warp], sm.cnt[warp]}, wex);
+}
+
 // Cuts a chunk of additions (element t ITEMS + k at thread t's a[k]) that
 // starts at about P0, `slack` units of its last place off at most, and writes
 // the pieces to out.  An element is a cut unless the approximate values before
@@ -277,7 +344,7 @@ struct ChunkSmem {
 // 2 FP64 numbers per SM and clock.  Bound by its dependent steps: ~25 us, where a
 // round per crossing (scan, search, one addition) took 4-9 us each and a first
 // chunk has a dozen (compressing o10v40's 160000 elements: the two walks 319 ->
-// 50 us, the sampling pass 130 -> 37, the chunk maps 17 -> 62; 613 -> 292 in all).
+// 28 us, the sampling pass 130 -> 37, the chunk maps 17 -> 41).
 template <int NT, int ITEMS>
 __device__ __forceinline__ int split_chunk(const double* a, int n_in, double P0, int64_t slack, SplitSmem& sm, Piece* out,
                                            Seg& pre, unsigned& cuts) {
@@ -337,47 +404,12 @@ __device__ __forceinline__ int split_chunk(const double* a, int n_in, double P0,
       p = q;
     }
   }
-  Seg inc = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const Seg w = seg_up(inc, o);
-    if (lane >= o) inc = then(w, inc);
-  }
-  Seg wex = seg_up(inc, 1);
-  if (lane == 0) wex = Seg{map_id(), 0, 0};
-  if (lane == 31) {
-    sm.m[warp] = inc.m;
-    sm.seg[warp] = inc.f;
-    sm.cnt[warp] = inc.n;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    Seg run = lane < NW ? Seg{sm.m[lane], sm.seg[lane], sm.cnt[lane]} : Seg{map_id(), 0, 0};
-#pragma unroll
-    for (int o = 1; o < NW; o <<= 1) {
-      const Seg w = seg_up(run, o);
-      if (lane >= o) run = then(w, run);
-    }
-    Seg e = seg_up(run, 1);
-    if (lane == 0) e = Seg{map_id(), 0, 0};
-    if (lane < NW) {
-      sm.m[lane] = e.m;
-      sm.seg[lane] = e.f;
-      sm.cnt[lane] = e.n;
-    }
-    if (lane == NW - 1) {
-      sm.m[NW] = run.m;
-      sm.seg[NW] = run.f;
-      sm.cnt[NW] = run.n;
-    }
-  }
-  __syncthreads();
-  pre = then(Seg{sm.m[warp], sm.seg[warp], sm.cnt[warp]}, wex);
+  pre = block_scan_seg<NT>(mine, sm);
   const int total = sm.cnt[NW] + 1;
-  if (total > PIECES) return 0;
+  if (total > PIECES || (sm.seg[NW] & CLASH)) return 0;
   if (cuts) {
     Map m = pre.m;
-    int f = pre.f & ~CUT, j = pre.n;
+    int f = pre.f & 0xffff, j = pre.n;
     p = P;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
@@ -397,7 +429,7 @@ __device__ __forceinline__ int split_chunk(const double* a, int n_in, double P0,
       }
     }
   }
-  if (t == 0) out[total - 1] = Piece{sm.m[NW], 0.0, sm.seg[NW] & ~CUT, 1};
+  if (t == 0) out[total - 1] = Piece{sm.m[NW], 0.0, sm.seg[NW] & 0xffff, 1};
   return total;
 }
 
@@ -412,6 +444,14 @@ template <class C, class = void>
 struct has_finish : std::false_type {};
 template <class C>
 struct has_finish<C, std::void_t<decltype(std::declval<C&>().finish())>> : std::true_type {};
+
+// A consumer that only looks for values the running sum passes has start(s), the
+// state at a thread's first element, and step(state, i, s), the sum after element i
+// (repeated past the chunk's end); runs() says whether they can be used.
+template <class C, class = void>
+struct has_run : std::false_type {};
+template <class C>
+struct has_run<C, std::void_t<decltype(std::declval<const C&>().runs())>> : std::true_type {};
 
 // A chain's length: n elements, or (dev) the count at dev[rep * stride],
 // never above n; nothing at all where the word skip[rep * sstride] is set.
@@ -457,11 +497,24 @@ __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, doub
     }
     const int b = binade_of(s);
     const int64_t n0 = n_of(s, b);
-    Map agg = map_id();
+    bool plain = b < 2047;
+    int64_t sum = 0;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       const int i = t * ITEMS + k;
-      if (i >= p && i < n_in) agg = compose(agg, elem_map(a[k], b, sub));
+      int64_t r;
+      plain &= plain_step(i >= p ? a[k] : 0.0, b, r);  // (zeros past n_in)
+      sum += r;
+    }
+    if (sub) sum = -sum;
+    Map agg{sum, sum};
+    if (!plain) {
+      agg = map_id();
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = t * ITEMS + k;
+        if (i >= p && i < n_in) agg = compose(agg, elem_map(a[k], b, sub));
+      }
     }
     Map tot;
     const Map pre = block_excl_scan_map<NT>(agg, sm.maps, &tot);
@@ -527,14 +580,31 @@ __device__ double block_exact_chunk(const Gen& gen, int64_t base, int n_in, doub
       istar = block_min<int>(first_bad, sm.imin);
       n = apply(pre, n0);
     }
+    bool done = false;
+    if constexpr (has_run<Cons>::value) {
+      if (plain && istar == INT_MAX && cons.runs()) {
+        auto run = cons.start(s_of(b, n));
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const int i = t * ITEMS + k;
-      if (i >= p && i < n_in && i < istar) {
-        int64_t nn;
-        step(n, a[k], b, sub, nn);
-        cons(base + i, s_of(b, n), s_of(b, nn), a[k]);
-        n = nn;
+        for (int k = 0; k < ITEMS; ++k) {
+          const int i = t * ITEMS + k;
+          int64_t r;
+          plain_step(i >= p ? a[k] : 0.0, b, r);
+          n += sub ? -r : r;
+          cons.step(run, base + i, s_of(b, n));
+        }
+        done = true;
+      }
+    }
+    if (!done) {
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = t * ITEMS + k;
+        if (i >= p && i < n_in && i < istar) {
+          int64_t nn;
+          step(n, a[k], b, sub, nn);
+          cons(base + i, s_of(b, n), s_of(b, nn), a[k]);
+          n = nn;
+        }
       }
     }
     if (istar == INT_MAX) {
@@ -585,7 +655,7 @@ __global__ void __launch_bounds__(256) k_chunk_sums(Gen gen0, Len ln, double* cs
 // additions, ~55 ns each on this part) took 58 us a call, three calls a
 // compression; now 4-5 us.
 static __global__ void __launch_bounds__(1024) k_classify(double* csum, Len ln, const double* s_init_dev,
-                                                   int sub, int* cbin, int slots, ChainStride cs) {
+                                                   int sub, int* cbin, ChainStride cs) {
   const int rep = blockIdx.x;
   const int64_t nch = fricc_cdiv(ln.get(rep), CH), cap = fricc_cdiv(ln.n, CH) + 1;
   csum += (int64_t)rep * cap;
@@ -636,7 +706,7 @@ static __global__ void __launch_bounds__(1024) k_classify(double* csum, Len ln, 
       const int b_lo = binade_of(lo), b_hi = binade_of(hi);
       if (b_lo == b_hi) b = b_lo;
     }
-    if (b == 0 && slots && !sub) {
+    if (b == 0 && !sub) {
       const int k = atomicAdd(&used, 1);
       if (k < SLOTS) b = -(k + 1);
       csum[c] = P0;
@@ -663,14 +733,14 @@ __global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, c
   __shared__ SplitSmem ssm;
   const int b = cbin[blockIdx.x];
   if (b == 0) return;  // uniform per block
-  if (b < 0) {
-    const int n_in = (int)(len - base < CH ? len - base : CH);
-    double a[ITEMS];
+  const int n_in = (int)(len - base < CH ? len - base : CH);
+  double a[ITEMS];
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const int i = threadIdx.x * ITEMS + k;
-      a[k] = i < n_in ? gen(base + i) : 0.0;
-    }
+  for (int k = 0; k < ITEMS; ++k) {
+    const int i = threadIdx.x * ITEMS + k;
+    a[k] = i < n_in ? gen(base + i) : 0.0;
+  }
+  if (b < 0) {
     Seg pre;
     unsigned cuts;
     slots += rep;
@@ -681,24 +751,34 @@ __global__ void __launch_bounds__(256) k_chunk_maps(Gen gen0, Len ln, int sub, c
     if (threadIdx.x == 0) slots->cnt[-b - 1] = cnt;
     return;
   }
-  Map agg = map_id();
+  bool plain = true;
+  int64_t sum = 0;
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
-    const int64_t i = base + threadIdx.x * ITEMS + k;
-    if (i < len) agg = compose(agg, elem_map(gen(i), b, sub != 0));
+    int64_t r;
+    plain &= plain_step(a[k], b, r);
+    sum += r;
+  }
+  if (sub) sum = -sum;
+  Map agg{sum, sum};
+  if (!plain) {
+    agg = map_id();
+#pragma unroll 1
+    for (int k = 0; k < ITEMS; ++k) {
+      const int64_t i = base + threadIdx.x * ITEMS + k;
+      if (i < len) agg = compose(agg, elem_map(gen(i), b, sub != 0));
+    }
   }
   Map tot;
   block_excl_scan_map<NT>(agg, smaps, &tot);
   if (threadIdx.x == 0) cmap[blockIdx.x] = tot;
 }
 
-// Up to this many chunks one thread applies their maps one after another
-// (~0.1 us each), where a block scan per binade takes ~4 us.
-constexpr int WALK_SERIAL = 256;
-
 // K_D (one block of 1024): the exact chain over chunks.  cstart[c] receives
 // the exact running value at the start of chunk c, cstart[nch] the total,
-// which also goes to *end (if given).
+// which also goes to *end (if given).  The loop over runs of chunks takes the
+// chains of subtractions, and an addition's from where a prediction fails.
+constexpr int WALK_Q = 256;  // pieces of all cut chunks
 template <class Gen>
 __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s_init_dev, int sub,
                                                const int* cbin, const Map* cmap, const Slots* slots, double* cstart,
@@ -718,47 +798,93 @@ __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s
   __shared__ Map smaps[33];
   __shared__ int simin[32];
   __shared__ ChunkSmem csm;
-  __shared__ Map cm[WALK_SERIAL];
-  __shared__ int cb[WALK_SERIAL], cnext;
+  __shared__ Piece q[WALK_Q];
+  __shared__ int64_t cut[PIECES], cfail;
+  __shared__ int off[SLOTS + 1];
   const int64_t nch = fricc_cdiv(len, CH);
-  const bool serial = nch <= WALK_SERIAL;
   double s = s_init;
   int64_t c = 0;
-  if (serial) {
-    for (int k = threadIdx.x; k < (int)nch; k += NT) {
-      cb[k] = cbin[k];
-      if (cb[k] > 0) cm[k] = cmap[k];
+  if (!sub) {  // all chunks at once: the segments between the cut ones by a scan, then one thread
+    SplitSmem& sm = csm.split;
+    const int64_t per = fricc_cdiv(nch, NT), c0 = threadIdx.x * per, c1 = c0 + per < nch ? c0 + per : nch;
+    Seg mine{map_id(), 0, 0};
+    for (int64_t k = c0; k < c1; ++k) {
+      const int b = cbin[k];
+      mine = then(mine, b > 0 ? Seg{cmap[k], b, 0} : Seg{map_id(), CUT, 1});
     }
-    __syncthreads();
+    const Seg pre = block_scan_seg<NT>(mine, sm);
+    const int ncut = sm.cnt[NT / 32];
+    if (ncut < PIECES && !(sm.seg[NT / 32] & CLASH)) {
+      Seg at = pre;
+      for (int64_t k = c0; k < c1; ++k) {
+        const int b = cbin[k];
+        if (b <= 0) {
+          sm.p[at.n] = Piece{at.m, 0.0, at.f & 0xffff, 0};
+          cut[at.n] = k;
+        }
+        at = then(at, b > 0 ? Seg{cmap[k], b, 0} : Seg{map_id(), CUT, 1});
+      }
+      if (threadIdx.x == 0) sm.p[ncut] = Piece{sm.m[NT / 32], 0.0, sm.seg[NT / 32] & 0xffff, 1};
+      // the cut chunks' pieces, slot by slot: a warp each
+      const int slot = (int)warp_id(), used = ncut < SLOTS ? ncut : SLOTS;
+      if (threadIdx.x < 32) {
+        const int v = (int)threadIdx.x < used ? slots->cnt[threadIdx.x] : 0;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int w = __shfl_up_sync(0xffffffffu, incl, o);
+          if ((int)threadIdx.x >= o) incl += w;
+        }
+        off[threadIdx.x + 1] = incl;
+        if (threadIdx.x == 0) off[0] = 0;
+      }
+      __syncthreads();
+      for (int k = (int)lane_id(); k < off[slot + 1] - off[slot]; k += 32)
+        if (off[slot] + k < WALK_Q) q[off[slot] + k] = slots->p[slot][k];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double v = s;
+        int64_t fail = nch;
+        for (int j = 0; j <= ncut; ++j) {
+          const int64_t first = j ? cut[j - 1] + 1 : 0;
+          const double before = v;
+          if (!walk_pieces(&sm.p[j], 1, v, nullptr)) {  // (its real addition is of zero)
+            fail = first;
+            v = before;
+            break;
+          }
+          sm.at[j] = make_double2(before, v);
+          if (j == ncut) break;
+          const int k = -cbin[cut[j]] - 1, o = k >= 0 ? off[k] : 0, cnt = k >= 0 ? off[k + 1] - o : 0;
+          const double at_cut = v;
+          if (cnt == 0 || o + cnt > WALK_Q || !walk_pieces(q + o, cnt, v, nullptr)) {
+            fail = cut[j];
+            v = at_cut;
+            break;
+          }
+        }
+        cfail = fail;
+        csm.s = v;
+      }
+      __syncthreads();
+      at = pre;
+      for (int64_t k = c0; k < c1 && k < cfail; ++k) {
+        const int b = cbin[k];
+        cstart[k] = b > 0 ? s_of(b, apply(at.m, n_of(sm.at[at.n].x, b))) : sm.at[at.n].y;
+        at = then(at, b > 0 ? Seg{cmap[k], b, 0} : Seg{map_id(), CUT, 1});
+      }
+      s = csm.s;
+      c = cfail;
+      __syncthreads();
+    }
   }
   for (int64_t guard = 0; guard <= 2 * nch && c < nch; ++guard) {
     if (sub && !(s > SUB_STOP)) break;
-    if (serial) {
-      if (threadIdx.x == 0) {
-        double v = s;
-        int k = (int)c;
-        for (; k < (int)nch && cb[k] > 0 && !(sub && !(v > SUB_STOP)); ++k) {
-          const int b = binade_of(v);
-          if (cb[k] != b) break;
-          const int64_t n = apply(cm[k], n_of(v, b));
-          if (!run_valid(n, b, sub != 0)) break;
-          cstart[k] = v;
-          v = s_of(b, n);
-        }
-        csm.s = v;
-        cnext = k;
-      }
-      __syncthreads();
-      s = csm.s;
-      c = cnext;
-      __syncthreads();
-      if (c == nch || (sub && !(s > SUB_STOP))) break;
-    }
     const int b = binade_of(s);
     const int64_t n0 = n_of(s, b);
     const int64_t ct = c + threadIdx.x;
-    const bool ok = !serial && ct < nch && cbin[ct] == b;
-    const int L = serial ? 0 : block_min<int>(ok ? INT_MAX : (int)threadIdx.x, simin);
+    const bool ok = ct < nch && cbin[ct] == b;
+    const int L = block_min<int>(ok ? INT_MAX : (int)threadIdx.x, simin);
     if (L > 0) {
       const Map mine = (ok && (int)threadIdx.x < L) ? cmap[ct] : map_id();
       Map tot;
@@ -782,25 +908,6 @@ __global__ void __launch_bounds__(1024) k_walk(Gen gen0, Len ln, const double* s
       }
     }
     if (threadIdx.x == 0) cstart[c] = s;
-    const int slot = -cbin[c] - 1, cnt = slot >= 0 ? slots->cnt[slot] : 0;
-    if (cnt > 0) {
-      if ((int)threadIdx.x < cnt) csm.split.p[threadIdx.x] = slots->p[slot][threadIdx.x];
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double v = s;
-        csm.split.ok = walk_pieces(csm.split.p, cnt, v, nullptr);
-        csm.s = v;
-      }
-      __syncthreads();
-      const bool done = csm.split.ok != 0;
-      const double v = csm.s;
-      __syncthreads();
-      if (done) {
-        s = v;
-        c += 1;
-        continue;
-      }
-    }
     const int64_t base = c * CH;
     const int n_in = (int)(len - base < CH ? len - base : CH);
     ConsNull none;
@@ -886,7 +993,7 @@ int run_chain(const Gen& gen, const Len& len, const double* s_init_dev, bool sub
   }
   const dim3 gch((unsigned)nch, (unsigned)R);
   if (!have_sums) k_chunk_sums<Gen><<<gch, 256, 0, st>>>(gen, len, sc.csum);
-  k_classify<<<R, 1024, 0, st>>>(sc.csum, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.slots != nullptr, cs);
+  k_classify<<<R, 1024, 0, st>>>(sc.csum, len, s_init_dev, sub ? 1 : 0, sc.cbin, cs);
   k_chunk_maps<Gen><<<gch, 256, 0, st>>>(gen, len, sub ? 1 : 0, sc.cbin, sc.cmap, sc.csum, sc.slots);
   k_walk<Gen><<<R, 1024, 0, st>>>(gen, len, s_init_dev, sub ? 1 : 0, sc.cbin, sc.cmap, sc.slots, sc.cstart, end,
                                   end_stride, cs);

@@ -48,7 +48,7 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 struct GenAbsNA {
   const double* x;
-  __device__ __forceinline__ double operator()(int64_t i) const { return fabs(x[i]); }
+  __device__ __forceinline__ double operator()(int64_t i) const { return exact::abs_bits(x[i]); }
 };
 
 struct ConsWriteNA {

@@ -1,7 +1,7 @@
 """The sequential sum where it crosses binades: chunks (4096 addends) cut at the
-crossings, more crossings than a chunk's 64 pieces, addends that land on a
-binade's edge, and chains around the length walked by one thread -- bit for bit
-numpy's left-to-right running sum."""
+crossings, more crossings than a chunk's 64 pieces, more such chunks than the 32
+with pieces, addends that land on a binade's edge, and long chains -- bit for
+bit numpy's left-to-right running sum."""
 import ctypes
 
 import numpy as np
@@ -10,7 +10,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-CH, SERIAL = 4096, 256 * 4096
+CH, LONG = 4096, 1024 * 4096   # elements of a chunk; chunks the walk's threads take one each
 
 
 def _addends(name):
@@ -25,6 +25,8 @@ def _addends(name):
         return np.concatenate([[2.0 ** 20 - 2.0 ** -20], np.full(9000, 2.0 ** -32), rng.random(9000)])
     if name == "ties":                # halves of a unit, odd and even
         return np.concatenate([[2.0 ** 52 - 3000], np.full(2 * CH, 0.5), np.full(2 * CH, 1.5)])
+    if name.startswith("growing"):    # each of that many chunks doubles the sum
+        return 2.0 ** (np.arange(float(int(name[7:]) * CH)) / CH) * rng.random(int(name[7:]) * CH)
     if name == "leading_zeros":
         return np.concatenate([np.zeros(CH + 100), rng.random(6000) * 1e-9, np.zeros(50), rng.random(6000)])
     if name == "subnormal":
@@ -40,9 +42,9 @@ def _addends(name):
     raise KeyError(name)
 
 
-@pytest.mark.parametrize("name", ["doubling", "many_crossings", "on_the_edge", "near_an_edge", "ties", "leading_zeros",
-                                  "subnormal", "to_infinity", "nan", "len1", "len7", f"len{CH - 1}", f"len{CH + 1}",
-                                  f"len{SERIAL}", f"len{SERIAL + 1}"])
+@pytest.mark.parametrize("name", ["doubling", "many_crossings", "on_the_edge", "near_an_edge", "ties",
+                                  "leading_zeros", "growing20", "growing45", "growing100", "subnormal", "to_infinity",
+                                  "nan", "len1", "len7", f"len{CH - 1}", f"len{CH + 1}", f"len{LONG}", f"len{LONG + 1}"])
 def test_sum_across_binades(gpulib, name):
     from fricc_gb300 import _lib
     x = np.ascontiguousarray(_addends(name))
