@@ -292,11 +292,48 @@ def sym_add(out: torch.Tensor, X: torch.Tensor, coef: float = 1.0) -> torch.Tens
     return out
 
 
-def _view5(t: torch.Tensor, shape):
-    """Element strides of ``t`` broadcast to ``shape``, padded to 5 dims."""
-    b = t.expand(*shape) if tuple(t.shape) != tuple(shape) else t
-    st = list(b.stride())
-    return [0] * (5 - len(st)) + st
+def _sig(ts):
+    return tuple((t.shape, t.stride()) for t in ts)
+
+
+def _strides5(shape, stride, to):
+    """Element strides of a (shape, stride) tensor broadcast to ``to``, padded
+    to 5 dims."""
+    n = len(to) - len(shape)
+    if n < 0 or any(a != b and a != 1 for a, b in zip(shape, to[n:])):
+        raise RuntimeError(f"combine: cannot broadcast {tuple(shape)} to {tuple(to)}")
+    return [0] * (5 - len(shape)) + [s if a == b else 0 for s, a, b in zip(stride, shape, to[n:])]
+
+
+# What the argument arrays of one combine call hold besides the pointers
+# depends on shapes and strides alone: an iteration makes ~45 such calls and
+# building them took ~15 of the ~25 us of each (o10v40 is bound by the host).
+# The library only reads the arrays, so threads share them.
+@functools.lru_cache(maxsize=4096)
+def _combine_plan(outs, xs, prod):
+    shape = tuple(outs[0][0])
+    if len(shape) > 5 or any(tuple(o[0]) != shape for o in outs):
+        raise ValueError("combine: outputs of one shape, at most 5 dims")
+    dims = [1] * (5 - len(shape)) + list(shape)
+    # walk the index space in the first output's memory order (its
+    # smallest stride innermost), so its reads and writes coalesce
+    s0 = _strides5(*outs[0], shape)
+    perm = sorted(range(5), key=lambda d: (dims[d] != 1, -s0[d]))
+
+    def strides(sig):
+        flat = []
+        for sh, st in sig:
+            s5 = _strides5(sh, st, shape)
+            flat.extend(s5[d] for d in perm)
+        return L.i64arr(flat if flat else [0])
+
+    return L.i64arr([dims[d] for d in perm]), strides(xs), strides(prod), strides(outs)
+
+
+def _ptrs(ts):
+    import ctypes
+
+    return (ctypes.c_void_p * (len(ts) or 1))(*[t.data_ptr() for t in ts])
 
 
 def combine(outs, xs=(), coefs=None, prod=(), accumulate=False):
@@ -308,42 +345,19 @@ def combine(outs, xs=(), coefs=None, prod=(), accumulate=False):
     Outputs must not overlap the inputs."""
     import ctypes
 
-    outs = list(outs)
-    xs = list(xs)
-    prod = list(prod)
-    shape = tuple(outs[0].shape)
-    if len(shape) > 5 or any(tuple(o.shape) != shape for o in outs):
-        raise ValueError("combine: outputs of one shape, at most 5 dims")
+    outs, xs, prod = list(outs), list(xs), list(prod)
     for t in outs + xs + prod:
-        if t.dtype != torch.float64 or t.device.type != "cuda":
+        if t.dtype != torch.float64 or not t.is_cuda:
             raise ValueError("combine: FP64 CUDA tensors only")
     nc = len(xs) + (1 if prod else 0)
     if coefs is None:
         coefs = [[1.0] * nc for _ in outs]
+    dims, sx, sp, so = _combine_plan(_sig(outs), _sig(xs), _sig(prod))
     if len(coefs) != len(outs) or any(len(c) != nc for c in coefs):
         raise ValueError("combine: one coefficient per input (and one for the product) per output")
-    dims = [1] * (5 - len(shape)) + list(shape)
-    vp = ctypes.c_void_p
-
-    def ptrs(ts):
-        return (vp * max(len(ts), 1))(*[t.data_ptr() for t in ts])
-
-    # walk the index space in the first output's memory order (its
-    # smallest stride innermost), so its reads and writes coalesce
-    s0 = _view5(outs[0], shape)
-    perm = sorted(range(5), key=lambda d: (dims[d] != 1, -s0[d]))
-
-    def strides(ts):
-        flat = []
-        for t in ts:
-            st = _view5(t, shape)
-            flat.extend(st[d] for d in perm)
-        return L.i64arr(flat if flat else [0])
-
     cf = (ctypes.c_double * (len(outs) * nc))(*[float(c) for row in coefs for c in row])
-    L.check(L.load().fricc_combine5(L.i64arr([dims[d] for d in perm]), len(xs), ptrs(xs), strides(xs), len(prod),
-                                    ptrs(prod), strides(prod), len(outs), ptrs(outs), strides(outs), cf,
-                                    int(bool(accumulate)), L.cur_stream()))
+    L.check(L.load().fricc_combine5(dims, len(xs), _ptrs(xs), sx, len(prod), _ptrs(prod), sp, len(outs), _ptrs(outs), so,
+                                    cf, int(bool(accumulate)), L.cur_stream()))
     return outs[0]
 
 
@@ -370,40 +384,45 @@ def _strides3(t: torch.Tensor):
     return (t.stride(1), t.stride(2), t.stride(0)), t.shape[0]
 
 
-def _bstrides(t: torch.Tensor):
+def _bstrides(shape, stride):
     """(row, col, batch, batch2) element strides and (batch, batch2) extents of
     a 2-D, 3-D ([batch, M, K]) or 4-D ([batch2, batch, M, K]) operand."""
-    if t.dim() == 2:
-        return (t.stride(0), t.stride(1), 0, 0), 1, 1
-    if t.dim() == 3:
-        return (t.stride(1), t.stride(2), t.stride(0), 0), t.shape[0], 1
-    if t.dim() == 4:
-        return (t.stride(2), t.stride(3), t.stride(1), t.stride(0)), t.shape[1], t.shape[0]
+    if len(shape) == 2:
+        return (stride[0], stride[1], 0, 0), 1, 1
+    if len(shape) == 3:
+        return (stride[1], stride[2], stride[0], 0), shape[0], 1
+    if len(shape) == 4:
+        return (stride[2], stride[3], stride[1], stride[0]), shape[1], shape[0]
     raise ValueError("gemm: operands are 2-D, 3-D or 4-D")
 
 
-def _gemm_call(fn, A, B, C, alpha, beta):
-    import ctypes
-
-    sA, bA, b2A = _bstrides(A)
-    sB, bB, b2B = _bstrides(B)
-    sC, batch, batch2 = _bstrides(C)
-    M, N = C.shape[-2], C.shape[-1]
-    K = A.shape[-1]
-    assert A.shape[-2] == M and B.shape[-2] == K and B.shape[-1] == N
+@functools.lru_cache(maxsize=4096)
+def _gemm_plan(A, B, C):
+    """(batch, batch2, M, N, K, stride arrays of three, of four) of operands
+    given as (shape, stride); the library only reads the arrays."""
+    sA, bA, b2A = _bstrides(*A)
+    sB, bB, b2B = _bstrides(*B)
+    sC, batch, batch2 = _bstrides(*C)
+    M, N = C[0][-2], C[0][-1]
+    K = A[0][-1]
+    assert A[0][-2] == M and B[0][-2] == K and B[0][-1] == N
     assert bA in (1, batch) and bB in (1, batch) and b2A in (1, batch2) and b2B in (1, batch2)
     # a size-1 batch level of an operand is shared: stride 0
     sA = (sA[0], sA[1], sA[2] if bA == batch and batch > 1 else 0, sA[3] if b2A == batch2 and batch2 > 1 else 0)
     sB = (sB[0], sB[1], sB[2] if bB == batch and batch > 1 else 0, sB[3] if b2B == batch2 and batch2 > 1 else 0)
+    return (batch, batch2, M, N, K, tuple(L.i64arr(x[:3]) for x in (sA, sB, sC)),
+            tuple(L.i64arr(x) for x in (sA, sB, sC)))
+
+
+def _gemm_call(fn, A, B, C, alpha, beta):
+    batch, batch2, M, N, K, s3, s4 = _gemm_plan(*_sig((A, B, C)))
     lib = L.load()
-    st = L.cur_stream()
-    pA, pB, pC = (ctypes.c_void_p(t.data_ptr()) for t in (A, B, C))
     if batch2 == 1:
-        L.check(getattr(lib, fn)(pA, pB, pC, batch, M, N, K, L.i64arr(sA[:3]), L.i64arr(sB[:3]), L.i64arr(sC[:3]),
-                                 float(alpha), float(beta), st))
+        L.check(getattr(lib, fn)(A.data_ptr(), B.data_ptr(), C.data_ptr(), batch, M, N, K, *s3, float(alpha), float(beta),
+                                 L.cur_stream()))
     else:
-        L.check(getattr(lib, fn + "_b2")(pA, pB, pC, batch, batch2, M, N, K, L.i64arr(sA), L.i64arr(sB),
-                                         L.i64arr(sC), float(alpha), float(beta), st))
+        L.check(getattr(lib, fn + "_b2")(A.data_ptr(), B.data_ptr(), C.data_ptr(), batch, batch2, M, N, K, *s4,
+                                         float(alpha), float(beta), L.cur_stream()))
     return C
 
 
@@ -420,21 +439,11 @@ def gemm_f64(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1
     ``a_mod`` / ``b_mod``: a 2-D operand prepared once (``mod_operand``)."""
     if a_mod is None and b_mod is None:
         return _gemm_call("fricc_gemm_f64", A, B, C, alpha, beta)
-    import ctypes
-
-    sA, bA, b2A = _bstrides(A)
-    sB, bB, b2B = _bstrides(B)
-    sC, batch, batch2 = _bstrides(C)
-    M, N, K = C.shape[-2], C.shape[-1], A.shape[-1]
-    assert A.shape[-2] == M and B.shape[-2] == K and B.shape[-1] == N
-    assert bA in (1, batch) and bB in (1, batch) and b2A in (1, batch2) and b2B in (1, batch2)
-    sA = (sA[0], sA[1], sA[2] if bA == batch and batch > 1 else 0, sA[3] if b2A == batch2 and batch2 > 1 else 0)
-    sB = (sB[0], sB[1], sB[2] if bB == batch and batch > 1 else 0, sB[3] if b2B == batch2 and batch2 > 1 else 0)
-    vp = ctypes.c_void_p
+    batch, batch2, M, N, K, _, s4 = _gemm_plan(*_sig((A, B, C)))
     L.check(L.load().fricc_gemm_f64_mod(
-        vp(A.data_ptr()), vp(a_mod.data_ptr()) if a_mod is not None else None, vp(B.data_ptr()),
-        vp(b_mod.data_ptr()) if b_mod is not None else None, vp(C.data_ptr()), batch, batch2, M, N, K, L.i64arr(sA),
-        L.i64arr(sB), L.i64arr(sC), float(alpha), float(beta), L.cur_stream()))
+        A.data_ptr(), a_mod.data_ptr() if a_mod is not None else None, B.data_ptr(),
+        b_mod.data_ptr() if b_mod is not None else None, C.data_ptr(), batch, batch2, M, N, K, *s4, float(alpha),
+        float(beta), L.cur_stream()))
     return C
 
 
@@ -484,14 +493,44 @@ def mod_operand(x: torch.Tensor, rows: int, k: int, row_stride: int, k_stride: i
 def _as3(x: torch.Tensor, shape3):
     """x (a permuted view) as a [batch, rows, cols] view, copied to a
     contiguous buffer by the library when its strides do not allow one."""
+    if _viewable(x.shape, x.stride(), shape3):
+        return x.view(shape3)
+    if not x.is_cuda:
+        return x.reshape(shape3)
+    buf = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    combine([buf], [x])
+    return buf.view(shape3)
+
+
+@functools.lru_cache(maxsize=4096)
+def _viewable(shape, stride, to) -> bool:
     try:
-        return x.view(*shape3)
+        torch.empty_strided(shape, stride, device="meta").view(to)
     except RuntimeError:
-        if x.device.type != "cuda":
-            return x.reshape(*shape3)
-        buf = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-        combine([buf], [x])
-        return buf.view(*shape3)
+        return False
+    return True
+
+
+@functools.lru_cache(maxsize=1024)
+def _einsum_plan(spec, shape_a, shape_b):
+    lhs, outs = spec.replace(" ", "").split("->")
+    a, b = lhs.split(",")
+    if len(set(a)) != len(a) or len(set(b)) != len(b):
+        raise ValueError(f"einsum_df: repeated index within an operand in {spec!r}")
+    size = {c: shape_a[a.index(c)] for c in a}
+    size.update({c: shape_b[b.index(c)] for c in b})
+    lone_a = [a.index(c) for c in a if c not in b and c not in outs]
+    lone_b = [b.index(c) for c in b if c not in a and c not in outs]
+    a = "".join(c for c in a if c in b or c in outs)
+    b = "".join(c for c in b if c in a or c in outs)
+    bt = [c for c in outs if c in a and c in b]
+    mi = [c for c in outs if c in a and c not in b]
+    ni = [c for c in outs if c in b and c not in a]
+    ki = [c for c in a if c in b and c not in outs]
+    nb, M, N, K = (math.prod(size[c] for c in idx) for idx in (bt, mi, ni, ki))
+    order = bt + mi + ni
+    return (lone_a, lone_b, [a.index(c) for c in bt + mi + ki], [b.index(c) for c in bt + ki + ni], (nb, M, K), (nb, K, N),
+            (nb, M, N), [size[c] for c in order], [outs.index(c) for c in order], [order.index(c) for c in outs])
 
 
 def einsum_df(spec: str, A: torch.Tensor, B: torch.Tensor, gemm=None, out=None, alpha: float = 1.0,
@@ -509,33 +548,17 @@ def einsum_df(spec: str, A: torch.Tensor, B: torch.Tensor, gemm=None, out=None, 
     order; with ``out`` (a tensor in the output's index order whose
     [batch, rows, cols] grouping is a view) the GEMM writes
     out = alpha * result + beta * out in place."""
-    lhs, outs = spec.replace(" ", "").split("->")
-    a, b = lhs.split(",")
-    if len(set(a)) != len(a) or len(set(b)) != len(b):
-        raise ValueError(f"einsum_df: repeated index within an operand in {spec!r}")
-    lone = [c for c in a if c not in b and c not in outs]
-    if lone:
-        A = A.sum(dim=[a.index(c) for c in lone])
-        a = "".join(c for c in a if c not in lone)
-    lone = [c for c in b if c not in a and c not in outs]
-    if lone:
-        B = B.sum(dim=[b.index(c) for c in lone])
-        b = "".join(c for c in b if c not in lone)
-    size = {c: A.shape[a.index(c)] for c in a}
-    size.update({c: B.shape[b.index(c)] for c in b})
-    bt = [c for c in outs if c in a and c in b]
-    mi = [c for c in outs if c in a and c not in b]
-    ni = [c for c in outs if c in b and c not in a]
-    ki = [c for c in a if c in b and c not in outs]
-    prod = lambda idx: math.prod(size[c] for c in idx)
-    nb, M, N, K = prod(bt), prod(mi), prod(ni), prod(ki)
-    Ap = _as3(A.permute([a.index(c) for c in bt + mi + ki]), (nb, M, K))
-    Bp = _as3(B.permute([b.index(c) for c in bt + ki + ni]), (nb, K, N))
-    order = bt + mi + ni
+    lone_a, lone_b, pa, pb, sa, sb, sc, size_c, pc, po = _einsum_plan(spec, A.shape, B.shape)
+    if lone_a:
+        A = A.sum(dim=lone_a)
+    if lone_b:
+        B = B.sum(dim=lone_b)
+    Ap, Bp = _as3(A.permute(pa), sa), _as3(B.permute(pb), sb)
+    K = sa[2]
     if out is not None:
-        C = out.permute([outs.index(c) for c in order]).view(nb, M, N)
+        C = out.permute(pc).view(sc)
     else:
-        C = torch.empty(nb, M, N, dtype=torch.float64, device=A.device)
+        C = torch.empty(sc, dtype=torch.float64, device=A.device)
         alpha, beta = 1.0, 0.0
     if C.numel():
         if K == 0:
@@ -545,7 +568,7 @@ def einsum_df(spec: str, A: torch.Tensor, B: torch.Tensor, gemm=None, out=None, 
             (gemm or gemm_df)(Ap, Bp, C, alpha, beta)
     if out is not None:
         return out
-    return C.view([size[c] for c in order]).permute([order.index(c) for c in outs])
+    return C.view(size_c).permute(po)
 
 
 def gemm_torch(A, B, C, alpha=1.0, beta=0.0):
