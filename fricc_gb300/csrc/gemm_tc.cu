@@ -544,9 +544,46 @@ __global__ void __launch_bounds__(NT, 1)
 // Row r = (r / ri, r % ri) and column j < k of x sit at
 // (r / ri) sro + (r % ri) sri + j sk: a transposed or batch-flattened view
 // becomes a K-major operand in the same pass.
+// x = hi + lo in BF16, each rounded to nearest even from the exact value, by
+// integers: the conversions and the subtraction are FP64 instructions, whose
+// unit bounded these passes (64 M elements 566 us, now 265).  The 53-bit
+// significand splits at bit 45 into hi's 8 bits and a signed remainder, whose
+// leading 8 bits are lo's.  Exponents where either would be subnormal or
+// infinite take the conversions.
+static __device__ __noinline__ unsigned split_bf16_conv(double x) {
+  const __nv_bfloat16 hi = __double2bfloat16(x);
+  const __nv_bfloat16 lo = __double2bfloat16(x - (double)__bfloat162float(hi));
+  return (unsigned)__bfloat16_as_ushort(hi) | ((unsigned)__bfloat16_as_ushort(lo) << 16);
+}
+// hi in the low half, lo in the high half
+__device__ __forceinline__ unsigned split_bf16(double x) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const int E = (int)((u >> 52) & 0x7ffu);
+  if (E < 949 || E > 1149) return (u << 1) ? split_bf16_conv(x) : (unsigned)(u >> 48);
+  const unsigned sgn = (unsigned)(u >> 48) & 0x8000u, top = (unsigned)(u >> 32) & 0xfffffu;
+  const unsigned h8 = 128u + (top >> 13);
+  const unsigned long long rem = u & ((1ull << 45) - 1), half = 1ull << 44;
+  const bool up = rem > half || (rem == half && (h8 & 1u));
+  const unsigned hi = sgn | (((unsigned)(E - 897) << 7) + h8 + (up ? 1u : 0u));
+  const unsigned long long a = up ? (1ull << 45) - rem : rem;  // |x - hi| 2^(1075 - E)
+  if (a == 0) return hi;
+  const int p = 63 - __clzll((long long)a);
+  unsigned q;
+  if (p > 7) {
+    const int sh = p - 7;
+    q = (unsigned)(a >> sh);
+    const unsigned long long r = a & ((1ull << sh) - 1), h = 1ull << (sh - 1);
+    q += (r > h || (r == h && (q & 1u))) ? 1u : 0u;
+  } else {
+    q = (unsigned)a << (7 - p);
+  }
+  const unsigned lo = (up ? sgn ^ 0x8000u : sgn) | (((unsigned)(E - 949 + p) << 7) + q);
+  return hi | (lo << 16);
+}
+
 __device__ __forceinline__ void split_put(double xv, int64_t k, __nv_bfloat16* ar, __nv_bfloat16* br) {
-  const __nv_bfloat16 hi = __double2bfloat16(xv);
-  const __nv_bfloat16 lo = __double2bfloat16(xv - (double)__bfloat162float(hi));
+  const unsigned s = split_bf16(xv);
+  const __nv_bfloat16 hi = __ushort_as_bfloat16((unsigned short)s), lo = __ushort_as_bfloat16((unsigned short)(s >> 16));
   if (ar) {
     ar[0] = hi;
     ar[k] = hi;
@@ -559,24 +596,58 @@ __device__ __forceinline__ void split_put(double xv, int64_t k, __nv_bfloat16* a
   }
 }
 
-// columns contiguous (or any layout): work items of (row, 1024 columns), a
-// block's threads over the columns, so a few very long rows spread as well
-__global__ void k_split_rows(const double* __restrict__ x, int64_t rows, int64_t k, int64_t ri, int64_t sro,
-                             int64_t sri, int64_t sk, int64_t kp, __nv_bfloat16* __restrict__ Ap,
-                             __nv_bfloat16* __restrict__ Bp) {
-  constexpr int64_t CH = 1024;
+// two adjacent columns of an even k: 4-byte stores
+__device__ __forceinline__ void split_put2(double x0, double x1, int64_t k, __nv_bfloat16* ar, __nv_bfloat16* br) {
+  const unsigned s0 = split_bf16(x0), s1 = split_bf16(x1);
+  const unsigned hi = __byte_perm(s0, s1, 0x5410), lo = __byte_perm(s0, s1, 0x7632);
+  if (ar) {
+    *reinterpret_cast<unsigned*>(ar) = hi;
+    *reinterpret_cast<unsigned*>(ar + k) = hi;
+    *reinterpret_cast<unsigned*>(ar + 2 * k) = lo;
+  }
+  if (br) {
+    *reinterpret_cast<unsigned*>(br) = hi;
+    *reinterpret_cast<unsigned*>(br + k) = lo;
+    *reinterpret_cast<unsigned*>(br + 2 * k) = hi;
+  }
+}
+
+// columns contiguous (or any layout): a warp per (row, 256 columns), so that
+// short rows keep a block busy and a few very long ones spread as well.
+// pair: two columns per lane (an even k, 4-byte aligned outputs)
+__global__ void __launch_bounds__(256) k_split_rows(const double* __restrict__ x, int64_t rows, int64_t k, int64_t ri,
+                                                    int64_t sro, int64_t sri, int64_t sk, int64_t kp,
+                                                    __nv_bfloat16* __restrict__ Ap, __nv_bfloat16* __restrict__ Bp,
+                                                    int pair) {
+  constexpr int64_t CH = 256;
+  const int lane = threadIdx.x & 31;
   const int64_t nch = fricc_cdiv(kp - 2 * k, CH);  // chunks over j < k, then the padding j >= 3k
-  for (int64_t w = blockIdx.x; w < rows * nch; w += gridDim.x) {
-    const int64_t r = w / nch, c = w - r * nch;
-    const int64_t ro = r / ri;
+  for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < rows * nch; w += (int64_t)gridDim.x * 8) {
+    const int64_t r = nch == 1 ? w : w / nch, c = w - r * nch;
+    const int64_t ro = ri == 1 ? r : r / ri;
     const double* xr = x + ro * sro + (r - ro * ri) * sri;
     __nv_bfloat16* ar = Ap ? Ap + r * kp : nullptr;
     __nv_bfloat16* br = Bp ? Bp + r * kp : nullptr;
     const int64_t j1 = (c + 1) * CH < k ? (c + 1) * CH : k;
-    for (int64_t j = c * CH + threadIdx.x; j < j1; j += blockDim.x)
-      split_put(xr[j * sk], k, ar ? ar + j : nullptr, br ? br + j : nullptr);
+    if (pair) {
+      double v[4][2];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int64_t j = c * CH + 64 * q + 2 * lane;
+        v[q][0] = j < j1 ? __ldg(xr + j * sk) : 0.0;
+        v[q][1] = j < j1 ? __ldg(xr + (j + 1) * sk) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int64_t j = c * CH + 64 * q + 2 * lane;
+        if (j < j1) split_put2(v[q][0], v[q][1], k, ar ? ar + j : nullptr, br ? br + j : nullptr);
+      }
+    } else {
+      for (int64_t j = c * CH + lane; j < j1; j += 32)
+        split_put(xr[j * sk], k, ar ? ar + j : nullptr, br ? br + j : nullptr);
+    }
     // padding: chunk c also zeroes columns 3k + [c*CH - k, ...) that fall in [3k, kp)
-    for (int64_t j = 3 * k + c * CH - k + threadIdx.x; j < kp && j < 3 * k + (c + 1) * CH - k; j += blockDim.x)
+    for (int64_t j = 3 * k + c * CH - k + lane; j < kp && j < 3 * k + (c + 1) * CH - k; j += 32)
       if (j >= 3 * k) {
         if (ar) ar[j] = __float2bfloat16(0.0f);
         if (br) br[j] = __float2bfloat16(0.0f);
@@ -584,30 +655,39 @@ __global__ void k_split_rows(const double* __restrict__ x, int64_t rows, int64_t
   }
 }
 
-// rows contiguous (sri == 1, within runs of ri rows): 32 x 32 tiles read
+// rows contiguous (sri == 1, within runs of ri rows): 32 x 64 tiles read
 // along r and written along j through shared memory
 __global__ void k_split_tr(const double* __restrict__ x, int64_t rows, int64_t k, int64_t ri, int64_t sro, int64_t sk,
-                           int64_t kp, __nv_bfloat16* __restrict__ Ap, __nv_bfloat16* __restrict__ Bp) {
-  __shared__ double tile[32][33];
-  const int64_t tiles_r = fricc_cdiv(rows, 32), tiles_k = fricc_cdiv(k, 32);
+                           int64_t kp, __nv_bfloat16* __restrict__ Ap, __nv_bfloat16* __restrict__ Bp,
+                           int pair) {
+  __shared__ double tile[64][33];
+  const int64_t tiles_r = fricc_cdiv(rows, 32), tiles_k = fricc_cdiv(k, 64);
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   for (int64_t t = blockIdx.x; t < tiles_r * tiles_k; t += gridDim.x) {
-    const int64_t r0 = (t / tiles_k) * 32, j0 = (t % tiles_k) * 32;
+    const int64_t r0 = (t / tiles_k) * 32, j0 = (t % tiles_k) * 64;
     __syncthreads();
-    for (int yy = ty; yy < 32; yy += 8) {  // tile[j][r]: read x(r0 + tx, j0 + yy)
-      const int64_t r = r0 + tx, j = j0 + yy;
-      double v = 0.0;
-      if (r < rows && j < k) {
-        const int64_t ro = r / ri;
-        v = x[ro * sro + (r - ro * ri) + j * sk];
+    {  // tile[j][r]: read x(r0 + tx, j0 + yy)
+      const int64_t r = r0 + tx, ro = r / ri;
+      const double* xr = x + ro * sro + (r - ro * ri);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int64_t j = j0 + ty + 8 * q;
+        tile[ty + 8 * q][tx] = r < rows && j < k ? xr[j * sk] : 0.0;
       }
-      tile[yy][tx] = v;
     }
     __syncthreads();
-    for (int yy = ty; yy < 32; yy += 8) {  // write row r0 + yy, columns j0 + tx
-      const int64_t r = r0 + yy, j = j0 + tx;
-      if (r < rows && j < k)
-        split_put(tile[tx][yy], k, Ap ? Ap + r * kp + j : nullptr, Bp ? Bp + r * kp + j : nullptr);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // write row r0 + yy, columns j0 + 2 tx, + 1
+      const int yy = ty + 8 * q;
+      const int64_t r = r0 + yy, j = j0 + 2 * tx;
+      if (r >= rows || j >= k) continue;
+      __nv_bfloat16 *ar = Ap ? Ap + r * kp + j : nullptr, *br = Bp ? Bp + r * kp + j : nullptr;
+      if (pair) {
+        split_put2(tile[2 * tx][yy], tile[2 * tx + 1][yy], k, ar, br);
+      } else {
+        split_put(tile[2 * tx][yy], k, ar, br);
+        if (j + 1 < k) split_put(tile[2 * tx + 1][yy], k, ar ? ar + 1 : nullptr, br ? br + 1 : nullptr);
+      }
     }
   }
   // padding columns
@@ -750,14 +830,15 @@ int fricc_split_bf16x3_strided(const double* x, int64_t rows, int64_t k, int64_t
   if (n == 0) return FRICC_OK;
   auto* a = static_cast<__nv_bfloat16*>(Ap);
   auto* b = static_cast<__nv_bfloat16*>(Bp);
+  const int pair = k % 2 == 0 && (reinterpret_cast<uintptr_t>(Ap) | reinterpret_cast<uintptr_t>(Bp)) % 4 == 0;
   if (sri == 1 && sk != 1 && ri >= 32) {
-    int64_t g = fricc_cdiv(rows, 32) * fricc_cdiv(k, 32);
+    int64_t g = fricc_cdiv(rows, 32) * fricc_cdiv(k, 64);
     if (g > 152 * 16) g = 152 * 16;
-    tc::k_split_tr<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(x, rows, k, ri, sro, sk, kp, a, b);
+    tc::k_split_tr<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(x, rows, k, ri, sro, sk, kp, a, b, pair);
   } else {
-    const int64_t items = rows * fricc_cdiv(kp - 2 * k, 1024);
-    const int64_t g = items < 152 * 16 ? items : 152 * 16;
-    tc::k_split_rows<<<(unsigned)g, 128, 0, (cudaStream_t)stream>>>(x, rows, k, ri, sro, sri, sk, kp, a, b);
+    const int64_t g = fricc_cdiv(rows * fricc_cdiv(kp - 2 * k, 256), 8);
+    tc::k_split_rows<<<(unsigned)(g < 152 * 32 ? g : 152 * 32), 256, 0, (cudaStream_t)stream>>>(x, rows, k, ri, sro, sri,
+                                                                                                sk, kp, a, b, pair);
   }
   fricc_note_launch();
   cudaError_t e = cudaGetLastError();
