@@ -33,7 +33,7 @@
 //
 // Measured on a GB300 (operands prepared; DFMA kernel): 900 x 22500 x 22500
 // 9.1 ms; 4500^3 2.05 ms (152 ms); 2000^3 0.26 ms (14.0 ms); 400^3 30 us
-// (279 us); 675000 x 30 x 150 0.97 ms (5.25 ms).  Converting an operand: 11-12 ps
+// (279 us); 675000 x 30 x 150 0.97 ms (5.25 ms).  Converting an operand: 10-11 ps
 // an element.  Error (2-norm, against 64 bits) of the o30v150 iteration: 7e-16,
 // 2.3e-15 on the FP64 pipe.
 #include <climits>
@@ -55,7 +55,7 @@ constexpr int MAX_KS = 64;    // K slices; their residues are summed in 32 bits
 
 struct Tab {
   int p[NP] = {};
-  int c[NP][4] = {};   // 2^(13 (j+1)) mod p, balanced
+  int c[NP][3] = {};   // 2^(16 (j+1)) mod p, balanced
   int f[NP][3] = {};   // round(2^96 y / p) in signed 32-bit limbs, y = (M/p)^-1 mod p
   unsigned long long mtop = 0;  // M >> 62, in [2^63, 2^64)
 };
@@ -71,8 +71,8 @@ constexpr Tab make_tab() {
   t.mtop = (unsigned long long)(M >> 62);
   for (int i = 0; i < NP; ++i) {
     int w = 1;
-    for (int j = 0; j < 4; ++j) {
-      for (int b = 0; b < 13; ++b) w = 2 * w % p[i];
+    for (int j = 0; j < 3; ++j) {
+      for (int b = 0; b < 16; ++b) w = 2 * w % p[i];
       t.c[i][j] = 2 * w > p[i] ? w - p[i] : w;
     }
     const int q = (int)((M / (unsigned)p[i]) % (unsigned)p[i]);
@@ -110,6 +110,11 @@ __device__ __forceinline__ float2 upk2(f32x2 r) {
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
@@ -306,45 +311,57 @@ __device__ __forceinline__ long long scaled(double x, int sh) {
   return (long long)u < 0 ? -(long long)v : (long long)v;
 }
 
-// X in 13-bit digits as floats: four unsigned ones and a signed leading one
-__device__ __forceinline__ void digits(long long X, float* a) {
-  const unsigned lo = (unsigned)X, hi = (unsigned)((unsigned long long)X >> 32);
-  const unsigned d[4] = {lo, lo >> 13, __funnelshift_r(lo, hi, 26), hi >> 7};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) a[j] = __uint_as_float((d[j] & 0x1fffu) | 0x4B000000u) - 8388608.0f;
-  a[4] = __int_as_float(0x4B400000 + ((int)hi >> 20)) - MAGIC;
+// X0 and X1 in signed 16-bit digits (the leading one of 14 bits) as floats
+__device__ __forceinline__ void digits(long long X0, long long X1, f32x2* d) {
+  const unsigned long long b0 = (unsigned long long)X0 + 0x800080008000ull, b1 = (unsigned long long)X1 + 0x800080008000ull;
+  const unsigned l0 = (unsigned)b0, l1 = (unsigned)b1, h0 = (unsigned)(b0 >> 32), h1 = (unsigned)(b1 >> 32);
+  constexpr unsigned E = 0x4B00u;  // 2^23 + field
+  const f32x2 bias = pk2(-8421376.0f, -8421376.0f);  // 2^23 + 2^15
+  d[0] = add2(pk2(__uint_as_float(__byte_perm(l0, E, 0x5410)), __uint_as_float(__byte_perm(l1, E, 0x5410))), bias);
+  d[1] = add2(pk2(__uint_as_float(__byte_perm(l0, E, 0x5432)), __uint_as_float(__byte_perm(l1, E, 0x5432))), bias);
+  d[2] = add2(pk2(__uint_as_float(__byte_perm(h0, E, 0x5410)), __uint_as_float(__byte_perm(h1, E, 0x5410))), bias);
+  d[3] = add2(pk2(__int_as_float(0x4B400000 + ((int)h0 >> 16)), __int_as_float(0x4B400000 + ((int)h1 >> 16))),
+              pk2(-MAGIC, -MAGIC));
 }
 
-// the residue of X modulo the i-th modulus: four exact FMAs (13-bit digits
-// times residues of 2^13j: below 2^23) and one reduction.  Scalar FMAs, whose
-// constants are immediates (a packed one would need them in register pairs)
+// The residues modulo the I-th modulus of SG pairs at once, two packed values an
+// instruction, and the constants' registers set up once for all of them: three
+// exact FMAs (sums below 2^15 (1 + 2 * 180) + 2^13 * 180 < 2^24) and one
+// reduction.  One pair at a time with 13-bit digits and scalar FMAs, the
+// conversion took 252 instructions an element and was bound by issuing them:
+// 20 M elements 200 us, now 170.
+constexpr int SG = 4;
 template <int I>
-__device__ __forceinline__ float residue(const float* a) {
-  float t = a[0];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) t = fmaf(a[j + 1], (float)TAB.c[I][j], t);
-  constexpr float inv = 1.0f / (float)TAB.p[I], negp = -(float)TAB.p[I];
-  return fmaf(fmaf(t, inv, MAGIC) - MAGIC, negp, t);
-}
-
-template <int I>
-__device__ __forceinline__ void put_residues(const float* a0, const float* a1, __nv_bfloat16* at, int64_t plane) {
+__device__ __forceinline__ void put_residues(const f32x2 (*d)[4], const bool* live, __nv_bfloat16* at, int64_t step,
+                                             int64_t plane) {
   if constexpr (I < NP) {
-    *reinterpret_cast<__nv_bfloat162*>(at) = __floats2bfloat162_rn(residue<I>(a0), residue<I>(a1));
-    put_residues<I + 1>(a0, a1, at + plane, plane);
+    constexpr float inv_ = 1.0f / (float)TAB.p[I], p_ = (float)TAB.p[I];
+    constexpr float c0 = (float)TAB.c[I][0], c1 = (float)TAB.c[I][1], c2 = (float)TAB.c[I][2];
+    const f32x2 inv = pk2(inv_, inv_), negp = pk2(-p_, -p_), k0 = pk2(c0, c0), k1 = pk2(c1, c1), k2 = pk2(c2, c2);
+#pragma unroll
+    for (int g = 0; g < SG; ++g) {
+      const float2 r = upk2(reduce2(fma2(d[g][3], k2, fma2(d[g][2], k1, fma2(d[g][1], k0, d[g][0]))), inv, negp));
+      if (live[g]) *reinterpret_cast<__nv_bfloat162*>(at + g * step) = __floats2bfloat162_rn(r.x, r.y);
+    }
+    put_residues<I + 1>(d, live, at + plane, step, plane);
   }
 }
 
-// two adjacent k of one row into every plane
-__device__ __forceinline__ void put_planes(double x0, double x1, int sh, __nv_bfloat16* at, int64_t plane) {
-  float a0[5], a1[5];
-  digits(scaled(x0, sh), a0);
-  digits(scaled(x1, sh), a1);
-  put_residues<0>(a0, a1, at, plane);
-  // the squares of x 2^(sh - 61) (the leading digits suffice: bf16)
-  const float s0 = (a0[4] * 8192.0f + a0[3]) * 0x1p-22f + (a0[2] * 8192.0f + a0[1]) * 0x1p-48f + a0[0] * 0x1p-61f;
-  const float s1 = (a1[4] * 8192.0f + a1[3]) * 0x1p-22f + (a1[2] * 8192.0f + a1[1]) * 0x1p-48f + a1[0] * 0x1p-61f;
-  *reinterpret_cast<__nv_bfloat162*>(at + NP * plane) = __floats2bfloat162_rn(s0 * s0, s1 * s1);
+// Two adjacent k of each of SG rows (`step` elements apart) into every plane.
+__device__ __forceinline__ void put_planes(const double (*x)[2], const int* sh, const bool* live, __nv_bfloat16* at,
+                                           int64_t step, int64_t plane) {
+  f32x2 d[SG][4];
+#pragma unroll
+  for (int g = 0; g < SG; ++g) digits(scaled(x[g][0], sh[g]), scaled(x[g][1], sh[g]), d[g]);
+  // the squares of x 2^(sh - 61)
+#pragma unroll
+  for (int g = 0; g < SG; ++g) {
+    f32x2 v = fma2(d[g][3], pk2(0x1p-13f, 0x1p-13f), mul2(d[g][2], pk2(0x1p-29f, 0x1p-29f)));
+    v = fma2(d[g][1], pk2(0x1p-45f, 0x1p-45f), fma2(d[g][0], pk2(0x1p-61f, 0x1p-61f), v));
+    const float2 q = upk2(mul2(v, v));
+    if (live[g]) *reinterpret_cast<__nv_bfloat162*>(at + g * step + NP * plane) = __floats2bfloat162_rn(q.x, q.y);
+  }
+  put_residues<0>(d, live, at, step, plane);
 }
 
 // x -> its planes, in tiles of 32 rows x 64 k (4 KB of each plane); one warp
@@ -360,17 +377,21 @@ __global__ void __launch_bounds__(256, 3) k_mod_split(const ModView v, int64_t R
   for (int64_t b = blockIdx.x; b < nrb * nkb; b += gridDim.x) {
     const int64_t kb = b / nrb, r0 = (b - kb * nrb) * 32, j0 = kb * BK;
     __nv_bfloat16* out = planes + (kb * R + r0) * BK + 2 * lane;
+    double x[SG][2];
+    int s[SG];
+    bool live[SG];
     if (KFAST) {
       const int64_t j = j0 + 2 * lane;
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
-        const int rr = warp + 8 * q;
-        if (r0 + rr < R) {
-          const double* xr = v.x + v.rows.at(r0 + rr);
-          const double x0 = j < k ? __ldg(xr + koff<K2>(v, j)) : 0.0, x1 = j + 1 < k ? __ldg(xr + koff<K2>(v, j + 1)) : 0.0;
-          put_planes(x0, x1, sh[r0 + rr], out + rr * BK, plane);
-        }
+#pragma unroll
+      for (int q = 0; q < SG; ++q) {
+        const int64_t r = r0 + warp + 8 * q;
+        live[q] = r < R;
+        const double* xr = v.x + (live[q] ? v.rows.at(r) : 0);
+        x[q][0] = live[q] && j < k ? __ldg(xr + koff<K2>(v, j)) : 0.0;
+        x[q][1] = live[q] && j + 1 < k ? __ldg(xr + koff<K2>(v, j + 1)) : 0.0;
+        s[q] = live[q] ? sh[r] : 0;
       }
+      put_planes(x, s, live, out + warp * BK, 8 * BK, plane);
     } else {
       __syncthreads();
       if (r0 + lane < R) {
@@ -382,11 +403,15 @@ __global__ void __launch_bounds__(256, 3) k_mod_split(const ModView v, int64_t R
         }
       }
       __syncthreads();
-#pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int q = 0; q < SG; ++q) {
         const int rr = warp + 8 * q;
-        if (r0 + rr < R) put_planes(t[2 * lane][rr], t[2 * lane + 1][rr], sh[r0 + rr], out + rr * BK, plane);
+        live[q] = r0 + rr < R;
+        x[q][0] = t[2 * lane][rr];
+        x[q][1] = t[2 * lane + 1][rr];
+        s[q] = live[q] ? sh[r0 + rr] : 0;
       }
+      put_planes(x, s, live, out + warp * BK, 8 * BK, plane);
     }
   }
 }
@@ -451,13 +476,20 @@ __global__ void __launch_bounds__(256, 3) k_mod_convert(const ModView v, int64_t
     }
     __syncthreads();
 #pragma unroll 1
-    for (int q = warp; q < 32 * nkb; q += 8) {
-      const int kb = q >> 5, rr = q & 31;
-      if (r0 + rr < R) {
-        const int j = kb * BK + 2 * lane;
-        put_planes(ct[j * 33 + rr], ct[(j + 1) * 33 + rr], ssh[rr], planes + ((int64_t)kb * R + r0 + rr) * BK + 2 * lane,
-                   plane);
+    for (int kb = 0; kb < nkb; ++kb) {
+      const int j = kb * BK + 2 * lane;
+      double x[SG][2];
+      int h[SG];
+      bool live[SG];
+#pragma unroll
+      for (int q = 0; q < SG; ++q) {
+        const int rr = warp + 8 * q;
+        live[q] = r0 + rr < R;
+        x[q][0] = ct[j * 33 + rr];
+        x[q][1] = ct[(j + 1) * 33 + rr];
+        h[q] = ssh[rr];
       }
+      put_planes(x, h, live, planes + ((int64_t)kb * R + r0 + warp) * BK + 2 * lane, 8 * BK, plane);
     }
   }
 }
