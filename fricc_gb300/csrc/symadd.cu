@@ -1,33 +1,43 @@
 // Fused symmetrised accumulation of the T2 residual:
 //   out[i,j,a,b] += coef * (X[i,j,a,b] + X[j,i,b,a])
 // for X any strided 4-index view (fricc/friccsd.py:245-267 builds these as
-// "tmp + tmp.transpose(1,0,3,2)" and adds them to t2new).  One pass over the
-// output: a CTA takes one (i,j) pair and a 32 x 32 tile of (a,b); each of
-// the two reads of X runs along whichever of its (a,b) indices is
-// contiguous, through a shared-memory transpose when that index is a, so
-// both stay coalesced; the output (C order) is read and written along b.
+// "tmp + tmp.transpose(1,0,3,2)" and adds them to t2new).  out[i,j,a,b] and
+// out[j,i,b,a] receive the same sum, so a CTA takes a pair i <= j and a
+// 32 x 32 tile of (a,b), reads the two tiles of X once, each along whichever of
+// its (a,b) indices is contiguous (through a shared-memory transpose), and
+// updates both outputs, the second along its own rows.  All of a thread's loads
+// are under way before the first use.  Bound by its bytes: 24 an element; with
+// one output per CTA, X was read twice (64 M elements 535 us, now 273).
 #include <cstdlib>
 
 #include "common.cuh"
 
 namespace {
 
-constexpr int TD = 32, TR = 8;  // 32 x 32 tile, 32 x 8 threads
+constexpr int TD = 32, TR = 8, NR = TD / TR;  // 32 x 32 tile, 32 x 8 threads
 
-// tile[a'][b'] = x(a0 + a', b0 + b') for the plane (p, q) of X, read along b
-// (rows of 32 b) or along a (then stored transposed)
-__device__ __forceinline__ void load_tile(double (*tile)[TD + 1], const double* __restrict__ X, int64_t base,
-                                          int64_t sa, int64_t sb, int64_t a0, int64_t b0, int64_t v_a, int64_t v_b,
-                                          bool along_b) {
+struct TileLoad {
+  double v[NR];
+};
+// the tile x(a0 + a', b0 + b') of the plane at `base`: row r of the registers is
+// read along b (a' = ty + TR r, b' = tx) or along a (a' = tx, b' = ty + TR r)
+__device__ __forceinline__ TileLoad load_tile(const double* __restrict__ X, int64_t base, int64_t sa, int64_t sb, int64_t a0,
+                                              int64_t b0, int64_t nv, bool along_b) {
+  TileLoad t;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int r = ty; r < TD; r += TR) {
-    if (along_b) {  // thread tx walks b
-      const int64_t a = a0 + r, b = b0 + tx;
-      tile[r][tx] = (a < v_a && b < v_b) ? X[base + a * sa + b * sb] : 0.0;
-    } else {        // thread tx walks a
-      const int64_t a = a0 + tx, b = b0 + r;
-      tile[tx][r] = (a < v_a && b < v_b) ? X[base + a * sa + b * sb] : 0.0;
-    }
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int64_t a = a0 + (along_b ? ty + TR * r : tx), b = b0 + (along_b ? tx : ty + TR * r);
+    t.v[r] = (a < nv && b < nv) ? __ldg(X + base + a * sa + b * sb) : 0.0;
+  }
+  return t;
+}
+__device__ __forceinline__ void put_tile(double (*tile)[TD + 1], const TileLoad& t, bool along_b) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (along_b) tile[ty + TR * r][tx] = t.v[r];
+    else tile[tx][ty + TR * r] = t.v[r];
   }
 }
 
@@ -36,24 +46,47 @@ __global__ void __launch_bounds__(TD* TR) k_symadd(double* __restrict__ out, con
                                                     double coef, int first_along_b, int second_along_b,
                                                     int64_t xr = 0) {
   __shared__ double t1[TD][TD + 1], t2[TD][TD + 1];
-  // replica batches: blockIdx.z = r o^2 + ij; replica r's X starts xr
-  // elements after the previous one's, its output o^2 v^2 after
-  const unsigned oo = (unsigned)(o * o);  // blockIdx.z < 65536: 32-bit divisions
-  const unsigned rep = blockIdx.z / oo;
-  const int64_t ij = blockIdx.z - rep * oo;
+  // replica batches: blockIdx.z = r o (o + 1) / 2 + pair; replica r's X starts
+  // xr elements after the previous one's, its output o^2 v^2 after
+  const unsigned np = (unsigned)(o * (o + 1) / 2);  // blockIdx.z < 65536: 32-bit divisions
+  const unsigned rep = blockIdx.z / np, pair = blockIdx.z - rep * np;
   X += rep * xr;
   out += rep * o * o * v * v;
-  const int64_t i = (unsigned)ij / (unsigned)o, j = ij - i * o;
+  unsigned j = (unsigned)((sqrtf(8.0f * (float)pair + 1.0f) - 1.0f) * 0.5f);  // j (j + 1) / 2 <= pair
+  while (j * (j + 1) / 2 > pair) --j;
+  while ((j + 1) * (j + 2) / 2 <= pair) ++j;
+  const int64_t i = pair - j * (j + 1) / 2;
   const int64_t a0 = (int64_t)blockIdx.y * TD, b0 = (int64_t)blockIdx.x * TD;
   // X[i,j,a,b] over (a,b): strides (s2, s3); X[j,i,b,a] over (a,b): strides (s3, s2)
-  load_tile(t1, X, i * s0 + j * s1, s2, s3, a0, b0, v, v, first_along_b != 0);
-  load_tile(t2, X, j * s0 + i * s1, s3, s2, a0, b0, v, v, second_along_b != 0);
-  __syncthreads();
+  const TileLoad x1 = load_tile(X, i * s0 + j * s1, s2, s3, a0, b0, v, first_along_b != 0);
+  const TileLoad x2 = load_tile(X, j * s0 + i * s1, s3, s2, a0, b0, v, second_along_b != 0);
+  double* o1 = out + ((i * o + j) * v) * v;  // [a][b]
+  double* o2 = out + ((j * o + i) * v) * v;  // [b][a]
   const int tx = threadIdx.x, ty = threadIdx.y;
-  double* orow = out + (ij * v) * v;
-  for (int r = ty; r < TD; r += TR) {
-    const int64_t a = a0 + r, b = b0 + tx;
-    if (a < v && b < v) orow[a * v + b] += coef * (t1[r][tx] + t2[r][tx]);
+  const bool two = i != (int64_t)j;
+  double y1[NR], y2[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int64_t q = ty + TR * r;
+    y1[r] = (a0 + q < v && b0 + tx < v) ? o1[(a0 + q) * v + b0 + tx] : 0.0;
+    y2[r] = (two && b0 + q < v && a0 + tx < v) ? o2[(b0 + q) * v + a0 + tx] : 0.0;
+  }
+  put_tile(t1, x1, first_along_b != 0);
+  put_tile(t2, x2, second_along_b != 0);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int q = ty + TR * r;
+    const double s = t1[q][tx] + t2[q][tx];
+    if (a0 + q < v && b0 + tx < v) o1[(a0 + q) * v + b0 + tx] = y1[r] + coef * s;
+    t1[q][tx] = s;
+  }
+  if (!two) return;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int q = ty + TR * r;
+    if (b0 + q < v && a0 + tx < v) o2[(b0 + q) * v + a0 + tx] = y2[r] + coef * t1[tx][q];
   }
 }
 
@@ -73,7 +106,7 @@ extern "C" int fricc_symadd(double* out, const double* X, int64_t nocc, int64_t 
   // the first read walks (a,b) with strides (s2, s3), the second with (s3, s2)
   const int first_along_b = std::llabs(s3) <= std::llabs(s2) ? 1 : 0;
   const int second_along_b = std::llabs(s2) <= std::llabs(s3) ? 1 : 0;
-  const dim3 grid((unsigned)fricc_cdiv(nvir, TD), (unsigned)fricc_cdiv(nvir, TD), (unsigned)(nocc * nocc));
+  const dim3 grid((unsigned)fricc_cdiv(nvir, TD), (unsigned)fricc_cdiv(nvir, TD), (unsigned)(nocc * (nocc + 1) / 2));
   k_symadd<<<grid, dim3(TD, TR), 0, (cudaStream_t)stream>>>(out, X, nocc, nvir, s0, s1, s2, s3, coef, first_along_b,
                                                            second_along_b);
   fricc_note_launch();
@@ -96,7 +129,7 @@ extern "C" int fricc_symadd_b(double* out, const double* X, int64_t R, int64_t n
   const int64_t s0 = strides[1], s1 = strides[2], s2 = strides[3], s3 = strides[4];
   const int first_along_b = std::llabs(s3) <= std::llabs(s2) ? 1 : 0;
   const int second_along_b = std::llabs(s2) <= std::llabs(s3) ? 1 : 0;
-  const dim3 grid((unsigned)fricc_cdiv(nvir, TD), (unsigned)fricc_cdiv(nvir, TD), (unsigned)(R * nocc * nocc));
+  const dim3 grid((unsigned)fricc_cdiv(nvir, TD), (unsigned)fricc_cdiv(nvir, TD), (unsigned)(R * (nocc * (nocc + 1) / 2)));
   k_symadd<<<grid, dim3(TD, TR), 0, (cudaStream_t)stream>>>(out, X, nocc, nvir, s0, s1, s2, s3, coef, first_along_b,
                                                            second_along_b, strides[0]);
   fricc_note_launch();
