@@ -431,14 +431,20 @@ __global__ void __launch_bounds__(1024) k_select_digit(const unsigned* __restric
   __shared__ int s_best;
   const int nb = 1 << bits, shift = 63 - bits, per = nb >> 10;  // bits >= 10
   // thread t owns the bins nb-1 - (t per + j), j < per: descending
+  // (all bins loaded at once: one after another, a thread's loads took 5 us)
+  constexpr int PER = NDIG >> 10;
+  const int top = nb - 1 - (int)threadIdx.x * per;
+  unsigned h[PER + 1];
+#pragma unroll
+  for (int j = 0; j <= PER; ++j) h[j] = j <= per && top - j >= 0 ? hist[top - j] : 0u;
   int64_t cnt = 0;
   double sum = 0.0;
-  for (int j = 0; j < per; ++j) {
-    const int b = nb - 1 - ((int)threadIdx.x * per + j);
-    const unsigned h = hist[b];
-    cnt += h;
-    if (h) sum += (double)h * __longlong_as_double((long long)((unsigned long long)(b + 1) << shift));
-  }
+#pragma unroll
+  for (int j = 0; j < PER; ++j)
+    if (j < per && h[j]) {
+      cnt += h[j];
+      sum += (double)h[j] * __longlong_as_double((long long)((unsigned long long)(top - j + 1) << shift));
+    }
   int64_t tot;
   int64_t C = block_excl_sum(cnt, sm, &tot);
   double incl = sum;
@@ -450,23 +456,25 @@ __global__ void __launch_bounds__(1024) k_select_digit(const unsigned* __restric
   if (lane_id() == 31) wsum[warp_id()] = incl;
   if (threadIdx.x == 0) s_best = INT_MAX;
   __syncthreads();
-  double S = 0.0;  // the sums of the warps before this one, then of the lanes
-  for (int w = 0; w < (int)warp_id(); ++w)
-    if (wsum[w] != 0.0) S += wsum[w];
+  // the sums of the warps before this one, then of the lanes
+  double S = (int)lane_id() < (int)warp_id() ? wsum[lane_id()] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
   {
     const double ex = __shfl_up_sync(0xffffffffu, incl, 1);
     if (lane_id() > 0) S += ex;
   }
   const double norm = fri ? c->norm : 0.0;
   const bool bound = fri && norm > 0.0 && norm < __longlong_as_double(0x7ff0000000000000ll);
-  for (int j = 0; j < per; ++j) {
-    const int b = nb - 1 - ((int)threadIdx.x * per + j);
-    const unsigned h = hist[b];
-    if (h) S += (double)h * __longlong_as_double((long long)((unsigned long long)(b + 1) << shift));
-    C += h;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if (j >= per) break;
+    const int b = top - j;
+    if (h[j]) S += (double)h[j] * __longlong_as_double((long long)((unsigned long long)(b + 1) << shift));
+    C += h[j];
     bool stop = C >= m;
     // only where the next bin holds something can the bound improve
-    if (!stop && bound && b > 0 && hist[b - 1]) {
+    if (!stop && bound && b > 0 && h[j + 1]) {
       const double e = __longlong_as_double((long long)((unsigned long long)b << shift));
       const double slack = norm * ((double)(C + 2) * 0x1p-52 + 0x1p-38);
       stop = (double)(m - C) * e < (norm - S - e - slack) * (1.0 - 0x1p-20);
@@ -505,8 +513,10 @@ __device__ __forceinline__ void set_d(Ctl* c, int64_t nd, double R, const unsign
 // The first chunks of the remaining-norm chain, in one block, until the
 // acceptance test first fails (D is usually a few thousand entries: one or
 // two chunks).  Sets c->found, and the chain's general kernels then have
-// nothing to do; a longer D leaves them the whole chain.
-constexpr int REM_CHUNKS = 4;
+// nothing to do; a longer D leaves them the whole chain.  Up to this many chunks
+// (m <= 32768) those kernels, ~15 us even with nothing to do, are not launched;
+// a chunk takes ~4 us here, so a D that fills them costs no more than they did.
+constexpr int REM_CHUNKS = 8;
 __global__ void __launch_bounds__(1024) k_rem_first(ConsAccept ca0, const unsigned long long* ckey,
                                                     const unsigned* cidx, Ctl* c, Rep rp = Rep{}) {
   const int rep = blockIdx.x;

@@ -10,7 +10,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-RANK_MAX, FIRST = 16384, 4 * 4096  # candidates ranked directly; chain elements of the first block
+RANK_MAX, FIRST = 16384, 8 * 4096  # candidates ranked directly; chain elements of the first block
 
 
 def _inputs(name):
