@@ -8,10 +8,11 @@
 // so its whole state is the history h = (r_{k-31}, ..., r_{k-1}) before the
 // next draw.  Advancing the history by one draw is a fixed 31x31 linear map M
 // over Z/2^32; by C draws it is J = M^C, built on the host by repeated
-// squaring.  One block walks the chunk starts h_{cC} = J h_{(c-1)C}, then one
-// thread per chunk produces its C uniforms from its start, the ring of 31
-// words held in registers (the loop is unrolled 31 deep so every ring index
-// is static).  The history after the last draw goes back to the caller, so a
+// squaring.  One block squares J up to the number of chunks, a warp per chunk
+// takes the powers of its number's binary digits to its start h_{cC} = J^c h_0,
+// and one thread per chunk produces its C words from there, the ring of 31 words
+// held in registers (the loop is unrolled 31 deep so every ring index is
+// static).  The history after the last draw goes back to the caller, so a
 // host-side copy of the stream continues exactly where the device stopped.
 #include <vector>
 
@@ -21,26 +22,45 @@ namespace {
 
 constexpr int RDEG = 31;
 constexpr int RSEP = 3;
-constexpr int64_t GCH = 31 * 64;  // draws per chunk (a multiple of the ring length)
+// Draws per chunk (a multiple of the ring length).  With the starts one after
+// another and 1984 draws each, the 549081 draws of o13v57 took 50 us of starts and
+// 51 of draws; now 17 (the powers), 9 and 8.
+constexpr int64_t GCH = 31 * 8;
 
-// out[c * 31 + t] = history at the start of chunk c (oldest first)
-__global__ void k_glibc_starts(const unsigned* __restrict__ J, const unsigned* __restrict__ h0, int64_t nch,
-                               unsigned* __restrict__ starts) {
-  __shared__ unsigned h[RDEG];
-  __shared__ unsigned Js[RDEG * RDEG];
-  const int t = threadIdx.x;
-  for (int i = t; i < RDEG * RDEG; i += blockDim.x) Js[i] = J[i];
-  if (t < RDEG) h[t] = h0[t];
-  __syncthreads();
-  for (int64_t c = 0; c < nch; ++c) {
-    unsigned nx = 0;
-    if (t < RDEG) {
-      starts[c * RDEG + t] = h[t];
-      for (int s = 0; s < RDEG; ++s) nx += Js[t * RDEG + s] * h[s];  // wraps mod 2^32
+// P[b][s * 31 + t] = J^(2^b)[t][s] for b < nb; 1024 threads
+__global__ void __launch_bounds__(1024) k_glibc_powers(const unsigned* __restrict__ J, int nb, unsigned* __restrict__ P) {
+  __shared__ unsigned A[RDEG * RDEG];
+  const int i = threadIdx.x, t = i / RDEG, s = i - t * RDEG;
+  const bool in = i < RDEG * RDEG;
+  if (in) A[i] = J[i];
+  for (int b = 0; b < nb; ++b) {
+    __syncthreads();
+    unsigned x = 0;
+    if (in) {
+      P[b * RDEG * RDEG + s * RDEG + t] = A[i];
+#pragma unroll
+      for (int q = 0; q < RDEG; ++q) x += A[t * RDEG + q] * A[q * RDEG + s];  // wraps mod 2^32
     }
     __syncthreads();
-    if (t < RDEG) h[t] = nx;
-    __syncthreads();
+    if (in) A[i] = x;
+  }
+}
+
+// starts[c * 31 + t] = history at the start of chunk c (oldest first)
+__global__ void __launch_bounds__(256) k_glibc_starts(const unsigned* __restrict__ P, const unsigned* __restrict__ h0,
+                                                      int64_t nch, unsigned* __restrict__ starts) {
+  const int lane = threadIdx.x & 31, t = lane < RDEG ? lane : 0;
+  for (int64_t c = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); c < nch; c += (int64_t)gridDim.x * 8) {
+    unsigned h = h0[t];
+    const unsigned* m = P;
+    for (int64_t q = c; q; q >>= 1, m += RDEG * RDEG)
+      if (q & 1) {
+        unsigned x = 0;
+#pragma unroll
+        for (int s = 0; s < RDEG; ++s) x += __ldg(m + s * RDEG + t) * __shfl_sync(0xffffffffu, h, s);
+        h = x;
+      }
+    if (lane < RDEG) starts[c * RDEG + lane] = h;
   }
 }
 
@@ -74,7 +94,7 @@ __global__ void k_glibc_gen(const unsigned* __restrict__ starts, int64_t nch, in
     // cnt draws leave the oldest word at ring index cnt % 31
     const int off = (int)(cnt % RDEG);
 #pragma unroll
-    for (int t = 0; t < RDEG; ++t) hist_out[t] = r[(off + t) % RDEG];
+    for (int t = 0; t < RDEG; ++t) hist_out[t >= off ? t - off : t - off + RDEG] = r[t];  // (static ring indices)
   }
 }
 
@@ -125,7 +145,9 @@ int fricc_glibc_uniforms_device(unsigned* hist, int64_t k, double* out, cudaStre
   const int64_t nch = fricc_cdiv(k, GCH);
   static const Mat J = step_power(GCH);
   unsigned *dJ = nullptr, *dh = nullptr, *starts = nullptr, *words = nullptr;
-  int rc = fricc_alloc_t(&dJ, RDEG * RDEG + 2 * RDEG, st);
+  int nb = 0;  // bits of the last chunk's number
+  while ((nch - 1) >> nb) ++nb;
+  int rc = fricc_alloc_t(&dJ, (size_t)(1 + nb) * RDEG * RDEG + 2 * RDEG, st);
   if (!rc) rc = fricc_alloc_t(&starts, nch * RDEG, st);
   if (!rc) rc = fricc_alloc_t(&words, k, st);
   if (rc) {
@@ -133,17 +155,20 @@ int fricc_glibc_uniforms_device(unsigned* hist, int64_t k, double* out, cudaStre
     fricc_free(starts, st);
     return rc;
   }
-  dh = dJ + RDEG * RDEG;
+  unsigned* const powers = dJ + RDEG * RDEG;
+  dh = powers + (size_t)nb * RDEG * RDEG;
   unsigned* dout = dh + RDEG;
   // pageable sources: the copies complete before cudaMemcpyAsync returns
   cudaError_t e = cudaMemcpyAsync(dJ, J.data(), sizeof(unsigned) * RDEG * RDEG, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dh, hist, sizeof(unsigned) * RDEG, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
-    k_glibc_starts<<<1, 32, 0, st>>>(dJ, dh, nch, starts);
+    const int64_t gs = fricc_cdiv(nch, 8);
+    k_glibc_powers<<<1, 1024, 0, st>>>(dJ, nb, powers);
+    k_glibc_starts<<<(unsigned)(gs < 152 * 8 ? gs : 152 * 8), 256, 0, st>>>(powers, dh, nch, starts);
     k_glibc_gen<<<(unsigned)fricc_cdiv(nch, 32), 32, 0, st>>>(starts, nch, k, words, dout);
     const int64_t g = fricc_cdiv(k, 256);
     k_glibc_uniform<<<(unsigned)(g < 152 * 16 ? g : 152 * 16), 256, 0, st>>>(words, k, out);
-    fricc_note_launch(3);
+    fricc_note_launch(4);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(hist, dout, sizeof(unsigned) * RDEG, cudaMemcpyDeviceToHost, st);
