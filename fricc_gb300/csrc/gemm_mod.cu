@@ -771,7 +771,14 @@ __device__ __forceinline__ void store_c(const CombineArgs& a, double* p, double 
   else *p = fma(a.out.beta, *p, x);
 }
 
-// The Chinese remainder sum of 14 residues as a signed 96-bit fraction of M,
+// v 2^e where that is subnormal or overflows (kept out of line: FP64
+// instructions)
+static __device__ __noinline__ double scaled_far(unsigned long long v, int e, bool neg) {
+  const double x = scalbn((double)v, e);
+  return neg ? -x : x;
+}
+
+// The Chinese remainder sum of 15 residues as a signed 96-bit fraction of M,
 // times M 2^-sh, rounded once to FP64 (integers only: FP64 operations on
 // this part cost more than the whole conversion).  *zero: the value is 0.
 __device__ __forceinline__ double crt(const int* r, int sh, bool* zero) {
@@ -786,45 +793,47 @@ __device__ __forceinline__ double crt(const int* r, int sh, bool* zero) {
   const unsigned l0 = (unsigned)a0;
   a1 += a0 >> 32;
   const unsigned l1 = (unsigned)a1;
-  a2 += a1 >> 32;
-  unsigned l2 = (unsigned)a2;
-  unsigned long long lo = ((unsigned long long)l1 << 32) | l0;
-  const bool neg = (int)l2 < 0;
-  if (neg) {
-    lo = 0ull - lo;
-    l2 = ~l2 + (lo == 0 ? 1u : 0u);
+  const unsigned l2 = (unsigned)(a2 + (a1 >> 32));
+  // |F| as three words, the top bits first
+  const unsigned sg = (unsigned)((int)l2 >> 31);
+  unsigned m0 = l0 ^ sg, m1 = l1 ^ sg, m2 = l2 ^ sg;
+  if (sg) {
+    m0 += 1u;
+    m1 += m0 == 0u ? 1u : 0u;
+    m2 += (m0 | m1) == 0u ? 1u : 0u;
   }
-  *zero = l2 == 0 && lo == 0;
-  if (*zero) return 0.0;
+  int lz = 0;
+  *zero = false;
+  if (m2 == 0u) {  // a small value, or none: whole words first
+    lz = 32;
+    m2 = m1;
+    m1 = m0;
+    m0 = 0u;
+    if (m2 == 0u) {
+      lz = 64;
+      m2 = m1;
+      m1 = 0u;
+      if (m2 == 0u) {
+        *zero = true;
+        return 0.0;
+      }
+    }
+  }
   // the top 64 bits of the magnitude, normalised: |F| = t 2^(32 - lz)
-  int lz;
-  unsigned long long t;
-  if (l2) {
-    lz = __clz((int)l2);
-    const unsigned long long hi = ((unsigned long long)l2 << 32) | (lo >> 32);
-    t = lz ? (hi << lz) | ((lo & 0xffffffffull) >> (32 - lz)) : hi;
-  } else {
-    const int z = __clzll((long long)lo);
-    lz = 32 + z;
-    t = lo << z;
-  }
+  const int z = __clz((int)m2);
+  lz += z;
+  const unsigned long long t = ((unsigned long long)__funnelshift_l(m1, m2, z) << 32) | __funnelshift_l(m0, m1, z);
   unsigned long long v = __umul64hi(t, TAB.mtop);  // value = v 2^(62 - lz - sh)
-  int e = 62 - lz - sh;
+  int be = 62 - lz - sh + 63 + 1023;
   if (!(v >> 63)) {
     v <<= 1;
-    --e;
+    --be;
   }
-  const int be = e + 63 + 1023;
-  double x;
-  if (be >= 1 && be <= 2045) {
-    const unsigned long long low = v & 0x7ff;
-    unsigned long long m = v >> 11;  // 53 bits
-    m += (low > 0x400 || (low == 0x400 && (m & 1))) ? 1 : 0;
-    x = __longlong_as_double((long long)(((unsigned long long)(be - 1) << 52) + m));
-  } else {
-    x = scalbn((double)v, e);
-  }
-  return neg ? -x : x;
+  if (be < 1 || be > 2045) return scaled_far(v, be - 1086, sg != 0);
+  const unsigned low = (unsigned)v & 0x7ffu;
+  unsigned long long m = v >> 11;  // 53 bits
+  m += (low + ((unsigned)m & 1u) > 0x400u) ? 1 : 0;  // half to even
+  return __longlong_as_double((long long)((((unsigned long long)(be - 1) << 52) + m) | ((unsigned long long)sg << 63)));
 }
 
 // K slices: slice 0 += the others (64 residues of at most 182 fit 16 bits)
@@ -858,13 +867,12 @@ constexpr float GUARD = 0x1p-16f;
 
 // One 32 x 64 tile of outputs per step: residues in, C out, and an entry on
 // the list for a tile with outputs to recompute (which are left alone).  A
-// warp reads 128-byte runs: 4 rows of a 16-column group, two adjacent columns
-// per lane.  Bound by its bytes (2 per plane in, 8-16 out per output) and
-// ~150 integer issues an output.
-// Masks: byte (column / 16) * 2 + (column & 1) of a row, bit (column % 16) / 2.
-__device__ __forceinline__ bool masked(const unsigned char* row, int c) {
-  return (row[(c >> 4) * 2 + (c & 1)] >> ((c & 15) >> 1)) & 1u;
-}
+// warp reads 256-byte runs: 8 rows of a 16-column group, four adjacent columns
+// per lane (128-byte runs and two columns took 288 us for 900 x 22500 outputs, 264
+// for 4500^2; now 231 and 244).  Its bytes (2 per plane in, 8-16 out per output)
+// would take 140; ~290 instructions an output keep it from them.
+// Masks: 64 column bits per row.
+__device__ __forceinline__ bool masked(const unsigned char* row, int c) { return (row[c >> 3] >> (c & 7)) & 1u; }
 
 __global__ void __launch_bounds__(256, 4) k_mod_combine(CombineArgs a, int64_t ntiles) {
   __shared__ double t[32][65];
@@ -873,61 +881,63 @@ __global__ void __launch_bounds__(256, 4) k_mod_combine(CombineArgs a, int64_t n
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t tn = fricc_cdiv(a.N, (int64_t)64), per = fricc_cdiv(a.M, (int64_t)32) * tn;
   const bool gave_up = *a.err != 0;
-  const int cg = warp & 3, cl = cg * 16 + 2 * (lane & 7);
+  const int cg = warp & 3, cl = cg * 16 + 4 * (lane & 3);
   for (int64_t b = blockIdx.x; b < ntiles; b += gridDim.x) {
     const int64_t rep = b / per, w = b - rep * per;
     const int64_t r0 = (w / tn) * 32, c0 = (w % tn) * 64;
     const int64_t c = c0 + cl;
-    int shb[2];
-    unsigned nb[2];
+    int shb[4];
+    unsigned nb[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < 4; ++h) {
       shb[h] = c + h < a.N ? a.shb[rep * a.b_rep + c + h] : 0;
       nb[h] = c + h < a.N ? a.cntb[rep * a.b_rep + c + h] : 0u;
     }
     unsigned any = 0;
 #pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-      const int rl = (warp >> 2) * 16 + 4 * q + (lane >> 3);
+    for (int q = 0; q < 2; ++q) {
+      const int rl = (warp >> 2) * 16 + 8 * q + (lane >> 2);
       const int64_t r = r0 + rl;
-      bool bad[2] = {false, false};
-      if (r < a.M && c < a.N) {  // (groups are whole: the pair's second residue exists)
-        const unsigned short* res = a.res + rep * a.rep_stride + (((c0 >> 4) + cg) * a.M + r) * 16 + 2 * (lane & 7);
-        unsigned w2[PLANES];
+      unsigned no = 0;
+      if (r < a.M && c < a.N) {  // (groups are whole: the other columns' residues exist)
+        const unsigned short* res = a.res + rep * a.rep_stride + (((c0 >> 4) + cg) * a.M + r) * 16 + 4 * (lane & 3);
+        uint2 w4[PLANES];
 #pragma unroll
-        for (int i = 0; i < PLANES; ++i)
-          w2[i] = __ldg(reinterpret_cast<const unsigned*>(res + i * a.plane_stride));
-        int ri[2][NP];
-        float s2[2] = {__uint_as_float(w2[NP] << 16), __uint_as_float(w2[NP] & 0xffff0000u)};
-#pragma unroll
-        for (int i = 0; i < NP; ++i) {
-          ri[0][i] = (short)w2[i];
-          ri[1][i] = (int)w2[i] >> 16;
-        }
+        for (int i = 0; i < PLANES; ++i) w4[i] = __ldg(reinterpret_cast<const uint2*>(res + i * a.plane_stride));
         const int sha = a.sha[rep * a.a_rep + r];
         const unsigned na = a.cnta[rep * a.a_rep + r];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          bool zero = false;
+        for (int h = 0; h < 4; ++h) {
+          int ri[NP];
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            const unsigned v = h < 2 ? w4[i].x : w4[i].y;
+            ri[i] = h & 1 ? (int)v >> 16 : (int)(short)v;
+          }
+          const unsigned v = h < 2 ? w4[NP].x : w4[NP].y;
+          const float s2 = __uint_as_float(h & 1 ? v & 0xffff0000u : v << 16);
+          bool zero = false, bad = false;
           double x = 0.0;
           if (gave_up || sha == SH_BAD || shb[h] == SH_BAD) {
-            bad[h] = c + h < a.N;
+            bad = c + h < a.N;
           } else {
-            x = crt(ri[h], sha + shb[h], &zero);
+            x = crt(ri, sha + shb[h], &zero);
             const float n = (float)(na < nb[h] ? na : nb[h]);
-            bad[h] = c + h < a.N && !(n * s2[h] >= GUARD) && !(zero && s2[h] == 0.0f);
+            bad = c + h < a.N && !(n * s2 >= GUARD) && !(zero && s2 == 0.0f);
           }
+          no |= bad ? 1u << h : 0u;
           t[rl][cl + h] = x;
         }
       }
-      const unsigned m0 = __ballot_sync(0xffffffffu, bad[0]), m1 = __ballot_sync(0xffffffffu, bad[1]);
-      if ((lane & 7) == 0) {
-        mask[rl][2 * cg] = (unsigned char)(m0 >> lane);
-        mask[rl][2 * cg + 1] = (unsigned char)(m1 >> lane);
-      }
-      any |= m0 | m1;
+      // the row's 16 bits of this group
+      no <<= 4 * (lane & 3);
+      no |= __shfl_xor_sync(0xffffffffu, no, 1);
+      no |= __shfl_xor_sync(0xffffffffu, no, 2);
+      if ((lane & 3) == 0) *reinterpret_cast<unsigned short*>(&mask[rl][2 * cg]) = (unsigned short)no;
+      any |= no;
     }
-    if (__syncthreads_or(any)) {
+    const bool bad = __syncthreads_or(any);
+    if (bad) {
       if (threadIdx.x == 0) {
         at = atomicAdd(a.count, 1u) * LIST_W;
         a.list[at] = (unsigned)b;
@@ -937,24 +947,22 @@ __global__ void __launch_bounds__(256, 4) k_mod_combine(CombineArgs a, int64_t n
     }
     double* C = a.out.C + a.out.rep.at(rep);
     if (a.col_fast) {
+      const bool in0 = c0 + lane < a.N, in1 = c0 + lane + 32 < a.N;
+      const int64_t cc0 = in0 ? a.out.col.at(c0 + lane) : 0, cc1 = in1 ? a.out.col.at(c0 + lane + 32) : 0;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = lane + 32 * h;
-        if (c0 + j < a.N) {
-          const int64_t cc = a.out.col.at(c0 + j);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int rl = warp + 8 * q;
-            if (r0 + rl < a.M && !masked(mask[rl], j)) store_c(a, C + a.out.row.at(r0 + rl) + cc, t[rl][j]);
-          }
-        }
+      for (int q = 0; q < 4; ++q) {
+        const int rl = warp + 8 * q;
+        if (r0 + rl >= a.M) break;
+        double* row = C + a.out.row.at(r0 + rl);
+        if (in0 && !(bad && masked(mask[rl], lane))) store_c(a, row + cc0, t[rl][lane]);
+        if (in1 && !(bad && masked(mask[rl], lane + 32))) store_c(a, row + cc1, t[rl][lane + 32]);
       }
     } else if (r0 + lane < a.M) {
       const int64_t rr = a.out.row.at(r0 + lane);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int j = warp + 8 * q;
-        if (c0 + j < a.N && !masked(mask[lane], j)) store_c(a, C + rr + a.out.col.at(c0 + j), t[lane][j]);
+        if (c0 + j < a.N && !(bad && masked(mask[lane], j))) store_c(a, C + rr + a.out.col.at(c0 + j), t[lane][j]);
       }
     }
     __syncthreads();  // before the next tile's values and masks
@@ -1103,15 +1111,15 @@ double fricc_mod_time_us(int64_t M, int64_t N, int64_t K, int64_t reps, bool a_s
                          bool conv_b) {
   if (K < 1 || K > mod::MAX_K) return 1e30;
   // measured on a GB300: the product at the model's clocks (1.7 GHz) or at
-  // 6 TB/s of planes, conversions at 12 ps an element, the combine at 17 ps
+  // 6 TB/s of planes, conversions at 10.5 ps an element, the combine at 12.5 ps
   // an output, ~8 us a kernel (its launch and scratch included: an o10v40
   // iteration is bound by the host)
   const mod::Plan p = mod::plan_for(M, N, K, reps, 152);
   const double kp = (double)fricc_cdiv(K, tc::BK) * tc::BK;
   const double ea = (double)(a_shared ? 1 : reps) * M * kp, eb = (double)(b_shared ? 1 : reps) * N * kp;
   const double planes = (ea + eb) * 2.0 * mod::PLANES / 6.0e6, mma = p.clocks / 1700.0;
-  return (mma > planes ? mma : planes) + 12e-6 * ((conv_a ? ea : 0.0) + (conv_b ? eb : 0.0)) +
-         17e-6 * (double)reps * M * N + 8.0 * (3 + (p.ks > 1) + ((conv_a ? 1 : 0) + (conv_b ? 1 : 0)) * (K > mod::SCH ? 3 : 1));
+  return (mma > planes ? mma : planes) + 10.5e-6 * ((conv_a ? ea : 0.0) + (conv_b ? eb : 0.0)) +
+         12.5e-6 * (double)reps * M * N + 8.0 * (3 + (p.ks > 1) + ((conv_a ? 1 : 0) + (conv_b ? 1 : 0)) * (K > mod::SCH ? 3 : 1));
 }
 
 // The scratch of one product is bounded: an operand of more than this many
