@@ -60,7 +60,6 @@ FP32_PEAK_FALLBACK = 74.2
 # Keys: (precision, workload) -> {term: bytes per launch}; "mean" is the
 # mean over the iteration's launches of that kernel.
 SPMM_TRAFFIC_CAPTURED = {
-    ("fp64", "o30v150"): {"mean": 3.97e9, "2323": 26.0e9, "XY": 9.64e9, "O3V3": 0.54e9},
     ("df64", "o30v150"): {"2323": 36.1e9, "XY": 13.85e9},
 }
 
@@ -578,10 +577,8 @@ def run_gpu(args):
             "frac": (achieved / peak) if achieved else None,
             "traffic": traffic.get("mean") if traffic else None,
             "traffic_per_launch_captured": traffic,
-            "traffic_note": ("DRAM bytes per launch (mean over the iteration's launches of the kernel) from one "
-                             "single-pass ncu capture of an iteration of this workload with this build, not measured "
-                             "by this run; the 2323 launch re-reads its W' (algorithmic 4.37 GB) ~6x without "
-                             "costing time: the kernel is bound by the FP64 pipe, not DRAM"),
+            "traffic_note": ("DRAM bytes per launch from one single-pass ncu capture of an iteration of this workload, "
+                             "not measured by this run") if traffic else None,
             "flops_counted": "2 m Q per launch (m nonzeros, Q outputs per nonzero): algorithmic, no padding",
             "launches": int(p_n.value), "kernel_ms": p_ms.value,
             "kernel_share_of_step": p_ms.value / ms if ms > 0 else None,
@@ -593,6 +590,25 @@ def run_gpu(args):
                 "achieved": g_ach, "peak": pk["fp64"], "unit": "TFLOP/s",
                 "frac": (g_ach / pk["fp64"]) if g_ach else None, "launches": int(g_n.value),
                 "kernel_ms": g_ms.value, "kernel_share_of_step": g_ms.value / ms if ms > 0 else None}
+    if args.precision in ("fp64", "df64") and t_n.value:
+        # the FP64-accurate products on the tensor cores carry the step where
+        # the sizes choose them; the FP64 / FP32-pair kernels have the rest
+        sus = measured_peaks().get("bf16_tflops_sustained")
+        tc_ach = (t_fl.value / (t_ms.value / 1000.0)) / 1e12 if t_ms.value > 0 else None
+        mod = {"kernel": "k_mod_gemm (tcgen05 modular GEMMs: the large sparse terms on the zero-filled compressed T2 "
+                         "and the large dense contractions, FP64-accurate)",
+               "bound": "tensor", "achieved": tc_ach, "peak": sus, "unit": "TFLOP/s",
+               "frac": (tc_ach / sus) if (tc_ach and sus) else None, "traffic": None,
+               "launches": int(t_n.value), "kernel_ms": t_ms.value,
+               "kernel_share_of_step": t_ms.value / ms if ms > 0 else None,
+               "flops_counted": "32 M N K per product (2 M N K for each of 15 moduli and the plane of squares), the "
+                                "zeros of the compressed T2 included, tile padding not",
+               "peak_source": "bf16_tflops_sustained of MEASURED_PEAKS.json (kernels timed inside the step)"}
+        if t_ms.value > p_ms.value:
+            mod["sparse_kernel"] = roof if roof.get("launches") else None
+            roof = mod
+        else:
+            roof["modular_gemm"] = mod
     if args.precision == "split":
         # the dominant kernel of the split form: the tensor-core GEMMs
         sus = measured_peaks().get("bf16_tflops_sustained")

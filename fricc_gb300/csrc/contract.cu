@@ -15,6 +15,10 @@
 // the bucketing is a stable sort, so each output element here receives its
 // contributions in the same order (fused multiply-add, one rounding per
 // term instead of two).
+//
+// Where the sizes choose it (fricc_spmm_takes_mod), a term runs instead as one
+// FP64-accurate product on the tensor cores with T as a zero-filled matrix
+// (gemm_mod.cu): its sums are of all the products, rounded once.
 #include <cmath>
 #include <cstring>
 
@@ -710,7 +714,7 @@ int fricc_sparse_bucketing(FriccSparse* T, int pa, int pb, cudaStream_t st, Buck
   if (!rc && fresh) rc = fricc_alloc_t(&slot->bptr, nb + 1, st);
   if (!rc) {
     k_pair_keys<<<grid_for(m, 256), 256, 0, st>>>(T->slots, m, pa, pb, T->dims[pb], keys, slot->order);
-    rc = radix::sort_pairs(keys, slot->order, ktmp, vtmp, m, bits, false, hist, st);
+    rc = radix::sort_pairs(keys, slot->order, ktmp, vtmp, m, bits, hist, st);
     fricc_note_launch(1);
   }
   if (!rc) {
@@ -1147,7 +1151,7 @@ int fricc_batch_bucketing(FriccSparseBatch* B, int which, int pa, int pb, cudaSt
     radix::Batch bt;
     bt.kv_stride = m;
     bt.hist_stride = hw;
-    rc = radix::sort_pairs(keys, slot->order, ktmp, vtmp, m, bits, false, hist, st, nullptr, R, bt);
+    rc = radix::sort_pairs(keys, slot->order, ktmp, vtmp, m, bits, hist, st, R, bt);
     fricc_note_launch(1);
     if (!rc) {
       k_bptr<<<dim3(grid_for(nb + 1, 256), R), 256, 0, st>>>(keys, m, nb, slot->bptr, rp);

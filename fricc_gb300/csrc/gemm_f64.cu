@@ -11,7 +11,8 @@
 // tile only has to keep enough warps on every SM.  Each output is summed in
 // k order (deterministic); a long K with few output tiles is split over
 // blockIdx.x (beside the N tiles; blockIdx.z is the batch) and the partial
-// tiles summed afterwards in slice order.
+// tiles summed afterwards in slice order.  Large products leave this pipe
+// altogether (fricc_mod_try, gemm_mod.cu).
 #include "gemm_mod.cuh"
 
 namespace {

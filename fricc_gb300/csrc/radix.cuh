@@ -1,10 +1,9 @@
-// Stable LSD radix sort of (uint64 key, uint32 value) pairs, 8-bit digits.
-//
-// Used twice on the FRI path: to order the top-m candidates by descending
-// |x| with ties in ascending flat index (the order a stable merge sort by
-// |x| gives, fri-cc src/fri_utils.cpp:22-25), and to bucket the nonzeros
-// of a SparseTensor4d by an index pair while keeping nonzero-slot order
-// inside each bucket (the accumulation order of src/sparse_tensor.cpp).
+// Stable sorts of (uint64 key, uint32 value) pairs on the FRI path: an LSD
+// radix sort, 8-bit digits, that buckets the nonzeros of a SparseTensor4d by an
+// index pair while keeping nonzero-slot order inside each bucket (the
+// accumulation order of src/sparse_tensor.cpp), and below it the descending sort
+// of a compression's candidates by |x| with ties in ascending flat index (the
+// order a stable merge sort by |x| gives, fri-cc src/fri_utils.cpp:22-25).
 #pragma once
 #include "common.cuh"
 
@@ -14,29 +13,21 @@ constexpr int NT = 256;
 constexpr int IPT = 8;
 constexpr int TILE = NT * IPT;
 
-__device__ __forceinline__ unsigned digit(unsigned long long k, int shift, int desc) {
-  const unsigned d = (unsigned)(k >> shift) & 255u;
-  return desc ? 255u - d : d;
-}
+__device__ __forceinline__ unsigned digit(unsigned long long k, int shift) { return (unsigned)(k >> shift) & 255u; }
 
-// n_dev (optional): the element count in device memory, overriding n; tiles
-// past it count nothing (and scatter nothing), so a sort can be launched for
-// a worst-case size without the host knowing the real one.
-//
 // Replica batches: blockIdx.y (blockIdx.x for k_scan_digits) is the replica;
 // its keys and values start kv_stride elements after the previous one's,
-// its histogram hist_stride words after, its n_dev n_stride int64s after.
+// its histogram hist_stride words after, its element count (of the sort that
+// reads it from the device) n_stride int64s after.
 struct Batch {
   int64_t kv_stride = 0, hist_stride = 0, n_stride = 0;
 };
 
 static __global__ void __launch_bounds__(NT) k_hist(const unsigned long long* __restrict__ keys, int64_t n, int shift,
-                                             int desc, unsigned* __restrict__ hist, int64_t ntiles,
-                                             const int64_t* __restrict__ n_dev, Batch bt) {
+                                             unsigned* __restrict__ hist, int64_t ntiles, Batch bt) {
   const int rep = blockIdx.y;
   keys += rep * bt.kv_stride;
   hist += rep * bt.hist_stride;
-  if (n_dev) n = n_dev[rep * bt.n_stride];
   __shared__ unsigned h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -44,7 +35,7 @@ static __global__ void __launch_bounds__(NT) k_hist(const unsigned long long* __
 #pragma unroll
   for (int r = 0; r < IPT; ++r) {
     const int64_t i = base + r * NT + threadIdx.x;
-    if (i < n) atomicAdd(&h[digit(keys[i], shift, desc)], 1u);
+    if (i < n) atomicAdd(&h[digit(keys[i], shift)], 1u);
   }
   __syncthreads();
   hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
@@ -84,9 +75,8 @@ static __global__ void __launch_bounds__(256) k_scan_digits(const unsigned* tota
 static __global__ void __launch_bounds__(NT) k_scatter(const unsigned long long* __restrict__ kin,
                                                 const unsigned* __restrict__ vin,
                                                 unsigned long long* __restrict__ kout, unsigned* __restrict__ vout,
-                                                int64_t n, int shift, int desc, const unsigned* __restrict__ offs,
-                                                int64_t ntiles, const unsigned* __restrict__ dbase,
-                                                const int64_t* __restrict__ n_dev, Batch bt) {
+                                                int64_t n, int shift, const unsigned* __restrict__ offs, int64_t ntiles,
+                                                const unsigned* __restrict__ dbase, Batch bt) {
   const int rep = blockIdx.y;
   kin += rep * bt.kv_stride;
   vin += rep * bt.kv_stride;
@@ -94,8 +84,6 @@ static __global__ void __launch_bounds__(NT) k_scatter(const unsigned long long*
   vout += rep * bt.kv_stride;
   offs += rep * bt.hist_stride;
   dbase += rep * bt.hist_stride;
-  if (n_dev) n = n_dev[rep * bt.n_stride];
-  if ((int64_t)blockIdx.x * TILE >= n) return;  // uniform per block
   constexpr int NW = NT / 32;
   __shared__ unsigned run[256];
   __shared__ unsigned wc[NW][256];
@@ -116,7 +104,7 @@ static __global__ void __launch_bounds__(NT) k_scatter(const unsigned long long*
     if (valid) {
       key = kin[i];
       val = vin[i];
-      d = digit(key, shift, desc);
+      d = digit(key, shift);
     }
     const unsigned peers = __match_any_sync(0xffffffffu, d);
     const unsigned lrank = __popc(peers & lt);
@@ -142,7 +130,7 @@ static __global__ void __launch_bounds__(NT) k_scatter(const unsigned long long*
   }
 }
 
-// Sorts n pairs on key bits [0, bits) (or *n_dev <= n pairs, when given).
+// Sorts n pairs on key bits [0, bits), ascending.
 // The result ends in (keys, vals); the tmp buffers must hold n entries, hist
 // hist_words(n) counts.
 inline int64_t hist_words(int64_t n) { return 256 * fricc_cdiv(n, TILE) + 512; }
@@ -151,8 +139,7 @@ inline int64_t hist_words(int64_t n) { return 256 * fricc_cdiv(n, TILE) + 512; }
 // each n long; hist holds R * hist_stride words, hist_stride >=
 // hist_words(n)).
 inline int sort_pairs(unsigned long long* keys, unsigned* vals, unsigned long long* ktmp, unsigned* vtmp,
-                      int64_t n, int bits, bool desc, unsigned* hist, cudaStream_t st,
-                      const int64_t* n_dev = nullptr, int R = 1, Batch bt = Batch{}) {
+                      int64_t n, int bits, unsigned* hist, cudaStream_t st, int R = 1, Batch bt = Batch{}) {
   if (n <= 1) return FRICC_OK;
   if (n > 0xffffffffLL || R < 1 || R > 65535) return FRICC_ERR_ARG;
   const int64_t ntiles = fricc_cdiv(n, TILE);
@@ -162,11 +149,11 @@ inline int sort_pairs(unsigned long long* keys, unsigned* vals, unsigned long lo
   for (int shift = 0; shift < bits; shift += 8, ++passes) {
     unsigned* totals = hist + 256 * ntiles;
     unsigned* base = totals + 256;
-    k_hist<<<dim3((unsigned)ntiles, (unsigned)R), NT, 0, st>>>(ka, n, shift, desc ? 1 : 0, hist, ntiles, n_dev, bt);
+    k_hist<<<dim3((unsigned)ntiles, (unsigned)R), NT, 0, st>>>(ka, n, shift, hist, ntiles, bt);
     k_scan_rows<<<dim3(256, (unsigned)R), 256, 0, st>>>(hist, ntiles, totals, bt);
     k_scan_digits<<<R, 256, 0, st>>>(totals, base, bt);
-    k_scatter<<<dim3((unsigned)ntiles, (unsigned)R), NT, 0, st>>>(ka, va, kb, vb, n, shift, desc ? 1 : 0, hist,
-                                                                  ntiles, base, n_dev, bt);
+    k_scatter<<<dim3((unsigned)ntiles, (unsigned)R), NT, 0, st>>>(ka, va, kb, vb, n, shift, hist, ntiles, base,
+                                                                  bt);
     fricc_note_launch(4);
     unsigned long long* tk = ka;
     ka = kb;
@@ -314,7 +301,7 @@ static __global__ void __launch_bounds__(NT) k_sort_coop(unsigned long long* ksr
 #pragma unroll
         for (int q = 0; q < IPT; ++q) {
           const int64_t i = t * TILE + q * NT + threadIdx.x;
-          if (i < n) atomicAdd(&h[digit(k[i], shift, 1)], 1u);
+          if (i < n) atomicAdd(&h[(255u - digit(k[i], shift))], 1u);
         }
         __syncthreads();
         hr[(int64_t)threadIdx.x * nt + t] = h[threadIdx.x];
@@ -361,7 +348,7 @@ static __global__ void __launch_bounds__(NT) k_sort_coop(unsigned long long* ksr
           const bool valid = i < n;
           const unsigned long long key = valid ? ka[o + i] : 0ull;
           const unsigned val = valid ? va[o + i] : 0u;
-          const unsigned d = valid ? digit(key, shift, 1) : 256u;
+          const unsigned d = valid ? (255u - digit(key, shift)) : 256u;
           const unsigned peers = __match_any_sync(0xffffffffu, d);
           const unsigned lrank = __popc(peers & lt);
           if (valid && lrank == 0) wc[w][d] = __popc(peers);
