@@ -80,7 +80,18 @@ def _split_view(x, rows, k, ri, sro, sri, sk, want_a, want_b):
     Bp = torch.empty(rows, kp, dtype=torch.bfloat16, device=x.device) if want_b else None
     L.check(L.load().fricc_split_bf16x3_strided(_p(x), rows, k, ri, sro, sri, sk, kp,
                                                 _p(Ap) if want_a else None, _p(Bp) if want_b else None, _st()))
-    return Ap if want_a else Bp
+    return (Ap, Bp) if want_a and want_b else (Ap if want_a else Bp)
+
+
+def split_factor(X: torch.Tensor, want_a: bool = True, want_b: bool = True):
+    """The split operands (A', B', or the one wanted) of a factor slice X [naux,
+    p, q], rows (p,q) and K = naux: straight from X where the transposing pass
+    takes it (rows of 32 contiguous q), else through a copy."""
+    naux, n1, n2 = X.shape
+    if n2 >= 32 and X.stride(2) == 1 and X.dtype == torch.float64 and X.is_cuda:
+        return _split_view(X, n1 * n2, naux, n2, X.stride(1), 1, X.stride(0), want_a, want_b)
+    AB = split_bf16x3(X.reshape(naux, -1).t().contiguous())
+    return AB if want_a and want_b else AB[0 if want_a else 1]
 
 
 # the tensor-core path needs enough work units to spread over the SMs: a
@@ -242,12 +253,6 @@ def dense_spmm(T, dims, pa, pb, ka, kb, coef, Bt: torch.Tensor, QS: int, Op: tor
     return True
 
 
-def lvv_t(Lf: torch.Tensor, nocc: int) -> torch.Tensor:
-    """L_vv^T [v*v, naux] (row c*v + a = L[:, a, c]) of a factor L [naux, nmo, nmo]."""
-    naux = Lf.shape[0]
-    return Lf[:, nocc:, nocc:].reshape(naux, -1).t().contiguous()
-
-
 class VvvvRebuild:
     """The (vv|vv) block rebuilt from the split factor: W[(c,d), (a,b)] =
     (ac|bd) in FP32 (rows of ``ldw`` = v*v floats, rounded up to even), on
@@ -257,7 +262,7 @@ class VvvvRebuild:
     def __init__(self, Lf: torch.Tensor, nocc: int):
         nmo = Lf.shape[1]
         self.v = nmo - nocc
-        self.Ap, self.Bp = split_bf16x3(lvv_t(Lf, nocc))
+        self.Ap, self.Bp = split_factor(Lf[:, nocc:, nocc:])  # row c*v + a = L[:, c, a]
         self.kp = self.Ap.shape[1]
         self.ldw = self.v * self.v + (self.v * self.v) % 2
         self.status = torch.zeros(1, dtype=torch.int32, device=Lf.device)
@@ -325,7 +330,7 @@ def split_eris(system, device="cuda"):
     ``VvvvRebuild`` for the O^2V^4 contraction; the small blocks (oo|oo),
     (ov|oo), (ov|ov) from the FP64 factor on the FP32-pair GEMM (~2^-40),
     (ov|vo) = (ov|ov) permuted (L is symmetric), sum_cd (ac|bd) in FP64."""
-    from .rccsd_dense import DeviceERIs, _dev_tensor
+    from .rccsd_dense import DeviceERIs, _dev_tensor, gemm_f64
     dev = torch.device(device)
     Lf = _dev_tensor(system.L, dev)
     o, nmo = system.nocc, system.nmo
@@ -347,10 +352,11 @@ def split_eris(system, device="cuda"):
         gemm_df(A, B.t(), C)
         return C.reshape(*n1, *n2)
 
+    R = VvvvRebuild(Lf, o)  # its B' is the (v,v) operand of both blocks below
+
     def tc_blk(name):
         p, q, r, t = name
-        A, _ = split_bf16x3(fac(p, q))
-        _, B = split_bf16x3(fac(r, t))
+        A, B = split_factor(Lf[:, sl[p], sl[q]], want_b=False), R.Bp
         n1 = (Lf[:, sl[p], sl[q]]).shape[1:]
         n2 = (Lf[:, sl[r], sl[t]]).shape[1:]
         return gemm_bf16_tn(A, B, f64=True).reshape(*n1, *n2)
@@ -360,8 +366,9 @@ def split_eris(system, device="cuda"):
     blocks["ovvv"] = tc_blk("ovvv")
     blocks["oovv"] = tc_blk("oovv")
     s = Lf[:, o:, o:].sum(dim=2)                      # [P, a] = sum_c L[P,a,c]
-    blocks["S0"] = s.t() @ s                          # sum_cd (ac|bd)
-    blocks["vvvv_rebuild"] = VvvvRebuild(Lf, o)
+    blocks["S0"] = torch.empty(s.shape[1], s.shape[1], dtype=torch.float64, device=dev)
+    gemm_f64(s.t(), s, blocks["S0"])                  # sum_cd (ac|bd)
+    blocks["vvvv_rebuild"] = R
     return DeviceERIs(_dev_tensor(system.fock, dev), _dev_tensor(system.mo_energy, dev), o, blocks, device)
 
 

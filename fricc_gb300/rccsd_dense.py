@@ -66,16 +66,23 @@ class DeviceERIs:
         self.g_ovov = 2.0 * ovov - ovov.permute(0, 3, 2, 1)               # 2(kc|ld) - (kd|lc)
         self.g_ovoo = 2.0 * ovoo - ovoo.permute(2, 1, 0, 3)               # [l,c,k,i]: 2(lc|ki) - (kc|li)
         # T1 O^2V^3 terms as one GEMM: G[k,c,d,a] = 2 (kd|ac) - (kc|ad)
-        self.G_t1 = (2.0 * ovvv.permute(0, 3, 1, 2) - ovvv.permute(0, 1, 3, 2)).contiguous()
-        # the same integral as [k,d,c,a]: X[c,a] = sum_kd t1[k,d] G[k,c,d,a] is one GEMV
-        # (it serves the t1.t1 T1 term and the ovvv part of Lvv)
-        self.G_t1_kdca = self.G_t1.permute(0, 2, 1, 3).contiguous()
+        # and as [k,d,c,a]: X[c,a] = sum_kd t1[k,d] G[k,c,d,a] is one GEMV
+        # (it serves the t1.t1 T1 term and the ovvv part of Lvv).  (The ovvv-sized
+        # layouts go through the library's elementwise pass: at o18v90 the
+        # torch expressions took 440 us.)
+        o, v = ovvv.shape[0], ovvv.shape[1]
+        new = functools.partial(torch.empty, dtype=ovvv.dtype, device=ovvv.device)
+        self.G_t1, self.G_t1_kdca = new(o, v, v, v), new(o, v, v, v)
+        _linear([self.G_t1, self.G_t1_kdca.permute(0, 2, 1, 3)], [ovvv.permute(0, 3, 1, 2), ovvv.permute(0, 1, 3, 2)],
+                [2.0, -1.0])
         # the T1 terms 2 sum_kc (kc|ai) t_kc - sum_kc (ki|ac) t_kc as one GEMV:
         # G1[k,c,i,a] = 2 (kc|ai) - (ki|ac)
         self.G_t1_kcia = (2.0 * self.ovvo.permute(0, 1, 3, 2) - self.oovv.permute(0, 3, 1, 2)).contiguous()
         # the t1 parts of Wvvvv, contracted with the compressed T2 instead of being
         # built densely: W'[c,d,(x,k,a)] = (kd|ac) for x=0 and (kc|ad) for x=1
-        self.ovvv_XY = torch.stack([ovvv.permute(3, 1, 0, 2), ovvv.permute(1, 3, 0, 2)], dim=2).contiguous()
+        self.ovvv_XY = new(v, v, 2, o, v)
+        _linear([self.ovvv_XY[:, :, 0]], [ovvv.permute(3, 1, 0, 2)], [1.0])
+        _linear([self.ovvv_XY[:, :, 1]], [ovvv.permute(1, 3, 0, 2)], [1.0])
         # sum_cd of the three Wvvvv pieces (for the reference's Wvvvv.t1.t1 term)
         self.S0 = self._S0 if self._S0 is not None else self.vvvvT.sum(dim=(0, 1))  # [a,b] = sum_cd (ac|bd)
         self.U = ovvv.sum(dim=(1, 3))                                     # [k,a] = sum_cd (kd|ac) = sum_cd (kc|ad)
@@ -86,8 +93,9 @@ class DeviceERIs:
         # GEMM-ready layouts for the dense O^2V^3 contractions
         self.g_klcd = self.g_ovov.permute(0, 2, 1, 3).contiguous()       # cc_Foo
         self.g_kldc = self.g_ovov.permute(0, 2, 3, 1).contiguous()       # cc_Fvv
-        self.ovvv_iabc = ovvv.permute(0, 1, 3, 2).contiguous()           # T2 driver term
-        self.ovvv_kacd = ovvv.permute(0, 2, 3, 1).contiguous()           # Wvovo t1 term
+        self.ovvv_iabc, self.ovvv_kacd = new(o, v, v, v), new(o, v, v, v)
+        _linear([self.ovvv_iabc], [ovvv.permute(0, 1, 3, 2)], [1.0])      # T2 driver term
+        _linear([self.ovvv_kacd], [ovvv.permute(0, 2, 3, 1)], [1.0])      # Wvovo t1 term
         self._dense_wvvvv = None
         self._splits = {}
         self._mod_bytes = 0
@@ -359,6 +367,17 @@ def combine(outs, xs=(), coefs=None, prod=(), accumulate=False):
     L.check(L.load().fricc_combine5(dims, len(xs), _ptrs(xs), sx, len(prod), _ptrs(prod), sp, len(outs), _ptrs(outs), so,
                                     cf, int(bool(accumulate)), L.cur_stream()))
     return outs[0]
+
+
+def _linear(outs, xs, coefs):
+    """Every out = sum_t coefs[t] xs[t]: one combine on the device, torch on a
+    host tensor."""
+    if outs[0].is_cuda:
+        combine(outs, xs, [list(coefs) for _ in outs])
+        return
+    r = sum(c * x for c, x in zip(coefs, xs))
+    for out in outs:
+        out.copy_(r)
 
 
 def zero(t: torch.Tensor) -> torch.Tensor:
