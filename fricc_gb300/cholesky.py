@@ -88,7 +88,7 @@ def split_factor(X: torch.Tensor, want_a: bool = True, want_b: bool = True):
     p, q], rows (p,q) and K = naux: straight from X where the transposing pass
     takes it (rows of 32 contiguous q), else through a copy."""
     naux, n1, n2 = X.shape
-    if n2 >= 32 and X.stride(2) == 1 and X.dtype == torch.float64 and X.is_cuda:
+    if n1 and n2 >= 32 and X.stride(2) == 1 and X.dtype == torch.float64 and X.is_cuda:
         return _split_view(X, n1 * n2, naux, n2, X.stride(1), 1, X.stride(0), want_a, want_b)
     AB = split_bf16x3(X.reshape(naux, -1).t().contiguous())
     return AB if want_a and want_b else AB[0 if want_a else 1]

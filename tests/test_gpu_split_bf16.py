@@ -51,3 +51,28 @@ def test_split_is_nearest(gpulib, layout, k, shift):
     for t, want in zip(out, (np.hstack([hi, hi, lo, pad]), np.hstack([hi, lo, hi, pad]))):
         got = t.cpu().numpy()[shift:shift + rows * kp].reshape(rows, kp)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("p,q", [((0, 5), (5, 36)), ((0, 5), (5, 37)), ((5, 38), (5, 38)), ((2, 3), (1, 34)), ((0, 0), (0, 33))])
+@pytest.mark.parametrize("flip", [False, True])
+def test_factor_slices_read_in_place(gpulib, p, q, flip):
+    """split_factor of a factor's slices -- rows too short for the transposing
+    pass, just long enough, offset, empty, or with transposed orbitals --
+    against the split of a copy."""
+    from fricc_gb300.cholesky import split_bf16x3, split_factor
+    rng = np.random.default_rng(p[1] + q[1])
+    L = torch.from_numpy(rng.standard_normal((19, 40, 40))).cuda()
+    X = L[:, p[0]:p[1], q[0]:q[1]]
+    if flip:
+        X = L.transpose(1, 2)[:, p[0]:p[1], q[0]:q[1]]
+    if X.numel() == 0:  # refused as the copy's split is
+        for f in (split_factor, lambda x: split_bf16x3(x.reshape(x.shape[0], -1).t().contiguous())):
+            with pytest.raises(ValueError):
+                f(X)
+        return
+    want = split_bf16x3(X.reshape(X.shape[0], -1).t().contiguous())
+    got = split_factor(X)
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    assert torch.equal(split_factor(X, want_b=False).view(torch.int16), want[0].view(torch.int16))
+    assert torch.equal(split_factor(X, want_a=False).view(torch.int16), want[1].view(torch.int16))
