@@ -26,8 +26,9 @@
 // terms commits about 0.2 n^1/2 2^-53 (sum x^2 y^2)^1/2.  The two part where
 // the large elements of x meet the small ones of y, so a 16th plane holds the
 // squares (BF16): every output is checked against n sum x^2 y^2 >= 2^-16
-// |x|^2 |y|^2, and one that fails, that belongs to a row that is not finite,
-// or whose pipeline gave up, is recomputed with FP64 FMAs (k_mod_fix).
+// |x|^2 |y|^2, and one that fails (true zeros apart: ZERO_SPAN), that belongs to
+// a row that is not finite, or whose pipeline gave up, is recomputed with FP64
+// FMAs (k_mod_fix).
 // Integer sums do not depend on their order: a result is the same in any
 // tiling, batch or split of K.
 //
@@ -129,8 +130,8 @@ __device__ __forceinline__ f32x2 reduce2(f32x2 x, f32x2 inv, f32x2 negp) {
 }
 
 // ------------------------------------------------------------ operands
-// Buffer of an operand: int sh[rows], unsigned cnt[rows] (nonzeros), then at
-// a 1 KB boundary the planes, [PLANES][nkb][rows][64] BF16 (K padded with
+// Buffer of an operand: int sh[rows], unsigned cnt[rows] (nonzeros, and in the
+// top byte the row's span, below), then at a 1 KB boundary the planes, [PLANES][nkb][rows][64] BF16 (K padded with
 // zeros to whole 64-wide blocks).  K-blocked, so that a TMA box of 256 rows is one
 // run of 32 KB and the conversion's stores are runs of 4 KB: with plain
 // K-major rows (45 KB apart at K = 22500) both missed the TLB on every row
@@ -157,12 +158,13 @@ __device__ __forceinline__ int64_t koff(const ModView& v, int64_t k) {
   else return k * v.sk;
 }
 
-// A row's (or a part of a row's) largest biased exponent (0: all zero),
-// nonzeros, and sum of (|x| 2^(1023 - emax))^2 in units of 2^-28, rounded up.
+// A row's (or a part of a row's) largest biased exponent (0: all zero), its
+// nonzeros' number and smallest exponent less 1 (all ones: none), and the sum of
+// (|x| 2^(1023 - emax))^2 in units of 2^-28, rounded up.
 struct RowStat {
   unsigned long long sum;
   int emax;
-  unsigned cnt;
+  unsigned short cnt, low;  // (of at most SCH elements)
 };
 constexpr int SCH = 256;  // k of one part: a thread's share stays in registers
 
@@ -186,7 +188,7 @@ __device__ __forceinline__ unsigned sq_units(unsigned long long u, int emax) {
 // rows.  (Two passes over the whole rows with atomics, the largest exponent
 // first, read x twice: 0.8 of the 1.9 ms that 20 M elements took to convert.)
 template <bool KFAST, bool K2>
-__global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, int64_t k, RowStat* __restrict__ part) {
+__global__ void __launch_bounds__(256, 2) k_mod_stat(const ModView v, int64_t R, int64_t k, RowStat* __restrict__ part) {
   const int64_t nch = fricc_cdiv(k, (int64_t)SCH);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (KFAST) {
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, in
       const double* xr = v.x + v.rows.at(r);
       unsigned long long u[SCH / 32];
       int e = 0;
-      unsigned cnt = 0;
+      unsigned cnt = 0, lo = ~0u;
 #pragma unroll
       for (int q = 0; q < SCH / 32; ++q) {
         const int64_t j = c * SCH + 32 * q + lane;
@@ -205,26 +207,28 @@ __global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, in
       for (int q = 0; q < SCH / 32; ++q) {
         const int ej = exp_of(u[q]);
         e = ej > e ? ej : e;
+        lo = min(lo, (unsigned)(ej - 1));
         cnt += ej ? 1u : 0u;
       }
       e = __reduce_max_sync(0xffffffffu, e);
+      lo = __reduce_min_sync(0xffffffffu, lo);
       cnt = __reduce_add_sync(0xffffffffu, cnt);
       unsigned long long s = 0;
 #pragma unroll
       for (int q = 0; q < SCH / 32; ++q) s += sq_units(u[q], e);
       s = warp_sum(s);
-      if (lane == 0) part[c * R + r] = RowStat{s, e, cnt};
+      if (lane == 0) part[c * R + r] = RowStat{s, e, (unsigned short)cnt, (unsigned short)lo};
     }
   } else {
     __shared__ unsigned long long ssum[8][33];
     __shared__ int se[8][33];
-    __shared__ unsigned sc[8][33];
+    __shared__ unsigned sc[8][33], sl[8][33];
     const int64_t nrb = fricc_cdiv(R, (int64_t)32);
     for (int64_t t = blockIdx.x; t < nrb * nch; t += gridDim.x) {
       const int64_t r = (t % nrb) * 32 + lane, c = t / nrb;
       unsigned long long u[SCH / 8];
       int e = 0;
-      unsigned cnt = 0;
+      unsigned cnt = 0, lo = ~0u;
       const double* xr = v.x + (r < R ? v.rows.at(r) : 0);
 #pragma unroll
       for (int q = 0; q < SCH / 8; ++q) {
@@ -235,11 +239,13 @@ __global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, in
       for (int q = 0; q < SCH / 8; ++q) {
         const int ej = exp_of(u[q]);
         e = ej > e ? ej : e;
+        lo = min(lo, (unsigned)(ej - 1));
         cnt += ej ? 1u : 0u;
       }
       __syncthreads();
       se[warp][lane] = e;
       sc[warp][lane] = cnt;
+      sl[warp][lane] = lo;
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < 8; ++q) e = se[q][lane] > e ? se[q][lane] : e;
@@ -252,8 +258,9 @@ __global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, in
         for (int q = 1; q < 8; ++q) {
           s += ssum[q][lane];
           cnt += sc[q][lane];
+          lo = min(lo, sl[q][lane]);
         }
-        part[c * R + r] = RowStat{s, e, cnt};
+        part[c * R + r] = RowStat{s, e, (unsigned short)cnt, (unsigned short)lo};
       }
     }
   }
@@ -261,11 +268,21 @@ __global__ void __launch_bounds__(256) k_mod_stat(const ModView v, int64_t R, in
 
 // the shift of each row: |x| 2^sh <= 2^61 for its norm (and > 2^60 but for
 // subnormal rows)
-__device__ __forceinline__ int shift_of(const RowStat& s) {
-  if (s.emax == 0) return 0;
-  if (s.emax >= 2047) return SH_BAD;
-  const int L = 64 - __clzll((long long)((s.sum - 1) | 1ull));  // sum <= 2^L
-  return 61 - (s.emax - 1023 - 14 + (L + 1) / 2);
+__device__ __forceinline__ int shift_of(unsigned long long sum, int emax) {
+  if (emax == 0) return 0;
+  if (emax >= 2047) return SH_BAD;
+  const int L = 64 - __clzll((long long)((sum - 1) | 1ull));  // sum <= 2^L
+  return 61 - (emax - 1023 - 14 + (L + 1) / 2);
+}
+
+// A row's word of `cnt`: its nonzeros, and in the top byte how many binary places
+// below the norm's bound 2^61 its smallest nonzero may lie (255: at least so
+// many; a subnormal's own places count).
+constexpr int SPAN_AT = 24;
+__device__ __forceinline__ unsigned cnt_word(unsigned cnt, unsigned low, int sh) {
+  if (cnt == 0 || sh == SH_BAD) return cnt;
+  const int span = 61 - ((int)low - 1022 + sh) + (low == 0 ? 52 : 0);
+  return cnt | (unsigned)min(max(span, 0), 255) << SPAN_AT;
 }
 
 // one warp per row: its parts combined (a long row has thousands)
@@ -280,19 +297,22 @@ __global__ void __launch_bounds__(256) k_mod_shift(const RowStat* __restrict__ p
     }
     e = __reduce_max_sync(0xffffffffu, e);
     unsigned long long s = 0;
-    unsigned n = 0;
+    unsigned n = 0, lo = ~0u;
     for (int64_t c = lane; c < nch; c += 32) {
       const RowStat p = part[c * R + r];
       if (p.cnt == 0) continue;
+      lo = min(lo, (unsigned)p.low);
       const int d = 2 * (e - p.emax);
       s += d > 62 ? 1ull : (p.sum >> d) + 1ull;
       n += p.cnt;
     }
     s = warp_sum(s);
     n = __reduce_add_sync(0xffffffffu, n);
+    lo = __reduce_min_sync(0xffffffffu, lo);
     if (lane == 0) {
-      sh[r] = shift_of(RowStat{s, e, n});
-      cnt[r] = n;
+      const int h = shift_of(s, e);
+      sh[r] = h;
+      cnt[r] = cnt_word(n, lo, h);
     }
   }
 }
@@ -426,7 +446,7 @@ __global__ void __launch_bounds__(256, 3) k_mod_convert(const ModView v, int64_t
   extern __shared__ double ct[];  // [64 nkb][33]
   __shared__ unsigned long long ssum[8][33];
   __shared__ int se[8][33], ssh[32];
-  __shared__ unsigned sc[8][33];
+  __shared__ unsigned sc[8][33], sl[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nkb = (int)fricc_cdiv(k, (int64_t)BK), kp = nkb * BK, kk = (int)k;
   const int64_t nrb = fricc_cdiv(R, (int64_t)32), plane = nkb * R * BK;
@@ -447,14 +467,16 @@ __global__ void __launch_bounds__(256, 3) k_mod_convert(const ModView v, int64_t
     }
     __syncthreads();
     int e = 0;
-    unsigned n = 0;
+    unsigned n = 0, lo = ~0u;
     for (int j = warp; j < kk; j += 8) {
       const int ej = exp_of((unsigned long long)__double_as_longlong(ct[j * 33 + lane]));
       e = ej > e ? ej : e;
+      lo = min(lo, (unsigned)(ej - 1));
       n += ej ? 1u : 0u;
     }
     se[warp][lane] = e;
     sc[warp][lane] = n;
+    sl[warp][lane] = lo;
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 8; ++q) e = se[q][lane] > e ? se[q][lane] : e;
@@ -466,12 +488,13 @@ __global__ void __launch_bounds__(256, 3) k_mod_convert(const ModView v, int64_t
       for (int q = 1; q < 8; ++q) {
         s += ssum[q][lane];
         n += sc[q][lane];
+        lo = min(lo, sl[q][lane]);
       }
-      const int h = shift_of(RowStat{s, e, n});
+      const int h = shift_of(s, e);
       ssh[lane] = h;
       if (r0 + lane < R) {
         sh[r0 + lane] = h;
-        cnt[r0 + lane] = n;
+        cnt[r0 + lane] = cnt_word(n, lo, h);
       }
     }
     __syncthreads();
@@ -864,6 +887,13 @@ __global__ void __launch_bounds__(256) k_mod_slices(unsigned* __restrict__ res, 
 }
 
 constexpr float GUARD = 0x1p-16f;
+// An output whose residues and whose sum of squares are zero is a true zero (no
+// nonzero of its row meets one of its column) where one of the two is empty, or
+// where the spans of both add up to no more than this: any two nonzeros that
+// meet then leave a square of at least 2^-124 (2^-126 is the smallest normal FP32
+// number).  Elsewhere the elements that meet may have been rounded to 0, or
+// their squares may have underflowed beside integers that cancel.
+constexpr unsigned ZERO_SPAN = 62;
 
 // One 32 x 64 tile of outputs per step: residues in, C out, and an entry on
 // the list for a tile with outputs to recompute (which are left alone).  A
@@ -922,8 +952,10 @@ __global__ void __launch_bounds__(256, 4) k_mod_combine(CombineArgs a, int64_t n
             bad = c + h < a.N;
           } else {
             x = crt(ri, sha + shb[h], &zero);
-            const float n = (float)(na < nb[h] ? na : nb[h]);
-            bad = c + h < a.N && !(n * s2 >= GUARD) && !(zero && s2 == 0.0f);
+            const unsigned ka = na & ((1u << SPAN_AT) - 1), kb = nb[h] & ((1u << SPAN_AT) - 1);
+            const float n = (float)(ka < kb ? ka : kb);
+            bad = c + h < a.N && !(n * s2 >= GUARD);
+            if (bad && zero && s2 == 0.0f) bad = n != 0.0f && (na >> SPAN_AT) + (nb[h] >> SPAN_AT) > ZERO_SPAN;
           }
           no |= bad ? 1u << h : 0u;
           t[rl][cl + h] = x;
