@@ -7,17 +7,17 @@
 //
 // * each row x of an operand is scaled by a power of two to integers
 //   X = rint(x 2^s) with 2^60 < |X|_2 <= 2^61 (one shift per row), and X is
-//   reduced modulo 15 pairwise coprime moduli <= 361 to balanced residues,
-//   integers of at most 181: exact in BF16.  Each modulus is one operand
+//   reduced modulo 15 pairwise coprime odd moduli <= 361 to balanced residues,
+//   integers of at most 180: exact in BF16.  Each modulus is one operand
 //   "plane";
 // * one persistent tcgen05 kernel multiplies the planes, modulus by modulus:
-//   512 products of at most 181^2 sum to less than 2^24, so FP32 accumulation
+//   512 products of at most 180^2 sum to less than 2^24, so FP32 accumulation
 //   in tensor memory is exact over 512 k; the epilogue warps drain it every
 //   512 k and reduce it modulo p in FP32 into registers.  (14 moduli up to 512
 //   need a drain every 256 k and were no faster: the drains, not the MMAs,
 //   set the pace.)
 // * by Cauchy-Schwarz |sum X Y| <= 2^122, below an eighth of the product of
-//   the moduli (2^125.8), so the 15 residues determine it: the Chinese
+//   the moduli (2^125.6), so the 15 residues determine it: the Chinese
 //   remainder sum is taken as a 96-bit binary fraction of that product (it
 //   wraps by itself) and rounded once to FP64.
 //
@@ -25,12 +25,16 @@
 // of 2^60.5, i.e. 2^-62 |x||y| in an output, where an FP64 FMA chain of n
 // terms commits about 0.2 n^1/2 2^-53 (sum x^2 y^2)^1/2.  The two part where
 // the large elements of x meet the small ones of y, so a 16th plane holds the
-// squares (BF16): every output is checked against n sum x^2 y^2 >= 2^-16
-// |x|^2 |y|^2, and one that fails (true zeros apart: ZERO_SPAN), that belongs to
+// squares (BF16): every output is checked against n s2 >= 2^-16 |x|^2 |y|^2, s2
+// the largest sum x^2 y^2 of a run of 512 k, and one that fails (true zeros apart: ZERO_SPAN), that belongs to
 // a row that is not finite, or whose pipeline gave up, is recomputed with FP64
 // FMAs (k_mod_fix).
-// Integer sums do not depend on their order: a result is the same in any
-// tiling, batch or split of K.
+// A result is the same in any tiling, batch or split of K: integer sums do not
+// depend on their order, a sum has one balanced residue whatever the order of its
+// reductions (make_tab), and the check compares the largest of the runs' squares,
+// which are the same runs in every split.  (With one of the moduli even, slices'
+// residues summed without a reduction and their squares added, the fraction's
+// rounding and the check's outcome followed the split, and so the batch.)
 //
 // Measured on a GB300 (operands prepared; DFMA kernel): 900 x 22500 x 22500
 // 9.1 ms; 4500^3 2.05 ms (152 ms); 2000^3 0.26 ms (14.0 ms); 400^3 30 us
@@ -61,9 +65,19 @@ struct Tab {
   unsigned long long mtop = 0;  // M >> 62, in [2^63, 2^64)
 };
 
+// The moduli are odd, and their FP32 reciprocals close enough that x - p rint(x
+// fl(1/p)) is the residue in (-p/2, p/2) for every |x| of a run (canonical()):
+// with 360, 349 or 343 a residue next to half of p could come out on either side,
+// depending on the run it was reduced in.
+constexpr bool canonical(int p) {
+  const int h = (p - 1) / 2;
+  const double e = (double)(1.0f / (float)p) * p - 1.0;  // exact
+  return p % 2 == 1 && 2.0 * (e < 0 ? -e : e) * (512.0 * h * h + h) < 1.0;
+}
+
 constexpr Tab make_tab() {
   Tab t;
-  const int p[NP] = {361, 360, 359, 353, 349, 347, 343, 341, 337, 331, 317, 313, 311, 307, 299};
+  const int p[NP] = {361, 359, 353, 347, 341, 339, 337, 335, 331, 329, 317, 313, 311, 307, 299};
   unsigned __int128 M = 1;
   for (int i = 0; i < NP; ++i) {
     t.p[i] = p[i];
@@ -92,8 +106,24 @@ constexpr Tab make_tab() {
 }
 __device__ constexpr Tab TAB = make_tab();
 static_assert((TAB.mtop >> 63) == 1, "the product of the moduli lies in [2^125, 2^126)");
+constexpr bool moduli_hold() {
+  for (int i = 0; i < NP; ++i) {
+    if (!canonical(make_tab().p[i])) return false;
+    for (int j = 0; j < i; ++j) {
+      int a = make_tab().p[i], b = make_tab().p[j];
+      while (b) {
+        const int r = a % b;
+        a = b;
+        b = r;
+      }
+      if (a != 1) return false;
+    }
+  }
+  return true;
+}
+static_assert(moduli_hold(), "pairwise coprime moduli with one balanced residue");
 
-__constant__ float c_p[NP] = {361, 360, 359, 353, 349, 347, 343, 341, 337, 331, 317, 313, 311, 307, 299};
+__constant__ float c_p[NP] = {361, 359, 353, 347, 341, 339, 337, 335, 331, 329, 317, 313, 311, 307, 299};
 
 constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: adding it rounds a float to an integer
 
@@ -720,12 +750,16 @@ __global__ void __launch_bounds__(MNT, 1)
           if ((w4 + 4 * c) * 16 < g.bn) {
             float r[16];
             tc_ld16(at + (uint32_t)(c * 64), r);
-            // (a run plus a residue stays below 2^24: 512 * 181^2 + 181)
+            if (sq) {  // the largest run's sum
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[c * 8 + j] = add2(acc[c * 8 + j], pk2(r[2 * j], r[2 * j + 1]));
-            if (!sq) {
+              for (int j = 0; j < 8; ++j) {
+                const float2 f = upk2(acc[c * 8 + j]);
+                acc[c * 8 + j] = pk2(fmaxf(f.x, r[2 * j]), fmaxf(f.y, r[2 * j + 1]));
+              }
+            } else {  // (a run plus a residue stays below 2^24: 512 * 180^2 + 180)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) acc[c * 8 + j] = reduce2(acc[c * 8 + j], inv, negp);
+              for (int j = 0; j < 8; ++j)
+                acc[c * 8 + j] = reduce2(add2(acc[c * 8 + j], pk2(r[2 * j], r[2 * j + 1])), inv, negp);
             }
           }
         }
@@ -859,29 +893,35 @@ __device__ __forceinline__ double crt(const int* r, int sh, bool* zero) {
   return __longlong_as_double((long long)((((unsigned long long)(be - 1) << 52) + m) | ((unsigned long long)sg << 63)));
 }
 
-// K slices: slice 0 += the others (64 residues of at most 182 fit 16 bits)
-__global__ void __launch_bounds__(256) k_mod_slices(unsigned* __restrict__ res, int64_t words, int64_t sq0, int ks) {
+// K slices: slice 0 = the sum of all (64 residues of at most 180), reduced to
+// the residue one slice would have left, or of the squares the largest.  One grid
+// row per plane; `words` of 2 values per plane, `slice` per slice.
+__global__ void __launch_bounds__(256) k_mod_slices(unsigned* __restrict__ res, int64_t words, int64_t slice, int ks) {
+  const int plane = blockIdx.y;
+  res += plane * words;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (int64_t)gridDim.x * 256) {
     const unsigned x = res[i];
-    if (i < sq0) {
+    if (plane < NP) {
       int lo = (short)x, hi = (int)x >> 16;
 #pragma unroll 8
       for (int s = 1; s < ks; ++s) {
-        const unsigned y = res[i + s * words];
+        const unsigned y = res[i + s * slice];
         lo += (short)y;
         hi += (int)y >> 16;
       }
+      const float p = c_p[plane], inv = 1.0f / p;
+      lo -= (int)p * __float2int_rn((float)lo * inv);
+      hi -= (int)p * __float2int_rn((float)hi * inv);
       res[i] = ((unsigned)lo & 0xffffu) | ((unsigned)hi << 16);
     } else {
       float lo = __uint_as_float(x << 16), hi = __uint_as_float(x & 0xffff0000u);
 #pragma unroll 8
       for (int s = 1; s < ks; ++s) {
-        const unsigned y = res[i + s * words];
-        lo += __uint_as_float(y << 16);
-        hi += __uint_as_float(y & 0xffff0000u);
+        const unsigned y = res[i + s * slice];
+        lo = fmaxf(lo, __uint_as_float(y << 16));
+        hi = fmaxf(hi, __uint_as_float(y & 0xffff0000u));
       }
-      const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-      res[i] = *reinterpret_cast<const unsigned*>(&h);
+      res[i] = (__float_as_uint(lo) >> 16) | (__float_as_uint(hi) & 0xffff0000u);
     }
   }
 }
@@ -1299,10 +1339,9 @@ int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out_, int64
         c.count = words + 1;
         c.list = words + 2;
         if (ks > 1) {
-          const int64_t words = g.slice_stride / 2;
-          const int64_t gs = fricc_cdiv(words, 256);
-          mod::k_mod_slices<<<(unsigned)(gs < 152 * 8 ? gs : 152 * 8), 256, 0, st>>>(
-              reinterpret_cast<unsigned*>(res), words, mod::NP * g.plane_stride / 2, ks);
+          const int64_t gs = fricc_cdiv(g.plane_stride / 2, 256);
+          mod::k_mod_slices<<<dim3((unsigned)(gs < 152 ? gs : 152), mod::PLANES), 256, 0, st>>>(
+              reinterpret_cast<unsigned*>(res), g.plane_stride / 2, g.slice_stride / 2, ks);
           fricc_note_launch();
         }
         const unsigned gc = (unsigned)(tiles < 152 * 8 ? tiles : 152 * 8);
