@@ -389,10 +389,11 @@ __global__ void k_densify_bf16x3(const int* __restrict__ slots, const double* __
 
 // The compressed T as a dense FP64 matrix [nP][R] in zeroed memory: the A
 // operand of the modular tensor-core product (gemm_mod.cu), which skips
-// elements whose bits are all zero, so a stored zero is written as -0.  (P, r)
-// is unique per nonzero but for the flat index 0, where every unmatched
-// sample of a systematic compression sits: those add up (equal values, or
-// an infinity among them, so their order does not matter).
+// elements whose bits are all zero, so a stored zero becomes -0.  Samples of a
+// systematic compression can share an element: every unmatched one sits at flat
+// index 0, and two can fall on a probability of 1 where the partial sums cross a
+// power of two.  Those add up (equal values, or an infinity among them, so their
+// order does not matter).
 __global__ void k_densify_f64(const int* __restrict__ slots, const double* __restrict__ vals, int64_t m, int pa, int pb,
                               int64_t dpb, int ka, int kb, int64_t dkb, int64_t R, double* __restrict__ out,
                               int64_t rep) {
@@ -404,8 +405,8 @@ __global__ void k_densify_f64(const int* __restrict__ slots, const double* __res
     const int sl[4] = {q.x, q.y, q.z, q.w};
     const double x = vals[s];
     const int64_t at = ((int64_t)sl[pa] * dpb + sl[pb]) * R + (int64_t)sl[ka] * dkb + sl[kb];
-    if (at == 0) atomicAdd(&out[0], x);
-    else out[at] = x == 0.0 ? -0.0 : x;
+    if (x == 0.0) atomicCAS(reinterpret_cast<unsigned long long*>(out + at), 0ull, 1ull << 63);
+    else atomicAdd(out + at, x);
   }
 }
 
