@@ -103,22 +103,35 @@ class DeviceERIs:
 
     SPLIT_BLOCKS = ("vvvvT", "ovvv_XY", "ovov", "ovov_0312", "ovov_0313_0113", "ovov_cdkl")
 
+    def _kept(self, key, make):
+        """The form of a constant block kept under ``key``, made once under a
+        lock and waited for before it can be seen: solvers on other threads and
+        streams never read one whose conversion is still in flight.  (``make``
+        may return None: nothing is kept.)"""
+        got = self._splits.get(key)
+        if got is None:
+            with self._lock:
+                got = self._splits.get(key)
+                if got is None:
+                    got = make()
+                    if got is not None:
+                        torch.cuda.current_stream().synchronize()
+                        self._splits[key] = got
+        return got
+
     def prepare_splits(self, names=None):
         """Build the (hi, lo) float-pair forms of constant W' blocks once (by
-        default those of FRI-CCSD), and wait for them: solvers on other
-        streams read them afterwards."""
-        names = self.SPLIT_BLOCKS if names is None else names
-        if any(n not in self._splits for n in names):
-            for name in names:
-                if name not in self._splits and getattr(self, name) is not None:
-                    self._splits[name] = split_f2(getattr(self, name))
-            torch.cuda.current_stream().synchronize()
+        default those of FRI-CCSD)."""
+        for name in self.SPLIT_BLOCKS if names is None else names:
+            if getattr(self, name) is not None:
+                self._kept(name, lambda: split_f2(getattr(self, name)))
 
     def pair_blocks(self, m, every, names=None):
         """The constant W' blocks a df64 solver keeping m entries contracts in
         float pairs: all of them with ``every`` (an autotuner compares the
         float-pair launches), else those whose term does not run as a modular
-        tensor-core product."""
+        tensor-core product (one that does only with the block converted counts
+        where that is kept, which is settled here, before the first iteration)."""
         names = self.SPLIT_BLOCKS if names is None else names
         if every:
             return names
@@ -129,7 +142,13 @@ class DeviceERIs:
                "ovov_cdkl": [(0, 1, 2, 3, o * o)], "oooo_klij": [(2, 3, 0, 1, o * o)],
                "lin_WA": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)], "lin_WB": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)],
                "lin_W2AB": [(1, 3, 0, 2, ov)]}
-        return tuple(n for n in names if not all(takes_mod((o, o, v, v), m, t, True, True) for t in use[n]))
+        dims = (o, o, v, v)
+
+        def modular(n, t):
+            return takes_mod(dims, m, t, False, True) or (takes_mod(dims, m, t, True, True) and
+                                                          self.mod_w(n, t[4]) is not None)
+        return tuple(n for n in names
+                     if getattr(self, n) is not None and not all(modular(n, t) for t in use[n]))
 
     LIN_BLOCKS = ("oooo_klij", "lin_WA", "lin_WB", "lin_W2AB")
 
@@ -148,42 +167,24 @@ class DeviceERIs:
                 torch.cuda.current_stream().synchronize()
 
     def prepare_f32(self, blocks: dict):
-        """Build the FP32 forms {name: qs} once, and wait for them (solvers
-        on other streams read them afterwards)."""
-        if any(("f32", n, q) not in self._splits for n, q in blocks.items()):
-            for n, q in blocks.items():
-                self.f32(n, q)
-            torch.cuda.current_stream().synchronize()
+        """Build the FP32 forms {name: qs} once."""
+        for n, q in blocks.items():
+            self.f32(n, q)
 
     def prepare_tc(self, operands: dict):
         """The split-BF16x3 operands of constant blocks for the split-precision
-        form's tensor-core GEMMs, made once and waited for:
+        form's tensor-core GEMMs, made once:
         {name: ("A" or "B", rows, cols)} with the block viewed as [rows, cols]."""
         from .cholesky import split_a, split_b
-        todo = {n: spec for n, spec in operands.items() if ("tc", n) not in self._splits}
-        if todo:
-            for n, (role, r, c) in todo.items():
-                x = getattr(self, n).reshape(r, c)
-                self._splits[("tc", n)] = (role, split_a(x) if role == "A" else split_b(x))
-            torch.cuda.current_stream().synchronize()
+        for n, (role, r, c) in operands.items():
+            self._kept(("tc", n), lambda: (role, (split_a if role == "A" else split_b)(getattr(self, n).reshape(r, c))))
 
     def tc_w(self, name, qs):
         """The split W^T ([hi|lo|hi], rows q) of a constant W' block viewed as
-        [rows][qs]: the B operand of the split-precision dense sparse terms.
-        Built on first use (the first, eager iteration) under a lock and
-        waited for, so solvers on other threads and streams never read a
-        block whose split is still in flight."""
+        [rows][qs]: the B operand of the split-precision dense sparse terms,
+        built on first use (the first, eager iteration)."""
         from .cholesky import split_b
-        key = ("tcW", name, qs)
-        got = self._splits.get(key)
-        if got is None:
-            with self._lock:
-                got = self._splits.get(key)
-                if got is None:
-                    got = split_b(getattr(self, name).reshape(-1, qs))
-                    torch.cuda.current_stream().synchronize()
-                    self._splits[key] = got
-        return got
+        return self._kept(("tcW", name, qs), lambda: split_b(getattr(self, name).reshape(-1, qs)))
 
     def tc(self, name, role):
         got = self._splits.get(("tc", name))
@@ -197,24 +198,18 @@ class DeviceERIs:
     MOD_BYTES = 40 << 30
 
     def _mod(self, key, name, rows, k, row_stride, k_stride):
-        got = self._splits.get(key)
-        if got is None:
-            with self._lock:
-                got = self._splits.get(key)
-                if got is None:
-                    need = L.load().fricc_mod_bytes(rows, k)
-                    if self._mod_bytes + need > self.MOD_BYTES:
-                        return None
-                    got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
-                    torch.cuda.current_stream().synchronize()
-                    self._mod_bytes += need
-                    self._splits[key] = got
-        return got
+        def make():
+            need = L.load().fricc_mod_bytes(rows, k)
+            if self._mod_bytes + need > self.MOD_BYTES:
+                return None
+            got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
+            self._mod_bytes += need
+            return got
+        return self._kept(key, make)
 
     def mod_w(self, name, qs):
         """A constant W' block viewed as [keys][qs], its rows q prepared for
-        the modular products, built on first use under a lock and waited for
-        (None past MOD_BYTES)."""
+        the modular products, built on first use (None past MOD_BYTES)."""
         return self._mod(("modW", name, qs), name, qs, getattr(self, name).numel() // qs, 1, qs)
 
     def mod_a(self, name, m, k):
@@ -228,10 +223,7 @@ class DeviceERIs:
     def f32(self, name, qs):
         """FP32 rows (qs columns, padded to even) of a constant block, built
         once: the W' operands of the split-precision form."""
-        key = ("f32", name, qs)
-        if key not in self._splits:
-            self._splits[key] = to_f32_rows(getattr(self, name), qs)
-        return self._splits[key]
+        return self._kept(("f32", name, qs), lambda: to_f32_rows(getattr(self, name), qs))
 
     def split(self, name):
         """The float-pair form of a constant block (prepare_splits() built it)."""
