@@ -1413,11 +1413,14 @@ int fricc_mod_try(const double* A, const double* B, double* C, int64_t batch, in
   out.col.outer(N, sC[1]);
   int64_t m = M, n = N, reps = 1;
   // a level that moves only A (or only B) is flattened into its rows; the
-  // levels that move both follow: replicas are the slowest index of the rows
+  // levels that move both follow: replicas are the slowest index of the rows.
+  // One that moves neither repeats A's rows, or, where those are prepared, B's:
+  // a prepared operand has its own rows and no more.
   for (int k = 0; k < 2; ++k) {
     const Level& l = lv[k];
     if (l.n == 1 || (l.a != 0 && l.b != 0)) continue;
-    if (l.b == 0) {
+    if (l.a == 0 && l.b == 0 && a_mod) vb.prepared = nullptr;
+    if (l.b == 0 && !(l.a == 0 && a_mod)) {
       va.rows.outer(l.n, l.a);
       out.row.outer(l.n, l.c);
       m *= l.n;
