@@ -56,6 +56,7 @@ SIGNATURES = [
                                             ctypes.c_int, ctypes.c_int]),
     ("fricc_mod_select", ctypes.c_int, [ctypes.c_int]),
     ("fricc_mod_mode", ctypes.c_int, []),
+    ("fricc_mod_scratch", ctypes.c_int, [_i64]),
     ("fricc_mod_bytes", _i64, [_i64, _i64]),
     ("fricc_mod_prepare", ctypes.c_int, [_dp, _i64, _i64, _i64, _i64, _vp, _vp]),
     ("fricc_gemm_f64_mod", ctypes.c_int, [_dp, _vp, _dp, _vp, _dp, _i64, _i64, _i64, _i64, _i64, _i64p, _i64p, _i64p,

@@ -146,6 +146,7 @@ int fricc_alloc(void** p, size_t bytes, cudaStream_t s) {
   cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, s);
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // reported here; not by the next launch's check
     return fricc_cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
   }
   return FRICC_OK;

@@ -647,13 +647,14 @@ bool fricc_spmm_takes_mod(const int64_t dims[4], int64_t m, int pa, int pb, int 
 namespace {
 
 // out[P][q] += coef sum_r T[P][r] W[r][q] as a modular product; W given as the view
-// of its rows q (and prepared or not), reps > 1: one T (and W unless shared) per replica
+// of its rows q (and prepared or not), reps > 1: one T (and W unless shared) per replica.
+// FRICC_MOD_NONE where its scratch could not be had: the sparse kernels need less.
 int spmm_mod(const int* slots, const double* vals, int64_t m, const int64_t dims[4], int pa, int pb, int ka, int kb,
              const ModView& W, ModOut out, int64_t QS, int64_t reps, bool w_shared, cudaStream_t st) {
   const int64_t nP = dims[pa] * dims[pb], R = dims[ka] * dims[kb];
   double* Td = nullptr;
-  int rc = fricc_alloc_t(&Td, (size_t)reps * nP * R, st);
-  if (rc) return rc;
+  if (fricc_alloc_t(&Td, (size_t)reps * nP * R, st)) return FRICC_MOD_NONE;
+  int rc = FRICC_OK;
   cudaError_t e = cudaMemsetAsync(Td, 0, sizeof(double) * (size_t)(reps * nP * R), st);
   if (e == cudaSuccess) {
     k_densify_f64<<<dim3(grid_for(m, 256), (unsigned)reps), 256, 0, st>>>(slots, vals, m, pa, pb, dims[pb], ka, kb,
@@ -797,7 +798,8 @@ int fricc_contract_device(const char* term, const double* Win, const int64_t Wd[
     o.row.outer(oe[0], osp[0]);
     o.col.outer(oe[3], osp[3]);
     o.col.outer(oe[2], osp[2]);
-    return spmm_mod(T->slots, T->vals, T->m, td, ts->pa, ts->pb, ts->ka, ts->kb, W, o, QS, 1, true, st);
+    rc = spmm_mod(T->slots, T->vals, T->m, td, ts->pa, ts->pb, ts->ka, ts->kb, W, o, QS, 1, true, st);
+    if (rc != FRICC_MOD_NONE) return rc;
   }
 
   Bucketing* bk = nullptr;
@@ -861,6 +863,7 @@ int fricc_spmm_device(FriccSparse* T, int pa, int pb, int ka, int kb, double coe
     return FRICC_ERR_ARG;
   }
   if (T->m == 0) return FRICC_OK;
+  int rc = FRICC_OK;
   if (fricc_spmm_takes_mod(T->dims, T->m, pa, pb, ka, kb, QS, w_mod != nullptr, false)) {
     ModView W;
     W.x = Wp;
@@ -873,10 +876,11 @@ int fricc_spmm_device(FriccSparse* T, int pa, int pb, int ka, int kb, double coe
     o.beta = 1.0;
     o.row.outer(T->dims[pa] * T->dims[pb], QS);
     o.col.outer(QS, 1);
-    return spmm_mod(T->slots, T->vals, T->m, T->dims, pa, pb, ka, kb, W, o, QS, 1, true, st);
+    rc = spmm_mod(T->slots, T->vals, T->m, T->dims, pa, pb, ka, kb, W, o, QS, 1, true, st);
+    if (rc != FRICC_MOD_NONE) return rc;
   }
   Bucketing* bk = nullptr;
-  int rc = fricc_sparse_bucketing(T, pa, pb, st, &bk);
+  rc = fricc_sparse_bucketing(T, pa, pb, st, &bk);
   if (rc) return rc;
   int* erow = nullptr;
   double* eval = nullptr;
@@ -1201,6 +1205,7 @@ int fricc_batch_spmm_device(FriccSparseBatch* B, int which, int pa, int pb, int 
   }
   const int R = B->R;
   const int64_t m = B->m;
+  int rc = FRICC_OK;
   // (one replica's estimate: a replica takes its lone call's route)
   if (!f2 && fricc_spmm_takes_mod(B->dims, m, pa, pb, ka, kb, QS, w_mod != nullptr, false)) {
     ModView W;
@@ -1220,11 +1225,11 @@ int fricc_batch_spmm_device(FriccSparseBatch* B, int which, int pa, int pb, int 
       W.rows.outer(R, w_stride);
       o.rep.outer(R, o_stride);
     }
-    return spmm_mod(B->slots[which], B->vals[which], m, B->dims, pa, pb, ka, kb, W, o, QS, R, w_stride == 0 || R == 1,
-                    st);
+    rc = spmm_mod(B->slots[which], B->vals[which], m, B->dims, pa, pb, ka, kb, W, o, QS, R, w_stride == 0 || R == 1, st);
+    if (rc != FRICC_MOD_NONE) return rc;
   }
   BatchBucketing* bk = nullptr;
-  int rc = fricc_batch_bucketing(B, which, pa, pb, st, &bk);
+  rc = fricc_batch_bucketing(B, which, pa, pb, st, &bk);
   if (rc) return rc;
   int* erow = nullptr;
   void* eval = nullptr;

@@ -1138,7 +1138,7 @@ int64_t fricc_mod_operand_bytes(int64_t rows, int64_t k) { return mod::layout(ro
 
 template <bool KFAST, bool K2>
 static int launch_operand(const ModView& v, int64_t rows, int64_t k, int* sh, unsigned* cnt, __nv_bfloat16* planes,
-                          cudaStream_t st) {
+                          mod::RowStat* part, cudaStream_t st) {
   auto cap = [](int64_t n) { return (unsigned)(n < 152 * 16 ? (n < 1 ? 1 : n) : 152 * 16); };
   const int64_t nkb = fricc_cdiv(k, tc::BK), nrb = fricc_cdiv(rows, 32);
   if (k <= mod::SCH) {
@@ -1154,29 +1154,39 @@ static int launch_operand(const ModView& v, int64_t rows, int64_t k, int* sh, un
     return fricc_cuda_check(cudaGetLastError(), "mod operand");
   }
   const int64_t nch = fricc_cdiv(k, mod::SCH);
-  mod::RowStat* part = nullptr;
-  int rc = fricc_alloc_t(&part, (size_t)(rows * nch), st);
-  if (rc) return rc;
   mod::k_mod_stat<KFAST, K2><<<cap(KFAST ? fricc_cdiv(rows * nch, 8) : nrb * nch), 256, 0, st>>>(v, rows, k, part);
   mod::k_mod_shift<<<cap(fricc_cdiv(rows, 8)), 256, 0, st>>>(part, rows, nch, sh, cnt);
   mod::k_mod_split<KFAST, K2><<<cap(nrb * nkb), 256, 0, st>>>(v, rows, k, sh, planes);
   fricc_note_launch(3);
-  rc = fricc_cuda_check(cudaGetLastError(), "mod operand");
-  fricc_free(part, st);
-  return rc;
+  return fricc_cuda_check(cudaGetLastError(), "mod operand");
 }
 
-int fricc_mod_operand(const ModView& v, int64_t rows, int64_t k, void* buf, cudaStream_t st) {
+// Scratch of a conversion (the statistics of rows of more than one part).
+static int64_t part_bytes(int64_t rows, int64_t k) {
+  return k <= mod::SCH ? 0 : rows * fricc_cdiv(k, mod::SCH) * (int64_t)sizeof(mod::RowStat);
+}
+
+static int convert(const ModView& v, int64_t rows, int64_t k, void* buf, void* part_buf, cudaStream_t st) {
+  auto* part = static_cast<mod::RowStat*>(part_buf);
   const mod::Layout l = mod::layout(rows, k);
   int* sh = static_cast<int*>(buf);
   unsigned* cnt = reinterpret_cast<unsigned*>(static_cast<char*>(buf) + l.off_cnt);
   auto* planes = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(buf) + l.off_planes);
   const bool kfast = v.sk == 1 || (v.rows.s0 != 1 && rows > 1);
   if (v.kn == 0)
-    return kfast ? launch_operand<true, false>(v, rows, k, sh, cnt, planes, st)
-                 : launch_operand<false, false>(v, rows, k, sh, cnt, planes, st);
-  return kfast ? launch_operand<true, true>(v, rows, k, sh, cnt, planes, st)
-               : launch_operand<false, true>(v, rows, k, sh, cnt, planes, st);
+    return kfast ? launch_operand<true, false>(v, rows, k, sh, cnt, planes, part, st)
+                 : launch_operand<false, false>(v, rows, k, sh, cnt, planes, part, st);
+  return kfast ? launch_operand<true, true>(v, rows, k, sh, cnt, planes, part, st)
+               : launch_operand<false, true>(v, rows, k, sh, cnt, planes, part, st);
+}
+
+int fricc_mod_operand(const ModView& v, int64_t rows, int64_t k, void* buf, cudaStream_t st) {
+  void* part = nullptr;
+  const int64_t bytes = part_bytes(rows, k);
+  int rc = bytes ? fricc_alloc(&part, bytes, st) : FRICC_OK;
+  if (!rc) rc = convert(v, rows, k, buf, part, st);
+  fricc_free(part, st);
+  return rc;
 }
 
 double fricc_mod_time_us(int64_t M, int64_t N, int64_t K, int64_t reps, bool a_shared, bool b_shared, bool conv_a,
@@ -1194,48 +1204,52 @@ double fricc_mod_time_us(int64_t M, int64_t N, int64_t K, int64_t reps, bool a_s
          12.5e-6 * (double)reps * M * N + 8.0 * (3 + (p.ks > 1) + ((conv_a ? 1 : 0) + (conv_b ? 1 : 0)) * (K > mod::SCH ? 3 : 1));
 }
 
-// The scratch of one product is bounded: an operand of more than this many
-// bytes of planes (or as many residues) is worked off in panels of its rows.
+// The scratch of one product is bounded: where its planes and residues would
+// take more than this, replicas are worked off in groups, and a single product
+// in panels of the rows of its larger operand (the smaller one is converted
+// whole).  All of it is taken before the first output is written, so a call that
+// cannot have it is left to the caller's other kernel.
 static constexpr int64_t MOD_PANEL_BYTES = 6ll << 30;
-
-int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out_, int64_t M, int64_t N, int64_t K,
-                   int64_t reps, bool a_shared, bool b_shared, bool skip_zero, cudaStream_t st) {
-  if (M <= 0 || N <= 0 || K <= 0 || K > mod::MAX_K || reps < 1) {
-    fricc_set_error("mod_gemm: bad arguments");
+static thread_local int64_t g_scratch = -1;
+int64_t fricc_mod_scratch_bound() { return g_scratch >= 0 ? g_scratch : MOD_PANEL_BYTES; }
+extern "C" int fricc_mod_scratch(int64_t bytes) {
+  if (bytes < -1) {
+    fricc_set_error("mod_scratch: a number of bytes, 0 (no modular products) or -1 (the default bound)");
     return FRICC_ERR_ARG;
   }
-  if (reps == 1) {
-    // (a prepared operand's planes are not cut: the other one's rows are)
-    const int64_t res_row = 2 * mod::PLANES;
-    const bool cut_b = !B.prepared && (A.prepared || N >= M);
-    const int64_t len = cut_b ? N : M;
-    int64_t per_row = res_row * (cut_b ? M : N);
-    if (!(cut_b ? B : A).prepared) per_row += 2 * mod::PLANES * fricc_cdiv(K, 64) * 64;
-    if (!(cut_b ? B : A).prepared && len > 2048 && len * per_row > MOD_PANEL_BYTES) {
-      int64_t panel = MOD_PANEL_BYTES / per_row / 256 * 256;
-      if (panel < 1024) panel = 1024;
-      ModView whole = cut_b ? A : B;
-      void* buf = nullptr;
-      int rc = FRICC_OK;
-      if (!whole.prepared) {
-        const int64_t rows = cut_b ? M : N;
-        rc = fricc_alloc(&buf, fricc_mod_operand_bytes(rows, K), st);
-        if (!rc) rc = fricc_mod_operand(whole, rows, K, buf, st);
-        whole.prepared = buf;
-      }
-      for (int64_t r0 = 0; r0 < len && !rc; r0 += panel) {
-        const int64_t n = len - r0 < panel ? len - r0 : panel;
-        ModView part = cut_b ? B : A;
-        ModOut o = out_;
-        part.rows.off += r0;
-        (cut_b ? o.col : o.row).off += r0;
-        rc = cut_b ? fricc_mod_gemm(whole, part, o, M, n, K, 1, true, true, skip_zero, st)
-                   : fricc_mod_gemm(part, whole, o, n, N, K, 1, true, true, skip_zero, st);
-      }
-      fricc_free(buf, st);
-      return rc;
-    }
+  g_scratch = bytes;
+  return FRICC_OK;
+}
+
+namespace {
+
+// The buffers of a product's pieces, which follow each other on one stream:
+// a first walk over the pieces finds the largest of each.
+struct Scratch {
+  enum { WHOLE, OPA, OPB, PART, RES, WORDS, N };
+  bool sizing = true;
+  int64_t need[N] = {};
+  void* buf[N] = {};
+  void* take(int which, int64_t bytes) {
+    if (sizing && bytes > need[which]) need[which] = bytes;
+    return buf[which];
   }
+  int get(cudaStream_t st) {
+    sizing = false;
+    for (int k = 0; k < N; ++k)
+      if (need[k])
+        if (int rc = fricc_alloc(&buf[k], need[k], st)) return rc;
+    return FRICC_OK;
+  }
+  void give_back(cudaStream_t st) {
+    for (int k = 0; k < N; ++k) fricc_free(buf[k], st);
+  }
+};
+
+// One launch of each kernel.  (sizing: only the scratch it takes; FRICC_MOD_NONE
+// where it is too large for one launch.)
+int mod_piece(const ModView& A, const ModView& B, const ModOut& out_, int64_t M, int64_t N, int64_t K, int64_t reps,
+              bool a_shared, bool b_shared, bool skip_zero, Scratch& scr, cudaStream_t st) {
   const int64_t rows_a = (a_shared ? 1 : reps) * M, rows_b = (b_shared ? 1 : reps) * N;
   const mod::Layout la = mod::layout(rows_a, K), lb = mod::layout(rows_b, K);
   int nsm = 0;
@@ -1252,19 +1266,19 @@ int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out_, int64
   const int64_t units = tm * tn * mod::PLANES * reps * ks;
   const int64_t tiles = reps * fricc_cdiv(m, 32) * fricc_cdiv(n, 64);
   if (units > 0x7fffffff || tiles * mod::LIST_W > 0x7fffffff || mod::PLANES * nk * rows_a + 256 > 0x7fffffff ||
-      mod::PLANES * nk * rows_b + 256 > 0x7fffffff) {
-    fricc_set_error("mod_gemm: problem too large for one launch");
-    return FRICC_ERR_ARG;
-  }
-  void *bufa = nullptr, *bufb = nullptr;
-  unsigned short* res = nullptr;
-  unsigned* words = nullptr;  // error word, list length, list
-  if (!A.prepared) rc = fricc_alloc(&bufa, la.bytes, st);
-  if (!rc && !B.prepared) rc = fricc_alloc(&bufb, lb.bytes, st);
-  if (!rc) rc = fricc_alloc_t(&res, (size_t)ks * mod::PLANES * reps * m * ng * 16, st);
-  if (!rc) rc = fricc_alloc_t(&words, 2 + tiles * mod::LIST_W, st);
-  if (!rc && !A.prepared) rc = fricc_mod_operand(A, rows_a, K, bufa, st);
-  if (!rc && !B.prepared) rc = fricc_mod_operand(B, rows_b, K, bufb, st);
+      mod::PLANES * nk * rows_b + 256 > 0x7fffffff)
+    return FRICC_MOD_NONE;
+  void* bufa = A.prepared ? nullptr : scr.take(Scratch::OPA, la.bytes);
+  void* bufb = B.prepared ? nullptr : scr.take(Scratch::OPB, lb.bytes);
+  void* part = scr.take(Scratch::PART, A.prepared ? 0 : part_bytes(rows_a, K));
+  part = scr.take(Scratch::PART, B.prepared ? 0 : part_bytes(rows_b, K));
+  auto* res = static_cast<unsigned short*>(
+      scr.take(Scratch::RES, (int64_t)ks * mod::PLANES * reps * m * ng * 16 * (int64_t)sizeof(unsigned short)));
+  // error word, list length, list
+  auto* words = static_cast<unsigned*>(scr.take(Scratch::WORDS, (2 + tiles * mod::LIST_W) * (int64_t)sizeof(unsigned)));
+  if (scr.sizing) return FRICC_OK;
+  if (!A.prepared) rc = convert(A, rows_a, K, bufa, part, st);
+  if (!rc && !B.prepared) rc = convert(B, rows_b, K, bufb, part, st);
   if (!rc) rc = fricc_cuda_check(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned), st), "mod_gemm");
   if (!rc) {
     const char* pa = static_cast<const char*>(A.prepared ? A.prepared : bufa);
@@ -1356,10 +1370,79 @@ int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out_, int64
       if (e != cudaSuccess) rc = fricc_cuda_fail(e, "mod_gemm", __FILE__, __LINE__);
     }
   }
-  fricc_free(bufa, st);
-  fricc_free(bufb, st);
-  fricc_free(res, st);
-  fricc_free(words, st);
+  return rc;
+}
+
+// A single product, in panels where it has to be.
+int mod_single(const ModView& A, const ModView& B, const ModOut& out, int64_t M, int64_t N, int64_t K, bool skip_zero,
+               Scratch& scr, cudaStream_t st) {
+  // (a prepared operand's planes are not cut: the other one's rows are)
+  const int64_t bound = fricc_mod_scratch_bound(), least = g_scratch >= 0 ? 256 : 1024;
+  const bool cut_b = !B.prepared && (A.prepared || N >= M);
+  const int64_t len = cut_b ? N : M;
+  const int64_t per_row = 2 * mod::PLANES * ((cut_b ? M : N) + fricc_cdiv(K, 64) * 64);
+  if ((cut_b ? B : A).prepared || len <= 2 * least || len * per_row <= bound)
+    return mod_piece(A, B, out, M, N, K, 1, true, true, skip_zero, scr, st);
+  int64_t panel = bound / per_row / 256 * 256;
+  if (panel < least) panel = least;
+  ModView whole = cut_b ? A : B;
+  int rc = FRICC_OK;
+  if (!whole.prepared) {
+    const int64_t rows = cut_b ? M : N;
+    void* buf = scr.take(Scratch::WHOLE, fricc_mod_operand_bytes(rows, K));
+    void* part = scr.take(Scratch::PART, part_bytes(rows, K));
+    if (!scr.sizing) rc = convert(whole, rows, K, buf, part, st);
+    whole.prepared = scr.sizing ? static_cast<const void*>(&scr) : buf;  // (not read while sizing)
+  }
+  for (int64_t r0 = 0; r0 < len && !rc; r0 += panel) {
+    const int64_t n = len - r0 < panel ? len - r0 : panel;
+    ModView cut = cut_b ? B : A;
+    ModOut o = out;
+    cut.rows.off += r0;
+    (cut_b ? o.col : o.row).off += r0;
+    rc = cut_b ? mod_piece(whole, cut, o, M, n, K, 1, true, true, skip_zero, scr, st)
+               : mod_piece(cut, whole, o, n, N, K, 1, true, true, skip_zero, scr, st);
+  }
+  return rc;
+}
+
+// The replicas, in groups where they have to be.
+int mod_groups(const ModView& A, const ModView& B, const ModOut& out, int64_t M, int64_t N, int64_t K, int64_t reps,
+               bool a_shared, bool b_shared, bool skip_zero, Scratch& scr, cudaStream_t st) {
+  if (reps == 1) return mod_single(A, B, out, M, N, K, skip_zero, scr, st);
+  const int64_t kp = fricc_cdiv(K, 64) * 64;
+  const int64_t per = 2 * mod::PLANES * (M * N + (a_shared ? 0 : M * kp) + (b_shared ? 0 : N * kp));
+  int64_t group = fricc_mod_scratch_bound() / per;
+  if (group >= reps) return mod_piece(A, B, out, M, N, K, reps, a_shared, b_shared, skip_zero, scr, st);
+  if (group < 1) group = 1;
+  int rc = FRICC_OK;
+  for (int64_t r0 = 0; r0 < reps && !rc; r0 += group) {
+    const int64_t n = reps - r0 < group ? reps - r0 : group;
+    ModView a = A, b = B;
+    ModOut o = out;
+    if (!a_shared) a.rows.off += r0 * M;
+    if (!b_shared) b.rows.off += r0 * N;
+    o.rep.off += r0;
+    rc = n == 1 ? mod_single(a, b, o, M, N, K, skip_zero, scr, st)
+                : mod_piece(a, b, o, M, N, K, n, a_shared, b_shared, skip_zero, scr, st);
+  }
+  return rc;
+}
+
+}  // namespace
+
+int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out, int64_t M, int64_t N, int64_t K, int64_t reps,
+                   bool a_shared, bool b_shared, bool skip_zero, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || K <= 0 || K > mod::MAX_K || reps < 1) {
+    fricc_set_error("mod_gemm: bad arguments");
+    return FRICC_ERR_ARG;
+  }
+  if (fricc_mod_scratch_bound() == 0) return FRICC_MOD_NONE;
+  Scratch scr;
+  int rc = mod_groups(A, B, out, M, N, K, reps, a_shared, b_shared, skip_zero, scr, st);
+  if (rc) return rc;
+  rc = scr.get(st) ? FRICC_MOD_NONE : mod_groups(A, B, out, M, N, K, reps, a_shared, b_shared, skip_zero, scr, st);
+  scr.give_back(st);
   return rc;
 }
 

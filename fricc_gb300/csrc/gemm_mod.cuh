@@ -59,6 +59,9 @@ struct ModOut {
 // A and B hold reps * M and (b_shared ? N : reps * N) rows, replica-major (A
 // likewise with a_shared).  skip_zero: elements of A whose bits are all
 // zero are absent (they multiply nothing, not even a NaN of B).
+// FRICC_MOD_NONE: its scratch could not be had (or it is too large for a
+// launch), and nothing was written.
+constexpr int FRICC_MOD_NONE = -1;
 int fricc_mod_gemm(const ModView& A, const ModView& B, const ModOut& out, int64_t M, int64_t N, int64_t K, int64_t reps,
                    bool a_shared, bool b_shared, bool skip_zero, cudaStream_t st);
 
@@ -82,8 +85,8 @@ bool fricc_mod_chosen(int64_t batch, int64_t M, int64_t N, int64_t K, bool a_bat
 // arguments; s2: the second batch level's strides or null) through
 // fricc_mod_gemm where that is chosen over the caller's kernel (FP64, or
 // FP32 pairs).  The choice does not depend on the second batch level, so a
-// replica takes the route of its lone product.  Returns a status, or -1 when
-// not taken.
+// replica takes the route of its lone product.  Returns a status, or
+// FRICC_MOD_NONE when not taken.
 int fricc_mod_try(const double* A, const double* B, double* C, int64_t batch, int64_t batch2, int64_t M, int64_t N,
                   int64_t K, const int64_t sA[3], const int64_t sB[3], const int64_t sC[3], const int64_t* s2,
                   double alpha, double beta, bool pairs, const void* a_mod, const void* b_mod, cudaStream_t st);

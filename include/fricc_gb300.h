@@ -197,6 +197,12 @@ int fricc_spmm(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, con
  * model (-1, the default). */
 int fricc_mod_select(int mode);
 int fricc_mod_mode(void); /* the calling thread's mode */
+/* The calling thread's bound, in bytes, on the scratch of one modular product
+ * beyond which it is worked off in pieces (results the same): -1 the default,
+ * 6 GB; 0: none may be taken, so every call runs on the FP64 or sparse kernels.
+ * The operand that is not cut is converted whole.  Where the scratch cannot be
+ * had, a call runs on those kernels too. */
+int fricc_mod_scratch(int64_t bytes);
 int64_t fricc_mod_bytes(int64_t rows, int64_t k);
 int fricc_mod_prepare(const double* x, int64_t rows, int64_t k, int64_t row_stride, int64_t k_stride, void* out,
                       void* stream);
