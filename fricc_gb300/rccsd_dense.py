@@ -192,24 +192,41 @@ class DeviceERIs:
             raise RuntimeError(f"split operand {role} of {name} missing: call prepare_tc() first")
         return got[1]
 
-    # device bytes of integral blocks kept converted for the modular products
-    # (all of them at o30v150 take 39 GB); a block beyond that is converted by
-    # each call that uses it
+    # device bytes of integral blocks kept converted for the modular products, at
+    # most (a seventh of the card; four times the FP64 blocks': all of them at
+    # o30v150 take 39 GB); a block beyond that is converted by each call that
+    # uses it
     MOD_BYTES = 40 << 30
 
+    @staticmethod
+    def _free_bytes():
+        """Device memory this process could still take: free, or cached unused."""
+        free, _ = torch.cuda.mem_get_info()
+        return free + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
+
     def _mod(self, key, name, rows, k, row_stride, k_stride):
+        # settled once per block: beyond the budget, or where as much again would
+        # not stay free (a solve that fits without it has to go on fitting), it is
+        # not kept
+        if ("not", key) in self._splits:
+            return None
+
         def make():
             need = L.load().fricc_mod_bytes(rows, k)
-            if self._mod_bytes + need > self.MOD_BYTES:
-                return None
-            got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
-            self._mod_bytes += need
-            return got
+            if self._mod_bytes + need <= self.MOD_BYTES and 2 * need <= self._free_bytes():
+                try:
+                    got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
+                    self._mod_bytes += need
+                    return got
+                except torch.OutOfMemoryError:
+                    pass
+            self._splits[("not", key)] = True
+            return None
         return self._kept(key, make)
 
     def mod_w(self, name, qs):
         """A constant W' block viewed as [keys][qs], its rows q prepared for
-        the modular products, built on first use (None past MOD_BYTES)."""
+        the modular products, built on first use (None where it is not kept)."""
         return self._mod(("modW", name, qs), name, qs, getattr(self, name).numel() // qs, 1, qs)
 
     def mod_a(self, name, m, k):
