@@ -202,22 +202,20 @@ def request_stream(n: int, rate: float, seed: int = 0, nocc=(5, 30), ratio=(4.0,
     return out
 
 
-def footprint_bytes(o: int, v: int, precision: str = "df64") -> int:
-    """HBM a resident solve needs: integral blocks and the layouts derived from
-    them (vvvv and its float-pair form, ovvv in nine layouts or forms),
-    amplitudes and work arrays (~16 o^2v^2), and the converted blocks and
-    scratch of the modular tensor-core products.  Split precision keeps (vv|vv)
-    only as the FP32 block it rebuilds (v^4 / 2 doubles) and adds the
-    BF16x3 operand splits (~4.5 o v^3 doubles)."""
+def footprint_bytes(o: int, v: int, precision: str = "df64", m: int | None = None) -> int:
+    """HBM a resident solve keeping m entries (default: a fifth of T2) needs:
+    integral blocks and the layouts derived from them (vvvv and its float-pair
+    form, ovvv in nine layouts or forms), amplitudes and work arrays (~16
+    o^2v^2), and what the modular tensor-core products take where its sizes
+    choose them.  Split precision keeps (vv|vv) only as the FP32 block it
+    rebuilds (v^4 / 2 doubles) and adds the BF16x3 operand splits (~4.5 o v^3
+    doubles)."""
     vvvv = 0.5 * v**4 if precision == "split" else 2 * v**4
     ovvv = 13.5 * o * v**3 if precision == "split" else 9 * o * v**3
     mod = 0
     if precision != "split":
-        # blocks kept converted for the modular products: 32 bytes an element of
-        # (vv|vv), the two halves of X/Y and four GEMM operands, up to
-        # DeviceERIs.MOD_BYTES, and the scratch of one product (two panels)
-        from .rccsd_dense import DeviceERIs
-        mod = min(32 * (v**4 + 6.5 * o * v**3), DeviceERIs.MOD_BYTES) + min(64 * v**4, 12 << 30)
+        from .rccsd_dense import converted_bytes
+        mod = converted_bytes(o, v, (o * v) ** 2 // 5 if m is None else int(m), precision == "df64")
     return int(8 * (vvvv + ovvv + 16 * o * o * v * v + 4 * o**4 + 8 * o**3 * v) + mod)
 
 
@@ -358,7 +356,7 @@ class SolveServer:
     # ----------------------------------------------------------- the stream
     def _release(self, req: Request) -> None:
         with self._cv:
-            self._in_use -= footprint_bytes(req.nocc, req.nvir, self.precision)
+            self._in_use -= footprint_bytes(req.nocc, req.nvir, self.precision, req.m)
             self._n_live -= 1
             self._cv.notify_all()
 
@@ -377,7 +375,7 @@ class SolveServer:
                 delay = r.arrival * time_scale - (time.perf_counter() - t0)
                 if delay > 0:
                     time.sleep(delay)
-                need = footprint_bytes(r.nocc, r.nvir, self.precision)
+                need = footprint_bytes(r.nocc, r.nvir, self.precision, r.m)
                 with self._cv:
                     while (self._in_use + need > self.budget or self._n_live >= cap) and self._n_live > 0:
                         self._cv.wait()

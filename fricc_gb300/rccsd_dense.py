@@ -136,12 +136,7 @@ class DeviceERIs:
         if every:
             return names
         o, v = self.nocc, self.mo_energy.numel() - self.nocc
-        ov = o * v
-        use = {"vvvvT": [(0, 1, 2, 3, v * v)], "ovvv_XY": [(0, 1, 2, 3, 2 * ov)], "ovov": [(3, 0, 1, 2, ov)],
-               "ovov_0312": [(3, 0, 1, 2, ov)], "ovov_0313_0113": [(2, 0, 1, 3, ov)],
-               "ovov_cdkl": [(0, 1, 2, 3, o * o)], "oooo_klij": [(2, 3, 0, 1, o * o)],
-               "lin_WA": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)], "lin_WB": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)],
-               "lin_W2AB": [(1, 3, 0, 2, ov)]}
+        use = sparse_uses(o, v)
         dims = (o, o, v, v)
 
         def modular(n, t):
@@ -473,6 +468,40 @@ def gemm_f64(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1
         b_mod.data_ptr() if b_mod is not None else None, C.data_ptr(), batch, batch2, M, N, K, *s4, float(alpha),
         float(beta), L.cur_stream()))
     return C
+
+
+def sparse_uses(o, v):
+    """The sparse terms (pa, pb, ka, kb, QS) each constant W' block serves."""
+    ov = o * v
+    return {"vvvvT": [(0, 1, 2, 3, v * v)], "ovvv_XY": [(0, 1, 2, 3, 2 * ov)], "ovov": [(3, 0, 1, 2, ov)],
+            "ovov_0312": [(3, 0, 1, 2, ov)], "ovov_0313_0113": [(2, 0, 1, 3, ov)], "ovov_cdkl": [(0, 1, 2, 3, o * o)],
+            "oooo_klij": [(2, 3, 0, 1, o * o)], "lin_WA": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)],
+            "lin_WB": [(1, 3, 0, 2, ov), (1, 2, 0, 3, ov)], "lin_W2AB": [(1, 3, 0, 2, ov)]}
+
+
+def dense_uses(o, v):
+    """The dense products (M, N, K) of FRI-CCSD with a constant block, and
+    which operand it is."""
+    return {"g_klcd": (o, o, o * v * v, "A"), "g_kldc": (v, v, o * o * v, "B"), "G_t1": (o, v, o * v * v, "B"),
+            "ovvv_iabc": (o * v * v, o, v, "A"), "ovvv": (o * v * v, o, v, "A"), "ovvv_kacd": (o * v * v, o, v, "A")}
+
+
+def converted_bytes(o, v, m, pairs) -> int:
+    """Device bytes a FRI-CCSD solve keeping m entries takes for the modular
+    products: the constant blocks its sizes let it keep converted
+    (DeviceERIs.MOD_BYTES at most), and the scratch of one product (planes and
+    residues of amplitude-sized operands).  0 where no term runs so."""
+    lib = L.load()
+    uses = sparse_uses(o, v)
+    kept, dims = 0, (o, o, v, v)
+    for name in DeviceERIs.SPLIT_BLOCKS:
+        pa, pb, ka, kb, qs = uses[name][0]
+        if takes_mod(dims, m, uses[name][0], True, pairs):
+            kept += lib.fricc_mod_bytes(qs, dims[ka] * dims[kb])
+    for M, N, K, side in dense_uses(o, v).values():
+        if _gemm_route(M, N, K, side == "A", side == "B", bool(pairs), lib.fricc_mod_mode()):
+            kept += lib.fricc_mod_bytes(M if side == "A" else N, K)
+    return min(kept, DeviceERIs.MOD_BYTES) + (104 * (o * v) ** 2 if kept else 0)
 
 
 def takes_mod(dims, m, term, prepared, pairs) -> bool:
