@@ -209,6 +209,8 @@ int fricc_tune_set(int knob, int value) {
   return FRICC_OK;
 }
 
+int fricc_tune_value(int knob) { return fricc_tune_get(knob); }
+
 void fricc_prof_enable(int on) {
   std::lock_guard<std::mutex> lk(g_prof_mu);
   g_prof.store(on != 0);

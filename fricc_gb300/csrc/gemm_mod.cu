@@ -1457,7 +1457,9 @@ double fricc_mod_alt_us(int64_t batch, int64_t M, int64_t N, int64_t K, bool pai
 bool fricc_mod_chosen(int64_t batch, int64_t M, int64_t N, int64_t K, bool a_batched, bool b_batched, bool a_prepared,
                       bool b_prepared, double alt_us) {
   const int force = fricc_mod_mode();
-  if (force == 0 || K > mod::MAX_K) return false;
+  // (up to four rows or columns are the GEMV kernels'; a tile set by a tuner is a
+  // choice of the other kernels)
+  if (force == 0 || M <= 4 || N <= 4 || K > mod::MAX_K || fricc_tune_get(FRICC_TUNE_GEMM_TILE) >= 0) return false;
   if (force == 1) return true;
   int64_t reps = 1;
   if (batch > 1) {
@@ -1471,10 +1473,9 @@ bool fricc_mod_chosen(int64_t batch, int64_t M, int64_t N, int64_t K, bool a_bat
 int fricc_mod_try(const double* A, const double* B, double* C, int64_t batch, int64_t batch2, int64_t M, int64_t N,
                   int64_t K, const int64_t sA[3], const int64_t sB[3], const int64_t sC[3], const int64_t* s2,
                   double alpha, double beta, bool pairs, const void* a_mod, const void* b_mod, cudaStream_t st) {
-  if (M <= 4 || N <= 4 || fricc_tune_get(FRICC_TUNE_GEMM_TILE) >= 0 ||
-      !fricc_mod_chosen(batch, M, N, K, sA[2] != 0, sB[2] != 0, a_mod != nullptr, b_mod != nullptr,
+  if (!fricc_mod_chosen(batch, M, N, K, sA[2] != 0, sB[2] != 0, a_mod != nullptr, b_mod != nullptr,
                         fricc_mod_alt_us(batch, M, N, K, pairs)))
-    return -1;
+    return FRICC_MOD_NONE;
   struct Level {
     int64_t n, a, b, c;
   };

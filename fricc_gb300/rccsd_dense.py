@@ -499,7 +499,7 @@ def converted_bytes(o, v, m, pairs) -> int:
         if takes_mod(dims, m, uses[name][0], True, pairs):
             kept += lib.fricc_mod_bytes(qs, dims[ka] * dims[kb])
     for M, N, K, side in dense_uses(o, v).values():
-        if _gemm_route(M, N, K, side == "A", side == "B", bool(pairs), lib.fricc_mod_mode()):
+        if gemm_takes_mod(M, N, K, side == "A", side == "B", pairs):
             kept += lib.fricc_mod_bytes(M if side == "A" else N, K)
     return min(kept, DeviceERIs.MOD_BYTES) + (104 * (o * v) ** 2 if kept else 0)
 
@@ -510,8 +510,12 @@ def takes_mod(dims, m, term, prepared, pairs) -> bool:
     return _spmm_route(tuple(dims), int(m), term, bool(prepared), bool(pairs), L.load().fricc_mod_mode())
 
 
-# (the routes are pure functions of the sizes and the thread's fricc_mod_select
-# mode; an iteration asks ~30 times, ~3 us each through ctypes)
+GEMM_TILE = 1  # fricc_tune_set's knob
+
+
+# (the routes are pure functions of the sizes, the thread's fricc_mod_select mode
+# and, for GEMMs, its tile knob; an iteration asks ~30 times, ~3 us each through
+# ctypes)
 @functools.lru_cache(maxsize=4096)
 def _spmm_route(dims, m, term, prepared, pairs, mode):
     pa, pb, ka, kb, qs = term
@@ -519,8 +523,16 @@ def _spmm_route(dims, m, term, prepared, pairs, mode):
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_route(M, N, K, a_prepared, b_prepared, pairs, mode):
+def _gemm_route(M, N, K, a_prepared, b_prepared, pairs, mode, tile):
     return bool(L.load().fricc_gemm_takes_mod(1, M, N, K, 0, 0, int(a_prepared), int(b_prepared), int(pairs)))
+
+
+def gemm_takes_mod(M, N, K, a_prepared, b_prepared, pairs) -> bool:
+    """Whether a dense product of this shape runs as a modular one
+    (fricc_gemm_takes_mod)."""
+    lib = L.load()
+    return _gemm_route(M, N, K, bool(a_prepared), bool(b_prepared), bool(pairs), lib.fricc_mod_mode(),
+                       lib.fricc_tune_value(GEMM_TILE))
 
 
 def mod_constants(E, A, B, C, const, const_b, pairs):
@@ -530,7 +542,7 @@ def mod_constants(E, A, B, C, const, const_b, pairs):
     if const is None and const_b is None:
         return None, None
     M, N, K = C.shape[-2], C.shape[-1], A.shape[-1]
-    if not _gemm_route(M, N, K, const is not None, const_b is not None, bool(pairs), L.load().fricc_mod_mode()):
+    if not gemm_takes_mod(M, N, K, const is not None, const_b is not None, pairs):
         return None, None
     return (E.mod_a(const, M, K) if const else None), (E.mod_b(const_b, K, N) if const_b else None)
 

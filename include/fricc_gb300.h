@@ -537,6 +537,7 @@ int fricc_stream_destroy(void* stream);
  * result's arithmetic except the GEMMs' tile and split, which reorder
  * their sums. */
 int fricc_tune_set(int knob, int value);
+int fricc_tune_value(int knob); /* the calling thread's; -1: the built-in choice */
 
 /* Instrumentation (no reference counterpart): the number of kernels this
  * library has launched so far; and CUDA-event timing of every sparse
