@@ -194,10 +194,11 @@ class DeviceERIs:
     MOD_BYTES = 40 << 30
 
     @staticmethod
-    def _free_bytes():
-        """Device memory this process could still take: free, or cached unused."""
+    def _free_bytes(enough):
+        """Device memory this process could still take: free, and (asked for,
+        ~150 us, only where that is not ``enough``) cached unused."""
         free, _ = torch.cuda.mem_get_info()
-        return free + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
+        return free if free >= enough else free + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
 
     def _mod(self, key, name, rows, k, row_stride, k_stride):
         # settled once per block: beyond the budget, or where as much again would
@@ -208,7 +209,9 @@ class DeviceERIs:
 
         def make():
             need = L.load().fricc_mod_bytes(rows, k)
-            if self._mod_bytes + need <= self.MOD_BYTES and 2 * need <= self._free_bytes():
+            # (a thousandth of the card is not worth the question)
+            roomy = need < 1 << 28 or 2 * need <= self._free_bytes(2 * need)
+            if self._mod_bytes + need <= self.MOD_BYTES and roomy:
                 try:
                     got = mod_operand(getattr(self, name), rows, k, row_stride, k_stride)
                     self._mod_bytes += need

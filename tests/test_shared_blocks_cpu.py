@@ -36,7 +36,7 @@ def shared(monkeypatch):
         monkeypatch.setattr(mod, name, lambda *a: "made")
     lib = types.SimpleNamespace(fricc_mod_bytes=lambda rows, k: 32 * rows * k)
     monkeypatch.setattr(D.L, "load", lambda *a: lib)
-    monkeypatch.setattr(D.DeviceERIs, "_free_bytes", staticmethod(lambda: 1 << 40))
+    monkeypatch.setattr(D.DeviceERIs, "_free_bytes", staticmethod(lambda *a: 1 << 40))
     return E, st
 
 
