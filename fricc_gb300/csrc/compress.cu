@@ -729,15 +729,16 @@ __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __res
 //
 // The tensor is cut into regions of S elements; a segment starts at the
 // first wrap of its region that the exact fixed-point prefix sums (mod 1, in
-// 2^-64) predict.  k_piv_walk<1> walks every segment from its predicted
-// start, once per parity, and leaves its map; k_piv_claims composes them to
-// the start of each segment; k_piv_walk<2> walks each segment again from
+// 2^-64) predict (k_piv_starts).  k_piv_walk<1> walks every segment from its
+// predicted start, once per parity, and leaves its map; k_piv_claims composes
+// them to the start of each segment; k_piv_walk<2> walks each segment again from
 // there with the sampler's own FP64 operations, writes a_j and the flags, and
 // compares its end with the next segment's start.  If they all agree the
 // recurrence holds from end to end: the result does not rest on the argument
 // above.  Where one does not (a prediction within ~1e-12 of a power of
 // two), the claims behind it are recomputed from its true end, twice; what
-// then remains (and p outside [0, 1], m' = 0) is left to the serial walk.
+// then remains (and p outside [0, 1], m' = 0, a stretch without a wrap through
+// half the tensor) is left to the serial walk.
 //
 // Bound by the latency of two dependent FP64 additions per element over one
 // segment (~70 ns each): o13v57 (549,081 elements) 73 ms serial, 60 us so.
@@ -806,14 +807,51 @@ __device__ __forceinline__ bool ge_one(double s) { return (__double_as_longlong(
 __device__ __forceinline__ bool piv_step(double& a, double p) {
   const double sum = __dadd_rn(a, p);
   const bool w = ge_one(sum);
-  a = w ? __dsub_rn(sum, 1.0) : sum;
+  a = __dadd_rn(sum, w ? -1.0 : 0.0);  // (sum >= +0: adding 0 leaves it)
   return w;
 }
 
-// One thread per segment.  PASS 1: find the start, walk both parities of the
-// predicted weight to the next segment's start, leave the map (segment 0:
-// its true end).  PASS 2: walk from the claimed weight, write a_j, the wrap
-// flags and their number, and report an end that is not the next claim.
+// The segments' starts, one thread each: the first wrap of the region that the
+// prefix sums predict, and the weight they predict after it.
+__global__ void __launch_bounds__(64) k_piv_starts(const double* __restrict__ P, PivSegs g, const Ctl* c) {
+  if (c->serial) return;
+  const int64_t s = (int64_t)blockIdx.x * 64 + threadIdx.x;
+  if (s >= g.nseg) return;
+  if (s == 0) {
+    g.start[0] = 0;
+    return;
+  }
+  const int64_t j0 = s * g.S, j1 = j0 + g.S < g.n ? j0 + g.S : g.n;
+  unsigned long long F = g.f[s];
+  int64_t at = -1;
+  constexpr int U = 8;  // elements loaded at once
+  for (int64_t j = j0; j < j1 && at < 0; j += U) {
+    double p[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) p[q] = j + q < j1 ? P[j + q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const unsigned long long F1 = F + frac64(p[q]);
+      if (at < 0) {
+        if (F1 < F) at = j + q;
+        F = F1;
+      }
+    }
+  }
+  g.start[s] = at;
+  if (at >= 0) g.claim[s] = (double)(long long)(F >> 12) * PW_ULP;
+}
+
+// One thread per segment.  PASS 1: walk both parities of the predicted weight to
+// the next segment's start, leave the map (segment 0: its true end).  PASS 2: walk
+// from the claimed weight, write a_j, the wrap flags and their number, and report
+// an end that is not the next claim.
+//
+// Both passes together take ~280 ns per element of the longest segment, the
+// serial walk ~136 per element of the tensor: a stretch without a wrap of more
+// than 15/32 of it (one or two samples; a long run of zeros) leaves the whole walk
+// to the serial one.  (549,081 elements, 1 sample: 155 ms, now 75; 3 samples, in
+// parallel: 52.)
 template <int PASS>
 __global__ void __launch_bounds__(64) k_piv_walk(const double* __restrict__ P, PivSegs g, Ctl* c,
                                                  double* __restrict__ A, unsigned char* __restrict__ code,
@@ -822,45 +860,33 @@ __global__ void __launch_bounds__(64) k_piv_walk(const double* __restrict__ P, P
   const int64_t s = (int64_t)blockIdx.x * 64 + threadIdx.x;
   if (s >= g.nseg) return;
   // a later round walks only what follows the segment that failed
-  int64_t first = 0;
   if (PASS == 2 && from_bad) {
-    first = from_bad == 1 ? g.cnt[g.nseg] : g.cnt[g.nseg + 1];  // the last round's bad segment
+    const int64_t first = from_bad == 1 ? g.cnt[g.nseg] : g.cnt[g.nseg + 1];  // the last round's bad segment
     if (first >= g.nseg || s <= first) return;
   }
-  int64_t j = s * g.S;
-  unsigned long long F = g.f[s];
+  const int64_t at = g.start[s];
+  if (at < 0) {
+    if (PASS == 1) g.map[s] = exact::map_id();
+    return;
+  }
+  // to the next segment's start
+  int64_t last = g.n - 1, nxt = g.nseg;
+  for (int64_t t = s + 1; t < g.nseg; ++t)
+    if (g.start[t] >= 0) {
+      last = g.start[t];
+      nxt = t;
+      break;
+    }
   double a0, a1 = 0.0;
   if (PASS == 1) {
-    if (s == 0) {
-      a0 = P[0];
-      F += frac64(a0);
-      g.start[0] = 0;
-      j = 1;
-    } else {
-      const int64_t j1 = j + g.S < g.n ? j + g.S : g.n;
-      int64_t at = -1;
-      for (; j < j1; ++j) {
-        const unsigned long long F1 = F + frac64(P[j]);
-        const bool w = F1 < F;
-        F = F1;
-        if (w) {
-          at = j++;
-          break;
-        }
-      }
-      g.start[s] = at;
-      if (at < 0) {
-        g.map[s] = exact::map_id();
-        return;
-      }
-      const unsigned long long n = F >> 12;  // the weight in units of 2^-52
-      a0 = (double)(long long)(n & ~1ull) * PW_ULP;
-      a1 = (double)(long long)(n | 1ull) * PW_ULP;
+    if ((last - at) * 32 > g.n * 15) {
+      c->serial = 1;
+      return;
     }
+    const long long n = s == 0 ? 0 : (long long)(g.claim[s] * 0x1p52);
+    a0 = s == 0 ? P[0] : (double)(n & ~1ll) * PW_ULP;
+    a1 = (double)(n | 1ll) * PW_ULP;
   } else {
-    const int64_t at = g.start[s];
-    if (at < 0) return;
-    j = at + 1;
     a0 = s == 0 ? P[0] : g.claim[s];
     if (s == 0) {
       A[0] = a0;
@@ -868,47 +894,38 @@ __global__ void __launch_bounds__(64) k_piv_walk(const double* __restrict__ P, P
     }
   }
   const double b0 = a0, b1 = a1;
-  // to the next segment's start: the first predicted wrap past this region
-  // (PASS 2 knows where it is)
-  int64_t last = g.n - 1, nxt = g.nseg;
-  if (PASS == 2) {
-    for (int64_t t = s + 1; t < g.nseg; ++t)
-      if (g.start[t] >= 0) {
-        last = g.start[t];
-        nxt = t;
-        break;
-      }
-  }
-  const int64_t edge = (s + 1) * g.S;
   int cnt = 0;
-  bool w0 = false, w1 = false, done = false;
+  bool w0 = false, w1 = false;
   constexpr int U = 8;  // elements loaded ahead
   double buf[U];
+  int64_t j = at + 1;
 #pragma unroll
   for (int q = 0; q < U; ++q) buf[q] = j + q <= last ? P[j + q] : 0.0;
-  while (j <= last && !done) {
-    double cur[U];
+  while (j <= last) {
+    // (another segment may have left the walk to the serial one; asked inside the
+    // inner loop, it cost 7% of the walk)
+    if (PASS == 1 && *(volatile int64_t*)&c->serial) return;
+    const int64_t stop = j + 128 * U <= last ? j + 128 * U : last + 1;
+    for (; j < stop; j += U) {
+      double cur[U];
 #pragma unroll
-    for (int q = 0; q < U; ++q) cur[q] = buf[q];
+      for (int q = 0; q < U; ++q) cur[q] = buf[q];
 #pragma unroll
-    for (int q = 0; q < U; ++q) buf[q] = j + U + q <= last ? P[j + U + q] : 0.0;
+      for (int q = 0; q < U; ++q) buf[q] = j + U + q <= last ? P[j + U + q] : 0.0;
 #pragma unroll
-    for (int q = 0; q < U; ++q) {
-      if (j + q <= last && !done) {
-        w0 = piv_step(a0, cur[q]);
-        if (PASS == 1) {
-          w1 = piv_step(a1, cur[q]);
-          const unsigned long long F1 = F + frac64(cur[q]);
-          done = F1 < F && j + q >= edge;
-          F = F1;
-        } else {
-          A[j + q] = a0;
-          code[j + q] = w0 ? PV_EMIT : 0;
-          cnt += w0 ? 1 : 0;
+      for (int q = 0; q < U; ++q) {
+        if (j + q <= last) {
+          w0 = piv_step(a0, cur[q]);
+          if (PASS == 1) {
+            w1 = piv_step(a1, cur[q]);
+          } else {
+            A[j + q] = a0;
+            code[j + q] = w0 ? PV_EMIT : 0;
+            cnt += w0 ? 1 : 0;
+          }
         }
       }
     }
-    j += U;
   }
   if (PASS == 1) {
     if (s == 0) {
@@ -1577,6 +1594,7 @@ static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsi
       const unsigned gw = (unsigned)fricc_cdiv(g.nseg, 64);
       k_piv_sums<<<grid_for(g.nseg, 8), 256, 0, st>>>(P, g, ctl);
       k_piv_prefix<<<1, 1024, 0, st>>>(g, ctl);
+      k_piv_starts<<<gw, 64, 0, st>>>(P, g, ctl);
       k_piv_walk<1><<<gw, 64, 0, st>>>(P, g, ctl, A, code, 0);
       for (int round = 0; round < 3; ++round) {
         k_piv_claims<<<1, 1024, 0, st>>>(g, ctl, round);
@@ -1584,7 +1602,7 @@ static int pivotal(int64_t n, const GenP& gp, Ctl* ctl, CompressScratch& s, unsi
       }
       k_piv_end<<<1, 1024, 0, st>>>(g, code, ctl);
       k_piv_chain<<<1, 32, 0, st>>>(P, n, ctl, A, code);
-      fricc_note_launch(12);
+      fricc_note_launch(13);
     }
   }
   if (!rc) {
