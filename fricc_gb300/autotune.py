@@ -4,7 +4,8 @@ The library exposes thread-local overrides of its launch configurations
 (``fricc_tune_set``): the float-pair sparse kernel's output pairs per thread,
 the FP32-pair GEMM's tile shape and split-K target, and the width of the
 compression's first select digit (how many candidates its exact top-m sort
-takes).  ``Autotuner`` times
+takes); and of the route to its modular tensor-core products
+(``fricc_mod_select``).  ``Autotuner`` times
 every candidate configuration of an operation the first time it meets that
 operation's shape -- on scratch copies of the outputs, so the real result is
 computed once, after the choice -- and replays the fastest configuration for
@@ -22,6 +23,7 @@ import torch
 from . import _lib as L
 
 SPMM_PPT, GEMM_TILE, GEMM_COVER, SELECT_BITS, SPMM_PERSIST = 0, 1, 2, 4, 5
+MOD = 100  # not a launch knob: fricc_mod_select
 
 # candidate configurations: {knob: value}; {} is the library's own choice.
 # The sparse kernel's gather tiles: pairs per thread (the q tile of a CTA is
@@ -32,19 +34,25 @@ GEMM_CANDIDATES = [{}] + [{GEMM_TILE: t, GEMM_COVER: c} for t, c in itertools.pr
 # the compression's top-m selection schedule: the first select digit's width
 # (candidates left for the exact sort), 12 bits by default
 COMPRESS_CANDIDATES = [{SELECT_BITS: b} for b in (10, 11, 12, 13)]
+# beside either list, where an untuned solver would take it (so a tuned one is
+# never the slower of the two): the modular tensor-core product
+MOD_CANDIDATE = {MOD: 1}
 
 
 @contextlib.contextmanager
 def knobs(cfg: dict):
     """Set the overrides of ``cfg`` for the launches inside the block."""
     lib = L.load()
+
+    def put(k, v):
+        return lib.fricc_mod_select(int(v)) if k == MOD else lib.fricc_tune_set(int(k), int(v))
     try:
         for k, v in cfg.items():
-            L.check(lib.fricc_tune_set(int(k), int(v)))
+            L.check(put(k, v))
         yield
     finally:
         for k in cfg:
-            lib.fricc_tune_set(int(k), -1)
+            put(k, -1)
 
 
 def _cuda_timer(fn):

@@ -245,12 +245,16 @@ class FRICCSDGPU:
         term = (pa, pb, ka, kb, int(QS))
         m = int(self.settings["m_keep"])
         Wm = None
-        if const and self._tuner is None and D.takes_mod(self._dims, m, term, True, self._df):
+        if const and D.takes_mod(self._dims, m, term, True, self._df):
             Wm = self.eris.mod_w(const, QS)
-        if Wm is not None or (self._tuner is None and D.takes_mod(self._dims, m, term, False, self._df)):
+        modular = Wm is not None or D.takes_mod(self._dims, m, term, False, self._df)
+
+        def launch_mod(outs):
             # FP64-accurate on the tensor cores (in either precision)
             L.check(self.lib.fricc_spmm_mod(T, pa, pb, ka, kb, float(coef), _ptr(Wp),
-                                            _ptr(Wm) if Wm is not None else None, int(QS), _ptr(Op), stream))
+                                            _ptr(Wm) if Wm is not None else None, int(QS), _ptr(outs[0]), stream))
+        if modular and self._tuner is None:
+            launch_mod([Op])
         elif self._df:
             if const:
                 self.eris.prepare_splits((const,))
@@ -258,11 +262,14 @@ class FRICCSDGPU:
             assert W2.numel() == (Wp.numel() // QS) * ((QS + 1) // 2) * 4, "float-pair W' split with another QS"
 
             def launch(outs):
+                if modular and self.lib.fricc_mod_mode() == 1:
+                    return launch_mod(outs)
                 L.check(self.lib.fricc_spmm_f2(T, pa, pb, ka, kb, float(coef), _ptr(W2), int(QS), _ptr(outs[0]),
                                                stream))
             if self._tuner is not None:
-                from .autotune import SPMM_CANDIDATES
-                self._tuner.run(("spmm", pa, pb, ka, kb, int(QS), self._dims), SPMM_CANDIDATES, launch, [Op])
+                from .autotune import MOD_CANDIDATE, SPMM_CANDIDATES
+                self._tuner.run(("spmm", pa, pb, ka, kb, int(QS), self._dims),
+                                SPMM_CANDIDATES + [MOD_CANDIDATE] * modular, launch, [Op])
             else:
                 launch([Op])
         else:
@@ -413,15 +420,21 @@ class FRICCSDGPU:
             tuner = self._tuner
 
             def mm(A_, B_, C_, alpha=1.0, beta=0.0, const=None, const_b=None):
+                Am, Bm = D.mod_constants(E, A_, B_, C_, const, const_b, self._df)
+                kept = Am is not None or Bm is not None
                 if tuner is None:
-                    Am, Bm = D.mod_constants(E, A_, B_, C_, const, const_b, self._df)
-                    if Am is not None or Bm is not None:
+                    if kept:
                         return D.gemm_f64(A_, B_, C_, alpha, beta, Am, Bm)
                     return mm0(A_, B_, C_, alpha, beta)
-                from .autotune import GEMM_CANDIDATES
+                from .autotune import GEMM_CANDIDATES, MOD_CANDIDATE
                 key = ("gemm", tuple(A_.shape), A_.stride(), tuple(B_.shape), B_.stride(), tuple(C_.shape),
-                       C_.stride(), beta != 0.0)
-                tuner.run(key, GEMM_CANDIDATES, lambda outs: mm0(A_, B_, outs[0], alpha, beta), [C_])
+                       C_.stride(), beta != 0.0, const, const_b)
+
+                def launch(outs):  # (without a kept operand the candidate {} takes the modular route by itself)
+                    if kept and self.lib.fricc_mod_mode() == 1:
+                        return D.gemm_f64(A_, B_, outs[0], alpha, beta, Am, Bm)
+                    return mm0(A_, B_, outs[0], alpha, beta)
+                tuner.run(key, GEMM_CANDIDATES + [MOD_CANDIDATE] * kept, launch, [C_])
                 return C_
 
         f64, dev = t2.dtype, t2.device
