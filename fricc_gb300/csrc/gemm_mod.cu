@@ -1230,6 +1230,19 @@ struct Scratch {
   bool sizing = true;
   int64_t need[N] = {};
   void* buf[N] = {};
+  // the last piece's plan, which the second walk mostly asks for again (~3 us)
+  int64_t shape[4] = {};
+  mod::Plan plan;
+  const mod::Plan& plan_of(int64_t M, int64_t Nn, int64_t K, int64_t reps, int nsm) {
+    if (shape[0] != M || shape[1] != Nn || shape[2] != K || shape[3] != reps) {
+      plan = mod::plan_for(M, Nn, K, reps, nsm);
+      shape[0] = M;
+      shape[1] = Nn;
+      shape[2] = K;
+      shape[3] = reps;
+    }
+    return plan;
+  }
   void* take(int which, int64_t bytes) {
     if (sizing && bytes > need[which]) need[which] = bytes;
     return buf[which];
@@ -1255,7 +1268,7 @@ int mod_piece(const ModView& A, const ModView& B, const ModOut& out_, int64_t M,
   int nsm = 0;
   int rc = tc::sm_count(&nsm);
   if (rc) return rc;
-  const mod::Plan pl = mod::plan_for(M, N, K, reps, nsm);
+  const mod::Plan pl = scr.plan_of(M, N, K, reps, nsm);
   const bool sw = pl.swap;  // the residues as [N][M] instead of [M][N]
   const int64_t m = sw ? N : M, n = sw ? M : N;
   const int64_t tm = fricc_cdiv(m, tc::BM), tn = fricc_cdiv(n, pl.bn);

@@ -201,6 +201,9 @@ class DeviceERIs:
         return free if free >= enough else free + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
 
     def _mod(self, key, name, rows, k, row_stride, k_stride):
+        got = self._splits.get(key)
+        if got is not None:
+            return got
         # settled once per block: beyond the budget, or where as much again would
         # not stay free (a solve that fits without it has to go on fitting), it is
         # not kept
