@@ -684,7 +684,7 @@ constexpr unsigned char PV_TAKE = 1, PV_EMIT = 2, PV_PIVOT = 4;
 // P = the p vector, with the p > 1 check and (psum, zeroed beforehand) the
 // approximate sum of each exact::CH chunk of the addends its chain takes.
 // Four blocks share a chunk, so that a small tensor's spread over the chip.  The
-// divisions by R run on the integer pipe (div_by): 20 M elements 503 -> 153 us,
+// divisions by R run on the integer pipe (div_by): 20 M elements 503 -> 144 us,
 // of which the FP64 multiplication and sum are 70.
 constexpr int PV_SUB = 4;
 __global__ void __launch_bounds__(256) k_pvec(GenP gp0, int64_t n, double* __restrict__ P, unsigned* err,

@@ -26,9 +26,13 @@
 // terms commits about 0.2 n^1/2 2^-53 (sum x^2 y^2)^1/2.  The two part where
 // the large elements of x meet the small ones of y, so a 16th plane holds the
 // squares (BF16): every output is checked against n s2 >= 2^-16 |x|^2 |y|^2, s2
-// the largest sum x^2 y^2 of a run of 512 k, and one that fails (true zeros apart: ZERO_SPAN), that belongs to
-// a row that is not finite, or whose pipeline gave up, is recomputed with FP64
-// FMAs (k_mod_fix).
+// the largest sum x^2 y^2 of a run of 512 k, and one that fails (true zeros
+// apart: ZERO_SPAN), that belongs to a row that is not finite, or whose pipeline
+// gave up, is recomputed with FP64 FMAs (k_mod_fix).  (At that line, where all
+// squares sit in one run, the error is two to three times one chain's, and by the
+// root of its slices more against the FP64 kernel's split sums; from 2^-14 up it
+// is below a chain's.  A line at 2^-13 listed 70 tiles an o30v150 iteration, 0.9
+// ms, and changed no measured error; 2^-12 took 56 ms.)
 // A result is the same in any tiling, batch or split of K: integer sums do not
 // depend on their order, a sum has one balanced residue whatever the order of its
 // reductions (make_tab), and the check compares the largest of the runs' squares,
@@ -39,8 +43,8 @@
 // Measured on a GB300 (operands prepared; DFMA kernel): 900 x 22500 x 22500
 // 9.1 ms; 4500^3 2.05 ms (152 ms); 2000^3 0.26 ms (14.0 ms); 400^3 30 us
 // (279 us); 675000 x 30 x 150 0.97 ms (5.25 ms).  Converting an operand: 10-11 ps
-// an element.  Error (2-norm, against 64 bits) of the o30v150 iteration: 7e-16,
-// 2.3e-15 on the FP64 pipe.
+// an element.  Error (2-norm, against 64 bits) of the o30v150 iteration over
+// several inputs: 7.0e-16 to 1.6e-15, 2.3e-15 on the FP64 pipe.
 #include <climits>
 
 #include "gemm_mod.cuh"
@@ -568,7 +572,7 @@ struct GemmArgs {
   int M;
   int a_rows, b_rows;    // rows of A and B (a K block of a plane)
   int a_rep, b_rep;      // rows per replica (0: shared)
-  int ks, chunks;        // K slices, 256-wide K runs in all
+  int ks, chunks;        // K slices, 512-wide K runs in all
   // the residues: [slice][plane][rep][ng][M][16], columns in groups of 16, so
   // that a warp's 32 rows store 1 KB runs (row-major, each lane's 16 bytes
   // went to a line of its own: 4096 store cycles a tile, the bound of every
@@ -598,10 +602,10 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs& g, int u) {
 
 // Work unit u = ((rep * PLANES + plane) * ks + slice) * tiles + tile.  Roles
 // as in gemm_tc.cu: TMA producer, MMA issuer, sixteen epilogue warps; the two
-// TMEM accumulators alternate per 256-wide K run, so a run is drained,
+// TMEM accumulators alternate per 512-wide K run, so a run is drained,
 // reduced modulo p and added to the warps' registers while the next one
-// accumulates.  A run of 128 x 256 outputs costs 2048 clocks of MMA and ~900
-// issue slots per scheduler of epilogue.
+// accumulates.  A run of 128 x 256 outputs costs 4096 clocks of MMA and ~1700 of
+// epilogue (plan_for).
 __global__ void __launch_bounds__(MNT, 1)
     k_mod_gemm(const __grid_constant__ CUtensorMap tma, const __grid_constant__ CUtensorMap tmb, GemmArgs g, int nunits,
                unsigned* err) {

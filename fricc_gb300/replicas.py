@@ -8,9 +8,10 @@ of every replica (fricc/friccsd.py:100-117) in one batched paired
 compression, every sparse term in one batched launch, the dense GEMMs with
 the replica as a second batch level, every elementwise pass over a 5-D index
 space, the energy of every replica in one launch.  Each replica's arithmetic
-is that of its own ``FRICCSDGPU`` iteration (the same kernels, tiles, K
-splits and summation orders), so each replica's trajectory is bit for bit
-the one its lone solve gives with the same seed.
+is that of its own ``FRICCSDGPU`` iteration (the same kernels and summation
+orders, or sums that no order changes), so each replica's trajectory is bit
+for bit the one its lone solve gives with the same seed (where neither runs
+short of scratch: a modular product that cannot have it runs elsewhere).
 
 The replicas' statistics are those of fricc/__init__.py:8-11 (``mcmc_std``
 of each trace; the replica mean and variance of E_corr).

@@ -180,9 +180,10 @@ int fricc_spmm(fricc_sparse* T, int pa, int pb, int ka, int kb, double coef, con
  * (FP64) and the dense fricc_gemm_f64 / fricc_gemm_df run as modular integer
  * products on the tensor cores: sums over the nonzeros (or k) taken exactly
  * on operands rounded at 2^-60 of their row's norm, then rounded once, which
- * no order of summation changes; outputs for which that could be less
- * accurate than an FP64 FMA chain, and rows with infinities or NaNs, are
- * recomputed in FP64 in index order.  No reference counterpart.
+ * no order of summation changes; outputs that are too small against their
+ * rows' norms for that (about 2^-8 of the norms' product, or an element lost to
+ * the rounding), and rows with infinities or NaNs, are recomputed in FP64 in
+ * index order.  No reference counterpart.
  *
  * A constant operand can be converted once: fricc_mod_prepare turns rows x k
  * FP64 elements (element (r, j) at x + r row_stride + j k_stride) into `out`
@@ -201,7 +202,7 @@ int fricc_mod_mode(void); /* the calling thread's mode */
  * beyond which it is worked off in pieces (results the same): -1 the default,
  * 6 GB; 0: none may be taken, so every call runs on the FP64 or sparse kernels.
  * The operand that is not cut is converted whole.  Where the scratch cannot be
- * had, a call runs on those kernels too. */
+ * had, a call runs on those kernels too (and agrees to rounding only). */
 int fricc_mod_scratch(int64_t bytes);
 int64_t fricc_mod_bytes(int64_t rows, int64_t k);
 int fricc_mod_prepare(const double* x, int64_t rows, int64_t k, int64_t row_stride, int64_t k_stride, void* out,

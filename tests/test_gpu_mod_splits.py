@@ -46,3 +46,27 @@ def test_outputs_at_the_check(gpulib, M, N, K):
     A[:, ::2] *= 2.0 ** -(4.0 + 8.0 * torch.rand(M, 1, generator=g, device="cuda", dtype=torch.float64))
     B[1::2] *= 2.0 ** -(4.0 + 8.0 * torch.rand(1, N, generator=g, device="cuda", dtype=torch.float64))
     _lone_and_batched(gpulib, A, B)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "df64"])
+def test_replicas_are_their_lone_solves(gpulib, precision):
+    """Twelve replicas at a size whose products are split differently alone."""
+    from fricc_gb300.batch import mp2_device
+    from fricc_gb300.friccsd import FRICCSDGPU
+    from fricc_gb300.rccsd_dense import DeviceERIs
+    from fricc_gb300.replicas import FusedReplicaBatch
+    from fricc_gb300.rng import GlibcRand
+    from fricc_gb300.synthetic import DeviceSystem
+    E = DeviceERIs.from_system(DeviceSystem(17, 83, 800, 0.04, seed=5))
+    m, seeds = 150_000, list(range(40, 52))
+    fb = FusedReplicaBatch(E, {"m_keep": m}, seeds, precision=precision)
+    for _ in range(2):
+        fb.step()
+    settings = {"compression": "fri", "sampling_method": "systematic", "verbose": False, "m_keep": m,
+                "compressed_contractions": ["O^2V^4", "O^3V^3", "O^4V^2"]}
+    for r in (0, 5, 11):
+        lone = FRICCSDGPU(E, settings, rn_draw=GlibcRand(seeds[r]), precision=precision)
+        t1, t2 = mp2_device(E)
+        for _ in range(2):
+            t1, t2 = lone.update_amps(t1, t2)
+        assert torch.equal(t1, fb.t1[r]) and torch.equal(t2, fb.t2[r]), r
